@@ -74,7 +74,10 @@ struct cz_batch {
   void* big_bw = nullptr;
   void* big_br = nullptr;
   uint8_t* big_aw = nullptr;
-  int *big_off = nullptr, *big_cnt = nullptr, *big_adj = nullptr;
+  int* big_adj = nullptr;
+  void* big_key = nullptr;
+  int big_csm = 0;       // contacts whose arrays k_resolve_big keeps in shared memory
+  size_t big_smem = 0;   // its shared memory per world
 
   // device buffers
   void* body = nullptr;
@@ -84,7 +87,7 @@ struct cz_batch {
   int *d_bstart = nullptr, *d_bcount = nullptr, *d_ccap = nullptr, *d_ccount = nullptr;
   long long* d_cstart = nullptr;
   uint32_t* d_wstatus = nullptr;
-  int *d_piters = nullptr, *d_viters = nullptr;
+  int *d_piters = nullptr, *d_viters = nullptr, *d_cost = nullptr;
   void* contact = nullptr;
   int* cbodies = nullptr;
   void* work = nullptr;
@@ -124,8 +127,10 @@ struct cz_batch {
 
   // tuning
   int np_threads = 128, np_grid = 1, rs_cs = 128, rs_grid = 1, rs_ctas_per_sm = 0, int_threads = 256;
-  int rs_lanes = 8;  // lanes per world in the resolver (32 / rs_lanes worlds per warp)
-  int big_lanes = 32; // lanes per world in the large-world resolver (16: two worlds per warp)
+  int rs_lanes = 8;  // resolver_lanes as set
+  // lanes per world in the resolver (32 / run_lanes() worlds per warp): an island takes eight
+  int run_lanes() const { return std::max(rs_lanes, 8); }
+  int big_lanes = 32; // large_world_lanes as set (both settings run one warp per world)
   int wait_limit = 1 << 22;  // polls of the narrowphase's bounded wait
   int wait_extra_tx = 0;     // test hook: bytes that wait expects beyond its copies
   int grid_min_bodies = 128; // narrowphase grid for worlds of at least this many bodies (0: never)
@@ -139,14 +144,15 @@ struct cz_batch {
   float* hv_labels = nullptr;
   unsigned long long* hv_count = nullptr;
   long long hv_cap = 0;
+  void* ws_imp = nullptr;
   void* ws_rows = nullptr;  // per-body warm-start / harvest scratch (allocated on first use)
   int* ws_int = nullptr;
-  uint8_t* ws_u8 = nullptr;
   uint8_t* ws_world = nullptr;
   float* ws_feat = nullptr;  // harvest features, allocated by the first cz_harvest
   int wf_grid = 1;           // k_warm_features CTAs
   int warm_shift = 2;        // warm-start worlds whose last solve used <= max_it >> warm_shift
-  size_t np_smem = 0, rs_smem = 0;
+  size_t np_smem = 0, rs_smem = 0;  // per narrowphase CTA; per resolver warp
+  int rs_wpc = 1;                    // warps per resolver CTA
 
   // graph cache: (nsteps, dt) -> executable graph
   std::map<std::pair<int, double>, cudaGraphExec_t> graphs;
@@ -179,6 +185,7 @@ struct cz_batch {
     v.world_status = d_wstatus;
     v.pos_iters = d_piters;
     v.vel_iters = d_viters;
+    v.cost = d_cost;
     v.contact = contact;
     v.contact_bodies = cbodies;
     v.work = work;
@@ -202,8 +209,8 @@ struct cz_batch {
     v.hv_count = hv_count;
     v.hv_cap = hv_cap;
     v.ws_rows = ws_rows;
+    v.ws_imp = ws_imp;
     v.ws_int = ws_int;
-    v.ws_u8 = ws_u8;
     v.ws_world = ws_world;
     v.ws_feat = ws_feat;
     v.warm_shift = warm_shift;
@@ -212,9 +219,8 @@ struct cz_batch {
     v.big_bw = big_bw;
     v.big_br = big_br;
     v.big_aw = big_aw;
-    v.big_off = big_off;
-    v.big_cnt = big_cnt;
     v.big_adj = big_adj;
+    v.big_key = big_key;
     v.wait_limit = wait_limit;
     v.wait_extra_tx = wait_extra_tx;
     v.grid_min_bodies = grid_min_bodies;
@@ -224,13 +230,13 @@ struct cz_batch {
 
 namespace {
 
-// Resolver queue for the next frame: worlds in decreasing adjustPositions +
-// adjustVelocities iterations of this frame (a counting sort in one CTA), so
-// that the worlds sharing a warp in lockstep have similar work.  The order of
-// independent worlds does not change any result.
+// Resolver queue for the next frame: worlds in decreasing rounds of this
+// frame's resolve (a counting sort in one CTA), so that the longest chains
+// start first and the worlds sharing a warp in lockstep have similar work (the
+// rounds of a world, not its iterations: its islands run side by side).  The
+// order of independent worlds does not change any result.
 constexpr int kReorderBuckets = 2048;
-__global__ void __launch_bounds__(1024) k_reorder(const int* __restrict__ pos_it, const int* __restrict__ vel_it,
-                                                  int W, int* __restrict__ order,
+__global__ void __launch_bounds__(1024) k_reorder(const int* __restrict__ cost, int W, int* __restrict__ order,
                                                   const uint8_t* __restrict__ plain_next = nullptr) {
   __shared__ int hist[kReorderBuckets];
   __shared__ int wsum[32];
@@ -242,7 +248,7 @@ __global__ void __launch_bounds__(1024) k_reorder(const int* __restrict__ pos_it
   // twice, and late in the queue that would be the frame's tail
   auto key_of_world = [&](int w) {
     if (plain_next && !plain_next[w]) return kReorderBuckets - 1;
-    return min(pos_it[w] + vel_it[w], kReorderBuckets - 1);
+    return min(cost[w], kReorderBuckets - 1);  // kExhausted: the longest chains, first
   };
   for (int w = tid; w < W; w += blockDim.x) atomicAdd(&hist[kReorderBuckets - 1 - key_of_world(w)], 1);
   __syncthreads();
@@ -285,10 +291,10 @@ void free_batch(cz_batch* b) {
   }
   void* dev[] = {
       b->d_offset,  b->d_off_stage, b->ws_feat,   b->d_units,     b->d_big,      b->big_bw,      b->big_br,
-      b->big_aw,    b->big_off,     b->big_cnt,   b->big_adj,     b->ws_rows,    b->ws_int,      b->ws_u8,
+      b->big_aw,    b->big_adj,     b->big_key,   b->ws_imp,      b->ws_rows,    b->ws_int,
       b->ws_world,  b->mlp_mem,     b->hv_features, b->hv_labels, b->hv_count,   b->snap_body,   b->snap_u8,
       b->body,      b->awake,       b->can_sleep, b->shape,       b->d_bstart,   b->d_bcount,    b->d_ccap,
-      b->d_ccount,  b->d_cstart,    b->d_wstatus, b->d_piters,    b->d_viters,   b->contact,     b->cbodies,
+      b->d_ccount,  b->d_cstart,    b->d_wstatus, b->d_piters,    b->d_viters,    b->d_cost,   b->contact,     b->cbodies,
       b->work,      b->wbodies,     b->kmat,      b->d_order,    b->d_order_rs,  b->d_queue,
       b->d_status,  b->d_counters,  b->d_h2p,     b->d_stage,     b->d_stage_u8, b->d_stage_i32, b->d_cstage,
       b->d_cstage_b, b->d_pow};
@@ -348,7 +354,7 @@ bool uses_frame(const cz_batch* b) {
 
 int launches_per_step(const cz_batch* b) {
   if (uses_frame(b)) return 1 + (b->nsmall > 1 ? 1 : 0);
-  return 2 + (b->nsmall > 0 ? 1 + (b->nsmall > 32 / b->rs_lanes ? 1 : 0) + (b->mode != 0 ? 1 : 0) : 0) +
+  return 2 + (b->nsmall > 0 ? 1 + (b->nsmall > 32 / b->run_lanes() ? 1 : 0) + (b->mode != 0 ? 1 : 0) : 0) +
          (b->big_ids.empty() ? 0 : 1);
 }
 
@@ -366,7 +372,7 @@ int launch_narrowphase(cz_batch* b) {
 // The resolver launches of one frame: k_resolve over the worlds that fit its
 // slot (then the re-queue of those worlds by cost), k_resolve_big over the
 // others.
-int launch_resolve_with(cz_batch* b, double dt, const cz::HostView& v, int cs, size_t smem) {
+int launch_resolve_with(cz_batch* b, double dt, const cz::HostView& v) {
   if (b->nsmall > 0) {
     if (v.mode != 0) {  // features (and, warm-starting, predictions) ahead of the resolver
       CZ_CUDA(cudaMemsetAsync(b->d_queue + 2, 0, sizeof(unsigned), b->stream));
@@ -374,23 +380,23 @@ int launch_resolve_with(cz_batch* b, double dt, const cz::HostView& v, int cs, s
       g_launches++;
     }
     CZ_CUDA(cudaMemsetAsync(b->d_queue + 1, 0, sizeof(unsigned), b->stream));
-    CZ_CUDA(b->ops->resolve(v, b->rs_nbs, cs, b->rs_lanes, b->rs_grid, smem, dt, b->stream));
+    CZ_CUDA(b->ops->resolve(v, b->rs_nbs, b->rs_cs, b->run_lanes(), b->rs_grid, b->rs_wpc, b->rs_smem, dt, b->stream));
     g_launches++;
-    if (b->nsmall > 32 / b->rs_lanes) {
-      k_reorder<<<1, 1024, 0, b->stream>>>(b->d_piters, b->d_viters, b->num_worlds, b->d_order_rs,
+    if (b->nsmall > 32 / b->run_lanes()) {
+      k_reorder<<<1, 1024, 0, b->stream>>>(b->d_cost, b->num_worlds, b->d_order_rs,
                                            v.mode == 2 ? v.ws_world : nullptr);
       CZ_CUDA(cudaGetLastError());
       g_launches++;
     }
   }
   if (!b->big_ids.empty()) {
-    CZ_CUDA(b->ops->resolve_big(v, (int)b->big_ids.size(), b->big_lanes, dt, b->stream));
+    CZ_CUDA(b->ops->resolve_big(v, (int)b->big_ids.size(), b->big_csm, b->big_smem, dt, b->stream));
     g_launches++;
   }
   return CZ_OK;
 }
 int launch_resolve(cz_batch* b, double dt, const cz::HostView* override_view = nullptr) {
-  return launch_resolve_with(b, dt, override_view ? *override_view : b->view(), b->rs_cs, b->rs_smem);
+  return launch_resolve_with(b, dt, override_view ? *override_view : b->view());
 }
 // The fused frame: integrate, narrowphase and resolve of every world in one
 // launch (then the re-queue by cost).
@@ -399,7 +405,7 @@ int launch_frame(cz_batch* b, double dt) {
   CZ_CUDA(b->ops->frame(b->view(), b->rs_nbs, b->rs_cs, b->fr_grid, b->fr_smem, dt, std::pow(0.5, dt), b->stream));
   g_launches++;
   if (b->nsmall > 1) {
-    k_reorder<<<1, 1024, 0, b->stream>>>(b->d_piters, b->d_viters, b->num_worlds, b->d_order_rs);
+    k_reorder<<<1, 1024, 0, b->stream>>>(b->d_cost, b->num_worlds, b->d_order_rs);
     CZ_CUDA(cudaGetLastError());
     g_launches++;
   }
@@ -422,27 +428,54 @@ int configure(cz_batch* b) {
   // resolver shared-memory tile: shrink the contact capacity until it fits
   int cs = std::min<long long>(b->rs_cs, round_up(b->max_cap, 32));
   cs = std::max(cs, 32);
-  while (cs > 32 && b->ops->rs_smem(b->rs_nbs, cs, b->rs_lanes, b->mode) > b->smem_optin) cs -= 32;
+  while (cs > 32 && b->ops->rs_smem(b->rs_nbs, cs, b->run_lanes()) > b->smem_optin) cs -= 32;
   b->rs_cs = cs;
-  b->rs_smem = b->ops->rs_smem(b->rs_nbs, cs, b->rs_lanes, b->mode);
+  b->rs_smem = b->ops->rs_smem(b->rs_nbs, cs, b->run_lanes());
   b->np_smem = b->ops->np_smem(b->nbs);
   if (b->np_smem > b->smem_optin || b->rs_smem > b->smem_optin)
     return fail(CZ_ERR_BODY_LIMIT, "world too large for the shared-memory tiles");
-  CZ_CUDA(b->ops->prepare(b->np_smem, b->rs_smem, b->rs_lanes));
   int npb = 0, rsb = 0;
-  CZ_CUDA(b->ops->occupancy(&npb, b->np_threads, b->np_smem, &rsb, b->rs_smem, b->rs_lanes, b->mode,
+  // Resolver warps are independent (each takes its own worlds), so a CTA holds
+  // as many as make the most resident warps per SM (the SM keeps 1 KB of
+  // shared memory per CTA), the fewest where several counts do; few worlds are
+  // spread over the SMs.
+  const int lanes = b->run_lanes();
+  const long long groups = (std::max(b->nsmall, 1) + 32 / lanes - 1) / (32 / lanes);
+  const int fit = (int)(b->smem_optin / b->rs_smem);
+  const int most = (int)std::min<long long>(std::min(b->ops->rs_wpc(lanes), fit),
+                                            (groups + b->sm_count - 1) / b->sm_count);
+  CZ_CUDA(b->ops->prepare(b->np_smem, std::max(most, 1) * b->rs_smem, lanes));
+  b->rs_wpc = 1;
+  for (int wpc = 1; wpc <= std::max(most, 1); ++wpc) {
+    int blocks = 0;
+    CZ_CUDA(b->ops->rs_occupancy(&blocks, wpc, b->rs_smem, lanes, b->mode));
+    if (wpc == 1 || blocks * wpc > rsb * b->rs_wpc) {
+      rsb = blocks;
+      b->rs_wpc = wpc;
+    }
+  }
+  CZ_CUDA(b->ops->occupancy(&npb, b->np_threads, b->np_smem,
                             b->grid_min_bodies > 0 && b->max_n >= b->grid_min_bodies));
   npb = std::max(npb, 1);
   rsb = std::max(rsb, 1);
   if (b->rs_ctas_per_sm > 0) rsb = std::min(rsb, b->rs_ctas_per_sm);
   b->np_grid = (int)std::min<long long>(b->num_worlds, (long long)npb * b->sm_count);
-  const long long groups = (std::max(b->nsmall, 1) + 32 / b->rs_lanes - 1) / (32 / b->rs_lanes);
-  const int wpc = b->ops->rs_wpc(b->rs_lanes);
-  b->rs_grid = (int)std::min<long long>((groups + wpc - 1) / wpc, (long long)rsb * b->sm_count);
+  b->rs_grid = (int)std::min<long long>((groups + b->rs_wpc - 1) / b->rs_wpc, (long long)rsb * b->sm_count);
   b->np_grid = std::max(b->np_grid, 1);
   b->rs_grid = std::max(b->rs_grid, 1);
   b->wf_grid = (int)std::min<long long>(std::max(b->nsmall, 1),
                                         (long long)b->ops->warm_features_blocks(b->rs_nbs) * b->sm_count);
+  if (!b->big_ids.empty()) {
+    // the large-world resolver's shared memory: half an SM's where several
+    // worlds share an SM (1024 bodies with 6 contacts each fit that), else all
+    int n = 0, cap = 0;
+    for (int w : b->big_ids) {
+      n = std::max(n, b->counts[w]);
+      cap = std::max(cap, b->ccap[w]);
+    }
+    const size_t budget = (int)b->big_ids.size() > b->sm_count ? (size_t)112 * 1024 : b->smem_optin;
+    CZ_CUDA(b->ops->big_smem(n, cap, budget, &b->big_csm, &b->big_smem));
+  }
   // the fused frame's slot holds the resolver's tile and the narrowphase's
   b->fr_smem = b->ops->frame_smem(b->rs_nbs, b->rs_cs);
   if (b->fr_smem > b->smem_optin) {
@@ -546,11 +579,10 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
   b->nsmall = b->num_worlds - (int)b->big_ids.size();
   b->rs_nbs = (int)std::max<long long>(round_up(max_small, 4), 4);
   b->np_threads = b->max_n >= 256 ? 256 : 128;
-  // defaults from the tuned precision workload: a world per warp in float32;
-  // two per warp in float64, which shares their float64 chains (the tuner
-  // may change both)
+  // a world per warp: its islands share the warp's instructions (the tuner may
+  // change it)
   b->rs_cs = 96;
-  b->rs_lanes = d->form == CZ_FORM_FP64 ? 16 : 32;
+  b->rs_lanes = 32;
   // world queue: decreasing body count (pair work grows as n^2)
   std::vector<int> order(b->num_worlds);
   std::iota(order.begin(), order.end(), 0);
@@ -570,9 +602,10 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
        dmalloc((void**)&b->d_ccap, sizeof(int) * W) && dmalloc((void**)&b->d_ccount, sizeof(int) * W) &&
        dmalloc((void**)&b->d_cstart, sizeof(long long) * W) && dmalloc((void**)&b->d_wstatus, sizeof(uint32_t) * W) &&
        dmalloc((void**)&b->d_piters, sizeof(int) * W) && dmalloc((void**)&b->d_viters, sizeof(int) * W) &&
+       dmalloc((void**)&b->d_cost, sizeof(int) * W) &&
        dmalloc((void**)&b->d_order, sizeof(int) * W) && dmalloc((void**)&b->d_order_rs, sizeof(int) * W);
   ok = ok && dmalloc(&b->contact, R * cz::C_NROWS * C) && dmalloc((void**)&b->cbodies, sizeof(int) * C);
-  ok = ok && dmalloc(&b->work, R * cz::W_NROWS * C) && dmalloc((void**)&b->wbodies, sizeof(int) * C);
+  ok = ok && dmalloc(&b->work, R * cz::CREC * C) && dmalloc((void**)&b->wbodies, sizeof(int) * C);
   ok = ok && dmalloc(&b->kmat, R * cz::K_ROW * C);
   ok = ok && dmalloc((void**)&b->d_queue, 4 * sizeof(unsigned)) && dmalloc((void**)&b->d_status, sizeof(uint32_t)) &&
        dmalloc((void**)&b->d_counters, 8 * sizeof(unsigned long long));
@@ -586,9 +619,9 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
   ok = ok && dmalloc(&b->snap_body, R * cz::B_NROWS * P) && dmalloc((void**)&b->snap_u8, 2 * P);
   if (!b->big_ids.empty()) {
     ok = ok && dmalloc((void**)&b->d_big, sizeof(int) * b->big_ids.size()) &&
-         dmalloc(&b->big_bw, sizeof(double) * 7 * P) && dmalloc(&b->big_br, R * 20 * P) &&
-         dmalloc((void**)&b->big_aw, P) && dmalloc((void**)&b->big_off, sizeof(int) * P) &&
-         dmalloc((void**)&b->big_cnt, sizeof(int) * P) && dmalloc((void**)&b->big_adj, sizeof(int) * 2 * C);
+         dmalloc(&b->big_bw, sizeof(double) * 7 * P) && dmalloc(&b->big_br, R * cz::BREC * P) &&
+         dmalloc((void**)&b->big_aw, P) && dmalloc((void**)&b->big_adj, sizeof(int) * 2 * C) &&
+         dmalloc(&b->big_key, R * C);
   }
   if (!ok) return bail(fail(CZ_ERR_CUDA, "device allocation failed"));
   ok = cudaMallocHost((void**)&b->h_stage, sizeof(double) * cz::SG_NDOUBLES * std::max<long long>(nb, 1)) ==
@@ -609,6 +642,7 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
       cudaMemsetAsync(b->d_wstatus, 0, sizeof(uint32_t) * W, s) != cudaSuccess ||
       cudaMemsetAsync(b->d_piters, 0, sizeof(int) * W, s) != cudaSuccess ||
       cudaMemsetAsync(b->d_viters, 0, sizeof(int) * W, s) != cudaSuccess ||
+      cudaMemsetAsync(b->d_cost, 0, sizeof(int) * W, s) != cudaSuccess ||
       cudaMemsetAsync(b->d_queue, 0, 4 * sizeof(unsigned), s) != cudaSuccess ||
       cudaMemsetAsync(b->d_status, 0, sizeof(uint32_t), s) != cudaSuccess ||
       cudaMemsetAsync(b->d_counters, 0, 8 * sizeof(unsigned long long), s) != cudaSuccess ||
@@ -1132,9 +1166,9 @@ int cz_step_timed(cz_batch* b, int32_t nsteps, double dt, double* total_ms, doub
 static int ensure_ws(cz_batch* b) {
   if (b->ws_rows) return CZ_OK;
   const size_t P = (size_t)b->nb_pad;
-  CZ_CUDA(cudaMalloc(&b->ws_rows, b->ops->real_size * 13 * P));
+  CZ_CUDA(cudaMalloc(&b->ws_rows, b->ops->real_size * 6 * P));
+  CZ_CUDA(cudaMalloc(&b->ws_imp, b->ops->real_size * 3 * (size_t)b->nc_total));
   CZ_CUDA(cudaMalloc((void**)&b->ws_int, sizeof(int) * cz::WS_NINT * P));
-  CZ_CUDA(cudaMalloc((void**)&b->ws_u8, 2 * P));
   CZ_CUDA(cudaMalloc((void**)&b->ws_world, (size_t)b->num_worlds));
   CZ_CUDA(cudaMemset(b->ws_world, 0, (size_t)b->num_worlds));
   return CZ_OK;
@@ -1212,10 +1246,6 @@ int cz_harvest(cz_batch* b, int32_t nsteps, double dt, int32_t every, float* fea
   if ((st = reset_status(b))) return st;
   // the plain resolver, writing features and applied impulses every `every` frames
   const int saved_mode = b->mode;
-  int cs = b->rs_cs;
-  while (cs > 32 && b->ops->rs_smem(b->rs_nbs, cs, b->rs_lanes, 1) > b->smem_optin) cs -= 32;
-  const size_t smem1 = b->ops->rs_smem(b->rs_nbs, cs, b->rs_lanes, 1);
-  CZ_CUDA(b->ops->prepare(b->np_smem, smem1, b->rs_lanes));
   for (int s = 0; s < nsteps && st == CZ_OK; ++s) {
     st = launch_integrate(b, dt);
     if (!st) st = launch_narrowphase(b);
@@ -1224,7 +1254,7 @@ int cz_harvest(cz_batch* b, int32_t nsteps, double dt, int32_t every, float* fea
       cz::HostView v = b->view();
       v.mode = h ? 1 : 0;
       v.hv_cap = b->hv_cap;
-      st = launch_resolve_with(b, dt, v, h ? cs : b->rs_cs, h ? smem1 : b->rs_smem);
+      st = launch_resolve_with(b, dt, v);
     }
   }
   b->mode = saved_mode;
@@ -1263,7 +1293,7 @@ int cz_batch_info(cz_batch* b, int64_t* info) {
   info[5] = b->np_grid;
   info[6] = b->rs_grid;
   info[7] = (int64_t)b->np_smem;
-  info[8] = (int64_t)b->rs_smem;
+  info[8] = (int64_t)(b->rs_wpc * b->rs_smem);
   return CZ_OK;
 }
 

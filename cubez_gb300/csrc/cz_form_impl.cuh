@@ -28,6 +28,7 @@ static BatchView<R> view_of(const HostView& h) {
   v.world_status = h.world_status;
   v.pos_iters = h.pos_iters;
   v.vel_iters = h.vel_iters;
+  v.cost = h.cost;
   v.contact = static_cast<R*>(h.contact);
   v.contact_bodies = h.contact_bodies;
   v.work = static_cast<R*>(h.work);
@@ -54,8 +55,8 @@ static BatchView<R> view_of(const HostView& h) {
   v.hv_count = h.hv_count;
   v.hv_cap = h.hv_cap;
   v.ws_rows = static_cast<R*>(h.ws_rows);
+  v.ws_imp = static_cast<R*>(h.ws_imp);
   v.ws_int = h.ws_int;
-  v.ws_u8 = h.ws_u8;
   v.ws_world = h.ws_world;
   v.ws_feat = h.ws_feat;
   v.warm_shift = h.warm_shift;
@@ -64,9 +65,8 @@ static BatchView<R> view_of(const HostView& h) {
   v.big_bw = h.big_bw;
   v.big_br = static_cast<R*>(h.big_br);
   v.big_aw = h.big_aw;
-  v.big_off = h.big_off;
-  v.big_cnt = h.big_cnt;
   v.big_adj = h.big_adj;
+  v.big_key = h.big_key;
   v.wait_limit = h.wait_limit;
   v.wait_extra_tx = h.wait_extra_tx;
   v.grid_min_bodies = h.grid_min_bodies;
@@ -187,19 +187,15 @@ __global__ void k_set_rows(BatchView<R> v, int row, int nrows, const double* __r
 }
 
 static size_t np_smem(int nbs) { return np_smem_bytes<R>(nbs); }
-// warps per resolver CTA for G lanes per world (rs_wpc)
+// most warps per resolver CTA for G lanes per world (rs_wpc)
 static int rs_wpc_of(int lanes) { return lanes == 32 ? rs_wpc<R, 32, false>() : 1; }
-static size_t rs_smem(int nbs, int cs, int lanes, int mode) {
-  (void)mode;  // the learned paths keep their scratch in global memory and registers
-  return (size_t)rs_wpc_of(lanes) * (32 / lanes) * rs_slot_bytes<R, W>(nbs, cs);
-}
+static size_t rs_smem(int nbs, int cs, int lanes) { return (size_t)(32 / lanes) * rs_slot_bytes<R, W>(nbs, cs); }
 
 // the resolver instantiation for G lanes per world, plain or with the
 // learned paths (harvest, warm start)
 static const void* resolve_fn_mode(int lanes, int mode) {
   const bool learn = mode != 0;
   switch (lanes) {
-    case 4: return learn ? (const void*)k_resolve<R, W, 4, true> : (const void*)k_resolve<R, W, 4, false>;
     case 8: return learn ? (const void*)k_resolve<R, W, 8, true> : (const void*)k_resolve<R, W, 8, false>;
     case 16: return learn ? (const void*)k_resolve<R, W, 16, true> : (const void*)k_resolve<R, W, 16, false>;
     case 32: return learn ? (const void*)k_resolve<R, W, 32, true> : (const void*)k_resolve<R, W, 32, false>;
@@ -253,17 +249,16 @@ static cudaError_t narrowphase(const HostView& h, int nbs, int threads, int grid
   return cudaGetLastError();
 }
 
-static cudaError_t resolve(const HostView& h, int nbs, int cs, int lanes, int grid, size_t smem, double dt,
+static cudaError_t resolve(const HostView& h, int nbs, int cs, int lanes, int grid, int wpc, size_t smem, double dt,
                            cudaStream_t s) {
   const BatchView<R> v = view_of(h);
   const bool learn = h.mode != 0;
 #define CZ_LAUNCH_RS(G)                                                                              \
   if (learn)                                                                                        \
-    k_resolve<R, W, G, true><<<grid, 32 * rs_wpc<R, G, false>(), smem, s>>>(v, nbs, cs, (R)dt);      \
+    k_resolve<R, W, G, true><<<grid, 32 * wpc, wpc * smem, s>>>(v, nbs, cs, (R)dt);                  \
   else                                                                                              \
-    k_resolve<R, W, G, false><<<grid, 32 * rs_wpc<R, G, false>(), smem, s>>>(v, nbs, cs, (R)dt);
+    k_resolve<R, W, G, false><<<grid, 32 * wpc, wpc * smem, s>>>(v, nbs, cs, (R)dt);
   switch (lanes) {
-    case 4: CZ_LAUNCH_RS(4) break;
     case 8: CZ_LAUNCH_RS(8) break;
     case 16: CZ_LAUNCH_RS(16) break;
     case 32: CZ_LAUNCH_RS(32) break;
@@ -330,13 +325,22 @@ static int warm_features_blocks(int nbs) {
   return blocks > 0 ? blocks : 1;
 }
 
-static cudaError_t resolve_big(const HostView& h, int nbig, int lanes, double dt, cudaStream_t s) {
+static cudaError_t resolve_big(const HostView& h, int nbig, int csm, size_t smem, double dt, cudaStream_t s) {
   if (nbig <= 0) return cudaSuccess;
-  if (lanes == 16)
-    k_resolve_big<R, W, 16><<<(nbig + 1) / 2, 32, 0, s>>>(view_of(h), (R)dt);
-  else
-    k_resolve_big<R, W, 32><<<nbig, 32, 0, s>>>(view_of(h), (R)dt);
+  k_resolve_big<R, W><<<nbig, 32, smem, s>>>(view_of(h), (R)dt, csm);
   return cudaGetLastError();
+}
+
+static cudaError_t big_smem(int n, int max_cap, size_t budget, int* csm, size_t* smem) {
+  const size_t fixed = big_fixed_bytes<R>(n);
+  *csm = 0;
+  *smem = fixed;
+  if (budget > fixed) {
+    const size_t fit = (budget - fixed) / big_contact_bytes<R>();
+    *csm = (int)(fit < (size_t)max_cap ? fit : (size_t)max_cap) & ~3;
+    *smem = fixed + *csm * big_contact_bytes<R>();
+  }
+  return raise_smem_limit((const void*)k_resolve_big<R, W>, *smem);
 }
 
 static cudaError_t upload(const HostView& h, const double* sg, const uint8_t* u8, const int* i32, const int* h2p,
@@ -353,13 +357,14 @@ static cudaError_t download(const HostView& h, double* sg, uint8_t* u8, int* i32
   return cudaGetLastError();
 }
 
-static cudaError_t occupancy(int* npb, int np_threads, size_t nps, int* rsb, size_t rss, int lanes, int mode,
-                             int grid) {
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(npb, narrowphase_fn(grid != 0), np_threads, nps);
-  if (e != cudaSuccess) return e;
+static cudaError_t occupancy(int* npb, int np_threads, size_t nps, int grid) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(npb, narrowphase_fn(grid != 0), np_threads, nps);
+}
+
+static cudaError_t rs_occupancy(int* rsb, int wpc, size_t rss, int lanes, int mode) {
   const void* f = resolve_fn_mode(lanes, mode);  // the instantiation that runs (registers differ)
   if (!f) return cudaErrorInvalidValue;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(rsb, f, 32 * rs_wpc_of(lanes), rss);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(rsb, f, 32 * wpc, wpc * rss);
 }
 
 static cudaError_t contacts_out(const HostView& h, long long start, int count, double* sg, int* bodies,
@@ -395,10 +400,12 @@ const FormOps CZ_FORM_OBJ = {sizeof(CZ_R),
                              CZ_FORM_NS::warm_features,
                              CZ_FORM_NS::warm_features_blocks,
                              CZ_FORM_NS::resolve_big,
+                             CZ_FORM_NS::big_smem,
                              CZ_FORM_NS::resolve,
                              CZ_FORM_NS::upload,
                              CZ_FORM_NS::download,
                              CZ_FORM_NS::occupancy,
+                             CZ_FORM_NS::rs_occupancy,
                              CZ_FORM_NS::contacts_out,
                              CZ_FORM_NS::contacts_in,
                              CZ_FORM_NS::set_rows,

@@ -30,6 +30,7 @@ struct HostView {
   uint32_t* world_status;
   int* pos_iters;
   int* vel_iters;
+  int* cost;
   void* contact;
   int* contact_bodies;
   void* work;
@@ -53,8 +54,8 @@ struct HostView {
   unsigned long long* hv_count;
   long long hv_cap;
   void* ws_rows;
+  void* ws_imp;
   int* ws_int;
-  uint8_t* ws_u8;
   uint8_t* ws_world;
   float* ws_feat;
   int warm_shift;
@@ -63,9 +64,8 @@ struct HostView {
   void* big_bw;
   void* big_br;
   uint8_t* big_aw;
-  int* big_off;
-  int* big_cnt;
   int* big_adj;
+  void* big_key;
   int wait_limit;
   int wait_extra_tx;
   int grid_min_bodies;
@@ -80,8 +80,8 @@ enum StageBlock : int {
 struct FormOps {
   size_t real_size;
   size_t (*np_smem)(int nbs);
-  size_t (*rs_smem)(int nbs, int cs, int lanes, int mode);  // per CTA (rs_wpc warps, 32 / lanes worlds each)
-  int (*rs_wpc)(int lanes);                                   // warps per resolver CTA
+  size_t (*rs_smem)(int nbs, int cs, int lanes);  // per warp (32 / lanes worlds)
+  int (*rs_wpc)(int lanes);                       // most warps per resolver CTA
   cudaError_t (*prepare)(size_t np_smem, size_t rs_smem, int lanes);  // function attributes
   cudaError_t (*integrate)(const HostView& v, double dt, double sleep_bias, int threads, cudaStream_t s);
   cudaError_t (*narrowphase)(const HostView& v, int nbs, int threads, int grid, size_t smem, cudaStream_t s);
@@ -91,9 +91,12 @@ struct FormOps {
   // the learned paths' features / predictions ahead of the resolver (k_warm_features)
   cudaError_t (*warm_features)(const HostView& v, int nbs, int grid, double dt, cudaStream_t s);
   int (*warm_features_blocks)(int nbs);  // resident CTAs per SM
-  // worlds above the shared-memory slot; `lanes` per world: 32, or 16 (two worlds per warp)
-  cudaError_t (*resolve_big)(const HostView& v, int nbig, int lanes, double dt, cudaStream_t s);
-  cudaError_t (*resolve)(const HostView& v, int nbs, int cs, int lanes, int grid, size_t smem, double dt,
+  // worlds above the shared-memory slot, one warp each; smem bytes hold csm contacts' arrays (big_smem)
+  cudaError_t (*resolve_big)(const HostView& v, int nbig, int csm, size_t smem, double dt, cudaStream_t s);
+  // the contacts whose arrays fit `budget` bytes beside those of n bodies, and the bytes for them (0: none fit)
+  cudaError_t (*big_smem)(int n, int max_cap, size_t budget, int* csm, size_t* smem);
+  // grid CTAs of wpc warps each, smem bytes per warp
+  cudaError_t (*resolve)(const HostView& v, int nbs, int cs, int lanes, int grid, int wpc, size_t smem, double dt,
                          cudaStream_t s);
   // `off` ([n][12] doubles, the collider Offsets) may be null; the upload
   // writes the Offset rows only when both it and v.offset are set
@@ -101,8 +104,8 @@ struct FormOps {
                         int nb, int has_iw, int has_lfa, const double* off, cudaStream_t s);
   cudaError_t (*download)(const HostView& v, double* stage, uint8_t* u8, int* i32, const int* h2p, int nb,
                           double* off, cudaStream_t s);
-  cudaError_t (*occupancy)(int* np_blocks, int np_threads, size_t np_smem, int* rs_blocks, size_t rs_smem,
-                           int lanes, int mode, int grid);
+  cudaError_t (*occupancy)(int* np_blocks, int np_threads, size_t np_smem, int grid);
+  cudaError_t (*rs_occupancy)(int* rs_blocks, int wpc, size_t rs_smem, int lanes, int mode);
   // contacts: device rows <-> AoS doubles staging (10 doubles + 2 ints per contact)
   cudaError_t (*contacts_out)(const HostView& v, long long start, int count, double* stage, int* bodies,
                               cudaStream_t s);

@@ -44,32 +44,30 @@ enum BodyRow : int {
 // Narrowphase output (Contact fields set by the colliders).
 enum ContactRow : int { C_PX, C_PY, C_PZ, C_NX, C_NY, C_NZ, C_PEN, C_FRIC, C_REST, C_NROWS };
 
-// Resolver working set (Contact's private fields, contact.go:38-50).  The
-// third basis column is never stored: calculateContactBasis (contact.go:
-// 118-156) derives it from the normal and the second column by the same
-// formulas.  The second column (W_TY*) is a function of the normal alone and
-// is stored: recomputing it where the basis is used freed three rows of the
-// resolver's shared-memory tile (10 instead of 9 CTAs per SM for the
-// precision form) but cost more on the update path than the occupancy gained
-// (measured: resolve +2.4 %).
-enum WorkRow : int {
-  W_PEN, W_DDV,
-  W_NX, W_NY, W_NZ,
-  W_R0X, W_R0Y, W_R0Z,
-  W_R1X, W_R1Y, W_R1Z,
-  W_CVX, W_CVY, W_CVZ,
-  W_TYX, W_TYY, W_TYZ,
-  W_J0, W_J1, W_J2,  // contact-frame impulse: predicted (warm start) or applied in total (harvest)
-  W_NROWS
+// Resolver working set (Contact's private fields, contact.go:38-50): one
+// record of CREC reals per contact, read in 16-byte pieces.  The basis's second
+// and third columns are functions of the normal (calculateContactBasis,
+// contact.go:114-156); they are kept, as recomputing them where the basis is
+// used costs more instructions than their loads.
+enum ContactRec : int {
+  CR_N = 0,     // contactToWorld's columns: normal,
+  CR_TY = 3,    //   tangent y,
+  CR_TZ = 6,    //   tangent z
+  CR_R0 = 9,    // relative contact positions
+  CR_R1 = 12,
+  CR_PEN = 15,  // penetration (adjustPositions); then
+  CR_VFA = 15,  // the frame velocity along the normal (adjustVelocities)
+  CR_CV = 16,   // contact velocity
+  CR_DDV = 19,  // desired delta velocity
+  CREC = 20
 };
+// Working state of a body, one record of BREC reals (position and orientation
+// are kept apart, in the island type)
+enum BodyRec : int { BR_VEL = 0, BR_ROT = 3, BR_IIT = 6, BR_INVM = 15, BR_LFA = 16, BR_MOTION = 19, BREC = 20 };
 // reals per contact of the friction solve's matrices (K: 9, the response's
 // first row: 3, padding: 4), contact-major, so the resolved contact's are one
 // aligned 64- (float32) or 128-byte (float64) block
 constexpr int K_ROW = 16;
-// whether the form stores the basis tangent row
-template <class R> __host__ __device__ constexpr bool stores_tangent() { return true; }
-// rows the resolver keeps per contact in its shared-memory tile
-template <class R> __host__ __device__ constexpr int w_rows_kept() { return stores_tangent<R>() ? W_J0 : W_TYX; }
 
 // World status bits (also OR-ed into the batch status word).
 enum : uint32_t {
@@ -79,6 +77,9 @@ enum : uint32_t {
   ST_TIMEOUT = 8u,          // a bounded wait gave up
   ST_BODY_LIMIT = 16u,      // world larger than the kernel's shared-memory tile
 };
+
+// in BatchView::cost: the world's last adjustVelocities used its whole budget
+constexpr int kExhausted = 1 << 30;
 
 // packed body pair of a contact: low 16 bits body 0, high 16 bits body 1
 // (0xFFFF = nil).  World-local indices, so a world holds at most 65535 bodies.
@@ -111,9 +112,10 @@ template <class R> struct BatchView {
   uint32_t* world_status;
   int* pos_iters;
   int* vel_iters;
+  int* cost;            // [num_worlds] the resolver's rounds in the last frame (k_reorder), and kExhausted
   R* contact;           // [C_NROWS][nc_total]
   int* contact_bodies;  // [nc_total]
-  R* work;              // [W_NROWS][nc_total]
+  R* work;              // [nc_total][CREC] contact records of the worlds above the shared tile
   R* kmat;              // [nc_total][16] reals per contact: K of its friction solve (9, inverted in the
                         // island type), the friction response's first row (3), padding (4)
   int* work_bodies;     // [nc_total]
@@ -138,21 +140,21 @@ template <class R> struct BatchView {
   long long hv_cap;
   // per-body scratch of the warm start and the harvest (modes 1, 2), indexed
   // like the body rows (row stride nb_pad)
-  R* ws_rows;            // [13]: saved velocity 0-2, rotation 3-5, motion 6; warm-start change 7-12
+  R* ws_rows;            // [6]: warm-start velocity and rotation change
+  R* ws_imp;             // [3][nc_total] contact-frame impulse: predicted (warm start) or applied in total (harvest)
   int* ws_int;           // [WS_NINT]
-  uint8_t* ws_u8;        // [2]: awake flags at the start of adjustVelocities, at prepareContacts
   uint8_t* ws_world;     // [num_worlds]: the world's last velocity solve used more than max_it >> warm_shift
   float* ws_feat;        // [nc_total][18] harvest features (k_warm_features, mode 1)
   int warm_shift;        // warm-start a world when its last solve used <= max_it >> warm_shift
   // worlds above the shared-memory slot of k_resolve, resolved by k_resolve_big
   const int* big_list;   // [big_count] world ids
   int big_count;
-  void* big_bw;          // [7][nb_pad] positions / orientations in the island type
-  R* big_br;             // [20][nb_pad] velocity, rotation, lfa, iitWorld, inverse mass, motion
+  void* big_bw;          // [nb_pad][7] positions / orientations in the island type
+  R* big_br;             // [nb_pad][BREC] body records
   uint8_t* big_aw;       // [nb_pad] awake flags
-  int* big_off;          // [nb_pad] start of each body's contact list in its world's segment
-  int* big_cnt;          // [nb_pad] end of each body's contact list
-  int* big_adj;          // [2 * nc_total] contact lists, a world's segment at 2 * contact_start
+  // of worlds whose contacts exceed k_resolve_big's shared memory:
+  int* big_adj;          // [2 * nc_total] contact lists per body, a world's segment at 2 * contact_start
+  void* big_key;         // [nc_total] argmax keys (as wide as R)
   // the narrowphase's bounded wait on its staging copies: polls before it
   // gives up, and extra bytes expected beyond those copied (0; a test raises
   // it so that the wait runs out with every real copy landed)

@@ -1,26 +1,25 @@
 // ResolveContacts (contact.go:204-445) for batches of worlds.
 //
-// One warp holds 32 / G worlds; the G lanes of a group own one world.  Within
-// a group the contacts are lane-strided: the argmax is a G-lane butterfly
-// (warp reductions for G = 32) whose tie-break is the reference's
-// first-maximum rule, and the per-iteration update of every contact touching
-// the two resolved bodies is lane-parallel (gathered to those contacts in the
-// float64 form).  The sequential part of an iteration (applyPositionChange
-// on lanes 0 and 1, one body each; applyVelocityChange on the group leader,
-// or on six lanes in the float64 form) runs for all groups at once, so each
-// instruction of that chain serves 32 / G worlds: on GB300 a float64 warp
-// instruction costs the same pipe time whatever its active mask, so packing
-// worlds into a warp divides the float64 cost of the plain form and of the
-// precision form's islands by 32 / G; with 16 or 32 lanes per world the
-// position and orientation updates are spread over 14 lanes of the group as
-// well (apply_position_change).  The friction solve's matrices do not change
-// during adjustVelocities and are computed once per contact, off the chain
-// (friction_prepare).  With one world per warp in float32 a CTA runs four
-// independent warps (rs_wpc).
+// One warp holds 32 / G worlds; the G lanes of a world solve its islands (the
+// connected components of its contacts, build_islands) side by side, eight
+// lanes to an island.  Within a group of lanes the contacts are lane-strided:
+// the argmax is a butterfly whose tie-break is the reference's first-maximum
+// rule, and the per-iteration update of every contact touching the two
+// resolved bodies is lane-parallel.  The change of the resolved contact's two
+// bodies is spread over the group: lane 4i + c forms component c of body i
+// (velocity_change, position_change), and the changes reach the updated
+// contacts by shuffles.  On GB300 a float64 warp instruction costs the same
+// pipe time whatever its active mask, and a float32 iteration is bound by the
+// instructions it issues, so both forms gain from lanes that work side by
+// side: several islands (or worlds) in one instruction, and one component per
+// lane instead of all of them on one.
 //
-// Groups of a warp advance in lockstep rounds; a group whose world is done
-// idles until the warp's last world finishes its phase.  Worlds are queued in
-// decreasing cost, so the worlds sharing a warp have similar iteration counts.
+// A contact's working values are one record (CREC reals), a body's another
+// (BREC): an update reads four or five 16-byte pieces of one record where the
+// rows of a structure of arrays took seventeen loads, each with its own
+// address.  The friction solve's matrices do not change during
+// adjustVelocities and are computed once per contact, off the chain
+// (friction_prepare).
 //
 // Also here: k_warm_features (the learned warm start's features, tensor-core
 // inference and plan, launched before k_resolve) and the shared pieces of
@@ -42,69 +41,101 @@ template <class R> __device__ __forceinline__ v3<R> contact_tangent(const v3<R>&
   const R s = (R)1 / sqrt_<R>(n.z * n.z + n.y * n.y);
   return V<R>((R)0, -n.z * s, n.y * s);
 }
+// its third column (contact.go:136-138, 149-151), from the first two
+template <class R> __device__ __forceinline__ v3<R> contact_bitangent(const v3<R>& n, const v3<R>& ty) {
+  if (fabs_<R>(n.x) > fabs_<R>(n.y)) return V<R>(n.y * ty.x, n.z * ty.x - n.x * ty.z, -n.y * ty.x);
+  return V<R>(n.y * ty.z - n.z * ty.y, -n.x * ty.z, n.x * ty.y);
+}
 
-template <class R, class W> struct RCtx {
-  W* bw;          // [7][nbs]: position xyz, orientation wxyz (island type)
-  R* br;          // [20][nbs]: vel 0-2, rot 3-5, lfa * dt 6-8, iitWorld 9-17, invMass 18, motion 19
-  uint8_t* aw;    // [nbs] awake
+// four consecutive reals of a record (16- or 32-byte aligned)
+template <class R> struct quad {
+  R a, b, c, d;
+};
+__device__ __forceinline__ quad<float> ld4(const float* p) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  return {t.x, t.y, t.z, t.w};
+}
+__device__ __forceinline__ quad<double> ld4(const double* p) {
+  const double2 s = reinterpret_cast<const double2*>(p)[0], t = reinterpret_cast<const double2*>(p)[1];
+  return {s.x, s.y, t.x, t.y};
+}
+__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
+  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
+  reinterpret_cast<double2*>(p)[0] = make_double2(a, b);
+  reinterpret_cast<double2*>(p)[1] = make_double2(c, d);
+}
+
+// The resolver's view of one world.
+template <class R, class W, bool SM> struct RCtx {
+  W* bw;        // [n][7]: position xyz, orientation wxyz (island type)
+  R* br;        // [n][BREC]: body records
+  uint8_t* aw;  // [n] awake
   int nbs;
-  R* cw;          // working rows of this world's contacts
-  int* cb;        // packed bodies of this world's contacts
-  long long cst;  // row stride of cw
-  R* bc;          // broadcast scratch [12]
-  // warm start / harvest (modes 1, 2): this world's per-body scratch in
-  // global memory (row stride wst) and its contacts' impulse rows
-  R* save;        // [7]: velocity 0-2, rotation 3-5, motion 6 at the start of adjustVelocities
-  R* delta;       // [6]: warm-start velocity and rotation change
-  int* wi;        // [WS_NINT] integer rows (WsInt)
+  R* cr;        // [C][CREC]: contact records
+  // packed bodies of this world's contacts.  SM (worlds of at most 64 bodies):
+  // bits 0-7 and 8-15 the bodies (0xFF: none), bits 16-31 the contact's index
+  // in the narrowphase's list (the records are in island order); else the
+  // narrowphase's packing (pack_bodies), and the records in its order
+  int* cb;
+  R* delta;  // warm start: [6] rows of the velocity and rotation change per body (row stride wst)
+  int* wi;   // [WS_NINT] integer rows (WsInt)
   long long wst;
-  R* jw;          // impulse rows J0..J2 (row stride jst)
+  R* jw;     // impulse rows J0..J2 of the learned paths, by the contact's list index (row stride jst)
   long long jst;
-  R* kw;          // per contact, K_ROW reals: K of the friction solve (inverted in W, kept in R), 9,
-                  // then the response matrix's first row, 3
+  R* kw;     // per contact, K_ROW reals: K of the friction solve (inverted in W, kept in R), 9,
+             // then the response matrix's first row, 3
   const R* gmat;  // friction / restitution rows of the contact list (null: 0.9 / 0.1)
   long long gst;
   R dt;
-  __device__ __forceinline__ W& P(int c, int i) const { return bw[c * nbs + i]; }
-  __device__ __forceinline__ R& Bf(int r, int i) const { return br[r * nbs + i]; }
-  __device__ __forceinline__ R& Cf(int f, int k) const { return cw[(long long)f * cst + k]; }
-  __device__ __forceinline__ R& J(int c, int k) const { return jw[(long long)c * jst + k]; }
-  __device__ __forceinline__ R& K(int q, int k) const { return kw[(long long)k * K_ROW + q]; }
-  __device__ __forceinline__ R& KD(int q, int k) const { return kw[(long long)k * K_ROW + 9 + q]; }
+  bool all_awake;  // every body of the warp's worlds was awake when loaded
+  static __device__ __forceinline__ int B0(int p) { return SM ? p & 0xFF : body0_of(p); }
+  static __device__ __forceinline__ int B1(int p) {
+    if (!SM) return body1_of(p);
+    const int b = (p >> 8) & 0xFF;
+    return b == 0xFF ? -1 : b;
+  }
+  __device__ __forceinline__ void set_pair(int k, int b0, int b1, int list_index) const {
+    cb[k] = SM ? (int)((b0 & 0xFFu) | ((b1 & 0xFFu) << 8) | ((unsigned)list_index << 16)) : pack_bodies(b0, b1);
+  }
+  __device__ __forceinline__ int pair(int k) const { return cb[k]; }
+  // the contact's index in the narrowphase's list
+  __device__ __forceinline__ int list_index(int k) const { return SM ? (int)((unsigned)cb[k] >> 16) : k; }
+  __device__ __forceinline__ W& P(int c, int i) const { return bw[i * 7 + c]; }
+  __device__ __forceinline__ R* body(int i) const { return br + i * BREC; }
+  __device__ __forceinline__ R* rec(int k) const { return cr + (long long)k * CREC; }
+  __device__ __forceinline__ R& J(int c, int o) const { return jw[(long long)c * jst + o]; }
+  __device__ __forceinline__ const R* krow(int k) const { return kw + (long long)k * K_ROW; }
   __device__ __forceinline__ int& WI(int r, int i) const { return wi[(long long)r * wst + i]; }
-  __device__ __forceinline__ R& Save(int r, int i) const { return save[(long long)r * wst + i]; }
   __device__ __forceinline__ R& Delta(int r, int i) const { return delta[(long long)r * wst + i]; }
-  __device__ __forceinline__ v3<R> Bv(int r, int i) const { return V<R>(Bf(r, i), Bf(r + 1, i), Bf(r + 2, i)); }
-  __device__ __forceinline__ v3<R> Cv(int f, int k) const { return V<R>(Cf(f, k), Cf(f + 1, k), Cf(f + 2, k)); }
-  __device__ __forceinline__ void setCv(int f, int k, const v3<R>& a) const {
-    Cf(f, k) = a.x; Cf(f + 1, k) = a.y; Cf(f + 2, k) = a.z;
+  __device__ __forceinline__ v3<R> Bv(int r, int i) const {
+    const R* b = body(i) + r;
+    return V<R>(b[0], b[1], b[2]);
   }
   __device__ __forceinline__ m3<R> iit(int i) const {
     m3<R> m;
+    const R* b = body(i) + BR_IIT;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) m.m[k] = Bf(9 + k, i);
+    for (int k = 0; k < 9; ++k) m.m[k] = b[k];
     return m;
   }
-  __device__ __forceinline__ R friction(int k) const { return gmat ? gmat[k] : (R)0.9; }
-  __device__ __forceinline__ R restitution(int k) const { return gmat ? gmat[gst + k] : (R)0.1; }
-  // contactToWorld: columns normal, tangent y, tangent z; the last is the
-  // reference's formula of the first two (contact.go:136-138, 149-151)
+  // materials, by list index
+  __device__ __forceinline__ R friction(int o) const { return gmat ? gmat[o] : (R)0.9; }
+  __device__ __forceinline__ R restitution(int o) const { return gmat ? gmat[gst + o] : (R)0.1; }
+  // contactToWorld: columns normal, tangent y, tangent z
   __device__ __forceinline__ m3<R> basis(int k) const {
-    const v3<R> n = Cv(W_NX, k);
-    const v3<R> ty = stores_tangent<R>() ? Cv(W_TYX, k) : contact_tangent(n);
+    const R* r = rec(k);
+    const quad<R> a = ld4(r), b = ld4(r + 4);
     m3<R> m;
-    m.m[0] = n.x; m.m[1] = n.y; m.m[2] = n.z;
-    m.m[3] = ty.x; m.m[4] = ty.y; m.m[5] = ty.z;
-    if (fabs_<R>(n.x) > fabs_<R>(n.y)) {
-      m.m[6] = n.y * ty.x;
-      m.m[7] = n.z * ty.x - n.x * ty.z;
-      m.m[8] = -n.y * ty.x;
-    } else {
-      m.m[6] = n.y * ty.z - n.z * ty.y;
-      m.m[7] = -n.x * ty.z;
-      m.m[8] = n.x * ty.y;
-    }
+    m.m[0] = a.a; m.m[1] = a.b; m.m[2] = a.c; m.m[3] = a.d;
+    m.m[4] = b.a; m.m[5] = b.b; m.m[6] = b.c; m.m[7] = b.d;
+    m.m[8] = r[8];
     return m;
+  }
+  __device__ __forceinline__ v3<R> rel(int side, int k) const {
+    const R* r = rec(k) + (side == 0 ? CR_R0 : CR_R1);
+    return V<R>(r[0], r[1], r[2]);
   }
 };
 
@@ -139,75 +170,78 @@ __device__ __forceinline__ void warp_first_max(unsigned long long& key, int& idx
   key = ((unsigned long long)mh << 32) | ml;
 }
 
-// Largest key over the G lanes of a group, smallest index among equal keys
+// Largest key over the L lanes of a group, smallest index among equal keys
 // (the first maximum of the reference's scan, contact.go:238-245, 394-402).
-template <int G, class K> __device__ __forceinline__ void group_first_max(K& key, int& idx) {
-  if constexpr (G == 32) {
+template <int L, class K> __device__ __forceinline__ void group_first_max(K& key, int& idx) {
+  if constexpr (L == 32) {
     warp_first_max(key, idx);
-    return;
-  }
+  } else {
 #pragma unroll
-  for (int off = G / 2; off > 0; off >>= 1) {
-    const K ok = __shfl_xor_sync(0xffffffffu, key, off);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-    if (ok > key || (ok == key && oi < idx)) {
-      key = ok;
-      idx = oi;
+    for (int off = L / 2; off > 0; off >>= 1) {
+      const K ok = __shfl_xor_sync(0xffffffffu, key, off);
+      const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
+      if (ok > key || (ok == key && oi < idx)) {
+        key = ok;
+        idx = oi;
+      }
     }
   }
 }
 
-// calculateDesiredDeltaVelocity, contact.go:87-112, of contact k between
-// bodies b0, b1 with normal n and contact velocity x component cvx (the
-// callers pass what they hold in registers).
-template <class R, class W>
-__device__ __forceinline__ R desired_dv_of(const RCtx<R, W>& x, int k, int b0, int b1, const v3<R>& n, R cvx) {
+// The last frame's acceleration along contact k's normal over the frame, of
+// its awake bodies (contact.go:88-101).  It changes only with the awake flags
+// of its bodies, so adjustVelocities keeps it in the record (CR_VFA) and
+// forms it again where a body woke.
+template <class R, class W, bool SM>
+__device__ __forceinline__ R frame_velocity(const RCtx<R, W, SM>& x, int b0, int b1, const v3<R>& n) {
   R vfa = (R)0;
-  // rows 6-8 hold LastFrameAcceleration * duration, formed when the body is
-  // loaded (the reference's product, once instead of at every use)
-  if (x.aw[b0]) vfa += dot(x.Bv(6, b0), n);
-  if (b1 >= 0 && x.aw[b1]) vfa -= dot(x.Bv(6, b1), n);
-  R rest = x.restitution(k);
-  if (fabs_<R>(cvx) < (R)0.25) rest = (R)0;
-  return -cvx - rest * (cvx - vfa);
+  // LastFrameAcceleration * duration, formed when the body is loaded (the
+  // reference's product, once instead of at every use)
+  if (x.aw[b0]) vfa += dot(x.Bv(BR_LFA, b0), n);
+  if (b1 >= 0 && x.aw[b1]) vfa -= dot(x.Bv(BR_LFA, b1), n);
+  return vfa;
 }
-template <class R, class W> __device__ __forceinline__ R desired_dv(const RCtx<R, W>& x, int k) {
-  const int bb = x.cb[k];
-  return desired_dv_of(x, k, body0_of(bb), body1_of(bb), x.Cv(W_NX, k), x.Cf(W_CVX, k));
+// calculateDesiredDeltaVelocity, contact.go:87-112
+template <class R> __device__ __forceinline__ R desired_dv(R cvx, R vfa, R restitution) {
+  const R rest = fabs_<R>(cvx) < (R)0.25 ? (R)0 : restitution;
+  return -cvx - rest * (cvx - vfa);
 }
 
 // calculateLocalVelocity, contact.go:158-182
-template <class R, class W>
-__device__ __forceinline__ v3<R> local_velocity(const RCtx<R, W>& x, int body, const v3<R>& rp, const m3<R>& C) {
-  v3<R> vel = cross(x.Bv(3, body), rp);
-  add(vel, x.Bv(0, body));
+template <class R, class W, bool SM>
+__device__ __forceinline__ v3<R> local_velocity(const RCtx<R, W, SM>& x, int body, const v3<R>& rp, const m3<R>& C) {
+  v3<R> vel = cross(x.Bv(BR_ROT, body), rp);
+  add(vel, x.Bv(BR_VEL, body));
   v3<R> cv = mulv_t(C, vel);
-  v3<R> acc = x.Bv(6, body);  // LastFrameAcceleration * duration
+  v3<R> acc = x.Bv(BR_LFA, body);  // LastFrameAcceleration * duration
   acc = mulv_t(C, acc);
   acc.x = (R)0;
   add(cv, acc);
   return cv;
 }
 
-// calculateInternals, contact.go:59-85, from the narrowphase rows.
-template <class R, class W>
-__device__ void prepare_contact(const RCtx<R, W>& x, const BatchView<R>& v, long long src, int k) {
+// calculateInternals, contact.go:59-85, of the contact at list index o (row
+// src of the narrowphase's rows), into record k.
+template <class R, class W, bool SM>
+__device__ void prepare_contact(const RCtx<R, W, SM>& x, const BatchView<R>& v, long long src, int k, int o) {
   const long long S = v.nc_total;
   const R* g = v.contact + src;
   v3<R> n = V<R>(g[C_NX * S], g[C_NY * S], g[C_NZ * S]);
   const v3<R> p = V<R>(g[C_PX * S], g[C_PY * S], g[C_PZ * S]);
-  int bb = v.contact_bodies[src];
-  int b0 = body0_of(bb), b1 = body1_of(bb);
+  const int raw = v.contact_bodies[src];
+  int b0 = body0_of(raw), b1 = body1_of(raw);
   if (b0 < 0) {
     mul_with(n, (R)-1);
     b0 = b1;
     b1 = -1;
-    bb = pack_bodies(b0, b1);
   }
-  x.cb[k] = bb;
-  x.setCv(W_NX, k, n);
-  if (stores_tangent<R>()) x.setCv(W_TYX, k, contact_tangent(n));  // calculateContactBasis
-  const m3<R> C = x.basis(k);
+  x.set_pair(k, b0, b1, o);
+  const v3<R> ty = contact_tangent(n);  // calculateContactBasis
+  const v3<R> tz = contact_bitangent(n, ty);
+  m3<R> C;
+  C.m[0] = n.x; C.m[1] = n.y; C.m[2] = n.z;
+  C.m[3] = ty.x; C.m[4] = ty.y; C.m[5] = ty.z;
+  C.m[6] = tz.x; C.m[7] = tz.y; C.m[8] = tz.z;
   v3<R> rp0 = p;
   sub(rp0, V<R>((R)(x.P(0, b0)), (R)(x.P(1, b0)), (R)(x.P(2, b0))));
   v3<R> cv = local_velocity(x, b0, rp0, C);
@@ -218,29 +252,45 @@ __device__ void prepare_contact(const RCtx<R, W>& x, const BatchView<R>& v, long
     v3<R> cv1 = local_velocity(x, b1, rp1, C);
     sub(cv, cv1);
   }
-  x.Cf(W_PEN, k) = g[C_PEN * S];
-  x.setCv(W_R0X, k, rp0);
-  x.setCv(W_R1X, k, rp1);
-  x.setCv(W_CVX, k, cv);
-  x.Cf(W_DDV, k) = desired_dv(x, k);
+  R* r = x.rec(k);
+  st4(r, n.x, n.y, n.z, ty.x);
+  st4(r + 4, ty.y, ty.z, tz.x, tz.y);
+  st4(r + 8, tz.z, rp0.x, rp0.y, rp0.z);
+  st4(r + 12, rp1.x, rp1.y, rp1.z, g[C_PEN * S]);
+  st4(r + 16, cv.x, cv.y, cv.z, desired_dv(cv.x, frame_velocity(x, b0, b1, n), x.restitution(o)));
 }
 
-// SetAwake(true) (rigidbody.go:182-187) through matchAwakeState (contact.go:184-202)
-template <class R, class W> __device__ __forceinline__ void match_awake(const RCtx<R, W>& x, int bb) {
-  const int b0 = body0_of(bb), b1 = body1_of(bb);
-  if (b1 < 0) return;
-  const bool a0 = x.aw[b0] != 0, a1 = x.aw[b1] != 0;
-  if ((a0 || a1) && !(a0 && a1)) {
-    const int t = a0 ? b1 : b0;
-    x.aw[t] = 1;
-    x.Bf(19, t) = (R)(0.3 * 2.0);
+// SetAwake(true) (rigidbody.go:182-187) through matchAwakeState
+// (contact.go:184-202), for the contact with pair bb, by the lanes of a group
+// with `on`; `first` marks the one that writes.  Every lane of the warp calls
+// it; true (for the whole warp) when a body woke.
+template <class R, class W, bool SM>
+__device__ __forceinline__ bool match_awake(const RCtx<R, W, SM>& x, int bb, bool on, bool first) {
+  if (x.all_awake) return false;  // no body falls asleep in the resolver
+  bool woke = false;
+  int t = 0;
+  if (on) {
+    const int b0 = x.B0(bb), b1 = x.B1(bb);
+    if (b1 >= 0) {
+      const bool a0 = x.aw[b0] != 0, a1 = x.aw[b1] != 0;
+      woke = a0 != a1;
+      t = a0 ? b1 : b0;
+    }
   }
+  if (!__any_sync(0xffffffffu, woke)) return false;
+  __syncwarp();
+  if (woke && first) {
+    x.aw[t] = 1;
+    x.body(t)[BR_MOTION] = (R)(0.3 * 2.0);
+  }
+  __syncwarp();
+  return true;
 }
 
 // CalculateDerivedData for a body that is asleep during adjustPositions
 // (contact.go:380-382): renormalise, refresh the world inverse inertia.
-template <class R, class W>
-__device__ void derive_asleep(const RCtx<R, W>& x, const BatchView<R>& v, int bstart, int body) {
+template <class R, class W, bool SM>
+__device__ __noinline__ void derive_asleep(RCtx<R, W, SM> x, const BatchView<R>& v, int bstart, int body) {
   q4<R> q{(R)x.P(3, body), (R)x.P(4, body), (R)x.P(5, body), (R)x.P(6, body)};
   q4<W> qw = cvtq<W>(q);
   qnormalize_island<R, W>(qw);
@@ -251,186 +301,131 @@ __device__ void derive_asleep(const RCtx<R, W>& x, const BatchView<R>& v, int bs
 #pragma unroll
   for (int k = 0; k < 9; ++k) ib.m[k] = v.body[(long long)(B_IB0 + k) * v.nb_pad + bstart + body];
   m3<R> iw = world_inertia(rm, ib);
+  R* b = x.body(body) + BR_IIT;
 #pragma unroll
-  for (int k = 0; k < 9; ++k) x.Bf(9 + k, body) = iw.m[k];
+  for (int k = 0; k < 9; ++k) b[k] = iw.m[k];
   x.P(3, body) = (W)q.w; x.P(4, body) = (W)q.x; x.P(5, body) = (W)q.y; x.P(6, body) = (W)q.z;
 }
 
-// applyPositionChange, contact.go:285-386, by lanes 0 and 1 of a group with
-// `on` (every lane of the warp calls it): lane i moves body i, so the two
-// bodies' float64 position / quaternion updates run side by side; their
-// inertias meet through a shuffle and the total is summed in the reference's
-// order (body 0, then body 1).  Each body's operations are the one-lane
-// formula's, so results are identical.  Lane i leaves body i's linear and
-// angular change in x.bc[3i..3i+2] and x.bc[6+3i..8+3i].
-//
-// With at least 16 lanes per world, the updates of position and orientation
-// are spread over the group: lanes 2-7 add one position component each (body
-// (gl-2)/3), lanes 8-15 one quaternion component each (body (gl-8)/4) and
-// square it; the quaternion's first lane sums the squares in the reference's
-// order and decides the renormalisation (the precision form's island, or
-// Normalize in the float64 form), which every component lane applies.  A
-// float64 warp instruction costs the pipe the same whatever its active
-// lanes, so this takes one float64 add for all fourteen components (seven
-// per body on one lane before) and one multiply for the squares, and in the
-// precision form each lane converts one value.  The operations on every
-// value are the one-lane formula's.
-template <class R, class W, int G>
-__device__ void apply_position_change(const RCtx<R, W>& x, const BatchView<R>& v, int bstart, int k, bool on, int gl) {
-  constexpr bool kSpread = G >= 16;
-  const bool mine = on && gl < 2;
+// Normalize (quaternion.go:77-99) of component c (w first) of a quaternion
+// whose squares sum to s: the component after it.  Out of line: in the
+// precision form's island it is rare.
+template <class W> __device__ __noinline__ W normalize_component(W s, W component, int c) {
+  W len = sqrt_<W>(s);
+  if (real_equal<W>((W)1, len)) return component;
+  if (len == (W)0) return c == 0 ? (W)1 : (W)0;
+  if (len == Lim<W>::inf()) len = Lim<W>::max_value();
+  return component * ((W)1 / len);
+}
+
+// applyPositionChange, contact.go:285-386, of contact k by the first eight
+// lanes (sl = 0..7) of a group with `on`; every lane of the warp calls it.
+// The four lanes 4i..4i+3 move body i: they form its inertia, its moves and
+// its changes alike (the two bodies meet by shuffles, and the total is summed
+// in the reference's order), then lane 4i + c adds position component c
+// (c < 3) and quaternion component c and squares the latter; the squares meet
+// by shuffles and every lane of the body decides the renormalisation alike
+// (the precision form's island, or Normalize in the float64 form).  A float64
+// warp instruction costs the pipe the same whatever its active lanes: two
+// adds and one multiply for both bodies' fourteen components, against seven
+// adds and four multiplies per body on one lane.  The operations on every
+// value are the one-lane formula's, so the bits are the same.  Lane 4i + c
+// returns component c of body i's linear and angular change.
+template <class R, class W, bool SM>
+__device__ void position_change(const RCtx<R, W, SM>& x, const BatchView<R>& v, int bstart, int k, bool on, int sl,
+                                R& linc, R& angc) {
+  const int i = (sl >> 2) & 1, c = sl & 3, src = sl & 4;
   const R z = (R)0;
+  linc = angc = z;
   int b = -1;
-  v3<R> n = V<R>(z, z, z), rp = V<R>(z, z, z);
+  v3<R> n = V<R>(z, z, z), rp = V<R>(z, z, z), ang = V<R>(z, z, z);
   R angI = z, linI = z, penetration = z;
-  if (mine) {
-    const int bb = x.cb[k];
-    b = gl == 0 ? body0_of(bb) : body1_of(bb);
-    n = x.Cv(W_NX, k);
-    rp = gl == 0 ? x.Cv(W_R0X, k) : x.Cv(W_R1X, k);
-    penetration = x.Cf(W_PEN, k);
+  if (on) {
+    const int bb = x.pair(k);
+    b = i == 0 ? x.B0(bb) : x.B1(bb);
+    const R* r = x.rec(k);
+    const quad<R> a = ld4(r);
+    n = V<R>(a.a, a.b, a.c);
+    rp = x.rel(i, k);
+    penetration = r[CR_PEN];
     if (b >= 0) {
-      v3<R> a = cross(rp, n);
-      a = mulv(x.iit(b), a);
-      a = cross(a, rp);
-      angI = dot(a, n);
-      linI = x.Bf(18, b);
+      ang = mulv(x.iit(b), cross(rp, n));
+      angI = dot(cross(ang, rp), n);
+      linI = x.body(b)[BR_INVM];
     }
   }
-  const R angO = __shfl_sync(0xffffffffu, angI, gl ^ 1, G);
-  const R linO = __shfl_sync(0xffffffffu, linI, gl ^ 1, G);
-  const int bO = __shfl_sync(0xffffffffu, b, gl ^ 1, G);
-  if (!kSpread && !mine) return;
-  v3<R> lin = V<R>(z, z, z), ang = V<R>(z, z, z);
-  if (mine) {
-    const int b0 = gl == 0 ? b : bO, b1 = gl == 0 ? bO : b;
+  const R angO = __shfl_xor_sync(0xffffffffu, angI, 4);
+  const R linO = __shfl_xor_sync(0xffffffffu, linI, 4);
+  const int bO = __shfl_xor_sync(0xffffffffu, b, 4);
+  const bool act = on && b >= 0;
+  W acc = (W)0;
+  R qr = z;
+  if (act) {
+    const int b0 = i == 0 ? b : bO, b1 = i == 0 ? bO : b;
     R total = z;
-    if (b0 >= 0) total += (gl == 0 ? linI : linO) + (gl == 0 ? angI : angO);
-    if (b1 >= 0) total += (gl == 0 ? linO : linI) + (gl == 0 ? angO : angI);
-    if (b >= 0) {
-      const R sign = gl != 0 ? (R)-1 : (R)1;
-      R am = sign * penetration * (angI / total);
-      R lm = sign * penetration * (linI / total);
-      v3<R> proj = rp;
-      add_scaled(proj, n, -dot(rp, n));
-      const R maxm = (R)0.2 * mag(proj);
-      if (am < -maxm) {
-        R tm = am + lm;
-        am = -maxm;
-        lm = tm - am;
-      } else if (am > maxm) {
-        R tm = am + lm;
-        am = maxm;
-        lm = tm - am;
-      }
-      if (am != (R)0) {
-        ang = mulv(x.iit(b), cross(rp, n));
-        mul_with(ang, am / angI);
-      }
-      lin = n;
-      mul_with(lin, lm);
-      if constexpr (!kSpread) {
-        // Position.AddScaled(normal, linearMove): product in R, accumulated in W
-        x.P(0, b) += cvt_fast<W>(n.x * lm);
-        x.P(1, b) += cvt_fast<W>(n.y * lm);
-        x.P(2, b) += cvt_fast<W>(n.z * lm);
-        q4<W> q{x.P(3, b), x.P(4, b), x.P(5, b), x.P(6, b)};
-        add_scaled_vector_island<R, W>(q, ang);
-        qnormalize_island<R, W>(q);
-        x.P(3, b) = q.w; x.P(4, b) = q.x; x.P(5, b) = q.y; x.P(6, b) = q.z;
-        if (!x.aw[b]) {
-          // CalculateDerivedData reads the stored (R-rounded) orientation
-          x.P(3, b) = (W)(R)q.w; x.P(4, b) = (W)(R)q.x; x.P(5, b) = (W)(R)q.y; x.P(6, b) = (W)(R)q.z;
-          derive_asleep(x, v, bstart, b);
-        }
-      }
+    if (b0 >= 0) total += (i == 0 ? linI : linO) + (i == 0 ? angI : angO);
+    if (b1 >= 0) total += (i == 0 ? linO : linI) + (i == 0 ? angO : angI);
+    const R sign = i != 0 ? (R)-1 : (R)1;
+    R am = sign * penetration * (angI / total);
+    R lm = sign * penetration * (linI / total);
+    v3<R> proj = rp;
+    add_scaled(proj, n, -dot(rp, n));
+    const R maxm = (R)0.2 * mag(proj);
+    if (am < -maxm) {
+      R tm = am + lm;
+      am = -maxm;
+      lm = tm - am;
+    } else if (am > maxm) {
+      R tm = am + lm;
+      am = maxm;
+      lm = tm - am;
     }
-    x.bc[3 * gl] = lin.x; x.bc[3 * gl + 1] = lin.y; x.bc[3 * gl + 2] = lin.z;
-    x.bc[6 + 3 * gl] = ang.x; x.bc[7 + 3 * gl] = ang.y; x.bc[8 + 3 * gl] = ang.z;
-  }
-  if constexpr (kSpread) {
-    const bool plane = gl >= 2 && gl < 8, qlane = gl >= 8 && gl < 16;
-    const int pc = (gl - 2) % 3, qc = (gl - 8) & 3;
-    const int src = plane ? (gl - 2) / 3 : (qlane ? (gl - 8) >> 2 : 0);  // the body's lane
-    const int bs = __shfl_sync(0xffffffffu, mine ? b : -1, src, G);
-    const bool act = (plane || qlane) && bs >= 0;
+    if (am != (R)0)
+      mul_with(ang, am / angI);
+    else
+      ang = V<R>(z, z, z);
+    linc = c == 3 ? z : (c == 0 ? n.x : (c == 1 ? n.y : n.z)) * lm;
+    angc = c == 0 ? ang.x : (c == 1 ? ang.y : ang.z);
     // the quaternion, narrowed by its component lanes for the increment
     // (add_scaled_vector_island's first step)
-    W acc = (W)0;
-    R qr = z;
-    if (act && qlane) {
-      acc = x.P(3 + qc, bs);
-      qr = cvt_fast<R>(acc);
+    acc = x.P(3 + c, b);
+    qr = cvt_fast<R>(acc);
+  }
+  q4<R> q;
+  q.w = __shfl_sync(0xffffffffu, qr, src, 8);
+  q.x = __shfl_sync(0xffffffffu, qr, src + 1, 8);
+  q.y = __shfl_sync(0xffffffffu, qr, src + 2, 8);
+  q.z = __shfl_sync(0xffffffffu, qr, src + 3, 8);
+  if (act) {
+    // Position.AddScaled(normal, linearMove), and the quaternion increment
+    if (c < 3) x.P(c, b) += cvt_fast<W>(linc);
+    q4<R> t{(R)0, ang.x * (R)1, ang.y * (R)1, ang.z * (R)1};
+    t = qmul(t, q);
+    acc += cvt_fast<W>((c == 0 ? t.w : (c == 1 ? t.x : (c == 2 ? t.y : t.z))) * (R)0.5);
+  }
+  // qnormalize_island on the four components
+  const W sq = act ? acc * acc : (W)0;
+  const W s0 = __shfl_sync(0xffffffffu, sq, src, 8), s1 = __shfl_sync(0xffffffffu, sq, src + 1, 8);
+  const W s2 = __shfl_sync(0xffffffffu, sq, src + 2, 8), s3 = __shfl_sync(0xffffffffu, sq, src + 3, 8);
+  bool asleep = false;
+  if (act) {
+    const W s = s0 + s1 + s2 + s3;
+    const W e = s - (W)1;
+    const W ae = fabs(e);
+    if (sizeof(R) != sizeof(W) && ae < (W)4e-7) {
+    } else if (sizeof(R) != sizeof(W) && ae < (W)0x1p-11) {
+      acc *= (W)1 + e * ((W)-0.5 + e * ((W)0.375 + e * ((W)-0.3125 + e * (W)0.2734375)));
+    } else {  // on the same sum
+      acc = normalize_component<W>(s, acc, c);
     }
-    const int qsrc = 8 + 4 * (gl & 1);
-    const R r0 = __shfl_sync(0xffffffffu, qr, qsrc, G), r1 = __shfl_sync(0xffffffffu, qr, qsrc + 1, G);
-    const R r2 = __shfl_sync(0xffffffffu, qr, qsrc + 2, G), r3 = __shfl_sync(0xffffffffu, qr, qsrc + 3, G);
-    R h0 = z, h1 = z, h2 = z, h3 = z;
-    if (mine && b >= 0) {
-      const q4<R> qq{r0, r1, r2, r3};
-      q4<R> t{(R)0, ang.x * (R)1, ang.y * (R)1, ang.z * (R)1};
-      t = qmul(t, qq);
-      h0 = t.w * (R)0.5; h1 = t.x * (R)0.5; h2 = t.y * (R)0.5; h3 = t.z * (R)0.5;
-    }
-    const R H0 = __shfl_sync(0xffffffffu, h0, src, G), H1 = __shfl_sync(0xffffffffu, h1, src, G);
-    const R H2 = __shfl_sync(0xffffffffu, h2, src, G), H3 = __shfl_sync(0xffffffffu, h3, src, G);
-    const R L0 = __shfl_sync(0xffffffffu, lin.x, src, G), L1 = __shfl_sync(0xffffffffu, lin.y, src, G);
-    const R L2 = __shfl_sync(0xffffffffu, lin.z, src, G);
-    // one float64 add: lanes 2-7 Position.AddScaled(normal, linearMove),
-    // lanes 8-15 the quaternion increment
-    if (act) {
-      R val;
-      if (plane) {
-        acc = x.P(pc, bs);
-        val = pc == 0 ? L0 : (pc == 1 ? L1 : L2);
-      } else {
-        val = qc == 0 ? H0 : (qc == 1 ? H1 : (qc == 2 ? H2 : H3));
-      }
-      acc += cvt_fast<W>(val);
-      if (plane) x.P(pc, bs) = acc;
-    }
-    // qnormalize_island: the squares on the component lanes, the sum in
-    // order and the decision on the quaternion's first lane
-    const W sq = act && qlane ? acc * acc : (W)0;
-    const W s1 = __shfl_sync(0xffffffffu, sq, gl + 1, G), s2 = __shfl_sync(0xffffffffu, sq, gl + 2, G);
-    const W s3 = __shfl_sync(0xffffffffu, sq, gl + 3, G);
-    int mode = 0;  // 0: leave, 1: scale by inv, 2: the identity (a zero quaternion)
-    W inv = (W)0;
-    if (act && qlane && qc == 0) {
-      const W s = sq + s1 + s2 + s3;
-      const W e = s - (W)1;
-      const W ae = fabs(e);
-      if (sizeof(R) != sizeof(W) && ae < (W)4e-7) {
-      } else if (sizeof(R) != sizeof(W) && ae < (W)0x1p-11) {
-        inv = (W)1 + e * ((W)-0.5 + e * ((W)0.375 + e * ((W)-0.3125 + e * (W)0.2734375)));
-        mode = 1;
-      } else {  // Normalize, quaternion.go:77-99, on the same sum
-        W len = sqrt_<W>(s);
-        if (real_equal<W>((W)1, len)) {
-        } else if (len == (W)0) {
-          mode = 2;
-        } else {
-          if (len == Lim<W>::inf()) len = Lim<W>::max_value();
-          inv = (W)1 / len;
-          mode = 1;
-        }
-      }
-    }
-    const int lead = qlane ? gl - qc : 0;
-    mode = __shfl_sync(0xffffffffu, mode, lead, G);
-    inv = __shfl_sync(0xffffffffu, inv, lead, G);
-    if (act && qlane) {
-      if (mode == 1) acc *= inv;
-      else if (mode == 2) acc = qc == 0 ? (W)1 : (W)0;
-      x.P(3 + qc, bs) = acc;
-    }
+    asleep = !x.all_awake && !x.aw[b];
+    // an asleep body's CalculateDerivedData reads the stored (R-rounded) orientation
+    x.P(3 + c, b) = asleep ? (W)(R)acc : acc;
+  }
+  if (!x.all_awake && __any_sync(0xffffffffu, asleep)) {
     __syncwarp();
-    if (mine && b >= 0 && !x.aw[b]) {
-      // CalculateDerivedData reads the stored (R-rounded) orientation
-#pragma unroll
-      for (int c = 3; c < 7; ++c) x.P(c, b) = (W)(R)x.P(c, b);
-      derive_asleep(x, v, bstart, b);
-    }
+    if (asleep && c == 0) derive_asleep(x, v, bstart, b);
+    __syncwarp();
   }
 }
 
@@ -444,21 +439,21 @@ template <class R> __device__ __forceinline__ m3<R> skew(const v3<R>& v) {  // c
 
 // The response matrix of calculateFrictionImpulse (contact.go:540-575): the
 // contact-frame velocity change per unit impulse of both bodies, in R.
-template <class R, class W>
-__device__ __forceinline__ m3<R> friction_response(const RCtx<R, W>& x, int k, int b0, int b1, const m3<R>& C) {
-  R inv_mass = x.Bf(18, b0);
-  m3<R> itt = skew(x.Cv(W_R0X, k));
+template <class R, class W, bool SM>
+__device__ __forceinline__ m3<R> friction_response(const RCtx<R, W, SM>& x, int k, int b0, int b1, const m3<R>& C) {
+  R inv_mass = x.body(b0)[BR_INVM];
+  m3<R> itt = skew(x.rel(0, k));
   m3<R> dvw = mulm(itt, x.iit(b0));
   dvw = mulm(dvw, itt);
   mulm_with(dvw, (R)-1);
   if (b1 >= 0) {
-    itt = skew(x.Cv(W_R1X, k));
+    itt = skew(x.rel(1, k));
     m3<R> d2 = mulm(itt, x.iit(b1));
     d2 = mulm(d2, itt);
     mulm_with(d2, (R)-1);
 #pragma unroll
     for (int q = 0; q < 9; ++q) dvw.m[q] += d2.m[q];
-    inv_mass += x.Bf(18, b1);
+    inv_mass += x.body(b1)[BR_INVM];
   }
   m3<R> dv = transpose(C);
   dv = mulm(dv, dvw);
@@ -469,328 +464,373 @@ __device__ __forceinline__ m3<R> friction_response(const RCtx<R, W>& x, int k, i
   return dv;
 }
 
-// The matrices of contact k's friction solve for the whole of
-// adjustVelocities: K = Invert(response) in W (contact.go:577-580,
+// What adjustVelocities needs of contact k and does not change: the matrices
+// of its friction solve, K = Invert(response) in W (contact.go:577-580,
 // matrix.go:125-153), kept in R for the solve, and the response's first row
-// (R).  They depend on the
-// relative positions, the basis, the inverse masses and the bodies' world
-// inverse inertia, none of which adjustVelocities changes, so computing them
+// (R); and its frame velocity (CR_VFA, in the place of the penetration, which
+// only adjustPositions uses).  They depend on the relative positions, the
+// basis, the inverse masses, the bodies' world inverse inertia and awake
+// flags, of which adjustVelocities changes only the last, so computing them
 // once, lane-parallel, at the start of the phase gives exactly the values the
 // reference recomputes at every iteration; the sequential chain then only
 // forms K * (desired delta velocity, -vy, -vz).
-template <class R, class W> __device__ __forceinline__ void friction_prepare(const RCtx<R, W>& x, int k) {
-  if (x.friction(k) == (R)0) return;  // calculateFrictionlessImpulse needs neither
-  const int bb = x.cb[k];
-  const m3<R> dv = friction_response(x, k, body0_of(bb), body1_of(bb), x.basis(k));
+template <class R, class W, bool SM> __device__ __forceinline__ void friction_prepare(const RCtx<R, W, SM>& x, int k) {
+  const int bb = x.pair(k);
+  const int b0 = x.B0(bb), b1 = x.B1(bb);
+  const m3<R> C = x.basis(k);
+  x.rec(k)[CR_VFA] = frame_velocity(x, b0, b1, V<R>(C.m[0], C.m[1], C.m[2]));
+  if (x.friction(x.list_index(k)) == (R)0) return;  // calculateFrictionlessImpulse needs neither
+  const m3<R> dv = friction_response(x, k, b0, b1, C);
   m3<W> dv_w;
 #pragma unroll
   for (int q = 0; q < 9; ++q) dv_w.m[q] = (W)(dv.m[q]);
   const m3<W> K = invert(dv_w);
-#pragma unroll
-  for (int q = 0; q < 9; ++q) x.K(q, k) = (R)(K.m[q]);
-  x.KD(0, k) = dv.m[0];
-  x.KD(1, k) = dv.m[3];
-  x.KD(2, k) = dv.m[6];
+  R* o = x.kw + (long long)k * K_ROW;
+  st4(o, (R)K.m[0], (R)K.m[1], (R)K.m[2], (R)K.m[3]);
+  st4(o + 4, (R)K.m[4], (R)K.m[5], (R)K.m[6], (R)K.m[7]);
+  st4(o + 8, (R)K.m[8], dv.m[0], dv.m[3], dv.m[6]);
 }
 
-// calculateFrictionImpulse, contact.go:533-606, from the matrices of
-// friction_prepare: the solve K * (desired delta velocity, -vy, -vz) in R,
-// then the dynamic-friction correction.
-// A contact's K (the first 9 reals of its K_ROW block) by 16-byte loads, and
-// the response's first row (reals 9-11), which only the dynamic-friction
-// branch reads.
-__device__ __forceinline__ void load_k(const float* p, float (&o)[9]) {
-  const float4* q = reinterpret_cast<const float4*>(p);
-  const float4 a = q[0], b = q[1];
-  o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-  o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-  o[8] = p[8];
-}
-__device__ __forceinline__ void load_k(const double* p, double (&o)[9]) {
-  const double2* q = reinterpret_cast<const double2*>(p);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const double2 t = q[i];
-    o[2 * i] = t.x; o[2 * i + 1] = t.y;
-  }
-  o[8] = p[8];
-}
-
-template <class R, class W> __device__ v3<R> friction_impulse(const RCtx<R, W>& x, int k) {
-  const R* row = x.kw + (long long)k * K_ROW;
-  m3<R> K;
-  load_k(row, K.m);
-  const R ddv = x.Cf(W_DDV, k);
-  const v3<R> kill = V<R>(ddv, -x.Cf(W_CVY, k), -x.Cf(W_CVZ, k));
-  v3<R> ic = mulv(K, kill);
-  const R fr = x.friction(k);
-  R planar = sqrt_<R>(ic.y * ic.y + ic.z * ic.z);
-  if (planar > ic.x * fr) {
-    ic.y /= planar;
-    ic.z /= planar;
-    ic.x = row[9] + row[10] * fr * ic.y + row[11] * fr * ic.z;
-    ic.x = ddv / ic.x;
-    ic.y *= fr * ic.x;
-    ic.z *= fr * ic.x;
-  }
-  return ic;
-}
-
-// applyVelocityChange, contact.go:447-494 (group leader); velocity and
-// rotation changes of both bodies go to x.bc[0..11].
-template <class R, class W, bool LEARN>
-__device__ void apply_velocity_change(const RCtx<R, W>& x, const BatchView<R>& v, int w, int k) {
-  const int bb = x.cb[k];
-  const int b0 = body0_of(bb), b1 = body1_of(bb);
-  const m3<R> C = x.basis(k);
-  v3<R> ic;
-  if (x.friction(k) == (R)0) {
-    // calculateFrictionlessImpulse, contact.go:496-531
-    v3<R> d = cross(x.Cv(W_R0X, k), x.Cv(W_NX, k));
-    d = mulv(x.iit(b0), d);
-    d = cross(d, x.Cv(W_R0X, k));
-    R dvel = dot(d, x.Cv(W_NX, k));
-    dvel += x.Bf(18, b0);
-    if (b1 < 0) {
-      atomicOr(&v.world_status[w], ST_FRICTIONLESS_NIL);
-      atomicOr(v.status, ST_FRICTIONLESS_NIL);
-    }
-    ic = V<R>(x.Cf(W_DDV, k) / dvel, (R)0, (R)0);
-  } else {
-    ic = friction_impulse(x, k);
-  }
-  if (LEARN && v.mode == 1) {  // harvest: total impulse applied at this contact
-    x.J(0, k) += ic.x;
-    x.J(1, k) += ic.y;
-    x.J(2, k) += ic.z;
-  }
-  const v3<R> imp = mulv(C, ic);
-  const R z = (R)0;
-  v3<R> vc0 = V<R>(z, z, z), vc1 = V<R>(z, z, z), rc1 = V<R>(z, z, z);
-  v3<R> rc0 = mulv(x.iit(b0), cross(x.Cv(W_R0X, k), imp));
-  add_scaled(vc0, imp, x.Bf(18, b0));
-  x.Bf(0, b0) += vc0.x; x.Bf(1, b0) += vc0.y; x.Bf(2, b0) += vc0.z;
-  x.Bf(3, b0) += rc0.x; x.Bf(4, b0) += rc0.y; x.Bf(5, b0) += rc0.z;
-  if (b1 >= 0) {
-    rc1 = mulv(x.iit(b1), cross(imp, x.Cv(W_R1X, k)));
-    add_scaled(vc1, imp, -x.Bf(18, b1));
-    x.Bf(0, b1) += vc1.x; x.Bf(1, b1) += vc1.y; x.Bf(2, b1) += vc1.z;
-    x.Bf(3, b1) += rc1.x; x.Bf(4, b1) += rc1.y; x.Bf(5, b1) += rc1.z;
-  }
-  x.bc[0] = vc0.x; x.bc[1] = vc0.y; x.bc[2] = vc0.z;
-  x.bc[3] = vc1.x; x.bc[4] = vc1.y; x.bc[5] = vc1.z;
-  x.bc[6] = rc0.x; x.bc[7] = rc0.y; x.bc[8] = rc0.z;
-  x.bc[9] = rc1.x; x.bc[10] = rc1.y; x.bc[11] = rc1.z;
-}
-
-
-// applyVelocityChange (contact.go:447-494) spread over lanes 0-5 of a group
-// with `on` (every lane of the warp calls it), for the float64 form, whose
-// chain runs on the float64 pipe: a float64 warp instruction costs the pipe
-// the same whatever its active lanes, so lane c (c = gl % 3) forms component
-// c of the friction solve's product and of the impulse, and lane 3i + c
-// forms component c of body i's velocity and rotation changes, where one
-// lane formed them all before.  Every component is the one-lane formula's
-// (mulv's row, cross's component, add_scaled), so the results are identical.
-// Lane 3i + c leaves body i's changes in x.bc[3i + c] and x.bc[6 + 3i + c].
-template <class R, class W, int G, bool LEARN>
-__device__ void apply_velocity_change_spread(const RCtx<R, W>& x, const BatchView<R>& v, int w, int k, bool on,
-                                             int gl) {
-  const int g0 = (threadIdx.x & 31) - gl;  // the group's first lane
-  const int c = gl % 3, i = gl / 3;
+// applyVelocityChange, contact.go:447-494, of contact k by the first eight
+// lanes (sl = 0..7) of a group with `on`; every lane of the warp calls it.
+// Lane 4i + c (c < 3) forms component c of the friction solve's product
+// (calculateFrictionImpulse, contact.go:533-606, from friction_prepare's
+// matrices), of the impulse, and of body i's velocity and rotation changes,
+// which it adds to the body and returns; the vectors in between meet by
+// shuffles, and the friction cone is decided on every lane alike.  Every
+// component is the one-lane formula's (mulv's row, cross's component,
+// add_scaled), so the bits are the same; one lane forming all of them issued
+// about twice the instructions.  err collects status bits.
+template <class R, class W, bool LEARN, bool SM>
+__device__ __forceinline__ void velocity_change(const RCtx<R, W, SM>& x, const BatchView<R>& v, int k, bool on, int sl,
+                                                R& vc, R& rc, uint32_t& err) {
+  const int i = (sl >> 2) & 1;
+  const bool comp = (sl & 3) != 3;
+  const int c = comp ? sl & 3 : 0;
   const int p = c == 2 ? 0 : c + 1, q = c == 0 ? 2 : c - 1;  // cross component c = a_p b_q - a_q b_p
-  const bool mine = on && gl < 6;
   const R z = (R)0;
-  int b0 = 0, b1 = -1;
-  m3<R> C;
-  v3<R> ic = V<R>(z, z, z);
-  R icc = z;
+  int b = -1, o = 0;
+  R icc = z, ddv = z, fr = (R)0.9;
+  // loaded ahead of the first shuffle, so that one latency covers them: the
+  // basis rows c, the relative position's other components, the body's rows
+  R nc = z, tyc = z, tzc = z, rp = z, rq = z, i0c = z, i1c = z, i2c = z, im = z, vel = z, rot = z;
+  R k9 = z, k10 = z, k11 = z;
   bool frictionless = false;
+  v3<R> ic = V<R>(z, z, z);
   if (on) {
-    const int bb = x.cb[k];
-    b0 = body0_of(bb);
-    b1 = body1_of(bb);
-    C = x.basis(k);
-    frictionless = x.friction(k) == (R)0;
+    const R* kr = x.krow(k);
+    const R kc0 = kr[c], kc1 = kr[3 + c], kc2 = kr[6 + c];
+    k9 = kr[9]; k10 = kr[10]; k11 = kr[11];
+    const R* r = x.rec(k);
+    const int bb = x.pair(k);
+    const int b0 = x.B0(bb), b1 = x.B1(bb);
+    b = i == 0 ? b0 : b1;
+    o = x.list_index(k);
+    fr = x.friction(o);
+    const quad<R> m = ld4(r + CR_CV);
+    nc = r[CR_N + c]; tyc = r[CR_TY + c]; tzc = r[CR_TZ + c];
+    const R* rel = r + (i == 0 ? CR_R0 : CR_R1);
+    rp = rel[p];
+    rq = rel[q];
+    if (b >= 0) {
+      const R* bd = x.body(b);
+      vel = bd[BR_VEL + c];
+      rot = bd[BR_ROT + c];
+      i0c = bd[BR_IIT + c]; i1c = bd[BR_IIT + 3 + c]; i2c = bd[BR_IIT + 6 + c];
+      im = bd[BR_INVM];
+    }
+    ddv = m.d;
+    frictionless = fr == z;
     if (frictionless) {
       // calculateFrictionlessImpulse, contact.go:496-531 (rare: every lane)
-      v3<R> d = cross(x.Cv(W_R0X, k), x.Cv(W_NX, k));
+      const v3<R> r0 = x.rel(0, k), n = V<R>(r[0], r[1], r[2]);
+      v3<R> d = cross(r0, n);
       d = mulv(x.iit(b0), d);
-      d = cross(d, x.Cv(W_R0X, k));
-      R dvel = dot(d, x.Cv(W_NX, k));
-      dvel += x.Bf(18, b0);
-      if (b1 < 0 && gl == 0) {
-        atomicOr(&v.world_status[w], ST_FRICTIONLESS_NIL);
-        atomicOr(v.status, ST_FRICTIONLESS_NIL);
-      }
-      ic = V<R>(x.Cf(W_DDV, k) / dvel, z, z);
+      d = cross(d, r0);
+      R dvel = dot(d, n);
+      dvel += x.body(b0)[BR_INVM];
+      if (b1 < 0 && sl == 0) err |= ST_FRICTIONLESS_NIL;
+      ic = V<R>(ddv / dvel, z, z);
     } else {
       // component c of K * (desired delta velocity, -vy, -vz) (mulv's row c)
-      const R* row = x.kw + (long long)k * K_ROW;
-      const R kx = x.Cf(W_DDV, k), ky = -x.Cf(W_CVY, k), kz = -x.Cf(W_CVZ, k);
-      icc = row[c] * kx + row[3 + c] * ky + row[6 + c] * kz;
+      icc = kc0 * ddv + kc1 * -m.b + kc2 * -m.c;
     }
   }
   {
-    const R i0 = __shfl_sync(FULL, icc, g0, 32), i1 = __shfl_sync(FULL, icc, g0 + 1, 32);
-    const R i2 = __shfl_sync(FULL, icc, g0 + 2, 32);
+    const R i0 = __shfl_sync(0xffffffffu, icc, 0, 4), i1 = __shfl_sync(0xffffffffu, icc, 1, 4);
+    const R i2 = __shfl_sync(0xffffffffu, icc, 2, 4);
     if (on && !frictionless) {
       ic = V<R>(i0, i1, i2);
-      // calculateFrictionImpulse's dynamic friction, contact.go:586-604 (every lane)
-      const R* row = x.kw + (long long)k * K_ROW;
-      const R fr = x.friction(k);
-      const R ddv = x.Cf(W_DDV, k);
-      R planar = sqrt_<R>(ic.y * ic.y + ic.z * ic.z);
+      // the dynamic friction of contact.go:586-604
+      const R planar = sqrt_<R>(ic.y * ic.y + ic.z * ic.z);
       if (planar > ic.x * fr) {
         ic.y /= planar;
         ic.z /= planar;
-        ic.x = row[9] + row[10] * fr * ic.y + row[11] * fr * ic.z;
+        ic.x = k9 + k10 * fr * ic.y + k11 * fr * ic.z;
         ic.x = ddv / ic.x;
         ic.y *= fr * ic.x;
         ic.z *= fr * ic.x;
       }
     }
   }
-  if (LEARN && on && v.mode == 1 && gl == 0) {  // harvest: total impulse applied at this contact
-    x.J(0, k) += ic.x;
-    x.J(1, k) += ic.y;
-    x.J(2, k) += ic.z;
+  if (LEARN && on && v.mode == 1 && sl == 0) {  // harvest: total impulse applied at this contact
+    x.J(0, o) += ic.x;
+    x.J(1, o) += ic.y;
+    x.J(2, o) += ic.z;
   }
-  // component c of the impulse C * ic (mulv's row c)
+  // component c of the impulse contactToWorld * ic (mulv's row c)
   R impc = z;
-  if (on) {
-    const R m0 = c == 0 ? C.m[0] : (c == 1 ? C.m[1] : C.m[2]);
-    const R m3 = c == 0 ? C.m[3] : (c == 1 ? C.m[4] : C.m[5]);
-    const R m6 = c == 0 ? C.m[6] : (c == 1 ? C.m[7] : C.m[8]);
-    impc = m0 * ic.x + m3 * ic.y + m6 * ic.z;
-  }
-  const R ix = __shfl_sync(FULL, impc, g0, 32), iy = __shfl_sync(FULL, impc, g0 + 1, 32);
-  const R iz = __shfl_sync(FULL, impc, g0 + 2, 32);
-  const v3<R> imp = V<R>(ix, iy, iz);
-  const int b = i == 0 ? b0 : b1;
-  const bool act = mine && b >= 0;
+  if (on) impc = nc * ic.x + tyc * ic.y + tzc * ic.z;
+  const R ip = __shfl_sync(0xffffffffu, impc, p, 4), iq = __shfl_sync(0xffffffffu, impc, q, 4);
+  const bool act = on && b >= 0;
   // component c of cross(r0, imp) (body 0) or cross(imp, r1) (body 1)
   R crc = z;
-  v3<R> r = V<R>(z, z, z);
   if (act) {
-    r = i == 0 ? x.Cv(W_R0X, k) : x.Cv(W_R1X, k);
-    const v3<R> a = i == 0 ? r : imp, bv = i == 0 ? imp : r;
-    const R ap = p == 0 ? a.x : (p == 1 ? a.y : a.z), aq = q == 0 ? a.x : (q == 1 ? a.y : a.z);
-    const R bp = p == 0 ? bv.x : (p == 1 ? bv.y : bv.z), bq = q == 0 ? bv.x : (q == 1 ? bv.y : bv.z);
-    crc = ap * bq - aq * bp;
+    const R m1 = rp * iq, m2 = rq * ip;
+    crc = i == 0 ? m1 - m2 : m2 - m1;
   }
-  const int t0 = g0 + 3 * (gl < 6 ? i : 0);
-  const R cx = __shfl_sync(FULL, crc, t0, 32), cy = __shfl_sync(FULL, crc, t0 + 1, 32);
-  const R cz = __shfl_sync(FULL, crc, t0 + 2, 32);
-  R vc = z, rc = z;
+  const R cx = __shfl_sync(0xffffffffu, crc, 0, 4), cy = __shfl_sync(0xffffffffu, crc, 1, 4);
+  const R cz = __shfl_sync(0xffffffffu, crc, 2, 4);
+  vc = rc = z;
   if (act) {
     // rc = iitWorld * cross (mulv's row c); vc = 0 + imp * (+-inverse mass)
-    rc = x.Bf(9 + c, b) * cx + x.Bf(12 + c, b) * cy + x.Bf(15 + c, b) * cz;
-    const R im = i == 0 ? x.Bf(18, b) : -x.Bf(18, b);
-    const R impc_own = c == 0 ? imp.x : (c == 1 ? imp.y : imp.z);
-    vc += impc_own * im;
-    x.Bf(c, b) += vc;
-    x.Bf(3 + c, b) += rc;
-  }
-  if (mine) {
-    x.bc[3 * i + c] = vc;
-    x.bc[6 + 3 * i + c] = rc;
+    rc = i0c * cx + i1c * cy + i2c * cz;
+    vc += impc * (i == 0 ? im : -im);
+    if (comp && sl < 8) {
+      R* bd = x.body(b);
+      bd[BR_VEL + c] = vel + vc;
+      bd[BR_ROT + c] = rot + rc;
+    }
   }
 }
 
+// Whether contact bodies (kb0, kb1) are the resolved bodies d0, d1 (d1 < 0:
+// none): x, y the resolved body that contact body 0, 1 is, else -1.  A contact
+// body is at most one of the two, so a contact takes at most two changes:
+// body 0's first, then body 1's, which is the order of the reference's (b, d)
+// loops (contact.go:254-280, 412-440).
+__device__ __forceinline__ int2 touching(int kb0, int kb1, int d0, int d1) {
+  int2 e;
+  e.x = kb0 == d0 ? 0 : (d1 >= 0 && kb0 == d1 ? 1 : -1);
+  e.y = kb1 < 0 ? -1 : (kb1 == d0 ? 0 : (d1 >= 0 && kb1 == d1 ? 1 : -1));
+  return e;
+}
 
-// A world's body rows from the batch rows into the working rows of x, by the
-// `step` lanes of a group (lane index `first`).
-template <class R, class W>
-__device__ __forceinline__ void load_bodies(const RCtx<R, W>& x, const BatchView<R>& v, long long bstart, int n,
+// The update of a contact after resolving a contact between bodies d0, d1:
+// its penetration (VEL false, contact.go:254-280) or contact velocity and
+// desired delta velocity (VEL true, contact.go:412-440).  update_load reads
+// what it needs of contact k (where `valid`), which the change of the resolved
+// contact does not touch, so the caller loads ahead of computing that change;
+// update_apply takes the change, of which lanes 4d + c of the group of L lanes
+// hold component c of resolved body d's, and returns the value the argmax
+// reads (penetration or desired delta velocity).  A contact touching neither
+// body is left alone.  Every lane of the warp calls both.
+// Most contacts touch one of the two bodies: one pass over the formula with
+// the side selected; the contacts between the two take a second.
+template <class R> struct Touched {
+  int k, bb;
+  int2 e;
+  bool valid;
+  quad<R> q0, q1, q2, q3, m;  // the record: basis, relative positions, penetration or frame velocity; cv, ddv
+};
+template <bool VEL, class R, class W, bool SM>
+__device__ __forceinline__ void update_load(const RCtx<R, W, SM>& x, Touched<R>& t, int k, bool valid, int d0, int d1) {
+  t.k = k;
+  t.valid = valid;
+  t.e = make_int2(-1, -1);
+  t.bb = 0;
+  t.m = t.q3 = quad<R>{(R)0, (R)0, (R)0, (R)0};
+  if (!valid) return;
+  t.bb = x.pair(k);
+  t.e = touching(x.B0(t.bb), x.B1(t.bb), d0, d1);
+  const R* r = x.rec(k);
+  if (VEL) t.m = ld4(r + CR_CV);
+  t.q3 = ld4(r + 12);
+  if (t.e.x < 0 && t.e.y < 0) return;
+  t.q0 = ld4(r);
+  t.q2 = ld4(r + 8);
+  if (VEL) t.q1 = ld4(r + 4);
+}
+template <bool VEL, class R, class W, bool SM>
+__device__ __forceinline__ R update_apply(const RCtx<R, W, SM>& x, Touched<R>& t, R lin, R ang, int L, bool woke) {
+  const bool hit = t.e.x >= 0 || t.e.y >= 0, both = t.e.x >= 0 && t.e.y >= 0;
+  R value = VEL ? t.m.d : t.q3.d;
+  if (!__any_sync(0xffffffffu, hit)) return value;
+  const int s1 = 4 * ((t.e.x >= 0 ? t.e.x : t.e.y) > 0);
+  const v3<R> dl = V<R>(__shfl_sync(0xffffffffu, lin, s1, L), __shfl_sync(0xffffffffu, lin, s1 + 1, L),
+                        __shfl_sync(0xffffffffu, lin, s1 + 2, L));
+  const v3<R> da = V<R>(__shfl_sync(0xffffffffu, ang, s1, L), __shfl_sync(0xffffffffu, ang, s1 + 1, L),
+                        __shfl_sync(0xffffffffu, ang, s1 + 2, L));
+  const bool first0 = t.e.x >= 0;  // the first change is contact body 0's
+  const m3<R> C{{t.q0.a, t.q0.b, t.q0.c, t.q0.d, t.q1.a, t.q1.b, t.q1.c, t.q1.d, t.q2.a}};
+  const v3<R> n = V<R>(t.q0.a, t.q0.b, t.q0.c);
+  if (hit) {
+    v3<R> dv = cross(da, first0 ? V<R>(t.q2.b, t.q2.c, t.q2.d) : V<R>(t.q3.a, t.q3.b, t.q3.c));
+    add(dv, dl);
+    if constexpr (VEL) {
+      const v3<R> a = mulv_t(C, dv);
+      t.m.a = first0 ? t.m.a + a.x : t.m.a - a.x;
+      t.m.b = first0 ? t.m.b + a.y : t.m.b - a.y;
+      t.m.c = first0 ? t.m.c + a.z : t.m.c - a.z;
+    } else {
+      const R a = dot(dv, n);
+      value = first0 ? value - a : value + a;
+    }
+  }
+  if (__any_sync(0xffffffffu, both)) {
+    const int s2 = 4 * (t.e.y > 0);
+    const v3<R> dl2 = V<R>(__shfl_sync(0xffffffffu, lin, s2, L), __shfl_sync(0xffffffffu, lin, s2 + 1, L),
+                           __shfl_sync(0xffffffffu, lin, s2 + 2, L));
+    const v3<R> da2 = V<R>(__shfl_sync(0xffffffffu, ang, s2, L), __shfl_sync(0xffffffffu, ang, s2 + 1, L),
+                           __shfl_sync(0xffffffffu, ang, s2 + 2, L));
+    if (both) {
+      v3<R> dv = cross(da2, V<R>(t.q3.a, t.q3.b, t.q3.c));
+      add(dv, dl2);
+      if constexpr (VEL) {
+        const v3<R> a = mulv_t(C, dv);
+        t.m.a -= a.x;
+        t.m.b -= a.y;
+        t.m.c -= a.z;
+      } else {
+        value += dot(dv, n);
+      }
+    }
+  }
+  if (hit) {
+    R* r = x.rec(t.k);
+    if constexpr (VEL) {
+      R vfa = t.q3.d;
+      if (woke) r[CR_VFA] = vfa = frame_velocity(x, x.B0(t.bb), x.B1(t.bb), n);
+      value = desired_dv(t.m.a, vfa, x.restitution(x.list_index(t.k)));
+      st4(r + CR_CV, t.m.a, t.m.b, t.m.c, value);
+    } else {
+      r[CR_PEN] = value;
+    }
+  }
+  return value;
+}
+
+// A world's bodies from the batch rows into the records of x, by the `step`
+// lanes of a group (lane index `first`).
+// Returns whether this lane's bodies are all awake.
+template <class R, class W, bool SM>
+__device__ __forceinline__ bool load_bodies(const RCtx<R, W, SM>& x, const BatchView<R>& v, long long bstart, int n,
                                             int first, int step) {
   const long long S = v.nb_pad;
+  bool awake = true;
+#pragma unroll 1
   for (int i = first; i < n; i += step) {
-    const long long g = bstart + i;
-    x.P(0, i) = (W)(v.body[B_PX * S + g]);
-    x.P(1, i) = (W)(v.body[B_PY * S + g]);
-    x.P(2, i) = (W)(v.body[B_PZ * S + g]);
-    x.P(3, i) = (W)(v.body[B_QW * S + g]);
-    x.P(4, i) = (W)(v.body[B_QX * S + g]);
-    x.P(5, i) = (W)(v.body[B_QY * S + g]);
-    x.P(6, i) = (W)(v.body[B_QZ * S + g]);
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      x.Bf(r, i) = v.body[(B_VX + r) * S + g];
-      x.Bf(3 + r, i) = v.body[(B_RX + r) * S + g];
-      x.Bf(6 + r, i) = v.body[(B_LX + r) * S + g] * x.dt;
-    }
-#pragma unroll
-    for (int r = 0; r < 9; ++r) x.Bf(9 + r, i) = v.body[(B_IW0 + r) * S + g];
-    x.Bf(18, i) = v.body[B_INVM * S + g];
-    x.Bf(19, i) = v.body[B_MOTION * S + g];
-    x.aw[i] = v.awake[g];
+    const R* g = v.body + bstart + i;
+    auto F = [&](int r) { return g[(long long)r * S]; };
+    x.P(0, i) = (W)F(B_PX); x.P(1, i) = (W)F(B_PY); x.P(2, i) = (W)F(B_PZ);
+    x.P(3, i) = (W)F(B_QW); x.P(4, i) = (W)F(B_QX); x.P(5, i) = (W)F(B_QY); x.P(6, i) = (W)F(B_QZ);
+    R* b = x.body(i);
+    st4(b, F(B_VX), F(B_VY), F(B_VZ), F(B_RX));
+    st4(b + 4, F(B_RY), F(B_RZ), F(B_IW0), F(B_IW1));
+    st4(b + 8, F(B_IW2), F(B_IW3), F(B_IW4), F(B_IW5));
+    st4(b + 12, F(B_IW6), F(B_IW7), F(B_IW8), F(B_INVM));
+    st4(b + 16, F(B_LX) * x.dt, F(B_LY) * x.dt, F(B_LZ) * x.dt, F(B_MOTION));
+    x.aw[i] = v.awake[bstart + i];
+    awake = awake && x.aw[i] != 0;
   }
+  return awake;
+}
+// ... and back
+template <class R, class W, bool SM>
+__device__ __forceinline__ void store_bodies(const RCtx<R, W, SM>& x, const BatchView<R>& v, long long bstart, int n,
+                                             int first, int step) {
+  const long long S = v.nb_pad;
+#pragma unroll 1
+  for (int i = first; i < n; i += step) {
+    R* g = v.body + bstart + i;
+#pragma unroll
+    for (int r = 0; r < 7; ++r) g[(long long)(B_PX + r) * S] = (R)x.P(r, i);
+    const R* b = x.body(i);
+    const quad<R> q0 = ld4(b), q1 = ld4(b + 4), q2 = ld4(b + 8), q3 = ld4(b + 12);
+    g[B_VX * S] = q0.a; g[B_VY * S] = q0.b; g[B_VZ * S] = q0.c;
+    g[B_RX * S] = q0.d; g[B_RY * S] = q1.a; g[B_RZ * S] = q1.b;
+    g[B_IW0 * S] = q1.c; g[B_IW1 * S] = q1.d; g[B_IW2 * S] = q2.a; g[B_IW3 * S] = q2.b; g[B_IW4 * S] = q2.c;
+    g[B_IW5 * S] = q2.d; g[B_IW6 * S] = q3.a; g[B_IW7 * S] = q3.b; g[B_IW8 * S] = q3.c;
+    g[B_MOTION * S] = b[BR_MOTION];
+    v.awake[bstart + i] = x.aw[i];
+  }
+}
+// ResolveContacts' effect on the caller's Contact values that the phases do
+// not produce: the swapped bodies and normal of calculateInternals.
+template <class R, class W, bool SM>
+__device__ __forceinline__ void write_back_contact(const RCtx<R, W, SM>& x, const BatchView<R>& v, long long cst,
+                                                   int k) {
+  const long long S = v.nc_total;
+  const R* r = x.rec(k);
+  const long long o = cst + x.list_index(k);
+  v.contact[C_NX * S + o] = r[0];
+  v.contact[C_NY * S + o] = r[1];
+  v.contact[C_NZ * S + o] = r[2];
+  v.contact_bodies[o] = pack_bodies(x.B0(x.pair(k)), x.B1(x.pair(k)));
 }
 
 // ---------------------------------------------------------------- world slots
-// Shared memory of one world: body rows (W and R), contact working rows,
-// broadcast scratch, packed bodies, awake flags.  The learned paths keep
-// their per-body scratch and the impulse rows in global memory, so they use
-// the same slot (and reach the same occupancy) as the plain resolver.
-// The float64 form (8 or more lanes per world) gathers the contacts touching
-// the two resolved bodies before updating them (see position_loop_g); room
-// for one gather.
+// Shared memory of one world: body and contact records, packed bodies, awake
+// flags, the island table.  The learned paths keep their per-body scratch and
+// the impulse rows in global memory, so they use the same slot (and reach the
+// same occupancy) as the plain resolver.
+// The float64 form gathers the contacts touching the two resolved bodies
+// before updating them (resolve_phase); room for one gather.
 constexpr int kTouchList = 64;
 template <class R> __host__ __device__ constexpr bool gathers_updates() { return sizeof(R) == 8; }
 
 template <class R, class W> __host__ __device__ inline size_t rs_slot_bytes(int nbs, int cs) {
-  const size_t nb16 = (size_t)((nbs + 15) & ~15);
   size_t b = (size_t)7 * nbs * sizeof(W);
-  b += (size_t)20 * nbs * sizeof(R);
-  b += (size_t)w_rows_kept<R>() * cs * sizeof(R);
-  b += 16 * sizeof(R);
+  b += (size_t)BREC * nbs * sizeof(R);
+  b += (size_t)CREC * cs * sizeof(R);
   b += (size_t)cs * sizeof(int);
-  b += nb16;
+  b += (size_t)((nbs + 15) & ~15);
   if (gathers_updates<R>()) b += (size_t)kTouchList * sizeof(int);
+  b += (size_t)(nbs + 4) * sizeof(uint16_t);      // first record of each island
+  b += (size_t)nbs * (sizeof(uint16_t) + 1);      // build_islands: cursors, labels
   return (b + 15) & ~(size_t)15;
 }
 
 template <class R, class W> struct Slot {
-  RCtx<R, W> x;
+  RCtx<R, W, true> x;
   int* ml;          // [kTouchList] contacts touching the two bodies just resolved (float64 form)
-  R* cw_s;
+  R* cr_s;
   int* cb_s;
-  uint8_t* aw_pos;  // awake flags at the start of adjustVelocities (global)
-  uint8_t* aw_pre;  // awake flags at prepareContacts (global)
+  uint16_t* ist;    // [nbs + 1] first record of each island
+  uint16_t* cur;    // [nbs] next free record of the island with smallest body i
+  uint8_t* lab;     // [nbs] smallest body of the body's island
 };
 
 template <class R, class W>
 __device__ __forceinline__ Slot<R, W> make_slot(unsigned char* base, int nbs, int cs, R dt) {
   Slot<R, W> s;
-  RCtx<R, W>& x = s.x;
+  RCtx<R, W, true>& x = s.x;
   x.nbs = nbs;
   x.dt = dt;
   x.bw = reinterpret_cast<W*>(base);
   x.br = reinterpret_cast<R*>(x.bw + 7 * nbs);
-  s.cw_s = x.br + 20 * nbs;
-  x.bc = s.cw_s + (size_t)w_rows_kept<R>() * cs;
-  s.cb_s = reinterpret_cast<int*>(x.bc + 16);
+  s.cr_s = x.br + BREC * nbs;
+  s.cb_s = reinterpret_cast<int*>(s.cr_s + (size_t)CREC * cs);
   x.aw = reinterpret_cast<uint8_t*>(s.cb_s + cs);
   s.ml = reinterpret_cast<int*>(x.aw + ((nbs + 15) & ~15));
-  x.save = x.delta = x.jw = nullptr;
+  s.ist = reinterpret_cast<uint16_t*>(s.ml + (gathers_updates<R>() ? kTouchList : 0));
+  s.cur = s.ist + nbs + 4;
+  s.lab = reinterpret_cast<uint8_t*>(s.cur + nbs);
+  x.delta = x.jw = nullptr;
   x.wi = nullptr;
   x.wst = x.jst = 0;
-  s.aw_pos = s.aw_pre = nullptr;
   return s;
 }
 
 template <class R, class W>
 __device__ __forceinline__ void bind_contacts(Slot<R, W>& s, const BatchView<R>& v, int C, int cs, long long cst) {
-  RCtx<R, W>& x = s.x;
+  RCtx<R, W, true>& x = s.x;
   if (C <= cs) {
-    x.cw = s.cw_s;
+    x.cr = s.cr_s;
     x.cb = s.cb_s;
-    x.cst = cs;
   } else {
-    x.cw = v.work + cst;
+    x.cr = v.work + cst * CREC;
     x.cb = v.work_bodies + cst;
-    x.cst = v.nc_total;
   }
   x.gmat = v.uniform_material ? nullptr : v.contact + (long long)C_FRIC * v.nc_total + cst;
   x.gst = (long long)(C_REST - C_FRIC) * v.nc_total;
@@ -799,16 +839,12 @@ __device__ __forceinline__ void bind_contacts(Slot<R, W>& s, const BatchView<R>&
 
 // the learned paths' global scratch of the world whose bodies start at bstart
 template <class R, class W>
-__device__ __forceinline__ void bind_ws(Slot<R, W>& s, const BatchView<R>& v, long long bstart, long long cst) {
-  RCtx<R, W>& x = s.x;
+__device__ __forceinline__ void bind_ws(RCtx<R, W, true>& x, const BatchView<R>& v, long long bstart, long long cst) {
   x.wst = v.nb_pad;
-  x.save = v.ws_rows + bstart;
-  x.delta = v.ws_rows + 7 * v.nb_pad + bstart;
+  x.delta = v.ws_rows + bstart;
   x.wi = v.ws_int + bstart;
-  x.jw = v.work + (long long)W_J0 * v.nc_total + cst;
+  x.jw = v.ws_imp + cst;
   x.jst = v.nc_total;
-  s.aw_pos = v.ws_u8 + bstart;
-  s.aw_pre = v.ws_u8 + v.nb_pad + bstart;
 }
 
 // The 18 features of a contact at the start of adjustVelocities, all in the
@@ -818,15 +854,16 @@ __device__ __forceinline__ void bind_ws(Slot<R, W>& s, const BatchView<R>& v, lo
 // would resolve the contact alone along its normal (desired delta velocity /
 // response nn), and per body the contacts touching it and their summed
 // positive desired delta velocities (2 + 2).
-template <class R, class W> __device__ void contact_features(const RCtx<R, W>& x, int k, float* f) {
-  const int bb = x.cb[k];
-  const int b0 = body0_of(bb), b1 = body1_of(bb);
-  const v3<R> cv = x.Cv(W_CVX, k);
-  const R ddv = x.Cf(W_DDV, k);
+template <class R, class W, bool SM> __device__ void contact_features(const RCtx<R, W, SM>& x, int k, float* f) {
+  const int bb = x.pair(k);
+  const int b0 = x.B0(bb), b1 = x.B1(bb);
+  const R* r = x.rec(k);
+  const v3<R> cv = V<R>(r[CR_CV], r[CR_CV + 1], r[CR_CV + 2]);
+  const R ddv = r[CR_DDV];
   f[0] = (float)x.WI(WS_NBB, b0);
   f[1] = b1 < 0 ? 1.f : 0.f;
   f[2] = (float)cv.x; f[3] = (float)cv.y; f[4] = (float)cv.z;
-  f[5] = (float)x.Cf(W_PEN, k);
+  f[5] = (float)r[CR_PEN];
   f[6] = (float)ddv;
   const m3<R> K = friction_response(x, k, b0, b1, x.basis(k));
   f[7] = (float)K.m[0]; f[8] = (float)K.m[4]; f[9] = (float)K.m[8];
@@ -866,13 +903,13 @@ template <int G> __device__ __forceinline__ int group_sum(int v) {
 //     warm start does nothing); warm_start_apply adds them.
 // The 32 lanes of a warp plan one world.  Adds this lane's warm-started bodies
 // and the sum of their scales to *nw and *ssum.
-template <class R, class W>
-__device__ void warm_start_plan(const RCtx<R, W>& x, int n, int C, int lane, int* nw, float* ssum) {
+template <class R, class W, bool SM>
+__device__ void warm_start_plan(const RCtx<R, W, SM>& x, int n, int C, int lane, int* nw, float* ssum) {
   const R z = (R)0, eps = (R)0.01;
   for (int k = lane; k < C; k += 32) {
-    const int bb = x.cb[k];
+    const int bb = x.pair(k);
     v3<R> J = V<R>(x.J(0, k), x.J(1, k), x.J(2, k));
-    if (body1_of(bb) >= 0 || x.WI(WS_NBB, body0_of(bb)) != 0 || !(J.x > z)) J = V<R>(z, z, z);  // also NaN
+    if (x.B1(bb) >= 0 || x.WI(WS_NBB, x.B0(bb)) != 0 || !(J.x > z)) J = V<R>(z, z, z);  // also NaN
     const R lim = x.friction(k) * J.x;
     const R planar = sqrt_<R>(J.y * J.y + J.z * J.z);
     if (planar > lim) {
@@ -891,15 +928,15 @@ __device__ void warm_start_plan(const RCtx<R, W>& x, int n, int C, int lane, int
     const int deg = x.WI(WS_DEG, i);
     if (x.WI(WS_NBB, i) == 0 && deg > 0) {
       const m3<R> I = x.iit(i);
-      const R invm = x.Bf(18, i);
+      const R invm = x.body(i)[BR_INVM];
       const int first = x.WI(WS_FIRST, i), last = x.WI(WS_LAST, i);
       const bool run = last - first + 1 == deg;
       for (int k = run ? first : 0; k <= (run ? last : C - 1); ++k) {
-        if (!run && body0_of(x.cb[k]) != i) continue;
+        if (!run && x.B0(x.pair(k)) != i) continue;
         const v3<R> J = V<R>(x.J(0, k), x.J(1, k), x.J(2, k));
         if (J.x == z) continue;
         const v3<R> imp = mulv(x.basis(k), J);
-        add(drot, mulv(I, cross(x.Cv(W_R0X, k), imp)));
+        add(drot, mulv(I, cross(x.rel(0, k), imp)));
         add_scaled(dvel, imp, invm);
       }
     }
@@ -914,9 +951,9 @@ __device__ void warm_start_plan(const RCtx<R, W>& x, int n, int C, int lane, int
   // contact velocity change at s = 1 (into the impulse rows) and the largest
   // scale each contact allows; a body's scale is the smallest of its contacts'
   for (int k = lane; k < C; k += 32) {
-    const int bb = x.cb[k];
-    const int b0 = body0_of(bb);
-    if (body1_of(bb) >= 0 || x.WI(WS_NBB, b0) != 0) {
+    const int bb = x.pair(k);
+    const int b0 = x.B0(bb);
+    if (x.B1(bb) >= 0 || x.WI(WS_NBB, b0) != 0) {
       x.J(0, k) = z;
       x.J(1, k) = z;
       x.J(2, k) = z;
@@ -925,19 +962,19 @@ __device__ void warm_start_plan(const RCtx<R, W>& x, int n, int C, int lane, int
     const m3<R> Ck = x.basis(k);
     const v3<R> dr = V<R>(x.Delta(3, b0), x.Delta(4, b0), x.Delta(5, b0));
     const v3<R> dl = V<R>(x.Delta(0, b0), x.Delta(1, b0), x.Delta(2, b0));
-    v3<R> dv = cross(dr, x.Cv(W_R0X, k));
+    v3<R> dv = cross(dr, x.rel(0, k));
     add(dv, dl);
     const v3<R> dcv = mulv_t(Ck, dv);
     x.J(0, k) = dcv.x;
     x.J(1, k) = dcv.y;
     x.J(2, k) = dcv.z;
     R sk = (R)1;
-    const R ddv = x.Cf(W_DDV, k);
+    const R ddv = x.rec(k)[CR_DDV];
     if (dcv.x > z) {
       const R q = ((ddv > z ? ddv : z) + eps) / dcv.x;
       if (q < sk) sk = q;
     }
-    const R ty = x.Cf(W_CVY, k), tz = x.Cf(W_CVZ, k);
+    const R ty = x.rec(k)[CR_CV + 1], tz = x.rec(k)[CR_CV + 2];
     const R a = dcv.y * dcv.y + dcv.z * dcv.z;
     if (a > z) {
       const R t2 = ty * ty + tz * tz;
@@ -967,9 +1004,9 @@ __device__ void warm_start_plan(const RCtx<R, W>& x, int n, int C, int lane, int
   }
   __syncwarp();
   for (int k = lane; k < C; k += 32) {
-    const int bb = x.cb[k];
-    const int b0 = body0_of(bb);
-    if (body1_of(bb) >= 0 || x.WI(WS_NBB, b0) != 0) continue;
+    const int bb = x.pair(k);
+    const int b0 = x.B0(bb);
+    if (x.B1(bb) >= 0 || x.WI(WS_NBB, b0) != 0) continue;
     const R sb = (R)__int_as_float(x.WI(WS_SCALE, b0));
 #pragma unroll
     for (int c = 0; c < 3; ++c) x.J(c, k) = x.J(c, k) != z ? sb * x.J(c, k) : z;
@@ -983,8 +1020,8 @@ __device__ void warm_start_plan(const RCtx<R, W>& x, int n, int C, int lane, int
 // its values bit for bit.  Every lane of the warp calls it (it synchronises
 // the warp); `on` selects the groups warm-starting.  Returns the bodies this
 // lane moved.
-template <class R, class W, int G>
-__device__ int warm_start_apply(const RCtx<R, W>& x, int n, int C, int gl, bool on) {
+template <class R, class W, int G, bool SM>
+__device__ int warm_start_apply(const RCtx<R, W, SM>& x, int n, int C, int gl, bool on) {
   const R z = (R)0;
   int moved = 0;
   for (int i = gl; on && i < n; i += G) {
@@ -994,252 +1031,415 @@ __device__ int warm_start_apply(const RCtx<R, W>& x, int n, int C, int gl, bool 
     if (!any) continue;
     ++moved;
 #pragma unroll
-    for (int r = 0; r < 6; ++r) x.Bf(r, i) += x.Delta(r, i);
+    for (int r = 0; r < 6; ++r) x.body(i)[BR_VEL + r] += x.Delta(r, i);
   }
   __syncwarp();
   for (int k = gl; on && k < C; k += G) {
-    const v3<R> dcv = V<R>(x.J(0, k), x.J(1, k), x.J(2, k));
+    const int o = x.list_index(k);
+    const v3<R> dcv = V<R>(x.J(0, o), x.J(1, o), x.J(2, o));
     if (dcv.x == z && dcv.y == z && dcv.z == z) continue;
-    v3<R> cv = x.Cv(W_CVX, k);
+    R* r = x.rec(k);
+    v3<R> cv = V<R>(r[CR_CV], r[CR_CV + 1], r[CR_CV + 2]);
     add(cv, dcv);
-    x.setCv(W_CVX, k, cv);
-    x.Cf(W_DDV, k) = desired_dv(x, k);
+    st4(r + CR_CV, cv.x, cv.y, cv.z, desired_dv(cv.x, r[CR_VFA], x.restitution(o)));
   }
   return moved;
 }
 
-// Which resolved body each body of contact k is: e[b] = d when contact body
-// b is resolved body d (d1 < 0: there is none), else -1.  A contact body is
-// at most one of the two, so a contact takes at most two changes: body 0's
-// first, then body 1's, which is the order of the reference's (b, d) loops
-// (contact.go:254-280, 412-440).  The updates below run one code block per
-// contact body, with d taken from e, instead of one per (b, d) pair: a warp
-// runs a block whenever any of its lanes needs it.
-__device__ __forceinline__ int2 touching(int bb, int d0, int d1) {
-  const int kb0 = body0_of(bb), kb1 = body1_of(bb);
-  int2 e;
-  e.x = kb0 == d0 ? 0 : (d1 >= 0 && kb0 == d1 ? 1 : -1);
-  e.y = kb1 < 0 ? -1 : (kb1 == d0 ? 0 : (d1 >= 0 && kb1 == d1 ? 1 : -1));
-  return e;
-}
+// ---------------------------------------------------------------- islands
+// The connected components of a world's contacts over its bodies ("islands";
+// the half-space is no body).  Resolving a contact reads and changes its two
+// bodies and the contacts touching them, so the reference's sequence of
+// resolved contacts, restricted to one island, depends on that island alone:
+// it is the island's own first-maximum sequence.  As long as the world's
+// iterations stay within its budget, the islands can therefore be solved side
+// by side, each by its own group of lanes, and every body, contact and count
+// comes out the same bit for bit.  Only when the budget runs out does the
+// order between the islands matter (which of them got the last iterations);
+// such a world is put back and solved as one list (resolve_phase, LIST false).
+//
+// Why: a settled world of 32 bodies has about 28 islands (spheres and cubes
+// resting alone, a few small heaps) and 130 iterations a frame, of which the
+// longest island has 25, and an iteration keeps 9 of 32 lanes busy.  Solved
+// one after the other, the iterations were 85 % of a frame.
 
-// adjustPositions' update of contact k after resolving a contact between
-// bodies d0, d1 (d1 < 0: none) whose linear / angular changes are in x.bc
-// (contact.go:254-280); a contact touching neither is left alone.
-template <class R, class W>
-__device__ __forceinline__ void penetration_update(const RCtx<R, W>& x, int k, int d0, int d1) {
-  const int2 e = touching(x.cb[k], d0, d1);
-  if (e.x < 0 && e.y < 0) return;
-  const v3<R> nk = x.Cv(W_NX, k);
-  R pen = x.Cf(W_PEN, k);
-#pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    const int d = b == 0 ? e.x : e.y;
-    if (d >= 0) {
-      const v3<R> r = b == 0 ? x.Cv(W_R0X, k) : x.Cv(W_R1X, k);
-      v3<R> dp = cross(d == 0 ? V<R>(x.bc[6], x.bc[7], x.bc[8]) : V<R>(x.bc[9], x.bc[10], x.bc[11]), r);
-      add(dp, d == 0 ? V<R>(x.bc[0], x.bc[1], x.bc[2]) : V<R>(x.bc[3], x.bc[4], x.bc[5]));
-      const R sign = b == 0 ? (R)-1 : (R)1;
-      pen += dot(dp, nk) * sign;
-    }
+// Lanes per island.  8: a resting cube has at most 8 contacts, and the eight
+// lanes are what the spread changes above use; worlds with fewer lanes are one
+// list.
+constexpr int kIslandLanes = 8;
+
+// Finds the islands of a world's C contacts (contact_bodies at list positions
+// cst..) and their places: island i's records are [ist[i], ist[i + 1]), the
+// ones with many contacts first; lab[b] is the smallest body of b's island,
+// cur[lab] the first record of that island (the caller advances it).  Returns
+// the number of islands.  sc: scratch of 3 * 64 ints.  The G lanes of a group
+// (gl) list one world of n <= 64 bodies; every lane of the warp calls it.
+template <int G, class R>
+__device__ __forceinline__ int build_islands(const BatchView<R>& v, long long cst, int n, int nbs, int C, int gl,
+                                             int* sc, uint16_t* ist, uint16_t* cur, uint8_t* lab8) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const unsigned gmask = G == 32 ? FULL : (((1u << G) - 1u) << (lane - gl));
+  int* lab = sc;        // smallest body of the island
+  int* cnt = sc + 64;   // at that body: the island's contacts
+  int* ord = sc + 128;  // islands (their smallest bodies) in order
+  const int* pairs = v.contact_bodies + cst;
+#pragma unroll 1
+  for (int i = gl; i < n; i += G) {
+    lab[i] = i;
+    cnt[i] = 0;
   }
-  x.Cf(W_PEN, k) = pen;
-}
-
-// adjustVelocities' update of contact k (contact.go:412-440), as above.
-template <class R, class W>
-__device__ __forceinline__ void velocity_update(const RCtx<R, W>& x, int k, int d0, int d1) {
-  const int bb = x.cb[k];
-  const int2 e = touching(bb, d0, d1);
-  if (e.x < 0 && e.y < 0) return;
-  const m3<R> Ck = x.basis(k);
-  v3<R> cv = x.Cv(W_CVX, k);
-#pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    const int d = b == 0 ? e.x : e.y;
-    if (d >= 0) {
-      const v3<R> r = b == 0 ? x.Cv(W_R0X, k) : x.Cv(W_R1X, k);
-      v3<R> dv = cross(d == 0 ? V<R>(x.bc[6], x.bc[7], x.bc[8]) : V<R>(x.bc[9], x.bc[10], x.bc[11]), r);
-      add(dv, d == 0 ? V<R>(x.bc[0], x.bc[1], x.bc[2]) : V<R>(x.bc[3], x.bc[4], x.bc[5]));
-      const R sign = b == 1 ? (R)-1 : (R)1;
-      v3<R> t = mulv_t(Ck, dv);
-      mul_with(t, sign);
-      add(cv, t);
-    }
-  }
-  x.setCv(W_CVX, k, cv);
-  x.Cf(W_DDV, k) = desired_dv_of(x, k, body0_of(bb), body1_of(bb), V<R>(Ck.m[0], Ck.m[1], Ck.m[2]), cv.x);
-}
-
-// adjustVelocities, contact.go:388-445, for the groups with run set; returns
-// the iterations used.
-template <class R, class W, int G, bool LEARN>
-__device__ int velocity_loop(const RCtx<R, W>& x, const BatchView<R>& v, int w, int C, int gl, int max_it, bool run) {
-  int used = 0;
-  // the lane's best key over its contacts (k = gl mod G): scanned once here,
-  // then by the update pass of each iteration, which visits the same contacts
-  // in the same order right after changing them (a contact's desired delta
-  // velocity changes only in its own lane), so the argmax is the same
-  auto best = key_of((R)0, (R)0);
-  int bidx = 0x7fffffff;
-  if (run)
+  __syncwarp();
+  // Labels only fall, to a body of the same island; done when every contact
+  // joins equal labels.  Each round also follows the labels' labels, so a
+  // chain of bodies takes few rounds.
+  for (bool more = true; __any_sync(FULL, more);) {
+    more = false;
+#pragma unroll 1
     for (int k = gl; k < C; k += G) {
-      const auto key = key_of(x.Cf(W_DDV, k), (R)0.01);
-      if (key > best) {
-        best = key;
-        bidx = k;
-      }
-    }
-  while (__any_sync(FULL, run)) {
-    group_first_max<G>(best, bidx);
-    if (best == 0) run = false;
-    if (run && gl == 0) {
-      match_awake(x, x.cb[bidx]);
-      apply_velocity_change<R, W, LEARN>(x, v, w, bidx);
+      const int bb = pairs[k];
+      const int b0 = body0_of(bb), b1 = body1_of(bb);
+      if (b0 < 0 || b1 < 0) continue;
+      const int l0 = lab[b0], l1 = lab[b1];
+      if (l0 == l1) continue;
+      const int lo = min(l0, l1);
+      atomicMin(&lab[max(l0, l1)], lo);
+      atomicMin(&lab[b0], lo);
+      atomicMin(&lab[b1], lo);
+      more = true;
     }
     __syncwarp();
-    auto nbest = key_of((R)0, (R)0);
-    int nidx = 0x7fffffff;
-    if (run) {
-      const int rb = x.cb[bidx];
-      const int d0 = body0_of(rb), d1 = body1_of(rb);
-      for (int k = gl; k < C; k += G) {
-        velocity_update(x, k, d0, d1);
-        const auto key = key_of(x.Cf(W_DDV, k), (R)0.01);
-        if (key > nbest) {
-          nbest = key;
-          nidx = k;
+#pragma unroll 1
+    for (int i = gl; i < n; i += G) atomicMin(&lab[i], lab[lab[i]]);
+    __syncwarp();
+  }
+#pragma unroll 1
+  for (int k = gl; k < C; k += G) {
+    const int bb = pairs[k];
+    const int b0 = body0_of(bb);
+    atomicAdd(&cnt[lab[b0 < 0 ? body1_of(bb) : b0]], 1);
+  }
+#pragma unroll 1
+  for (int i = gl; i < n; i += G) lab8[i] = (uint8_t)lab[i];
+  __syncwarp();
+  int ni = 0;
+#pragma unroll 1
+  for (int c = 0; c < 5; ++c)
+#pragma unroll 1
+    for (int base = 0; base < nbs; base += G) {
+      const int i = base + gl;
+      const int m = i < n ? cnt[i] : 0;
+      const bool hit = m > 0 && c == (m >= 24 ? 0 : m >= 12 ? 1 : m >= 6 ? 2 : m >= 3 ? 3 : 4);
+      const unsigned bal = __ballot_sync(FULL, hit) & gmask;
+      if (hit) ord[ni + __popc(bal & below)] = i;
+      ni += __popc(bal);
+    }
+  __syncwarp();
+  int carry = 0;
+#pragma unroll 1
+  for (int base = 0; base < nbs; base += G) {
+    const int p = base + gl;
+    const int r = p < ni ? ord[p] : 0;
+    const int len = p < ni ? cnt[r] : 0;
+    int sum = len;
+#pragma unroll
+    for (int d = 1; d < G; d <<= 1) {
+      const int y = __shfl_up_sync(FULL, sum, d, G);
+      if (gl >= d) sum += y;
+    }
+    if (p < ni) {
+      ist[p] = (uint16_t)(carry + sum - len);
+      cur[r] = (uint16_t)(carry + sum - len);
+    }
+    carry += __shfl_sync(FULL, sum, G - 1, G);
+  }
+  if (gl == 0) ist[ni] = (uint16_t)C;
+  __syncwarp();
+  return ni;
+}
+
+// The record of contact k of a world in island order: its island's next free
+// one.  Called with k ascending over the lanes of a world, G at a time (`on`
+// where there is one), so an island's records keep the list's order.  Every
+// lane of the warp calls it.
+template <int G, class R>
+__device__ __forceinline__ int next_record(const BatchView<R>& v, long long cst, int k, bool on, int gl, uint16_t* cur,
+                                           const uint8_t* lab) {
+  const int lane = threadIdx.x & 31;
+  int r = 0;
+  if (on) {
+    const int bb = v.contact_bodies[cst + k];
+    const int b0 = body0_of(bb);
+    r = lab[b0 < 0 ? body1_of(bb) : b0];
+  }
+  const unsigned same = __match_any_sync(FULL, on ? (lane - gl) * 64 + r : -1 - lane);
+  const int p = on ? cur[r] + __popc(same & ((1u << lane) - 1u)) : 0;
+  __syncwarp();
+  if (on && (same >> lane) == 1u) cur[r] = (uint16_t)(p + 1);
+  __syncwarp();
+  return p;
+}
+
+// adjustPositions (VEL false, contact.go:231-283) or adjustVelocities (VEL
+// true, contact.go:388-445) of the worlds with `run` set, G lanes per world.
+// Every lane of the warp calls it.
+//
+// The groups of L = 8 lanes each take the next island when their own is done;
+// when no world of the warp has more than one island left, all its G lanes
+// take that one (L = G): the islands left last are the long ones, and a round
+// of theirs is then one update pass instead of one per eight contacts.  With
+// `whole`, the world is one list for all G lanes from the start, the
+// reference's own order of work.  Equal values go to the contact that comes
+// first in the narrowphase's list.  `over` is set when the iterations wanted
+// exceed max_it.
+//
+// One body of code serves every width: with an instance each for the islands,
+// the last island and the whole list, the warps of an SM ran from so much code
+// that 8 of 15 stall cycles per instruction were instruction fetches.
+//
+// A lane's best key covers its contacts of the range in order (strict >, so
+// its own first maximum).  In float32 the update pass, which visits them all,
+// also finds the next one.  The float64 form first gathers the contacts
+// touching the resolved bodies (a ballot per L contacts) and updates those,
+// one per lane: walking all of them costs a whole warp instruction on the
+// float64 pipe for every position with a match anywhere in the warp; the next
+// argmax is then a separate scan.  The reference's loop visits every contact
+// but changes only these, and each update touches only its own contact
+// (contact.go:254-280, 412-440), so the result is the same bit for bit.
+struct Progress {
+  int used;    // iterations
+  int rounds;  // rounds this world took part in
+  bool over;   // the world wants more than max_it iterations
+};
+template <class R, class W, int G, bool VEL, bool LEARN>
+__device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, const BatchView<R>& v, int bstart, int C,
+                                                  int gl, int max_it, bool run, bool whole, int ni,
+                                                  const uint16_t* ist, int* ml_world, uint32_t& err) {
+  using Key = decltype(key_of((R)0, (R)0));
+  constexpr bool kGather = gathers_updates<R>();
+  constexpr int kValue = VEL ? CR_DDV : CR_PEN;
+  const int lane = threadIdx.x & 31;
+  const unsigned wmask = G == 32 ? FULL : (((1u << G) - 1u) << (lane - gl));
+  Progress pr{0, 0, false};
+  int L = G, sl = gl, s = 0, e = C, next = 0, len = 0, cap = kTouchList;
+  unsigned lmask = wmask;
+  int* ml = ml_world;
+  if (G > kIslandLanes && !whole) {
+    L = kIslandLanes;
+    sl = gl % L;
+    lmask = 0xFFu << (lane - sl);
+    cap = kTouchList / (G / L);
+    ml = ml_world + gl / L * cap;
+    e = 0;  // no island yet: the first round's maxima are zero
+  } else {
+    ni = 0;
+  }
+  bool have = run, scan = true;
+  Key best = 0;
+  int bidx = 0x7fffffff;
+  auto consider = [&](int k, int bb, R value) {
+    const Key key = key_of(value, (R)0.01);
+    const int id = (int)((unsigned)bb & 0xFFFF0000u) | k;  // by list index
+    if (key > best || (key == best && id < bidx)) {
+      best = key;
+      bidx = id;
+    }
+  };
+#pragma unroll 1
+  for (;;) {
+    if (__any_sync(FULL, scan)) {
+      if (scan) {
+        best = 0;
+        bidx = 0x7fffffff;
+#pragma unroll 1
+        for (int k = s + sl; have && k < e; k += L) consider(k, x.pair(k), x.rec(k)[kValue]);
+      }
+      scan = false;
+      len = (int)__reduce_max_sync(FULL, (unsigned)(have ? e - s : 0));  // the longest of the warp's groups'
+    }
+    if (G > kIslandLanes && L == kIslandLanes)
+      group_first_max<kIslandLanes>(best, bidx);
+    else
+      group_first_max<G>(best, bidx);
+    const unsigned leaders = __ballot_sync(FULL, sl == 0) & wmask;
+    const bool fin = have && best == 0;
+    const unsigned done = __ballot_sync(FULL, fin);
+    if (done) {
+      const unsigned m = done & leaders;
+      if (fin) {  // the next island, in the order of the groups
+        const int isl = next + __popc(m & ((1u << (lane - sl)) - 1u));
+        have = isl < ni;
+        if (have) {
+          s = ist[isl];
+          e = ist[isl + 1];
+        }
+        scan = true;
+      }
+      next += __popc(m);
+      continue;
+    }
+    const unsigned live = __ballot_sync(FULL, have);
+    if (!live) break;
+    const int act = __popc(live & leaders);
+    if (G > kIslandLanes && L == kIslandLanes && __all_sync(FULL, act <= 1 && next >= ni)) {
+      // all lanes of the world on its last island
+      const unsigned held = live & wmask;
+      const int from = held ? __ffs(held) - 1 : lane;
+      s = __shfl_sync(FULL, s, from);
+      e = __shfl_sync(FULL, e, from);
+      have = held != 0;
+      L = G;
+      sl = gl;
+      lmask = wmask;
+      cap = kTouchList;
+      ml = ml_world;
+      scan = true;
+      continue;
+    }
+    if (act && pr.used + act > max_it) pr.over = true;
+    pr.used += act;
+    pr.rounds += act > 0;
+    if (pr.over) have = false;
+    const int k = bidx & 0xFFFF;
+    const int bb = have ? x.pair(k) : 0;
+    const int d0 = have ? x.B0(bb) : -2, d1 = have ? x.B1(bb) : -2;
+    R lin, ang;
+    bool woke = false;
+    auto change = [&]() {
+      woke = match_awake(x, bb, have, sl == 0);
+      if constexpr (VEL)
+        velocity_change<R, W, LEARN>(x, v, k, have && sl < 8, sl, lin, ang, err);
+      else
+        position_change(x, v, bstart, k, have && sl < 8, sl, lin, ang);
+    };
+    if constexpr (kGather) {
+      change();
+      int m = 0;
+#pragma unroll 1
+      for (int base = 0; base < len; base += L) {
+        const int j = s + base + sl;
+        bool hit = false;
+        if (have && j < e) {
+          const int kb = x.pair(j);
+          const int2 h = touching(x.B0(kb), x.B1(kb), d0, d1);
+          hit = h.x >= 0 || h.y >= 0;
+        }
+        const unsigned bal = __ballot_sync(FULL, hit) & lmask;
+        if (hit) ml[m + __popc(bal & ((1u << lane) - 1u))] = j;
+        m += __popc(bal);
+        if (__any_sync(FULL, m > cap - L) || base + L >= len) {
+          __syncwarp();
+          const int mm = (int)__reduce_max_sync(FULL, (unsigned)m);
+#pragma unroll 1
+          for (int q = sl; q - sl < mm; q += L) {
+            Touched<R> t;
+            update_load<VEL>(x, t, q < m ? ml[q] : 0, q < m, d0, d1);
+            update_apply<VEL>(x, t, lin, ang, L, woke);
+          }
+          __syncwarp();
+          m = 0;
         }
       }
+      scan = have;
+    } else {
+      best = 0;
+      bidx = 0x7fffffff;
+#pragma unroll 1
+      for (int base = 0; base < len; base += L) {
+        // the first contacts' records load while the change is computed
+        Touched<R> t;
+        update_load<VEL>(x, t, s + base + sl, have && s + base + sl < e, d0, d1);
+        if (base == 0) change();
+        const R value = update_apply<VEL>(x, t, lin, ang, L, woke);
+        if (t.valid) consider(t.k, t.bb, value);
+      }
     }
     __syncwarp();
-    if (run && ++used >= max_it) run = false;
-    best = nbest;
-    bidx = nidx;
   }
-  return used;
+  return pr;
 }
 
-// ---------------------------------------------------------------- gathered updates
-// The float64 form updates, after a resolved contact, only the contacts
-// touching its two bodies: gathered in contact order (a ballot per G
-// contacts of each world) and updated one per lane of the world's group,
-// instead of every lane walking all its contacts, where a matching contact's
-// float64 update ran once per loop position with a match anywhere in the
-// warp, at the cost of a whole warp instruction on the float64 pipe for
-// each.  The reference's loop visits every contact but changes only these,
-// and each update touches only its own contact (contact.go:254-280,
-// 412-440), so the result is the same bit for bit.  The next argmax is then
-// a separate scan of the world's keys.  With G < 32 the worlds of a warp do
-// this side by side (lockstep, as the other loops).  (In float32 the gather
-// did not pay: the same number of instructions, and more registers.)
-
-// Applies upd(k) to every contact k of the group's world touching body d0 or
-// d1 (nothing where `on` is false).  Every lane of the warp calls it.
-template <int G, class R, class W, class F>
-__device__ __forceinline__ void update_touching(const RCtx<R, W>& x, int C, int gl, int d0, int d1, int* ml, bool on,
-                                                F&& upd) {
-  const int lane = threadIdx.x & 31;
-  const unsigned gmask = G == 32 ? FULL : (((1u << G) - 1u) << (lane - gl));
-  const int Cg = on ? C : 0;
-  int Cmax = Cg;  // the warp's trip count: the largest of its worlds'
-#pragma unroll
-  for (int off = G; off < 32; off <<= 1) Cmax = max(Cmax, __shfl_xor_sync(FULL, Cmax, off));
-  int m = 0;
-  for (int base = 0; base < Cmax; base += G) {
-    const int k = base + gl;
-    bool hit = false;
-    if (k < Cg) {
-      const int bb = x.cb[k];
-      const int kb0 = body0_of(bb), kb1 = body1_of(bb);
-      hit = kb0 == d0 || (d1 >= 0 && kb0 == d1) || (kb1 >= 0 && (kb1 == d0 || kb1 == d1));
+// A phase of the worlds with `run` set: their islands side by side (unless
+// they are all `hard`: their last solve ran out of iterations); then, as
+// one list, the worlds whose islands want more iterations than the budget,
+// after restart(over) has put them back (not with `once`: such a world only
+// reports the whole budget used).
+template <class R, class W, int G, bool VEL, bool LEARN, class F>
+__device__ __forceinline__ Progress resolve_worlds(const RCtx<R, W, true>& x, const BatchView<R>& v, int bstart, int C,
+                                                   int gl, int max_it, bool run, int ni, const uint16_t* ist, int* ml,
+                                                   bool hard, bool once, uint32_t& err, F&& restart) {
+  Progress pr{0, 0, false};
+  uint32_t er = 0;
+  bool on = run;
+#pragma unroll 1
+  for (bool whole = G == kIslandLanes || __all_sync(FULL, !run || hard);; whole = true) {
+    const Progress p = resolve_phase<R, W, G, VEL, LEARN>(x, v, bstart, C, gl, max_it, on, whole, ni, ist, ml, er);
+    if (on) {
+      pr.rounds += p.rounds;
+      pr.used = p.over ? max_it : p.used;
     }
-    const unsigned bal = __ballot_sync(FULL, hit) & gmask;
-    if (hit) ml[m + __popc(bal & ((1u << lane) - 1u))] = k;
-    m += __popc(bal);
-    if (__any_sync(FULL, m > kTouchList - G) || base + G >= Cmax) {
-      __syncwarp();
-      for (int j = gl; j < m; j += G) upd(ml[j]);
-      __syncwarp();
-      m = 0;
-    }
+    // as one list, the budget's end is the reference's
+    pr.over = pr.over || (on && p.over);
+    on = on && p.over && !whole && !once;
+    if (!__any_sync(FULL, on)) break;
+    restart(on);
+    if (on) er = 0;
   }
+  err |= er;
+  return pr;
 }
 
-// The group's first maximum of a row's keys (W_PEN or W_DDV) over its
-// world's contacts (key 0 where `on` is false).
-template <int G, class R, class W>
-__device__ __forceinline__ void group_row_first_max(const RCtx<R, W>& x, int row, int C, int gl, bool on,
-                                                    decltype(key_of((R)0, (R)0))& best, int& bidx) {
-  best = key_of((R)0, (R)0);
-  bidx = 0x7fffffff;
-  for (int k = gl; on && k < C; k += G) {
-    const auto key = key_of(x.Cf(row, k), (R)0.01);
-    if (key > best) {
-      best = key;
-      bidx = k;
-    }
-  }
-  group_first_max<G>(best, bidx);
-}
-
-// adjustPositions (contact.go:231-283) with gathered updates, G lanes per
-// world; returns the iterations used.
+// Puts the worlds with `on` back to the state adjustVelocities starts from:
+// velocities, rotations, motion and awake flags (the batch rows still hold the
+// values before the solve; awake_bits are the flags after adjustPositions,
+// whose matchAwakeState may have woken bodies), and the contact velocities and
+// desired delta velocities prepareContacts left (same velocities, relative
+// positions, basis and awake flags).  Harvested impulse totals start again at
+// zero.  Every lane of the warp calls it.
+// (Rare, so its code stays out of the kernel's: __noinline__, by value.)
 template <class R, class W, int G>
-__device__ int position_loop_g(const RCtx<R, W>& x, const BatchView<R>& v, int bstart, int C, int gl, int max_it,
-                               bool run, int* ml) {
-  int used = 0;
-  while (__any_sync(FULL, run)) {
-    decltype(key_of((R)0, (R)0)) best;
-    int bidx;
-    group_row_first_max<G>(x, W_PEN, C, gl, run, best, bidx);
-    if (best == 0) run = false;
-    if (run && gl == 0) match_awake(x, x.cb[bidx]);
-    __syncwarp();
-    apply_position_change<R, W, G>(x, v, bstart, bidx, run, gl);
-    __syncwarp();
-    int d0 = -2, d1 = -2;
-    if (run) {
-      const int rb = x.cb[bidx];
-      d0 = body0_of(rb);
-      d1 = body1_of(rb);
+__device__ __noinline__ void restart_velocities(RCtx<R, W, true> x, const R* body, const uint8_t* awake, long long S,
+                                                long long bstart, int n, int C, int gl, bool on, unsigned awake_bits,
+                                                bool harvest) {
+  const R* g = body + bstart;
+  __syncwarp();
+  for (int i = gl; on && i < n; i += G) {
+    R* b = x.body(i);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      b[BR_VEL + r] = g[(B_VX + r) * S + i];
+      b[BR_ROT + r] = g[(B_RX + r) * S + i];
     }
-    update_touching<G>(x, C, gl, d0, d1, ml, run, [&](int k) { penetration_update(x, k, d0, d1); });
-    if (run && ++used >= max_it) run = false;
+    x.aw[i] = awake[bstart + i];
   }
-  return used;
-}
-
-// adjustVelocities (contact.go:388-445) with gathered updates, G lanes per
-// world; returns the iterations used.
-template <class R, class W, int G, bool LEARN>
-__device__ int velocity_loop_g(const RCtx<R, W>& x, const BatchView<R>& v, int w, int C, int gl, int max_it,
-                               bool run, int* ml) {
-  int used = 0;
-  while (__any_sync(FULL, run)) {
-    decltype(key_of((R)0, (R)0)) best;
-    int bidx;
-    group_row_first_max<G>(x, W_DDV, C, gl, run, best, bidx);
-    if (best == 0) run = false;
-    if constexpr (sizeof(R) == 8) {
-      if (run && gl == 0) match_awake(x, x.cb[bidx]);
-      __syncwarp();
-      apply_velocity_change_spread<R, W, G, LEARN>(x, v, w, bidx, run, gl);
-    } else if (run && gl == 0) {
-      match_awake(x, x.cb[bidx]);
-      apply_velocity_change<R, W, LEARN>(x, v, w, bidx);
+  __syncwarp();
+  for (int k = gl; on && k < C; k += G) {
+    const int bb = x.pair(k), o = x.list_index(k);
+    const int b0 = x.B0(bb), b1 = x.B1(bb);
+    const m3<R> Ck = x.basis(k);
+    v3<R> cv = local_velocity(x, b0, x.rel(0, k), Ck);
+    if (b1 >= 0) sub(cv, local_velocity(x, b1, x.rel(1, k), Ck));
+    const R vfa = frame_velocity(x, b0, b1, V<R>(Ck.m[0], Ck.m[1], Ck.m[2]));
+    st4(x.rec(k) + CR_CV, cv.x, cv.y, cv.z, desired_dv(cv.x, vfa, x.restitution(o)));
+    if (harvest) {
+      x.J(0, o) = (R)0;
+      x.J(1, o) = (R)0;
+      x.J(2, o) = (R)0;
     }
-    __syncwarp();
-    int d0 = -2, d1 = -2;
-    if (run) {
-      const int rb = x.cb[bidx];
-      d0 = body0_of(rb);
-      d1 = body1_of(rb);
-    }
-    update_touching<G>(x, C, gl, d0, d1, ml, run, [&](int k) { velocity_update(x, k, d0, d1); });
-    if (run && ++used >= max_it) run = false;
   }
-  return used;
+  __syncwarp();
+  for (int i = gl, j = 0; on && i < n; i += G, ++j) {
+    const bool was = x.aw[i] != 0, now = (awake_bits >> j) & 1u;
+    x.body(i)[BR_MOTION] = now && !was ? (R)(0.3 * 2.0) : g[B_MOTION * S + i];
+    if (now && !was) x.aw[i] = 1;
+  }
+  __syncwarp();
+  for (int k = gl; on && k < C; k += G) {
+    const int bb = x.pair(k);
+    const R* r = x.rec(k);
+    x.rec(k)[CR_VFA] = frame_velocity(x, x.B0(bb), x.B1(bb), V<R>(r[0], r[1], r[2]));
+  }
+  __syncwarp();
 }
 
 // v.mode: 0 plain, 1 harvest (plain, copying k_warm_features' features and
@@ -1300,19 +1500,17 @@ __device__ void frame_front(const BatchView<R>& v, int w, int n, int bstart, int
 // fused frame): each world's integrate and narrowphase first
 // (frame_front), so one launch runs a whole frame (one world per warp, plain
 // resolver).
-// Warps per CTA: one world per warp in float32 runs four independent warps
-// per CTA (each its own slot and its own worlds from the queue), so the SM's
-// per-CTA shared-memory reserve is paid once per four slots: 5 CTAs of 4
-// warps (20 warps) fit where 18 one-warp CTAs did.
+// Most warps per CTA (each its own slot and its own worlds from the queue; the
+// host picks the count).  Registers: float32 with one world per warp has 128,
+// 16 warps per SM: at 96 (18 warps, what shared memory allows) the loops'
+// spills missed the little L1 that the slots leave.
 template <class R, int G, bool FRAME> __host__ __device__ constexpr int rs_wpc() {
-  return sizeof(R) == 4 && G == 32 && !FRAME ? 4 : 1;
+  return sizeof(R) == 4 && G == 32 && !FRAME ? 8 : 1;
 }
-// Registers: one world per warp in float32 is bounded to 20 warps per SM (96
-// registers, a few spilled), the count its shared-memory slots allow.
 template <class R, class W, int G, bool LEARN, bool FRAME = false>
 __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
-                                  FRAME ? (sizeof(R) == 4 ? 18 : 8)
-                                        : (G == 32 && sizeof(R) == 4 ? 5 : (LEARN ? 16 : 0)))
+                                  FRAME ? (sizeof(R) == 4 ? 16 : 8)
+                                        : (G == 32 && sizeof(R) == 4 ? 2 : 8))
     k_resolve(BatchView<R> v, int nbs, int cs, R dt, R sleep_bias = (R)0) {
   static_assert(!FRAME || (G == 32 && !LEARN), "the fused frame runs one world per warp, plain");
   extern __shared__ __align__(128) unsigned char smem[];
@@ -1322,8 +1520,7 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
   const int mode = LEARN ? v.mode : 0;
   const size_t slot_bytes = FRAME ? frame_slot_bytes<R, W>(nbs, cs) : rs_slot_bytes<R, W>(nbs, cs);
   Slot<R, W> sl = make_slot<R, W>(smem + (size_t)((threadIdx.x >> 5) * NG + grp) * slot_bytes, nbs, cs, dt);
-  RCtx<R, W>& x = sl.x;
-  const long long S = v.nb_pad;
+  RCtx<R, W, true>& x = sl.x;
   for (;;) {
     unsigned q0 = 0;
     if (lane == 0) q0 = atomicAdd(&v.queue[1], (unsigned)NG);
@@ -1340,12 +1537,16 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
       __syncwarp();
     }
     int C = has ? v.contact_count[w] : 0;
+    // about half of the worlds whose adjustVelocities ran out of its budget do
+    // so again in the next frame: they are solved as one list at once
+    const bool hard = has && (v.cost[w] & kExhausted) != 0;
     if (has) {
       const int cap = v.contact_cap[w];
       if (C > cap) C = cap;  // the world is already flagged ST_CAPACITY
       if (gl == 0) {
         v.pos_iters[w] = 0;
         v.vel_iters[w] = 0;
+        v.cost[w] = 0;
       }
     }
     bool active = has && C > 0 && dt > (R)0;  // ResolveContacts guards, contact.go:210-212
@@ -1358,85 +1559,60 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
     }
     const long long cst = has ? v.contact_start[w] : 0;
     bind_contacts(sl, v, C, cs, cst);
-    if (LEARN && mode) bind_ws(sl, v, bstart, cst);
-    if (active) {
-      load_bodies(x, v, bstart, n, gl, G);
-      if (mode)
-        for (int i = gl; i < n; i += G) sl.aw_pre[i] = x.aw[i];
-    }
+    if (LEARN && mode) bind_ws(x, v, bstart, cst);
+    constexpr int L = kIslandLanes;
+    constexpr bool kIslands = G > L;
+    const int Ca = active ? C : 0;
+    x.all_awake = __all_sync(FULL, !active || load_bodies(x, v, bstart, n, gl, G));
+    int ni = 0;
+    // (its scratch is the contact tile, which prepare_contact fills next)
+    if constexpr (kIslands)
+      ni = build_islands<G>(v, cst, active ? n : 0, nbs, Ca, gl, reinterpret_cast<int*>(sl.cr_s), sl.ist, sl.cur,
+                            sl.lab);
     __syncwarp();
-    if (active)
-      for (int k = gl; k < C; k += G) prepare_contact(x, v, cst + k, k);
+    int Cmax = Ca;  // next_record needs every lane of the warp
+    if (G < 32) Cmax = (int)__reduce_max_sync(FULL, (unsigned)Cmax);
+#pragma unroll 1
+    for (int base = 0; base < Cmax; base += G) {
+      const int k = base + gl;
+      int p = k;
+      if constexpr (kIslands) p = next_record<G>(v, cst, k, k < Ca, gl, sl.cur, sl.lab);
+      if (k < Ca) prepare_contact(x, v, cst + k, p, k);
+    }
     __syncwarp();
     const int max_it = v.max_iterations >= 0 ? v.max_iterations : C * v.iter_mult;
-    constexpr bool kGather = G >= 8 && gathers_updates<R>();
-    // ---------------- adjustPositions, contact.go:231-283
-    int used = 0;
-    if constexpr (kGather) {
-      used = position_loop_g<R, W, G>(x, v, bstart, C, gl, max_it, active && max_it > 0, sl.ml);
-    } else {
-    bool run = active && max_it > 0;
-    // as in velocity_loop: the update pass also finds the next argmax
-    auto best = key_of((R)0, (R)0);
-    int bidx = 0x7fffffff;
-    if (run)
-      for (int k = gl; k < C; k += G) {
-        const auto key = key_of(x.Cf(W_PEN, k), (R)0.01);
-        if (key > best) {
-          best = key;
-          bidx = k;
-        }
-      }
-    while (__any_sync(FULL, run)) {
-      group_first_max<G>(best, bidx);
-      if (best == 0) run = false;
-      if (run && gl == 0) match_awake(x, x.cb[bidx]);
-      __syncwarp();
-      apply_position_change<R, W, G>(x, v, bstart, bidx, run, gl);
-      __syncwarp();
-      auto nbest = key_of((R)0, (R)0);
-      int nidx = 0x7fffffff;
-      if (run) {
-        const int rb = x.cb[bidx];
-        const int d0 = body0_of(rb), d1 = body1_of(rb);
-        for (int k = gl; k < C; k += G) {
-          penetration_update(x, k, d0, d1);
-          const auto key = key_of(x.Cf(W_PEN, k), (R)0.01);
-          if (key > nbest) {
-            nbest = key;
-            nidx = k;
-          }
-        }
-      }
-      __syncwarp();
-      if (run && ++used >= max_it) run = false;
-      best = nbest;
-      bidx = nidx;
-    }
-    }
-    const int pos_used = used;
     const bool solve = active && max_it > 0;
+    uint32_t err = 0;
+    // ---------------- adjustPositions, contact.go:231-283
+    const Progress pos = resolve_worlds<R, W, G, false, LEARN>(
+        x, v, bstart, C, gl, max_it, solve, ni, sl.ist, sl.ml, false, false, err, [&](bool over) {
+          if (over) {
+            load_bodies(x, v, bstart, n, gl, G);
+#pragma unroll 1
+            for (int k = gl; k < C; k += G)
+              x.rec(k)[CR_PEN] = v.contact[C_PEN * v.nc_total + cst + x.list_index(k)];
+          }
+          __syncwarp();
+        });
+    const int pos_used = pos.used;
+    if (active && v.contact_writeback)  // the caller's Contact.Penetration after ResolveContacts
+      for (int k = gl; k < C; k += G) v.contact[C_PEN * v.nc_total + cst + x.list_index(k)] = x.rec(k)[CR_PEN];
     if (solve)
+#pragma unroll 1
       for (int k = gl; k < C; k += G) friction_prepare(x, k);
     __syncwarp();
+    // awake flags after adjustPositions, of this lane's bodies (restart_velocities)
+    unsigned awake_bits = 0;
+    for (int i = gl, j = 0; solve && i < n; i += G, ++j) awake_bits |= (x.aw[i] ? 1u : 0u) << j;
     // ---------------- learned warm start / harvest set-up
     long long hv_base = -1;
-    if (LEARN && mode) {
-      // the state before adjustVelocities, for the fallback; the per-body
-      // aggregates and the predicted impulses come from k_warm_features
-      for (int i = gl; solve && i < n; i += G) {
-        sl.aw_pos[i] = x.aw[i];
-#pragma unroll
-        for (int r = 0; r < 6; ++r) x.Save(r, i) = x.Bf(r, i);
-        x.Save(6, i) = x.Bf(19, i);
+    // the per-body aggregates and the predicted impulses come from k_warm_features
+    if (LEARN && mode == 1)  // harvest: the impulse totals start at zero
+      for (int k = gl; solve && k < C; k += G) {
+        x.J(0, k) = (R)0;
+        x.J(1, k) = (R)0;
+        x.J(2, k) = (R)0;
       }
-      if (mode == 1)  // harvest: the impulse totals start at zero
-        for (int k = gl; solve && k < C; k += G) {
-          x.J(0, k) = (R)0;
-          x.J(1, k) = (R)0;
-          x.J(2, k) = (R)0;
-        }
-    }
     __syncwarp();
     if (LEARN && mode == 1) {
       // every lane takes part in the shuffle; only solving groups reserve rows
@@ -1465,54 +1641,38 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
       warmed = group_sum<G>(nw) > 0;
     }
     // ---------------- adjustVelocities, contact.go:388-445
-    if constexpr (kGather)
-      used = velocity_loop_g<R, W, G, LEARN>(x, v, w, C, gl, max_it, solve, sl.ml);
-    else
-      used = velocity_loop<R, W, G, LEARN>(x, v, w, C, gl, max_it, solve);
-    int vel_used = used;
-    if (LEARN && mode == 2) {
-      // the plain resolver has the last word: a warm-started world that used
-      // all its iterations is solved again by the plain path from the saved
-      // state (a world without a warm-started body was solved plainly)
-      const bool fb = solve && warmed && used >= max_it;
-      if (solve && gl == 0) v.ws_world[w] = ((long long)used << v.warm_shift) > max_it;
-      if (__any_sync(FULL, fb)) {
-        if (fb) {
-          for (int i = gl; i < n; i += G) {
-#pragma unroll
-            for (int r = 0; r < 6; ++r) x.Bf(r, i) = x.Save(r, i);
-            x.Bf(19, i) = x.Save(6, i);
-            x.aw[i] = sl.aw_pos[i];
-          }
+    auto restart = [&](bool over) {
+      if (__any_sync(FULL, over))
+        restart_velocities<R, W, G>(x, v.body, v.awake, v.nb_pad, bstart, n, C, gl, over, awake_bits,
+                                    LEARN && mode == 1);
+    };
+    int vel_used = 0, rounds = 2 * pos.rounds;
+    bool exhausted = false;
+    bool todo = solve;
+    for (bool first = true; __any_sync(FULL, todo); first = false) {
+      const Progress vel = resolve_worlds<R, W, G, true, LEARN>(x, v, bstart, C, gl, max_it, todo, ni, sl.ist, sl.ml,
+                                                                hard, first && warmed, err, restart);
+      bool again = false;
+      if (todo) {
+        vel_used += vel.used;
+        rounds += vel.rounds;
+        exhausted = vel.over;
+        if (LEARN && mode == 2 && first) {
+          // the plain resolver has the last word: a warm-started world that
+          // used all its iterations is solved again by the plain path (a
+          // world without a warm-started body was solved plainly)
+          if (gl == 0) v.ws_world[w] = ((long long)vel.used << v.warm_shift) > max_it;
+          again = warmed && vel.used >= max_it;
+          if (again && gl == 0) atomicAdd(&v.counters[4], 1ull);
         }
-        __syncwarp();
-        if (fb) {
-          // contact velocities as prepareContacts left them (same velocities,
-          // relative positions and basis), desired delta velocity with the
-          // awake flags of that moment
-          uint8_t* aw_now = x.aw;
-          x.aw = sl.aw_pre;
-          for (int k = gl; k < C; k += G) {
-            const int bb = x.cb[k];
-            const int b0 = body0_of(bb), b1 = body1_of(bb);
-            const m3<R> Ck = x.basis(k);
-            v3<R> cv = local_velocity(x, b0, x.Cv(W_R0X, k), Ck);
-            if (b1 >= 0) sub(cv, local_velocity(x, b1, x.Cv(W_R1X, k), Ck));
-            x.setCv(W_CVX, k, cv);
-            x.Cf(W_DDV, k) = desired_dv(x, k);
-          }
-          x.aw = aw_now;
-        }
-        __syncwarp();
-        int used2;
-        if constexpr (kGather)
-          used2 = velocity_loop_g<R, W, G, LEARN>(x, v, w, C, gl, max_it, fb, sl.ml);
-        else
-          used2 = velocity_loop<R, W, G, LEARN>(x, v, w, C, gl, max_it, fb);
-        if (fb) vel_used += used2;
-        if (fb && gl == 0) atomicAdd(&v.counters[4], 1ull);
       }
-      if (warm_ok && gl == 0) atomicAdd(&v.counters[5], 1ull);
+      if (LEARN) restart(again);
+      todo = again;
+    }
+    if (LEARN && mode == 2 && warm_ok && gl == 0) atomicAdd(&v.counters[5], 1ull);
+    if (err) {
+      atomicOr(&v.world_status[w], err);
+      atomicOr(v.status, err);
     }
     if (LEARN && mode == 1 && hv_base >= 0) {
       for (int k = gl; k < C; k += G) {
@@ -1524,45 +1684,15 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
     }
     if (has && gl == 0) {
       v.pos_iters[w] = pos_used;
+      v.cost[w] = rounds | (exhausted ? kExhausted : 0);
       v.vel_iters[w] = vel_used;
       atomicAdd(&v.counters[1], (unsigned long long)pos_used);
       atomicAdd(&v.counters[2], (unsigned long long)vel_used);
       atomicAdd(&v.counters[3], (unsigned long long)C);
     }
-    if (active && v.contact_writeback) {
-      // the caller's Contact values after ResolveContacts (penetration,
-      // swapped bodies and normal of calculateInternals)
-      const long long CS = v.nc_total;
-      for (int k = gl; k < C; k += G) {
-        R* o = v.contact + cst + k;
-        o[C_NX * CS] = x.Cf(W_NX, k);
-        o[C_NY * CS] = x.Cf(W_NY, k);
-        o[C_NZ * CS] = x.Cf(W_NZ, k);
-        o[C_PEN * CS] = x.Cf(W_PEN, k);
-        v.contact_bodies[cst + k] = x.cb[k];
-      }
-    }
-    if (active) {
-      for (int i = gl; i < n; i += G) {
-        const long long g = bstart + i;
-        v.body[B_PX * S + g] = (R)(x.P(0, i));
-        v.body[B_PY * S + g] = (R)(x.P(1, i));
-        v.body[B_PZ * S + g] = (R)(x.P(2, i));
-        v.body[B_QW * S + g] = (R)(x.P(3, i));
-        v.body[B_QX * S + g] = (R)(x.P(4, i));
-        v.body[B_QY * S + g] = (R)(x.P(5, i));
-        v.body[B_QZ * S + g] = (R)(x.P(6, i));
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          v.body[(B_VX + r) * S + g] = x.Bf(r, i);
-          v.body[(B_RX + r) * S + g] = x.Bf(3 + r, i);
-        }
-#pragma unroll
-        for (int r = 0; r < 9; ++r) v.body[(B_IW0 + r) * S + g] = x.Bf(9 + r, i);
-        v.body[B_MOTION * S + g] = x.Bf(19, i);
-        v.awake[g] = x.aw[i];
-      }
-    }
+    if (active && v.contact_writeback)
+      for (int k = gl; k < C; k += G) write_back_contact(x, v, cst, k);
+    if (active) store_bodies(x, v, bstart, n, gl, G);
     __syncwarp();
   }
 }
@@ -1586,7 +1716,7 @@ constexpr int kWfWarps = 4;                       // worlds in flight per CTA
 
 // bytes of one warp's body rows, and of a CTA
 template <class R, class W> __host__ __device__ inline size_t wf_slot_bytes(int nbs) {
-  return ((size_t)7 * nbs * sizeof(W) + (size_t)20 * nbs * sizeof(R) + (size_t)((nbs + 15) & ~15) + 15) & ~(size_t)15;
+  return ((size_t)7 * nbs * sizeof(W) + (size_t)BREC * nbs * sizeof(R) + (size_t)((nbs + 15) & ~15) + 15) & ~(size_t)15;
 }
 template <class R, class W> __host__ __device__ inline size_t wf_smem_bytes(int nbs) {
   return WF_BYTES + kWfWarps * wf_slot_bytes<R, W>(nbs);
@@ -1647,15 +1777,15 @@ __global__ void __launch_bounds__(32 * kWfWarps) k_warm_features(BatchView<R> v,
   const float* isg = reinterpret_cast<const float*>(smem + WF_IS);
   const float* osc = reinterpret_cast<const float*>(smem + WF_OS);
   unsigned char* slot = smem + WF_BYTES + (size_t)wid * wf_slot_bytes<R, W>(nbs);
-  RCtx<R, W> x;
+  RCtx<R, W, true> x;
   x.nbs = nbs;
   x.dt = dt;
   x.bw = reinterpret_cast<W*>(slot);
   x.br = reinterpret_cast<R*>(x.bw + 7 * nbs);
-  x.aw = reinterpret_cast<uint8_t*>(x.br + 20 * nbs);
-  x.bc = nullptr;
-  x.save = x.delta = nullptr;
+  x.aw = reinterpret_cast<uint8_t*>(x.br + BREC * nbs);
+  x.delta = nullptr;
   x.kw = nullptr;
+  x.all_awake = false;
   const bool harvest = v.mode == 1;
   for (;;) {
     unsigned q = 0;
@@ -1672,16 +1802,11 @@ __global__ void __launch_bounds__(32 * kWfWarps) k_warm_features(BatchView<R> v,
     if (C <= 0 || dt <= (R)0 || n > nbs || max_it <= 0 || (!harvest && v.ws_world[w])) continue;
     const long long bstart = v.body_start[w];
     const long long cst = v.contact_start[w];
-    x.cw = v.work + cst;
+    x.cr = v.work + cst * CREC;
     x.cb = v.work_bodies + cst;
-    x.cst = v.nc_total;
     x.gmat = v.uniform_material ? nullptr : v.contact + (long long)C_FRIC * v.nc_total + cst;
     x.gst = (long long)(C_REST - C_FRIC) * v.nc_total;
-    x.wi = v.ws_int + bstart;
-    x.wst = v.nb_pad;
-    x.jw = v.work + (long long)W_J0 * v.nc_total + cst;
-    x.jst = v.nc_total;
-    x.delta = v.ws_rows + 7 * v.nb_pad + bstart;
+    bind_ws(x, v, bstart, cst);
     load_bodies(x, v, bstart, n, lane, 32);
     for (int i = lane; i < n; i += 32) {
       x.WI(WS_DEG, i) = 0;
@@ -1692,10 +1817,10 @@ __global__ void __launch_bounds__(32 * kWfWarps) k_warm_features(BatchView<R> v,
     }
     __syncwarp();
     for (int k = lane; k < C; k += 32) {
-      prepare_contact(x, v, cst + k, k);
-      const int bb = x.cb[k];
-      const int b0 = body0_of(bb), b1 = body1_of(bb);
-      const float dd = (float)x.Cf(W_DDV, k);
+      prepare_contact(x, v, cst + k, k, k);
+      const int bb = x.pair(k);
+      const int b0 = x.B0(bb), b1 = x.B1(bb);
+      const float dd = (float)x.rec(k)[CR_DDV];
       const int fx = dd > 0.f ? (int)(fminf(dd, 100.f) * kLoadScale + 0.5f) : 0;
       atomicAdd(&x.WI(WS_DEG, b0), 1);
       atomicAdd(&x.WI(WS_LOAD, b0), fx);

@@ -1,282 +1,241 @@
 // ResolveContacts (contact.go:204-445) for worlds whose bodies do not fit the
 // shared-memory slot of k_resolve (hundreds to thousands of bodies).
 //
-// One warp per world, or one per two worlds (16 lanes each).  Body and
-// contact working rows live in global memory (L2-resident at these sizes).
-// The argmax over a world's contacts is a lane-strided scan (four interleaved
-// chains per lane) and the first-maximum butterfly of k_resolve.  After
-// prepareContacts every body gets the list of its contacts (counting sort by
-// body, in global memory), so the update after each resolved contact visits
-// only the contacts of the two resolved bodies instead of all C: the
-// reference's loop over every contact skips the others, so the visited set
-// and each contact's arithmetic are the same (penetration_update /
-// velocity_update), and the float64 form stays bit-identical.  The order of
-// the visits does not matter: each contact's update reads only its own rows
-// and the resolved contact's broadcast changes.
+// One warp per world: such a world is mostly one island, so its iterations are
+// one chain, and what counts is the latency of an iteration.
+//   * Body and contact records are in global memory (L1/L2); a record is two
+//     cache lines at most, where rows took a line per value.
+//   * The argmax is over chunk maxima in shared memory (at most kBigChunks),
+//     kept by refreshing the chunks of the contacts an iteration changed,
+//     instead of a scan over every contact's value.
+//   * After prepareContacts every body gets the list of its contacts (counting
+//     sort by body), so the update after each resolved contact visits only the
+//     contacts of the two resolved bodies: the reference's loop over every
+//     contact skips the others, so the visited set and each contact's
+//     arithmetic are the same (contact_update), and the bits too.  The order
+//     of the visits does not matter: each contact's update reads only its own
+//     record and the resolved contact's changes.
+//   * The packed bodies, the keys and the lists are in shared memory where the
+//     world's contacts fit it, so the records an update will need are known,
+//     and loaded, while the resolved contact's change is computed.
 #pragma once
 #include "cz_resolve.cuh"
 
 namespace cz {
 
-// Visit every contact of bodies d0 and d1 once (lists adj[off[b] .. end[b]))
-// with the G lanes of a group.
-template <int G, class R, class W, class F>
-__device__ __forceinline__ void for_pair_contacts(const RCtx<R, W>& x, const int* __restrict__ adj, const int* off,
-                                                  const int* end, int d0, int d1, int gl, F f) {
-  const int o0 = off[d0], l0 = end[d0] - o0;
-  const int o1 = d1 >= 0 ? off[d1] : 0, l1 = d1 >= 0 ? end[d1] - o1 : 0;
-  for (int e = gl; e < l0 + l1; e += G) {
-    int k;
-    if (e < l0) {
-      k = adj[o0 + e];
-    } else {
-      k = adj[o1 + e - l0];
-      const int bb = x.cb[k];
-      if (body0_of(bb) == d0 || body1_of(bb) == d0) continue;  // visited in d0's list
-    }
-    f(k);
-  }
-}
+constexpr int kBigChunks = 512;  // chunks of a world's contacts (16 each up to 8192 contacts)
 
-// The lane's first maximum of key_of(row[k], 0.01) over its contacts k = gl,
-// gl + G, ...: four interleaved running maxima (four independent compare
-// chains instead of one), each keeping its first maximum, merged by key and
-// then the smaller index.  The result is what one in-order scan of the
-// lane's contacts finds.
-template <int G, class R, class W>
-__device__ __forceinline__ void lane_first_max(const RCtx<R, W>& x, int row, int C, int gl,
-                                               decltype(key_of((R)0, (R)0))& best, int& bidx) {
-  using K = decltype(key_of((R)0, (R)0));
-  K b[4];
-  int ix[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    b[q] = 0;
-    ix[q] = 0x7fffffff;
-  }
-  int k = gl;
-  for (; k + 3 * G < C; k += 4 * G) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const K key = key_of(x.Cf(row, k + G * q), (R)0.01);
-      if (key > b[q]) {
-        b[q] = key;
-        ix[q] = k + G * q;
+// shared memory ahead of the per-contact arrays: chunk maxima and their first
+// contacts, list starts and ends of n bodies
+template <class R> __host__ __device__ inline size_t big_fixed_bytes(int n) {
+  return (size_t)kBigChunks * (sizeof(R) + sizeof(int)) + (size_t)2 * ((n + 3) & ~3) * sizeof(int);
+}
+// per contact: key, packed bodies, two list entries
+template <class R> __host__ __device__ constexpr size_t big_contact_bytes() { return sizeof(R) + 3 * sizeof(int); }
+
+// The chunk maxima of a world's keys and the first contact holding each.
+template <class Key> struct BigKeys {
+  Key* key;     // [C]
+  Key* cmax;    // [kBigChunks]
+  int* cfirst;  // [kBigChunks]
+  int C, shift;  // chunk of contact k: k >> shift
+  // the chunk's first maximum again, by one lane
+  __device__ __forceinline__ void refresh(int ch) const {
+    const int k0 = ch << shift, k1 = min(C, k0 + (1 << shift));
+    Key best = 0;
+    int at = k0;
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) {
+      const Key q = key[k];
+      if (q > best) {
+        best = q;
+        at = k;
       }
     }
+    cmax[ch] = best;
+    cfirst[ch] = at;
   }
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {  // at most three contacts left
-    const int kq = k + G * q;
-    if (kq < C) {
-      const K key = key_of(x.Cf(row, kq), (R)0.01);
-      if (key > b[q]) {
-        b[q] = key;
-        ix[q] = kq;
-      }
-    }
-  }
-#pragma unroll
-  for (int q = 1; q < 4; ++q) {
-    if (b[q] > b[0] || (b[q] == b[0] && ix[q] < ix[0])) {
-      b[0] = b[q];
-      ix[0] = ix[q];
-    }
-  }
-  best = b[0];
-  bidx = ix[0];
-}
+};
 
-// One warp, 32 / G worlds of the large-world list (world blockIdx.x * 32 / G
-// + group), G lanes each.  With G = 16 the two worlds of a warp run their
-// iterations in lockstep, so the sequential part of each iteration (the
-// leader's float64 island arithmetic) is issued once for both.  Control flow
-// is uniform across the warp: a group whose world is missing or finished
-// keeps taking part in the warp-wide shuffles and barriers with its `run`
-// flag cleared.
-template <class R, class W, int G>
-__global__ void __launch_bounds__(32) k_resolve_big(BatchView<R> v, R dt) {
-  constexpr int NG = 32 / G;
-  __shared__ R bcs[NG][16];
+// adjustPositions (VEL false) or adjustVelocities (VEL true) of one world by
+// its warp; returns the iterations used.
+template <class R, class W, bool VEL, class Key>
+__device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const BatchView<R>& v, int bstart,
+                                         const BigKeys<Key>& bk, const int* off, const int* end, const int* adj,
+                                         int max_it, uint32_t& err) {
   const int lane = threadIdx.x;
-  const int grp = lane / G, gl = lane % G;
-  const int wi = blockIdx.x * NG + grp;
-  const bool has = wi < v.big_count;
-  const int w = has ? v.big_list[wi] : 0;
-  const int n = has ? v.body_count[w] : 0;
-  const int bstart = has ? v.body_start[w] : 0;
-  const long long cst = has ? v.contact_start[w] : 0;
-  const long long S = v.nb_pad;
-  int C = has ? v.contact_count[w] : 0;
-  const int cap = has ? v.contact_cap[w] : 0;
-  if (C > cap) C = cap;  // the world is already flagged ST_CAPACITY
-  RCtx<R, W> x;
-  x.nbs = (int)S;  // row stride of the global body rows
+  const int C = bk.C;
+  const int nch = (C + (1 << bk.shift) - 1) >> bk.shift;
+  for (int k = lane; k < C; k += 32) bk.key[k] = key_of(x.rec(k)[VEL ? CR_DDV : CR_PEN], (R)0.01);
+  __syncwarp();
+  for (int ch = lane; ch < nch; ch += 32) bk.refresh(ch);
+  __syncwarp();
+  int used = 0;
+  while (used < max_it) {
+    Key best = 0;
+    int ch = 0x7fffffff;
+    for (int c = lane; c < nch; c += 32) {
+      const Key q = bk.cmax[c];
+      if (q > best) {
+        best = q;
+        ch = c;
+      }
+    }
+    warp_first_max(best, ch);
+    if (best == 0) break;
+    const int k = bk.cfirst[ch];
+    const int bb = x.pair(k);
+    const int d0 = x.B0(bb), d1 = x.B1(bb);
+    const int o0 = off[d0], l0 = end[d0] - o0;
+    const int o1 = d1 >= 0 ? off[d1] : 0, l1 = d1 >= 0 ? end[d1] - o1 : 0;
+    // this lane's contact of the two bodies' lists (32 at a time); one that
+    // touches both bodies is visited in d0's list
+    auto entry = [&](int e) {
+      if (e >= l0 + l1) return -1;
+      const int q = e < l0 ? adj[o0 + e] : adj[o1 + e - l0];
+      if (e >= l0) {
+        const int qb = x.pair(q);
+        if (x.B0(qb) == d0 || x.B1(qb) == d0) return -1;
+      }
+      return q;
+    };
+    // its record loads while the resolved contact's change is computed
+    Touched<R> t;
+    const int q = entry(lane);
+    update_load<VEL>(x, t, q, q >= 0, d0, d1);
+    const bool woke = match_awake(x, bb, true, lane == 0);
+    R lin, ang;
+    if constexpr (VEL)
+      velocity_change<R, W, false>(x, v, k, lane < 8, lane, lin, ang, err);
+    else
+      position_change(x, v, bstart, k, lane < 8, lane, lin, ang);
+    for (int base = 0; base < l0 + l1; base += 32) {
+      if (base > 0) {
+        const int r = entry(base + lane);
+        update_load<VEL>(x, t, r, r >= 0, d0, d1);
+      }
+      const R value = update_apply<VEL>(x, t, lin, ang, 32, woke);
+      if (t.valid) bk.key[t.k] = key_of(value, (R)0.01);
+      __syncwarp();
+      if (t.valid) bk.refresh(t.k >> bk.shift);  // lanes of one chunk find the same
+      __syncwarp();
+    }
+    ++used;
+  }
+  return used;
+}
+
+template <class R, class W>
+__global__ void __launch_bounds__(32, 4) k_resolve_big(BatchView<R> v, R dt, int csm) {
+  using Key = decltype(key_of((R)0, (R)0));
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int lane = threadIdx.x;
+  const int w = v.big_list[blockIdx.x];
+  const int n = v.body_count[w];
+  const int bstart = v.body_start[w];
+  const long long cst = v.contact_start[w];
+  int C = v.contact_count[w];
+  if (C > v.contact_cap[w]) C = v.contact_cap[w];  // the world is already flagged ST_CAPACITY
+  if (C <= 0 || dt <= (R)0) {                      // ResolveContacts guards, contact.go:210-212
+    if (lane == 0) {
+      v.pos_iters[w] = 0;
+      v.vel_iters[w] = 0;
+      atomicAdd(&v.counters[3], (unsigned long long)C);
+    }
+    return;
+  }
+  BigKeys<Key> bk;
+  bk.C = C;
+  bk.shift = 4;
+  while (((C - 1) >> bk.shift) >= kBigChunks) ++bk.shift;
+  bk.cmax = reinterpret_cast<Key*>(smem);
+  bk.cfirst = reinterpret_cast<int*>(bk.cmax + kBigChunks);
+  // list starts and ends (first the counts, then the fill cursors)
+  int* off = bk.cfirst + kBigChunks;
+  int* end = off + ((n + 3) & ~3);
+  unsigned char* tile = reinterpret_cast<unsigned char*>(end + ((n + 3) & ~3));
+  RCtx<R, W, false> x;
+  x.nbs = n;
   x.dt = dt;
-  x.bw = reinterpret_cast<W*>(v.big_bw) + bstart;
-  x.br = v.big_br + bstart;
+  x.bw = reinterpret_cast<W*>(v.big_bw) + (long long)bstart * 7;
+  x.br = v.big_br + (long long)bstart * BREC;
   x.aw = v.big_aw + bstart;
-  x.bc = bcs[grp];
-  x.cw = v.work + cst;
-  x.cb = v.work_bodies + cst;
-  x.cst = v.nc_total;
+  x.cr = v.work + cst * CREC;
   x.gmat = v.uniform_material ? nullptr : v.contact + (long long)C_FRIC * v.nc_total + cst;
   x.gst = (long long)(C_REST - C_FRIC) * v.nc_total;
-  x.save = x.delta = x.jw = nullptr;
+  x.delta = x.jw = nullptr;
   x.wi = nullptr;
   x.wst = x.jst = 0;
   x.kw = v.kmat + cst * K_ROW;
-  const bool active = has && C > 0 && dt > (R)0;  // ResolveContacts guards, contact.go:210-212
-  if (has && !active && gl == 0) {
-    v.pos_iters[w] = 0;
-    v.vel_iters[w] = 0;
-    atomicAdd(&v.counters[3], (unsigned long long)C);
+  int* adj;
+  if (C <= csm) {
+    bk.key = reinterpret_cast<Key*>(tile);
+    x.cb = reinterpret_cast<int*>(bk.key + csm);
+    adj = x.cb + csm;
+  } else {
+    bk.key = static_cast<Key*>(v.big_key) + cst;
+    x.cb = v.work_bodies + cst;
+    adj = v.big_adj + 2 * cst;
   }
-  const int na = active ? n : 0;
-  const int Ca = active ? C : 0;
-  for (int i = gl; i < na; i += G) {
-    const long long g = bstart + i;
-    x.P(0, i) = (W)v.body[B_PX * S + g];
-    x.P(1, i) = (W)v.body[B_PY * S + g];
-    x.P(2, i) = (W)v.body[B_PZ * S + g];
-    x.P(3, i) = (W)v.body[B_QW * S + g];
-    x.P(4, i) = (W)v.body[B_QX * S + g];
-    x.P(5, i) = (W)v.body[B_QY * S + g];
-    x.P(6, i) = (W)v.body[B_QZ * S + g];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      x.Bf(r, i) = v.body[(B_VX + r) * S + g];
-      x.Bf(3 + r, i) = v.body[(B_RX + r) * S + g];
-      x.Bf(6 + r, i) = v.body[(B_LX + r) * S + g] * x.dt;  // LastFrameAcceleration * duration
-    }
-#pragma unroll
-    for (int r = 0; r < 9; ++r) x.Bf(9 + r, i) = v.body[(B_IW0 + r) * S + g];
-    x.Bf(18, i) = v.body[B_INVM * S + g];
-    x.Bf(19, i) = v.body[B_MOTION * S + g];
-    x.aw[i] = v.awake[g];
-  }
+  x.all_awake = __all_sync(FULL, load_bodies(x, v, bstart, n, lane, 32));
   __syncwarp();
-  for (int k = gl; k < Ca; k += G) prepare_contact(x, v, cst + k, k);
+  for (int k = lane; k < C; k += 32) prepare_contact(x, v, cst + k, k, k);
+  for (int i = lane; i < n; i += 32) end[i] = 0;
   __syncwarp();
   // contact lists per body: count, exclusive scan, fill
-  int* off = v.big_off + bstart;
-  int* end = v.big_cnt + bstart;  // counts, then the fill cursor, then the list ends
-  int* adj = v.big_adj + 2 * cst;
-  for (int i = gl; i < na; i += G) end[i] = 0;
-  __syncwarp();
-  for (int k = gl; k < Ca; k += G) {
-    const int bb = x.cb[k];
-    atomicAdd(&end[body0_of(bb)], 1);
-    if (body1_of(bb) >= 0) atomicAdd(&end[body1_of(bb)], 1);
+  for (int k = lane; k < C; k += 32) {
+    const int bb = x.pair(k);
+    atomicAdd(&end[x.B0(bb)], 1);
+    if (x.B1(bb) >= 0) atomicAdd(&end[x.B1(bb)], 1);
   }
   __syncwarp();
-  const int nmax = __reduce_max_sync(FULL, (unsigned)na);  // the scan's shuffles need every lane
   int carry = 0;
-  for (int base = 0; base < nmax; base += G) {
-    const int i = base + gl;
-    const int c = i < na ? end[i] : 0;
+  for (int base = 0; base < n; base += 32) {
+    const int i = base + lane;
+    const int c = i < n ? end[i] : 0;
     int s = c;
 #pragma unroll
-    for (int d = 1; d < G; d <<= 1) {
-      const int y = __shfl_up_sync(FULL, s, d, G);
-      if (gl >= d) s += y;
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(FULL, s, d);
+      if (lane >= d) s += y;
     }
-    if (i < na) {
+    if (i < n) {
       off[i] = carry + s - c;
       end[i] = carry + s - c;
     }
-    carry += __shfl_sync(FULL, s, G - 1, G);
+    carry += __shfl_sync(FULL, s, 31);
   }
   __syncwarp();
-  for (int k = gl; k < Ca; k += G) {
-    const int bb = x.cb[k];
-    adj[atomicAdd(&end[body0_of(bb)], 1)] = k;
-    if (body1_of(bb) >= 0) adj[atomicAdd(&end[body1_of(bb)], 1)] = k;
+  for (int k = lane; k < C; k += 32) {
+    const int bb = x.pair(k);
+    adj[atomicAdd(&end[x.B0(bb)], 1)] = k;
+    if (x.B1(bb) >= 0) adj[atomicAdd(&end[x.B1(bb)], 1)] = k;
   }
   __syncwarp();
-  const int max_it = active ? (v.max_iterations >= 0 ? v.max_iterations : C * v.iter_mult) : 0;
-  // ---------------- adjustPositions, contact.go:231-283
-  int pos_used = 0;
-  bool run = active && max_it > 0;
-  while (__any_sync(FULL, run)) {
-    auto best = key_of((R)0, (R)0);
-    int bidx = 0x7fffffff;
-    if (run) lane_first_max<G>(x, W_PEN, C, gl, best, bidx);
-    group_first_max<G>(best, bidx);
-    if (best == 0) run = false;
-    if (run && gl == 0) match_awake(x, x.cb[bidx]);
-    __syncwarp();
-    apply_position_change<R, W, G>(x, v, bstart, bidx, run, gl);
-    __syncwarp();
-    if (run) {
-      const int rb = x.cb[bidx];
-      const int d0 = body0_of(rb), d1 = body1_of(rb);
-      for_pair_contacts<G>(x, adj, off, end, d0, d1, gl, [&](int k) { penetration_update(x, k, d0, d1); });
-    }
-    __syncwarp();
-    if (run && ++pos_used >= max_it) run = false;
-  }
-  for (int k = gl; k < Ca; k += G) friction_prepare(x, k);
+  const int max_it = v.max_iterations >= 0 ? v.max_iterations : C * v.iter_mult;
+  uint32_t err = 0;
+  const int pos_used = big_phase<R, W, false>(x, v, bstart, bk, off, end, adj, max_it, err);
   __syncwarp();
-  // ---------------- adjustVelocities, contact.go:388-445
-  int vel_used = 0;
-  run = active && max_it > 0;
-  while (__any_sync(FULL, run)) {
-    auto best = key_of((R)0, (R)0);
-    int bidx = 0x7fffffff;
-    if (run) lane_first_max<G>(x, W_DDV, C, gl, best, bidx);
-    group_first_max<G>(best, bidx);
-    if (best == 0) run = false;
-    if (run && gl == 0) {
-      match_awake(x, x.cb[bidx]);
-      apply_velocity_change<R, W, false>(x, v, w, bidx);
-    }
-    __syncwarp();
-    if (run) {
-      const int rb = x.cb[bidx];
-      const int d0 = body0_of(rb), d1 = body1_of(rb);
-      for_pair_contacts<G>(x, adj, off, end, d0, d1, gl, [&](int k) { velocity_update(x, k, d0, d1); });
-    }
-    __syncwarp();
-    if (run && ++vel_used >= max_it) run = false;
+  if (v.contact_writeback)
+    for (int k = lane; k < C; k += 32) v.contact[C_PEN * v.nc_total + cst + k] = x.rec(k)[CR_PEN];
+  for (int k = lane; k < C; k += 32) friction_prepare(x, k);
+  __syncwarp();
+  const int vel_used = big_phase<R, W, true>(x, v, bstart, bk, off, end, adj, max_it, err);
+  __syncwarp();
+  if (err) {
+    atomicOr(&v.world_status[w], err);
+    atomicOr(v.status, err);
   }
-  if (active && gl == 0) {
+  if (lane == 0) {
     v.pos_iters[w] = pos_used;
     v.vel_iters[w] = vel_used;
     atomicAdd(&v.counters[1], (unsigned long long)pos_used);
     atomicAdd(&v.counters[2], (unsigned long long)vel_used);
     atomicAdd(&v.counters[3], (unsigned long long)C);
   }
-  if (v.contact_writeback) {
-    const long long CS = v.nc_total;
-    for (int k = gl; k < Ca; k += G) {
-      R* o = v.contact + cst + k;
-      o[C_NX * CS] = x.Cf(W_NX, k);
-      o[C_NY * CS] = x.Cf(W_NY, k);
-      o[C_NZ * CS] = x.Cf(W_NZ, k);
-      o[C_PEN * CS] = x.Cf(W_PEN, k);
-      v.contact_bodies[cst + k] = x.cb[k];
-    }
-  }
-  for (int i = gl; i < na; i += G) {
-    const long long g = bstart + i;
-    v.body[B_PX * S + g] = (R)x.P(0, i);
-    v.body[B_PY * S + g] = (R)x.P(1, i);
-    v.body[B_PZ * S + g] = (R)x.P(2, i);
-    v.body[B_QW * S + g] = (R)x.P(3, i);
-    v.body[B_QX * S + g] = (R)x.P(4, i);
-    v.body[B_QY * S + g] = (R)x.P(5, i);
-    v.body[B_QZ * S + g] = (R)x.P(6, i);
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      v.body[(B_VX + r) * S + g] = x.Bf(r, i);
-      v.body[(B_RX + r) * S + g] = x.Bf(3 + r, i);
-    }
-#pragma unroll
-    for (int r = 0; r < 9; ++r) v.body[(B_IW0 + r) * S + g] = x.Bf(9 + r, i);
-    v.body[B_MOTION * S + g] = x.Bf(19, i);
-    v.awake[g] = x.aw[i];
-  }
+  if (v.contact_writeback)
+    for (int k = lane; k < C; k += 32) write_back_contact(x, v, cst, k);
+  store_bodies(x, v, bstart, n, lane, 32);
 }
 
 }  // namespace cz

@@ -46,7 +46,7 @@ constexpr size_t kOffAwake = align256(kOffBody + sizeof(double) * cz::B_NROWS * 
 constexpr size_t kOffContact = align256(kOffAwake + kStaticMaxBodies);
 constexpr size_t kOffCBodies = align256(kOffContact + sizeof(double) * cz::C_NROWS * kStaticMaxContacts);
 constexpr size_t kOffWork = align256(kOffCBodies + sizeof(int) * kStaticMaxContacts);
-constexpr size_t kOffWBodies = align256(kOffWork + sizeof(double) * cz::W_NROWS * kStaticMaxContacts);
+constexpr size_t kOffWBodies = align256(kOffWork + sizeof(double) * cz::CREC * kStaticMaxContacts);
 constexpr size_t kOffKmat = align256(kOffWBodies + sizeof(int) * kStaticMaxContacts);
 constexpr size_t kOffMeta = align256(kOffKmat + sizeof(double) * cz::K_ROW * kStaticMaxContacts);
 constexpr size_t kScratchBytes = align256(kOffMeta + 256);
@@ -59,7 +59,7 @@ struct Meta {
   unsigned long long counters[8];
   int body_start, body_count, contact_cap, contact_count;
   uint32_t world_status, status;
-  int pos_iters, vel_iters, order, order_rs;
+  int pos_iters, vel_iters, cost, order, order_rs;
   unsigned queue[4];
 };
 static_assert(sizeof(Meta) <= 256, "metadata section");
@@ -216,6 +216,7 @@ cz::HostView static_view(unsigned char* scratch, int n) {
   v.world_status = &m->world_status;
   v.pos_iters = &m->pos_iters;
   v.vel_iters = &m->vel_iters;
+  v.cost = &m->cost;
   v.contact = scratch + kOffContact;
   v.contact_bodies = reinterpret_cast<int*>(scratch + kOffCBodies);
   v.work = scratch + kOffWork;
@@ -258,7 +259,7 @@ int resolve_static(const cz::FormOps& ops, int32_t max_iterations, cz_contact* c
     return cz::set_error(CZ_ERR_CUDA, "cz_resolve_contacts_static: input kernels", e);
   cz::HostView v = static_view<R>(scratch, n);
   v.max_iterations = max_iterations < 0 ? 0 : max_iterations;
-  const size_t smem = ops.rs_smem(kStaticMaxBodies, kStaticContactTile, 32, 0);
+  const size_t smem = ops.rs_smem(kStaticMaxBodies, kStaticContactTile, 32);
   // the kernel's dynamic shared-memory limit may have been set by a batch:
   // raise it when this launch needs more, never lower it
   const void* fn = ops.resolve_kernel(32);
@@ -268,7 +269,7 @@ int resolve_static(const cz::FormOps& ops, int32_t max_iterations, cz_contact* c
   if ((size_t)attr.maxDynamicSharedSizeBytes < smem &&
       (e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
     return cz::set_error(CZ_ERR_CUDA, "cz_resolve_contacts_static: resolver shared-memory limit", e);
-  if ((e = ops.resolve(v, kStaticMaxBodies, kStaticContactTile, 32, 1, smem, duration, s)) != cudaSuccess)
+  if ((e = ops.resolve(v, kStaticMaxBodies, kStaticContactTile, 32, 1, 1, smem, duration, s)) != cudaSuccess)
     return cz::set_error(CZ_ERR_CUDA, "cz_resolve_contacts_static: resolver launch", e);
   k_static_out<R><<<blocks, threads, 0, s>>>(scratch, *bodies, contacts, n, nc);
   if ((e = cudaGetLastError()) != cudaSuccess)

@@ -263,15 +263,16 @@ int cz_mlp_predict(cz_mlp* mlp, const float* features, int64_t n, float* impulse
 typedef struct cz_tuning {
   int32_t narrowphase_threads; /* CTA size of the narrowphase */
   int32_t resolver_contacts;   /* contacts kept in shared memory per world */
-  int32_t resolver_ctas_per_sm;/* resident resolver CTAs per SM (a CTA is 4 independent warps in the
-                                  float32 form with 32 lanes per world, else 1 warp) */
+  int32_t resolver_ctas_per_sm;/* resident resolver CTAs per SM (a CTA is 1 warp, or up to 8 independent ones in
+                                  the float32 form with 32 lanes per world) */
   int32_t integrate_threads;
-  int32_t resolver_lanes;      /* lanes per world in the resolver: 4, 8, 16 or 32 */
+  int32_t resolver_lanes;      /* lanes per world in the resolver: 4, 8, 16 or 32 (its islands of touching
+                                  bodies take 8 lanes each; 4 runs as 8) */
   int32_t warm_start_budget_shift; /* learned warm start: a world is warm-started when its last
                                       solve used at most max_iterations >> shift iterations
                                       (1 to 8; default 2) */
-  int32_t large_world_lanes;   /* lanes per world of more than 64 bodies: 32 (the default) or
-                                  16 (two worlds per warp in lockstep) */
+  int32_t large_world_lanes;   /* worlds of more than 64 bodies: 32 (the default) or 16; one warp per world
+                                  either way */
   int32_t broadphase_min_bodies; /* the narrowphase bins the bodies of worlds of at least this many
                                     bodies in a uniform grid and tests only pairs of neighbouring
                                     cells (default 128; -1 = never).  The grid drops only pairs the
