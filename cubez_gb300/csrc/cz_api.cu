@@ -68,6 +68,16 @@ struct cz_batch {
   // others by k_resolve with a shared-memory slot of rs_nbs bodies
   int rs_nbs = 4, nsmall = 0;
   std::vector<int> big_ids;
+  // Rollouts run the batch in parts, each its own chain of launches (part_rule)
+  struct Part {
+    int w0, w1;           // worlds
+    long long b0, b1;     // padded bodies
+    int nsmall, big0, nbig;
+  };
+  std::vector<Part> parts;
+  std::vector<cudaStream_t> part_streams;  // of parts 1.. (part 0: the batch's)
+  int* d_order_part = nullptr;             // the parts' narrowphase queues, one after the other
+  int* d_order_rs_part = nullptr;          // ... and their resolver queues
   int* d_big = nullptr;
   int* d_units = nullptr;  // cz_collide's unit list
   long long units_cap = 0;
@@ -175,6 +185,9 @@ struct cz_batch {
     v.shape = shape;
     v.offset = has_offset ? d_offset : nullptr;
     v.nb_pad = nb_pad;
+    v.first_body = 0;
+    v.nb_run = nb_pad;
+    v.first_world = 0;
     v.num_worlds = num_worlds;
     v.max_bodies = max_n;
     v.body_start = d_bstart;
@@ -226,6 +239,19 @@ struct cz_batch {
     v.grid_min_bodies = grid_min_bodies;
     return v;
   }
+  // the view of one part of the batch
+  cz::HostView view(const Part& p, int index) const {
+    cz::HostView v = view();
+    v.first_body = p.b0;
+    v.nb_run = p.b1 - p.b0;
+    v.first_world = p.w0;
+    v.num_worlds = p.w1 - p.w0;
+    v.order = d_order_part + p.w0;
+    v.order_rs = d_order_rs_part + p.w0;
+    v.queue = d_queue + 4 * index;
+    v.big_list = d_big + p.big0;
+    return v;
+  }
 };
 
 namespace {
@@ -236,7 +262,8 @@ namespace {
 // rounds of a world, not its iterations: its islands run side by side).  The
 // order of independent worlds does not change any result.
 constexpr int kReorderBuckets = 2048;
-__global__ void __launch_bounds__(1024) k_reorder(const int* __restrict__ cost, int W, int* __restrict__ order,
+__global__ void __launch_bounds__(1024) k_reorder(const int* __restrict__ cost, int w0, int W,
+                                                  int* __restrict__ order,
                                                   const uint8_t* __restrict__ plain_next = nullptr) {
   __shared__ int hist[kReorderBuckets];
   __shared__ int wsum[32];
@@ -250,7 +277,7 @@ __global__ void __launch_bounds__(1024) k_reorder(const int* __restrict__ cost, 
     if (plain_next && !plain_next[w]) return kReorderBuckets - 1;
     return min(cost[w], kReorderBuckets - 1);  // kExhausted: the longest chains, first
   };
-  for (int w = tid; w < W; w += blockDim.x) atomicAdd(&hist[kReorderBuckets - 1 - key_of_world(w)], 1);
+  for (int w = w0 + tid; w < w0 + W; w += blockDim.x) atomicAdd(&hist[kReorderBuckets - 1 - key_of_world(w)], 1);
   __syncthreads();
   // exclusive scan of 2048 buckets, two per thread
   const int a = hist[2 * tid], c = hist[2 * tid + 1];
@@ -278,7 +305,8 @@ __global__ void __launch_bounds__(1024) k_reorder(const int* __restrict__ cost, 
   hist[2 * tid] = excl;
   hist[2 * tid + 1] = excl + a;
   __syncthreads();
-  for (int w = tid; w < W; w += blockDim.x) order[atomicAdd(&hist[kReorderBuckets - 1 - key_of_world(w)], 1)] = w;
+  for (int w = w0 + tid; w < w0 + W; w += blockDim.x)
+    order[atomicAdd(&hist[kReorderBuckets - 1 - key_of_world(w)], 1)] = w;
 }
 
 void free_batch(cz_batch* b) {
@@ -295,7 +323,7 @@ void free_batch(cz_batch* b) {
       b->ws_world,  b->mlp_mem,     b->hv_features, b->hv_labels, b->hv_count,   b->snap_body,   b->snap_u8,
       b->body,      b->awake,       b->can_sleep, b->shape,       b->d_bstart,   b->d_bcount,    b->d_ccap,
       b->d_ccount,  b->d_cstart,    b->d_wstatus, b->d_piters,    b->d_viters,    b->d_cost,   b->contact,     b->cbodies,
-      b->work,      b->wbodies,     b->kmat,      b->d_order,    b->d_order_rs,  b->d_queue,
+      b->work,      b->wbodies,     b->kmat,      b->d_order,    b->d_order_rs,  b->d_order_part, b->d_order_rs_part, b->d_queue,
       b->d_status,  b->d_counters,  b->d_h2p,     b->d_stage,     b->d_stage_u8, b->d_stage_i32, b->d_cstage,
       b->d_cstage_b, b->d_pow};
   for (void* p : dev)
@@ -304,6 +332,7 @@ void free_batch(cz_batch* b) {
                   b->h_cstage,     b->h_cstage_b, b->h_pow,      b->h_status};
   for (void* p : host)
     if (p) cudaFreeHost(p);
+  for (cudaStream_t s : b->part_streams) cudaStreamDestroy(s);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }
@@ -352,51 +381,82 @@ bool uses_frame(const cz_batch* b) {
   return b->fused && b->fr_smem > 0 && b->big_ids.empty() && b->rs_lanes == 32 && b->mode == 0 && b->nsmall > 0;
 }
 
-int launches_per_step(const cz_batch* b) {
-  if (uses_frame(b)) return 1 + (b->nsmall > 1 ? 1 : 0);
-  return 2 + (b->nsmall > 0 ? 1 + (b->nsmall > 32 / b->run_lanes() ? 1 : 0) + (b->mode != 0 ? 1 : 0) : 0) +
-         (b->big_ids.empty() ? 0 : 1);
+// Frames in one graph where the batch runs in parts (longer rollouts launch it
+// again: the parts meet that often, and the graph has at most 4096 launches).
+constexpr int kPartFrames = 32;
+// The re-queue by cost matters where a launch's worlds do not all start at once.
+constexpr int kReorderWorlds = 256;
+
+// One frame's launches over a view of the batch (the whole of it, or a part),
+// on a stream.
+struct Chain {
+  cz::HostView v;
+  int nsmall, nbig;
+  bool requeue;  // sort the worlds by cost for the next frame
+  cudaStream_t s;
+};
+bool requeues(const cz_batch* b, int nsmall) { return nsmall > 32 / b->run_lanes(); }
+Chain whole(cz_batch* b) {
+  return {b->view(), b->nsmall, (int)b->big_ids.size(), requeues(b, b->nsmall), b->stream};
 }
 
-int launch_integrate(cz_batch* b, double dt) {
-  CZ_CUDA(b->ops->integrate(b->view(), dt, std::pow(0.5, dt), b->int_threads, b->stream));
+// CTAs for a view's worlds, of a kernel that takes `per_cta` worlds at a time
+// and fills the GPU with `most`.
+int chain_grid(int worlds, int per_cta, int most) {
+  return std::max(1, std::min((worlds + per_cta - 1) / per_cta, most));
+}
+
+int launches_of(const cz_batch* b, int nsmall, int nbig, bool requeue) {
+  return 2 + (nsmall > 0 ? 1 + (requeue ? 1 : 0) + (b->mode != 0 ? 1 : 0) : 0) + (nbig > 0 ? 1 : 0);
+}
+int launches_per_step(const cz_batch* b, bool in_parts) {
+  if (uses_frame(b)) return 1 + (b->nsmall > 1 ? 1 : 0);
+  if (!in_parts || b->parts.size() == 1)
+    return launches_of(b, b->nsmall, (int)b->big_ids.size(), requeues(b, b->nsmall));
+  int n = 0;
+  for (const auto& p : b->parts) n += launches_of(b, p.nsmall, p.nbig, p.nsmall > kReorderWorlds);
+  return n;
+}
+
+int launch_integrate(cz_batch* b, const Chain& c, double dt) {
+  CZ_CUDA(b->ops->integrate(c.v, dt, std::pow(0.5, dt), b->int_threads, c.s));
   g_launches++;
   return CZ_OK;
 }
-int launch_narrowphase(cz_batch* b) {
-  CZ_CUDA(cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned), b->stream));
-  CZ_CUDA(b->ops->narrowphase(b->view(), b->nbs, b->np_threads, b->np_grid, b->np_smem, b->stream));
+// `reset`: zero the queue first (in a frame, the integrate launch has)
+int launch_narrowphase(cz_batch* b, const Chain& c, bool reset) {
+  if (reset) CZ_CUDA(cudaMemsetAsync(c.v.queue, 0, sizeof(unsigned), c.s));
+  CZ_CUDA(b->ops->narrowphase(c.v, b->nbs, b->np_threads, chain_grid(c.v.num_worlds, 1, b->np_grid), b->np_smem, c.s));
   g_launches++;
   return CZ_OK;
 }
 // The resolver launches of one frame: k_resolve over the worlds that fit its
 // slot (then the re-queue of those worlds by cost), k_resolve_big over the
 // others.
-int launch_resolve_with(cz_batch* b, double dt, const cz::HostView& v) {
-  if (b->nsmall > 0) {
-    if (v.mode != 0) {  // features (and, warm-starting, predictions) ahead of the resolver
-      CZ_CUDA(cudaMemsetAsync(b->d_queue + 2, 0, sizeof(unsigned), b->stream));
-      CZ_CUDA(b->ops->warm_features(v, b->rs_nbs, b->wf_grid, dt, b->stream));
+int launch_resolve(cz_batch* b, const Chain& c, double dt, bool reset) {
+  if (c.nsmall > 0) {
+    const int worlds_per_warp = 32 / b->run_lanes();
+    if (reset) CZ_CUDA(cudaMemsetAsync(c.v.queue + 1, 0, 2 * sizeof(unsigned), c.s));
+    if (c.v.mode != 0) {  // features (and, warm-starting, predictions) ahead of the resolver
+      CZ_CUDA(b->ops->warm_features(c.v, b->rs_nbs, chain_grid(c.v.num_worlds, 1, b->wf_grid), dt, c.s));
       g_launches++;
     }
-    CZ_CUDA(cudaMemsetAsync(b->d_queue + 1, 0, sizeof(unsigned), b->stream));
-    CZ_CUDA(b->ops->resolve(v, b->rs_nbs, b->rs_cs, b->run_lanes(), b->rs_grid, b->rs_wpc, b->rs_smem, dt, b->stream));
+    CZ_CUDA(b->ops->resolve(c.v, b->rs_nbs, b->rs_cs, b->run_lanes(),
+                            chain_grid(c.v.num_worlds, worlds_per_warp * b->rs_wpc, b->rs_grid), b->rs_wpc, b->rs_smem,
+                            dt, c.s));
     g_launches++;
-    if (b->nsmall > 32 / b->run_lanes()) {
-      k_reorder<<<1, 1024, 0, b->stream>>>(b->d_cost, b->num_worlds, b->d_order_rs,
-                                           v.mode == 2 ? v.ws_world : nullptr);
+    if (c.requeue) {
+      k_reorder<<<1, 1024, 0, c.s>>>(b->d_cost, c.v.first_world, c.v.num_worlds, const_cast<int*>(c.v.order_rs),
+                                     c.v.mode == 2 ? c.v.ws_world : nullptr);
       CZ_CUDA(cudaGetLastError());
       g_launches++;
     }
   }
-  if (!b->big_ids.empty()) {
-    CZ_CUDA(b->ops->resolve_big(v, (int)b->big_ids.size(), b->big_csm, b->big_smem, dt, b->stream));
+  if (c.nbig > 0) {
+    CZ_CUDA(b->ops->resolve_big(c.v, c.nbig, b->big_csm, b->big_smem, dt, c.s));
     g_launches++;
   }
   return CZ_OK;
-}
-int launch_resolve(cz_batch* b, double dt, const cz::HostView* override_view = nullptr) {
-  return launch_resolve_with(b, dt, override_view ? *override_view : b->view());
 }
 // The fused frame: integrate, narrowphase and resolve of every world in one
 // launch (then the re-queue by cost).
@@ -405,11 +465,25 @@ int launch_frame(cz_batch* b, double dt) {
   CZ_CUDA(b->ops->frame(b->view(), b->rs_nbs, b->rs_cs, b->fr_grid, b->fr_smem, dt, std::pow(0.5, dt), b->stream));
   g_launches++;
   if (b->nsmall > 1) {
-    k_reorder<<<1, 1024, 0, b->stream>>>(b->d_cost, b->num_worlds, b->d_order_rs);
+    k_reorder<<<1, 1024, 0, b->stream>>>(b->d_cost, 0, b->num_worlds, b->d_order_rs);
     CZ_CUDA(cudaGetLastError());
     g_launches++;
   }
   return CZ_OK;
+}
+
+// How many parts a rollout runs the batch in: parallel branches of its graph,
+// each a chain of frames over its own worlds.  Worlds are independent, but a
+// launch over all of them ends with its longest world, and a frame's next
+// launch waited for that: half of a resolver launch was its tail (8192 worlds
+// of 32 bodies, float32: 0.62 of 1.2 ms with the SMs busy).  With parts, one
+// part's tail runs beside the others' work.  At least 64 worlds each; at most
+// 32 parts in float64, where 4096 worlds of 8 to 64 bodies x 30 frames took
+// 221, 189, 179 and 165 ms with 1, 4, 8 and 32 parts, and 8 in float32, whose
+// launches are short (16384 x 32 bodies x 60 frames: 142, 119, 122 and 132 ms;
+// 8192 worlds with the warm start x 30: 48.3, 40.2, 39.3 and 40.7 ms).
+int part_rule(int form, int num_worlds) {
+  return std::max(1, std::min(num_worlds / 64, form == CZ_FORM_FP64 ? 32 : 8));
 }
 
 // The captured graphs hold the kernels' parameters (the batch view); drop them
@@ -586,7 +660,23 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
   // world queue: decreasing body count (pair work grows as n^2)
   std::vector<int> order(b->num_worlds);
   std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return b->counts[a] > b->counts[c]; });
+  const auto larger = [&](int a, int c) { return b->counts[a] > b->counts[c]; };
+  std::vector<int> order_part(order);
+  std::stable_sort(order.begin(), order.end(), larger);
+  // parts: consecutive worlds, about as many in each
+  const int nparts = part_rule(b->form, b->num_worlds);
+  for (int p = 0; p < nparts; ++p) {
+    cz_batch::Part part{};
+    part.w0 = (int)((long long)b->num_worlds * p / nparts);
+    part.w1 = (int)((long long)b->num_worlds * (p + 1) / nparts);
+    part.b0 = b->bstart[part.w0];
+    part.b1 = part.w1 < b->num_worlds ? b->bstart[part.w1] : b->nb_pad;
+    for (int w = part.w0; w < part.w1; ++w) part.nbig += b->counts[w] > kBigWorld;
+    part.nsmall = part.w1 - part.w0 - part.nbig;
+    part.big0 = (int)(std::lower_bound(b->big_ids.begin(), b->big_ids.end(), part.w0) - b->big_ids.begin());
+    std::stable_sort(order_part.begin() + part.w0, order_part.begin() + part.w1, larger);
+    b->parts.push_back(part);
+  }
 
   const size_t R = b->ops->real_size;
   const long long P = b->nb_pad, C = b->nc_total, W = b->num_worlds;
@@ -595,6 +685,12 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
     return true;
   };
   bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess;
+  for (int p = 1; ok && p < nparts; ++p) {
+    cudaStream_t s = nullptr;
+    ok = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+    if (ok) b->part_streams.push_back(s);
+  }
+  ok = ok && dmalloc((void**)&b->d_order_part, sizeof(int) * W) && dmalloc((void**)&b->d_order_rs_part, sizeof(int) * W);
   ok = ok && dmalloc(&b->body, R * cz::B_NROWS * P);
   ok = ok && dmalloc((void**)&b->awake, P) && dmalloc((void**)&b->can_sleep, P) &&
        dmalloc((void**)&b->shape, sizeof(int) * P);
@@ -607,7 +703,7 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
   ok = ok && dmalloc(&b->contact, R * cz::C_NROWS * C) && dmalloc((void**)&b->cbodies, sizeof(int) * C);
   ok = ok && dmalloc(&b->work, R * cz::CREC * C) && dmalloc((void**)&b->wbodies, sizeof(int) * C);
   ok = ok && dmalloc(&b->kmat, R * cz::K_ROW * C);
-  ok = ok && dmalloc((void**)&b->d_queue, 4 * sizeof(unsigned)) && dmalloc((void**)&b->d_status, sizeof(uint32_t)) &&
+  ok = ok && dmalloc((void**)&b->d_queue, 4 * sizeof(unsigned) * nparts) && dmalloc((void**)&b->d_status, sizeof(uint32_t)) &&
        dmalloc((void**)&b->d_counters, 8 * sizeof(unsigned long long));
   ok = ok && dmalloc((void**)&b->d_h2p, sizeof(int) * std::max<long long>(nb, 1));
   ok = ok && dmalloc((void**)&b->d_stage, sizeof(double) * cz::SG_NDOUBLES * std::max<long long>(nb, 1)) &&
@@ -643,7 +739,7 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
       cudaMemsetAsync(b->d_piters, 0, sizeof(int) * W, s) != cudaSuccess ||
       cudaMemsetAsync(b->d_viters, 0, sizeof(int) * W, s) != cudaSuccess ||
       cudaMemsetAsync(b->d_cost, 0, sizeof(int) * W, s) != cudaSuccess ||
-      cudaMemsetAsync(b->d_queue, 0, 4 * sizeof(unsigned), s) != cudaSuccess ||
+      cudaMemsetAsync(b->d_queue, 0, 4 * sizeof(unsigned) * nparts, s) != cudaSuccess ||
       cudaMemsetAsync(b->d_status, 0, sizeof(uint32_t), s) != cudaSuccess ||
       cudaMemsetAsync(b->d_counters, 0, 8 * sizeof(unsigned long long), s) != cudaSuccess ||
       cudaMemsetAsync(b->cbodies, 0xFF, sizeof(int) * C, s) != cudaSuccess ||
@@ -654,6 +750,9 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
           cudaSuccess ||
       cudaMemcpyAsync(b->d_order, order.data(), sizeof(int) * W, cudaMemcpyHostToDevice, s) != cudaSuccess ||
       cudaMemcpyAsync(b->d_order_rs, order.data(), sizeof(int) * W, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+      cudaMemcpyAsync(b->d_order_part, order_part.data(), sizeof(int) * W, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+      cudaMemcpyAsync(b->d_order_rs_part, order_part.data(), sizeof(int) * W, cudaMemcpyHostToDevice, s) !=
+          cudaSuccess ||
       (!b->big_ids.empty() && cudaMemcpyAsync(b->d_big, b->big_ids.data(), sizeof(int) * b->big_ids.size(),
                                               cudaMemcpyHostToDevice, s) != cudaSuccess) ||
       (nb > 0 &&
@@ -856,7 +955,7 @@ int cz_integrate(cz_batch* b, double dt) {
   int st = ensure_pows(b, dt);
   if (st) return st;
   if ((st = reset_status(b))) return st;
-  if ((st = launch_integrate(b, dt))) return st;
+  if ((st = launch_integrate(b, whole(b), dt))) return st;
   return finish(b);
 }
 
@@ -865,7 +964,7 @@ int cz_narrowphase(cz_batch* b) {
   CZ_CUDA(cudaSetDevice(b->device));
   int st = reset_status(b);
   if (st) return st;
-  if ((st = launch_narrowphase(b))) return st;
+  if ((st = launch_narrowphase(b, whole(b), true))) return st;
   return finish(b);
 }
 
@@ -874,8 +973,52 @@ int cz_resolve(cz_batch* b, double dt) {
   CZ_CUDA(cudaSetDevice(b->device));
   int st = reset_status(b);
   if (st) return st;
-  if ((st = launch_resolve(b, dt))) return st;
+  if ((st = launch_resolve(b, whole(b), dt, true))) return st;
   return finish(b);
+}
+
+// One frame of a chain.
+static int launch_step(cz_batch* b, const Chain& c, double dt) {
+  int st = launch_integrate(b, c, dt);
+  if (!st) st = launch_narrowphase(b, c, false);
+  if (!st) st = launch_resolve(b, c, dt, false);
+  return st;
+}
+
+// The batch's parts as parallel branches of the graph being captured on its
+// stream, each its own chain of frames.
+static int capture_parts(cz_batch* b, int nsteps, double dt) {
+  cudaEvent_t fork = nullptr;
+  std::vector<cudaEvent_t> joins;
+  auto run = [&]() -> int {
+    CZ_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    CZ_CUDA(cudaEventRecord(fork, b->stream));
+    for (size_t p = 0; p < b->parts.size(); ++p) {
+      const cz_batch::Part& part = b->parts[p];
+      const Chain c{b->view(part, (int)p), part.nsmall, part.nbig, part.nsmall > kReorderWorlds,
+                    p == 0 ? b->stream : b->part_streams[p - 1]};
+      if (p > 0) CZ_CUDA(cudaStreamWaitEvent(c.s, fork, 0));
+      for (int s = 0; s < nsteps; ++s)
+        if (int st = launch_step(b, c, dt)) return st;
+      if (p > 0) {
+        cudaEvent_t e = nullptr;
+        CZ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        joins.push_back(e);
+        CZ_CUDA(cudaEventRecord(e, c.s));
+      }
+    }
+    for (cudaEvent_t e : joins) CZ_CUDA(cudaStreamWaitEvent(b->stream, e, 0));
+    return CZ_OK;
+  };
+  const int st = run();
+  if (fork) cudaEventDestroy(fork);
+  for (cudaEvent_t e : joins) cudaEventDestroy(e);
+  return st;
+}
+
+// Frames the next graph of a rollout with `left` frames to go holds.
+static int graph_frames(const cz_batch* b, int left) {
+  return !uses_frame(b) && b->parts.size() > 1 ? std::min(left, kPartFrames) : left;
 }
 
 // Capture (once per (nsteps, dt)) the plain rollout graph.
@@ -890,14 +1033,13 @@ static int get_graph(cz_batch* b, int nsteps, double dt, cudaGraphExec_t* out) {
   const long long before = g_launches.load();
   int cst = CZ_OK;
   const bool fused = uses_frame(b);
-  for (int s = 0; s < nsteps && cst == CZ_OK; ++s) {
-    if (fused) {
-      cst = launch_frame(b, dt);
-      continue;
-    }
-    cst = launch_integrate(b, dt);
-    if (!cst) cst = launch_narrowphase(b);
-    if (!cst) cst = launch_resolve(b, dt);
+  if (fused) {
+    for (int s = 0; s < nsteps && cst == CZ_OK; ++s) cst = launch_frame(b, dt);
+  } else if (b->parts.size() > 1) {
+    cst = capture_parts(b, nsteps, dt);
+  } else {
+    const Chain c = whole(b);
+    for (int s = 0; s < nsteps && cst == CZ_OK; ++s) cst = launch_step(b, c, dt);
   }
   g_launches.store(before);  // captured launches are counted when the graph runs
   cudaGraph_t graph = nullptr;
@@ -935,6 +1077,7 @@ static int get_timed(cz_batch* b, int nsteps, double dt, cz_batch::Timed** out) 
   };
   int cst = record(0);
   const bool fused = uses_frame(b);
+  const Chain c = whole(b);
   for (int s = 0; s < nsteps && cst == CZ_OK; ++s) {
     if (fused) {  // one launch: its time is reported as the resolve phase
       cst = record(3 * s + 1);
@@ -943,11 +1086,11 @@ static int get_timed(cz_batch* b, int nsteps, double dt, cz_batch::Timed** out) 
       if (!cst) cst = record(3 * s + 3);
       continue;
     }
-    cst = launch_integrate(b, dt);
+    cst = launch_integrate(b, c, dt);
     if (!cst) cst = record(3 * s + 1);
-    if (!cst) cst = launch_narrowphase(b);
+    if (!cst) cst = launch_narrowphase(b, c, false);
     if (!cst) cst = record(3 * s + 2);
-    if (!cst) cst = launch_resolve(b, dt);
+    if (!cst) cst = launch_resolve(b, c, dt, false);
     if (!cst) cst = record(3 * s + 3);
   }
   g_launches.store(before);
@@ -975,10 +1118,14 @@ int cz_step(cz_batch* b, int32_t nsteps, double dt) {
   int st = ensure_pows(b, dt);
   if (st) return st;
   if ((st = reset_status(b))) return st;
-  cudaGraphExec_t exec = nullptr;
-  if ((st = get_graph(b, nsteps, dt, &exec))) return st;
-  CZ_CUDA(cudaGraphLaunch(exec, b->stream));
-  g_launches += (long long)launches_per_step(b) * nsteps;
+  for (int left = nsteps; left > 0;) {
+    const int n = graph_frames(b, left);
+    cudaGraphExec_t exec = nullptr;
+    if ((st = get_graph(b, n, dt, &exec))) return st;
+    CZ_CUDA(cudaGraphLaunch(exec, b->stream));
+    left -= n;
+  }
+  g_launches += (long long)launches_per_step(b, true) * nsteps;
   return finish(b);
 }
 
@@ -988,7 +1135,9 @@ int cz_prepare_rollout(cz_batch* b, int32_t nsteps, double dt) {
   int st = ensure_pows(b, dt);
   if (st) return st;
   cudaGraphExec_t exec = nullptr;
-  if ((st = get_graph(b, nsteps, dt, &exec))) return st;
+  if ((st = get_graph(b, graph_frames(b, nsteps), dt, &exec))) return st;
+  const int rest = nsteps % graph_frames(b, nsteps);
+  if (rest > 0 && (st = get_graph(b, rest, dt, &exec))) return st;
   cz_batch::Timed* t = nullptr;
   return get_timed(b, nsteps, dt, &t);
 }
@@ -1078,11 +1227,11 @@ int cz_resolve_contacts(cz_batch* b, int32_t max_iterations, cz_contact* contact
   g_launches++;
   CZ_CUDA(cudaMemcpyAsync(b->d_ccount, &ncontacts, sizeof(int), cudaMemcpyHostToDevice, b->stream));
   if ((st = reset_status(b))) return st;
-  cz::HostView v = b->view();
-  v.max_iterations = std::max(max_iterations, 0);
-  v.contact_writeback = 1;
-  v.uniform_material = 0;
-  if ((st = launch_resolve(b, duration, &v))) return st;
+  Chain c = whole(b);
+  c.v.max_iterations = std::max(max_iterations, 0);
+  c.v.contact_writeback = 1;
+  c.v.uniform_material = 0;
+  if ((st = launch_resolve(b, c, duration, true))) return st;
   st = finish(b);
   if (st != CZ_OK && st != CZ_ERR_FRICTIONLESS) return st;
   const int st2 = cz_download_bodies(b, bodies);
@@ -1139,7 +1288,7 @@ int cz_step_timed(cz_batch* b, int32_t nsteps, double dt, double* total_ms, doub
   cz_batch::Timed* t = nullptr;
   if ((st = get_timed(b, nsteps, dt, &t))) return st;
   CZ_CUDA(cudaGraphLaunch(t->exec, b->stream));
-  g_launches += (long long)launches_per_step(b) * nsteps;
+  g_launches += (long long)launches_per_step(b, false) * nsteps;
   st = finish(b);
   double ph[3] = {0, 0, 0};
   const bool fused = uses_frame(b);
@@ -1247,15 +1396,10 @@ int cz_harvest(cz_batch* b, int32_t nsteps, double dt, int32_t every, float* fea
   // the plain resolver, writing features and applied impulses every `every` frames
   const int saved_mode = b->mode;
   for (int s = 0; s < nsteps && st == CZ_OK; ++s) {
-    st = launch_integrate(b, dt);
-    if (!st) st = launch_narrowphase(b);
-    if (!st) {
-      const bool h = (s % every) == every - 1;
-      cz::HostView v = b->view();
-      v.mode = h ? 1 : 0;
-      v.hv_cap = b->hv_cap;
-      st = launch_resolve_with(b, dt, v);
-    }
+    Chain c = whole(b);
+    c.v.mode = (s % every) == every - 1 ? 1 : 0;
+    c.v.hv_cap = b->hv_cap;
+    st = launch_step(b, c, dt);
   }
   b->mode = saved_mode;
   if (st) return st;

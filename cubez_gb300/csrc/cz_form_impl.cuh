@@ -1,6 +1,8 @@
 // Kernel instantiation and launch wrappers for one form; included by
 // cz_fp64.cu / cz_fp32.cu with CZ_R, CZ_W and CZ_FORM_NAME defined.
 #pragma once
+#include <algorithm>
+
 #include "cz_forms.h"
 #include "cz_kernels.cuh"
 
@@ -18,6 +20,9 @@ static BatchView<R> view_of(const HostView& h) {
   v.shape = h.shape;
   v.offset = static_cast<const R*>(h.offset);
   v.nb_pad = h.nb_pad;
+  v.first_body = h.first_body;
+  v.nb_run = h.nb_run;
+  v.first_world = h.first_world;
   v.num_worlds = h.num_worlds;
   v.max_bodies = h.max_bodies;
   v.body_start = h.body_start;
@@ -235,8 +240,8 @@ static cudaError_t prepare(size_t np, size_t rs, int lanes) {
 }
 
 static cudaError_t integrate(const HostView& h, double dt, double bias, int threads, cudaStream_t s) {
-  const long long nb = h.nb_pad;
-  const int grid = (int)((nb + threads - 1) / threads);
+  const long long nb = h.nb_run;
+  const int grid = (int)std::max<long long>(1, (nb + threads - 1) / threads);
   k_integrate<R, W><<<grid, threads, 0, s>>>(view_of(h), (R)dt, (R)bias);
   return cudaGetLastError();
 }

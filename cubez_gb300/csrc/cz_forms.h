@@ -20,6 +20,8 @@ struct HostView {
   int32_t* shape;
   const void* offset;  // [12][nb_pad] collider Offset rows, or null (identity)
   long long nb_pad;
+  long long first_body, nb_run;
+  int first_world;
   int num_worlds;
   int max_bodies;
   const int* body_start;

@@ -87,8 +87,10 @@ __device__ __forceinline__ void integrate_body(const BatchView<R>& v, long long 
 template <class R, class W>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 0) k_integrate(BatchView<R> v, R dt, R sleep_bias) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= v.nb_pad) return;
-  integrate_body<R, W>(v, i, dt, sleep_bias);
+  // the work queues of the frame's launches that follow on the stream
+  if (i < 4) v.queue[i] = 0;
+  if (i >= v.nb_run) return;
+  integrate_body<R, W>(v, v.first_body + i, dt, sleep_bias);
 }
 
 // ============================================================== narrowphase

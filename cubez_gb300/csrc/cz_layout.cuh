@@ -102,6 +102,10 @@ template <class R> struct BatchView {
   int32_t* shape;       // [nb_pad] 0 sphere, 1 cube, -1 padding
   const R* offset;      // [12][nb_pad] collider Offset (column-major 3x4), null = identity for every body
   long long nb_pad;
+  // the worlds a launch covers: num_worlds of them from first_world, whose
+  // bodies are the nb_run padded rows from first_body
+  long long first_body, nb_run;
+  int first_world;
   int num_worlds;
   int max_bodies;       // largest world
   const int* body_start;
@@ -122,7 +126,7 @@ template <class R> struct BatchView {
   long long nc_total;
   const int* order;     // narrowphase queue: worlds in decreasing body count
   const int* order_rs;  // resolver queue: worlds in decreasing iterations of the previous frame
-  unsigned* queue;      // [0] narrowphase, [1] resolver, [2..3] spare
+  unsigned* queue;      // [0] narrowphase, [1] resolver, [2] features, [3] spare (k_integrate zeroes them)
   uint32_t* status;     // batch status word
   unsigned long long* counters;  // [0] contacts generated, [1] adjustPositions iterations,
                                  // [2] adjustVelocities iterations, [3] contacts resolved,

@@ -1792,7 +1792,7 @@ __global__ void __launch_bounds__(32 * kWfWarps) k_warm_features(BatchView<R> v,
     if (lane == 0) q = atomicAdd(&v.queue[2], 1u);
     q = __shfl_sync(FULL, q, 0);
     if (q >= (unsigned)v.num_worlds) break;
-    const int w = (int)q;
+    const int w = v.first_world + (int)q;
     const int n = v.body_count[w];
     int C = v.contact_count[w];
     const int cap = v.contact_cap[w];

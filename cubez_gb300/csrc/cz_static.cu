@@ -206,6 +206,9 @@ cz::HostView static_view(unsigned char* scratch, int n) {
   v.can_sleep = nullptr;
   v.shape = nullptr;
   v.nb_pad = kStaticMaxBodies;
+  v.first_body = 0;
+  v.nb_run = kStaticMaxBodies;
+  v.first_world = 0;
   v.num_worlds = 1;
   v.max_bodies = n;
   v.body_start = &m->body_start;
