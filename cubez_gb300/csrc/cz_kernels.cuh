@@ -85,7 +85,7 @@ __device__ __forceinline__ void integrate_body(const BatchView<R>& v, long long 
 }
 
 template <class R, class W>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 0) k_integrate(BatchView<R> v, R dt, R sleep_bias) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_integrate(BatchView<R> v, R dt, R sleep_bias) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   // the work queues of the frame's launches that follow on the stream
   if (i < 4) v.queue[i] = 0;
@@ -114,9 +114,21 @@ template <class R> struct NPTile {
     for (int r = 0; r < 12; ++r) t.m[r] = T[r * nbs + i];
     return t;
   }
+  // column c of body i's transform (an axis, or with c = 3 the centre), for any c
+  __device__ __forceinline__ v3<R> axis(int i, int c) const {
+    const R* t = T + (size_t)(3 * c) * nbs + i;
+    return V<R>(t[0], t[nbs], t[2 * nbs]);
+  }
   __device__ __forceinline__ v3<R> half(int i) const { return V<R>(s(7, i), s(8, i), s(9, i)); }
   __device__ __forceinline__ R radius(int i) const { return s(10, i); }
 };
+
+// Integer keys in the order of non-negative values (both zeros alike).
+__device__ __forceinline__ unsigned sort_key(float v) { return v == 0.f ? 0u : __float_as_uint(v); }
+__device__ __forceinline__ unsigned long long sort_key(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return (b << 1) == 0ull ? 0ull : b;
+}
 
 template <class R>
 __device__ __forceinline__ R transform_to_axis(const xf<R>& t, const v3<R>& h, const v3<R>& axis) {
@@ -125,40 +137,94 @@ __device__ __forceinline__ R transform_to_axis(const xf<R>& t, const v3<R>& h, c
          h.z * fabs_<R>(dot(axis, t.axis(2)));
 }
 
-// tryAxis, colliders.go:458-477 (false = separating axis found)
+// The outcome of CollisionCube.CheckAgainstCube's axes for a pair of boxes
+// (colliders.go:575-627), in both orders of the pair: the axis of smallest
+// penetration (0-2 and 3-5 the boxes' own, 6 + 3i + j the edge pairs; 255:
+// none) and the smallest of the first six alone.
+template <class R> struct SatResult {
+  R pen;
+  int code;  // best | best_single << 8 of (one, two), and << 16, << 24 of (two, one); kSatApart: a separating axis
+};
+constexpr int kSatApart = -1;
+
+// tryAxis (colliders.go:458-477) for the fifteen axes of a pair of boxes, an
+// axis per lane of a group of 16 (l = 0..15), the smallest penetration (the
+// first of equal ones, as the reference's loop keeps) by shuffles.  Every lane
+// of the warp calls it.  The axes of (two, one) are the same vectors or their
+// negatives, and every term of a penetration is the same or its magnitude is,
+// so one set of fifteen serves both orders; only the order in which equal
+// penetrations are met differs.
+// On one lane the fifteen axes are one chain (about 60 us of float64 latency),
+// and a warp runs it for the twenty or so box pairs of a small world, most of
+// them in both orders: 15 axes' instructions for 20 lanes, against half of 10.
 template <class R>
-__device__ __forceinline__ bool try_axis(const xf<R>& t1, const v3<R>& h1, const xf<R>& t2, const v3<R>& h2,
-                                         v3<R> axis, const v3<R>& tc, int index, R& smallest, int& best) {
-  if (sqmag(axis) < Lim<R>::eps()) return true;
-  normalize(axis);
-  R one = transform_to_axis(t1, h1, axis);
-  R two = transform_to_axis(t2, h2, axis);
-  R dist = fabs_<R>(dot(tc, axis));
-  R p = one + two - dist;  // penetrationOnAxis, colliders.go:445-456
-  if (p < (R)0) return false;
-  if (p < smallest) {
-    smallest = p;
-    best = index;
+__device__ __forceinline__ SatResult<R> sat_axes(const NPTile<R>& tl, int i1, int i2, int l) {
+  using Key = decltype(sort_key((R)0));
+  const unsigned gmask = 0xFFFFu << (threadIdx.x & 16);
+  const int ei = (l - 6) / 3, ej = (l - 6) % 3;  // edge axes
+  v3<R> axis = tl.axis(l < 3 || l > 5 ? i1 : i2, l < 3 ? l : (l < 6 ? l - 3 : (l < 15 ? ei : 0)));
+  if (l > 5) axis = cross(axis, tl.axis(i2, l < 15 ? ej : 0));
+  const xf<R> t1 = tl.xform(i1), t2 = tl.xform(i2);
+  const v3<R> h1 = tl.half(i1), h2 = tl.half(i2);
+  v3<R> tc = t2.axis(3);
+  sub(tc, t1.axis(3));
+  R p = (R)0;
+  bool tried = l < 15 && !(sqmag(axis) < Lim<R>::eps());
+  if (tried) {
+    normalize(axis);
+    const R one = transform_to_axis(t1, h1, axis);
+    const R two = transform_to_axis(t2, h2, axis);
+    const R dist = fabs_<R>(dot(tc, axis));
+    p = one + two - dist;  // penetrationOnAxis, colliders.go:445-456
   }
-  return true;
+  SatResult<R> r;
+  r.pen = (R)0;
+  r.code = kSatApart;
+  const bool apart = (__ballot_sync(FULL, tried && p < (R)0) & gmask) != 0;
+  tried = tried && p < Lim<R>::max_value();  // a candidate (NaN never is)
+  // integer keys of the (here non-negative) penetrations
+  const Key none = ~(Key)0;
+  const Key key = tried && !(p < (R)0) ? sort_key(p) : none;
+  Key all = key, own = l < 6 ? key : none;
+#pragma unroll
+  for (int d = 8; d > 0; d >>= 1) {
+    const Key a = __shfl_xor_sync(FULL, all, d, 16), o = __shfl_xor_sync(FULL, own, d, 16);
+    all = a < all ? a : all;
+    own = o < own ? o : own;
+  }
+  // the first axis with the smallest value, in the pair's order and in the other's
+  const int back = l < 3 ? l + 3 : (l < 6 ? l - 3 : 6 + 3 * ej + ei);
+  const unsigned at_all = __ballot_sync(FULL, key == all && all != none) & gmask;
+  const unsigned at_own = __ballot_sync(FULL, l < 6 && key == own && own != none) & gmask;
+  int b_all = key == all && all != none ? back : 255, b_own = l < 6 && key == own && own != none ? back : 255;
+#pragma unroll
+  for (int d = 8; d > 0; d >>= 1) {
+    b_all = min(b_all, __shfl_xor_sync(FULL, b_all, d, 16));
+    b_own = min(b_own, __shfl_xor_sync(FULL, b_own, d, 16));
+  }
+  const int best = at_all ? (__ffs(at_all) - 1) & 15 : 255, single = at_own ? (__ffs(at_own) - 1) & 15 : 255;
+  r.pen = __shfl_sync(FULL, p, best & 15, 16);
+  if (!apart) r.code = best | single << 8 | b_all << 16 | (b_own & 0x7F) << 24;
+  return r;
 }
 
-// fillPointFaceBoxBox, colliders.go:479-517
+// fillPointFaceBoxBox, colliders.go:479-517, of boxes one and two
 template <class R>
-__device__ __forceinline__ void fill_point_face(const xf<R>& one, const xf<R>& two, const v3<R>& h2, const v3<R>& tc,
-                                                int best, R pen, int b0, int b1, NPContact<R>& c) {
-  v3<R> nrm = one.axis(best);
+__device__ __forceinline__ void fill_point_face(const NPTile<R>& tl, int one, int two, const v3<R>& tc, int best, R pen,
+                                                NPContact<R>& c) {
+  v3<R> nrm = tl.axis(one, best);
   if (dot(nrm, tc) > (R)0) mul_with(nrm, (R)-1);
-  v3<R> vv = h2;
-  if (dot(two.axis(0), nrm) < (R)0) vv.x = -vv.x;
-  if (dot(two.axis(1), nrm) < (R)0) vv.y = -vv.y;
-  if (dot(two.axis(2), nrm) < (R)0) vv.z = -vv.z;
-  v3<R> p = xf_mul(two, vv);
+  const xf<R> t = tl.xform(two);
+  v3<R> vv = tl.half(two);
+  if (dot(t.axis(0), nrm) < (R)0) vv.x = -vv.x;
+  if (dot(t.axis(1), nrm) < (R)0) vv.y = -vv.y;
+  if (dot(t.axis(2), nrm) < (R)0) vv.z = -vv.z;
+  v3<R> p = xf_mul(t, vv);
   c.px = p.x; c.py = p.y; c.pz = p.z;
   c.nx = nrm.x; c.ny = nrm.y; c.nz = nrm.z;
   c.pen = pen;
-  c.b0 = b0;
-  c.b1 = b1;
+  c.b0 = one;
+  c.b1 = two;
 }
 
 // contactPoint, colliders.go:519-573
@@ -189,49 +255,32 @@ __device__ __forceinline__ v3<R> edge_contact_point(const v3<R>& p1, const v3<R>
   return c1;
 }
 
-// CollisionCube.CheckAgainstCube, colliders.go:575-710
+// CollisionCube.CheckAgainstCube past its axes (colliders.go:628-710): the
+// contact for the axis `best` of penetration `pen` (sat_axes).
 template <class R>
-__device__ int cube_cube(const xf<R>& t1, const v3<R>& h1, int i1, const xf<R>& t2, const v3<R>& h2, int i2,
-                         NPContact<R>& c, uint32_t& err) {
-  v3<R> tc = t2.axis(3);
-  sub(tc, t1.axis(3));
-  R pen = Lim<R>::max_value();
-  int best = 0xffffff;
-#pragma unroll 1
-  for (int i = 0; i < 3; ++i)
-    if (!try_axis(t1, h1, t2, h2, t1.axis(i), tc, i, pen, best)) return 0;
-#pragma unroll 1
-  for (int i = 0; i < 3; ++i)
-    if (!try_axis(t1, h1, t2, h2, t2.axis(i), tc, i + 3, pen, best)) return 0;
-  const int best_single = best;
-#pragma unroll 1
-  for (int i = 0; i < 3; ++i) {
-#pragma unroll 1
-    for (int j = 0; j < 3; ++j) {
-      if (!try_axis(t1, h1, t2, h2, cross(t1.axis(i), t2.axis(j)), tc, i * 3 + j + 6, pen, best)) return 0;
-    }
-  }
-  if (best < 3) {
-    fill_point_face(t1, t2, h2, tc, best, pen, i1, i2, c);
-    return 1;
-  }
-  if (best < 6) {
-    v3<R> nc = tc;
-    mul_with(nc, (R)-1);
-    fill_point_face(t2, t1, h1, nc, best - 3, pen, i2, i1, c);
-    return 1;
-  }
-  if (best == 0xffffff) {  // only with non-finite transforms; the reference panics here
+__device__ int cube_contact(const NPTile<R>& tl, int i1, int i2, int best, int best_single, R pen, NPContact<R>& c,
+                            uint32_t& err) {
+  if (best > 14) {  // only with non-finite transforms; the reference panics here
     err |= ST_NONFINITE;
     return 0;
   }
+  v3<R> tc = tl.axis(i2, 3);
+  sub(tc, tl.axis(i1, 3));
+  if (best < 6) {
+    const bool second = best > 2;
+    if (second) mul_with(tc, (R)-1);
+    fill_point_face(tl, second ? i2 : i1, second ? i1 : i2, tc, second ? best - 3 : best, pen, c);
+    return 1;
+  }
   best -= 6;
   const int ai = best / 3, bi = best % 3;
-  v3<R> oa = t1.axis(ai);
-  v3<R> ob = t2.axis(bi);
+  v3<R> oa = tl.axis(i1, ai);
+  v3<R> ob = tl.axis(i2, bi);
   v3<R> axis = cross(oa, ob);
   normalize(axis);
   if (dot(axis, tc) > (R)0) mul_with(axis, (R)-1);
+  const xf<R> t1 = tl.xform(i1), t2 = tl.xform(i2);
+  const v3<R> h1 = tl.half(i1), h2 = tl.half(i2);
   R e1[3] = {h1.x, h1.y, h1.z};
   R e2[3] = {h2.x, h2.y, h2.z};
 #pragma unroll
@@ -318,66 +367,50 @@ __device__ __forceinline__ int sphere_sphere(const v3<R>& p1, R r1, int i1, cons
   return 1;
 }
 
-// Vertex sign table, colliders.go:319-327 (bit k set = negative component k)
-__device__ __forceinline__ v3<float> vsign(int k) {
-  return V<float>((k & 1) ? -1.f : 1.f, (k & 2) ? -1.f : 1.f, (k & 4) ? -1.f : 1.f);
+// CollisionSphere.CheckAgainstHalfSpace (colliders.go:178-207)
+template <class R>
+__device__ __forceinline__ int plane_sphere(const NPTile<R>& tl, int i, const BatchView<R>& v, NPContact<R>& c) {
+  const v3<R> pn = V<R>(v.plane_nx, v.plane_ny, v.plane_nz);
+  const v3<R> pos = V<R>(tl.T[9 * tl.nbs + i], tl.T[10 * tl.nbs + i], tl.T[11 * tl.nbs + i]);
+  const R r = tl.radius(i);
+  const R d = dot(pn, pos) - r;
+  if (!(d <= v.plane_offset)) return 0;
+  v3<R> p = pn;
+  mul_with(p, d + r * (R)-1);
+  add(p, pos);
+  c.px = p.x; c.py = p.y; c.pz = p.z;
+  c.nx = pn.x; c.ny = pn.y; c.nz = pn.z;
+  c.pen = -d;
+  c.b0 = i;
+  c.b1 = -1;
+  return 1;
 }
 
-// Plane tests: CollisionSphere/CollisionCube.CheckAgainstHalfSpace
-// (colliders.go:178-207, 306-366, 750-760).  Returns the number of contacts;
-// with `out` non-null it also writes them (in vertex order) at out[0..].
+// Vertex k of CollisionCube.CheckAgainstHalfSpace (colliders.go:306-366,
+// 750-760; bit b of k set: component b negative): whether it gives a contact,
+// and the contact.
 template <class R>
-__device__ int plane_contacts(const NPTile<R>& tl, int i, const BatchView<R>& v, R* out, int* outb, long long stride,
-                              int room) {
+__device__ __forceinline__ bool plane_vertex(const NPTile<R>& tl, int i, int k, const BatchView<R>& v,
+                                             NPContact<R>& c) {
   const v3<R> pn = V<R>(v.plane_nx, v.plane_ny, v.plane_nz);
   const R off = v.plane_offset;
   const xf<R> t = tl.xform(i);
-  const v3<R> pos = t.axis(3);
-  if (tl.shape[i] == 0) {
-    const R r = tl.radius(i);
-    R d = dot(pn, pos) - r;
-    if (!(d <= off)) return 0;
-    if (out && room > 0) {
-      v3<R> p = pn;
-      mul_with(p, d + r * (R)-1);
-      add(p, pos);
-      out[C_PX * stride] = p.x; out[C_PY * stride] = p.y; out[C_PZ * stride] = p.z;
-      out[C_NX * stride] = pn.x; out[C_NY * stride] = pn.y; out[C_NZ * stride] = pn.z;
-      out[C_PEN * stride] = -d;
-      out[C_FRIC * stride] = (R)0.9;
-      out[C_REST * stride] = (R)0.1;
-      outb[0] = pack_bodies(i, -1);
-    }
-    return 1;
-  }
   const v3<R> h = tl.half(i);
-  R proj = transform_to_axis(t, h, pn);
-  R cd = dot(pn, pos) - proj;
-  if (!(cd <= off)) return 0;
-  int cnt = 0;
-#pragma unroll 1
-  for (int k = 0; k < 8; ++k) {
-    v3<float> sg = vsign(k);
-    v3<R> vv = V<R>((R)sg.x * h.x, (R)sg.y * h.y, (R)sg.z * h.z);
-    v3<R> vp = xf_mul(t, vv);
-    R vd = dot(vp, pn);
-    if (vd <= off) {
-      if (out && cnt < room) {
-        v3<R> p = pn;
-        mul_with(p, vd - off);
-        add(p, vp);
-        R* o = out + cnt;
-        o[C_PX * stride] = p.x; o[C_PY * stride] = p.y; o[C_PZ * stride] = p.z;
-        o[C_NX * stride] = pn.x; o[C_NY * stride] = pn.y; o[C_NZ * stride] = pn.z;
-        o[C_PEN * stride] = off - vd;
-        o[C_FRIC * stride] = (R)0.9;
-        o[C_REST * stride] = (R)0.1;
-        outb[cnt] = pack_bodies(i, -1);
-      }
-      ++cnt;
-    }
-  }
-  return cnt;
+  const R proj = transform_to_axis(t, h, pn);
+  const R cd = dot(pn, t.axis(3)) - proj;
+  if (!(cd <= off)) return false;
+  const v3<R> vp = xf_mul(t, V<R>((k & 1) ? -h.x : h.x, (k & 2) ? -h.y : h.y, (k & 4) ? -h.z : h.z));
+  const R vd = dot(vp, pn);
+  if (!(vd <= off)) return false;
+  v3<R> p = pn;
+  mul_with(p, vd - off);
+  add(p, vp);
+  c.px = p.x; c.py = p.y; c.pz = p.z;
+  c.nx = pn.x; c.ny = pn.y; c.nz = pn.z;
+  c.pen = off - vd;
+  c.b0 = i;
+  c.b1 = -1;
+  return true;
 }
 
 // Conservative float32 rejection tests.  Each returns true only when the
@@ -430,26 +463,19 @@ template <class R> __device__ __forceinline__ bool pair_culled(const NPTile<R>& 
   return si == 0 ? cl.box_sphere(j, i) : cl.boxes(i, j);
 }
 
-// One ordered pair (i, j) past the culls: CheckForCollisions(collider i,
-// collider j) (colliders.go:718-747 with the forwarding of colliders.go:209-213).
+// One ordered pair (i, j) past the culls with a sphere in it:
+// CheckForCollisions(collider i, collider j) (colliders.go:718-747 with the
+// forwarding of colliders.go:209-213).
 template <class R>
-__device__ int pair_full(const NPTile<R>& tl, int i, int j, const BatchView<R>& v, int bstart, NPContact<R>& c,
-                         uint32_t& err) {
+__device__ int sphere_pair(const NPTile<R>& tl, int i, int j, const BatchView<R>& v, int bstart, NPContact<R>& c) {
   const int si = tl.shape[i], sj = tl.shape[j];
   if (si == 0 && sj == 0)
     return sphere_sphere(V<R>(tl.T[9 * tl.nbs + i], tl.T[10 * tl.nbs + i], tl.T[11 * tl.nbs + i]), tl.radius(i), i,
                          V<R>(tl.T[9 * tl.nbs + j], tl.T[10 * tl.nbs + j], tl.T[11 * tl.nbs + j]), tl.radius(j), j, c);
-  if (si != 0 && sj != 0) return cube_cube(tl.xform(i), tl.half(i), i, tl.xform(j), tl.half(j), j, c, err);
   // a cube and a sphere, in either order: one call site
   const int bx = si != 0 ? i : j, sp = si != 0 ? j : i;
   return cube_sphere(tl.xform(bx), tl.half(bx), bx, tl.xform(sp), tl.radius(sp), sp,
                      v.body + (long long)B_VX * v.nb_pad + bstart + sp, v.nb_pad, c);
-}
-
-template <class R>
-__device__ __forceinline__ int pair_test(const NPTile<R>& tl, int i, int j, const BatchView<R>& v, int bstart,
-                                         NPContact<R>& c, uint32_t& err) {
-  return pair_culled(tl, i, j) ? 0 : pair_full(tl, i, j, v, bstart, c, err);
 }
 
 // Whether a float32 cull rules out any contact of body i with the half-space
@@ -504,9 +530,12 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 // (up to 1024 units) on top of a partly filled list, and at least one body's
 // units (the grid path lists a body's units together).
 constexpr int kSurvivors = 1280;
-// np_flush's scratch for a CTA of bd threads: the chunk's order by kind of
-// test, its counts, and per-kind counts of each warp (6 kinds x 8 warps)
-__host__ __device__ constexpr int np_sort_ints(int bd) { return 2 * bd + 64; }
+// np_flush's scratch for a CTA of bd threads: the box pairs' penetrations,
+// outcomes and the unit that holds them, the chunk's order by kind of test, its
+// counts, and per-kind counts of each warp (6 kinds x 8 warps)
+template <class R> __host__ __device__ constexpr int np_sort_ints(int bd) {
+  return (int)(sizeof(R) / 4) * bd + 4 * bd + 64;
+}
 __host__ __device__ inline int np_surv_cap(int nbs) { return nbs + 1 > kSurvivors ? ((nbs + 32) & ~31) : kSurvivors; }
 
 template <class R> __host__ __device__ inline size_t np_smem_bytes(int nbs) {
@@ -516,7 +545,7 @@ template <class R> __host__ __device__ inline size_t np_smem_bytes(int nbs) {
   b += (size_t)5 * nbs * sizeof(float);           // cull data
   b += 2 * 33 * sizeof(int);                      // scan scratch (double-buffered) + world id + wait outcome
   b += (size_t)np_surv_cap(nbs) * sizeof(int);    // units past the culls, awaiting their full tests
-  b += (size_t)np_sort_ints(256) * sizeof(int);   // np_flush's sort of a chunk by kind of test
+  b += (size_t)np_sort_ints<R>(256) * sizeof(int) + 8;  // np_flush's scratch (aligned)
   return b;
 }
 
@@ -606,44 +635,46 @@ __device__ __forceinline__ void np_chunk_scan(int cnt, int* scan, int parity, in
   *total = wt[nwarps - 1];
 }
 
-// Write one unit's contacts (a pair's single contact or a half-space test's
-// 0..8) at slot `off` of the world's contact slab, within its capacity.
+// Write a contact at slot `off` of the world's contact slab, within its
+// capacity.
 template <class R>
-__device__ __forceinline__ void np_emit(const NPTile<R>& tl, const BatchView<R>& v, long long cs, int cap, int off,
-                                        int cnt, int i, bool plane, const NPContact<R>& c) {
-  if (cnt <= 0) return;
-  const int room = cap - off;
-  if (room <= 0) return;
+__device__ __forceinline__ void np_emit(const BatchView<R>& v, long long cs, int cap, int off, const NPContact<R>& c) {
+  if (off >= cap) return;
   R* o = v.contact + cs + off;
-  int* ob = v.contact_bodies + cs + off;
-  if (plane) {
-    plane_contacts<R>(tl, i, v, o, ob, v.nc_total, room);
-  } else {
-    const long long S = v.nc_total;
-    o[C_PX * S] = c.px; o[C_PY * S] = c.py; o[C_PZ * S] = c.pz;
-    o[C_NX * S] = c.nx; o[C_NY * S] = c.ny; o[C_NZ * S] = c.nz;
-    o[C_PEN * S] = c.pen;
-    o[C_FRIC * S] = (R)0.9;
-    o[C_REST * S] = (R)0.1;
-    ob[0] = pack_bodies(c.b0, c.b1);
-  }
+  const long long S = v.nc_total;
+  o[C_PX * S] = c.px; o[C_PY * S] = c.py; o[C_PZ * S] = c.pz;
+  o[C_NX * S] = c.nx; o[C_NY * S] = c.ny; o[C_NZ * S] = c.nz;
+  o[C_PEN * S] = c.pen;
+  o[C_FRIC * S] = (R)0.9;
+  o[C_REST * S] = (R)0.1;
+  v.contact_bodies[cs + off] = pack_bodies(c.b0, c.b1);
 }
 
 // The full tests of the listed units (unit u = i * n + k: k = 0 the
 // half-space, else the pair with j = k - 1, skipping i), in chunks of the
 // CTA's size, emitting their contacts in list order at out onwards.  Within a
-// chunk the units are taken in order of their kind of test (half-space with
-// a sphere, with a cube; sphere-sphere, sphere-cube, cube-cube), stably, so
-// the lanes of a warp mostly run one test's code; the counts are then
-// scanned in list order, so every contact lands where the list order puts
-// it (the reference's contact order).  sortw: np_sort_ints(blockDim.x) ints.
+// chunk the units are taken in order of their kind of test (half-space with a
+// sphere, with a cube; sphere-sphere, sphere-cube, cube-cube), stably, so the
+// lanes of a warp mostly run one test's code; the counts are then scanned in
+// list order, so every contact lands where the list order puts it (the
+// reference's contact order).  The two tests with many parts are spread over
+// lanes: a cube's half-space test takes a lane per vertex (eight), which keeps
+// its vertex's contact until the scan says where it goes, and a cube pair's
+// axes take sixteen (sat_axes).  On a thread each, a warp ran the eight
+// vertices twice (count, write) and the fifteen axes one after the other for
+// whatever few lanes had them.  Narrowphase of 8192 worlds x 32 bodies, float64
+// 1.50 -> 0.73 ms a frame, float32 0.176 -> 0.170; of one world of 20 cubes in
+// float64 84 -> 43 us.  sortw: np_sort_ints(blockDim.x) ints.
 template <class R>
 __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart, int n, long long cs, int cap,
                          const int* surv, int nsurv, int* scan, int& parity, int& out, uint32_t& err, int* sortw) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, bd = blockDim.x, nwarps = (bd + 31) >> 5;
-  int* perm = sortw;
-  int* cntb = sortw + bd;
-  int* wcnt = sortw + 2 * bd;  // [kind * 8 + warp]
+  R* satp = reinterpret_cast<R*>(((size_t)sortw + 7) & ~(size_t)7);
+  int* satc = reinterpret_cast<int*>(satp + bd);  // outcome of the pair held here
+  int* satr = satc + bd;                          // the unit holding this unit's outcome; a cube's vertices (bits)
+  int* perm = satr + bd;
+  int* cntb = perm + bd;
+  int* wcnt = cntb + bd;  // [kind * 8 + warp]
   for (int sb = 0; sb < nsurv; sb += bd) {
     const int m = nsurv - sb < bd ? nsurv - sb : bd;
     int key = 5;  // no unit
@@ -666,25 +697,78 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
       if (lane == 0) wcnt[q * 8 + wid] = __popc(bal);
     }
     __syncthreads();
-    int dst = rank;
-    for (int q = 0; q < key; ++q)
-      for (int w2 = 0; w2 < nwarps; ++w2) dst += wcnt[q * 8 + w2];
-    for (int w2 = 0; w2 < wid; ++w2) dst += wcnt[key * 8 + w2];
+    int dst = rank, n0 = 0, n1 = 0, n23 = 0, n4 = 0;
+    for (int w2 = 0; w2 < nwarps; ++w2) {
+      const int a = wcnt[w2], b = wcnt[8 + w2], c2 = wcnt[16 + w2], c3 = wcnt[24 + w2], d = wcnt[32 + w2];
+      n0 += a;
+      n1 += b;
+      n23 += c2 + c3;
+      n4 += d;
+      dst += (key > 0 ? a : 0) + (key > 1 ? b : 0) + (key > 2 ? c2 : 0) + (key > 3 ? c3 : 0) + (key > 4 ? d : 0);
+      if (w2 < wid) dst += wcnt[key * 8 + w2];
+    }
     perm[dst] = tid;
     __syncthreads();
+    // cube pairs: an axis per lane
+#pragma unroll 1
+    for (int g = tid >> 4; g < ((n4 + 1) & ~1); g += bd >> 4) {  // both groups of a warp together
+      const bool on = g < n4;
+      const int at = perm[n0 + n1 + n23 + (on ? g : 0)], l = tid & 15;
+      const int uu = surv[sb + at];
+      const int i = uu / n, k = uu - i * n;
+      const int j = k - 1 >= i ? k : k - 1;
+      // (i, j) with i > j takes the outcome of (j, i) where the chunk has it
+      int other = -1;
+      if (on && i > j)
+        for (int q = l; q < m; q += 16)
+          if (surv[sb + q] == j * n + i) other = q;  // j's k is i: i > j
+      const unsigned have = __ballot_sync(FULL, other >= 0) & (0xFFFFu << (lane & 16));
+      other = __shfl_sync(FULL, other, have ? __ffs(have) - 1 : lane);
+      const bool need = on && !have;
+      if (__any_sync(FULL, need)) {
+        const SatResult<R> r = sat_axes(tl, i, j, l);
+        if (need && l == 0) {
+          satp[at] = r.pen;
+          satc[at] = r.code;
+        }
+      }
+      if (on && l == 0) satr[at] = have ? other : at;
+    }
+    // half-space with a cube: a vertex per lane, kept by the last pass
+    NPContact<R> vc;
+    bool vhit = false;
+    const int passes = (8 * n1 + bd - 1) / bd;
+#pragma unroll 1
+    for (int q = 0; q < passes; ++q) {
+      const int g = (q * bd + tid) >> 3;
+      const int at = perm[n0 + (g < n1 ? g : 0)];
+      vhit = g < n1 && plane_vertex(tl, surv[sb + at] / n, tid & 7, v, vc);
+      const unsigned bits = (__ballot_sync(FULL, vhit) >> (lane & 24)) & 0xFFu;
+      if (g < n1 && (tid & 7) == 0) satr[at] = (int)bits;
+    }
+    __syncthreads();
     const int src = perm[tid];  // this thread tests the chunk's unit src
-    int cnt = 0, i = 0, k = 0;
+    int cnt = 0;
+    bool cube_plane = false;
     NPContact<R> c;
     if (src < m) {
       const int uu = surv[sb + src];
-      i = uu / n;
-      k = uu - i * n;
-      if (k == 0) {
-        cnt = plane_contacts<R>(tl, i, v, nullptr, nullptr, 0, 0);
+      const int i = uu / n, k = uu - i * n;
+      const int j = k - 1 >= i ? k : k - 1;
+      cube_plane = k == 0 && tl.shape[i] != 0;
+      if (cube_plane) {
+        cnt = __popc((unsigned)satr[src]);
+      } else if (k == 0) {
+        cnt = plane_sphere(tl, i, v, c);
+      } else if (tl.shape[i] != 0 && tl.shape[j] != 0) {
+        const int at = satr[src];
+        int code = satc[at];
+        if (code != kSatApart) {
+          if (at != src) code = (int)((unsigned)code >> 16);  // the pair's other order
+          cnt = cube_contact(tl, i, j, code & 0xFF, (code >> 8) & 0x7F, satp[at], c, err);
+        }
       } else {
-        int j = k - 1;
-        if (j >= i) ++j;
-        cnt = pair_full<R>(tl, i, j, v, bstart, c, err);
+        cnt = sphere_pair(tl, i, j, v, bstart, c);
       }
     }
     cntb[src] = cnt;
@@ -694,7 +778,16 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
     parity ^= 1;
     cntb[tid] = excl;
     __syncthreads();
-    np_emit<R>(tl, v, cs, cap, out + cntb[src], cnt, i, k == 0, c);
+    if (cnt > 0 && !cube_plane) np_emit<R>(v, cs, cap, out + cntb[src], c);
+#pragma unroll 1
+    for (int q = passes - 1; q >= 0; --q) {
+      const int g = (q * bd + tid) >> 3;
+      if (g < n1) {
+        const int at = perm[n0 + g];
+        if (q < passes - 1) vhit = plane_vertex(tl, surv[sb + at] / n, tid & 7, v, vc);
+        if (vhit) np_emit<R>(v, cs, cap, out + cntb[at] + __popc((unsigned)satr[at] & ((1u << (tid & 7)) - 1u)), vc);
+      }
+    }
     out += total;
     __syncthreads();  // perm and cntb are reused by the next chunk
   }
@@ -978,10 +1071,11 @@ __device__ void np_world(const NPTile<R>& tl, const BatchView<R>& v, int w, int 
 
 // GRID = false compiles the all-pairs path alone (worlds too small for the
 // grid), so its registers and occupancy stay those of that path; in float32
-// it is bounded to 64 registers (8 CTAs of 128 threads per SM instead of 6;
-// a few registers spill), which hides more of its barrier waits.
+// it is bounded to 80 registers (6 CTAs of 128 threads per SM; a few registers
+// spill): 0.190 ms for 8192 worlds of 32 bodies, against 0.200 with 64 (320
+// bytes spilled) and 0.201 with 109 (no spills, 4 CTAs).
 template <class R, bool GRID>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 && !GRID ? 4 : 0) k_narrowphase(BatchView<R> v, int nbs) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 && !GRID ? 3 : 0) k_narrowphase(BatchView<R> v, int nbs) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem);
   NPTile<R> tl;
@@ -1084,24 +1178,28 @@ __global__ void __launch_bounds__(256) k_collide(BatchView<R> v, int w, const in
   __syncthreads();
   const long long cs = v.contact_start[w];
   const int cap = v.contact_cap[w];
-  int out = 0, parity = 0;
+  int* surv = scan + 66;
+  const int scap = np_surv_cap(nbs);
+  int out = 0, parity = 0, nsurv = 0;
   uint32_t err = 0;
   for (int base = 0; base < nunits; base += blockDim.x) {
     const int u = base + tid;
-    int cnt = 0, i = 0;
-    bool plane = false;
-    NPContact<R> c;
+    bool keep = false;
+    int2 un = make_int2(0, 0);
     if (u < nunits) {
-      const int2 un = units[u];
-      i = un.x;
-      plane = un.y < 0;
-      cnt = plane ? plane_contacts<R>(tl, i, v, nullptr, nullptr, 0, 0) : pair_test<R>(tl, i, un.y, v, bstart, c, err);
+      un = units[u];
+      keep = un.y < 0 ? !plane_culled(tl, un.x, v) : !pair_culled(tl, un.x, un.y);
     }
     int excl, total;
-    np_chunk_scan(cnt, scan, parity, &excl, &total);
+    np_chunk_scan(keep ? 1 : 0, scan, parity, &excl, &total);
     parity ^= 1;
-    np_emit<R>(tl, v, cs, cap, out + excl, cnt, i, plane, c);
-    out += total;
+    if (keep) surv[nsurv + excl] = un.x * n + (un.y < 0 ? 0 : (un.y < un.x ? un.y + 1 : un.y));
+    nsurv += total;
+    if (nsurv + (int)blockDim.x <= scap && base + (int)blockDim.x < nunits) continue;
+    __syncthreads();
+    np_flush(tl, v, bstart, n, cs, cap, surv, nsurv, scan, parity, out, err, surv + scap);
+    nsurv = 0;
+    __syncthreads();
   }
   if (err) {
     atomicOr(&v.world_status[w], err);
