@@ -310,9 +310,14 @@ __device__ __noinline__ void derive_asleep(RCtx<R, W, SM> x, const BatchView<R>&
 // Normalize (quaternion.go:77-99) of component c (w first) of a quaternion
 // whose squares sum to s: the component after it.  Out of line: in the
 // precision form's island it is rare.
+// RealEqual(1, len) is |1 - len| / (1 + len) < 1e-7: certain without the
+// division below 1e-7 (1 + len is at least 1) and above 4e-7 (with len < 2.9
+// the divisor is at most 3.9), which is nearly always.
 template <class W> __device__ __noinline__ W normalize_component(W s, W component, int c) {
   W len = sqrt_<W>(s);
-  if (real_equal<W>((W)1, len)) return component;
+  const W diff = fabs_<W>((W)1 - len);
+  if (diff < (W)1e-7) return component;
+  if (!(diff > (W)4e-7 && len < (W)2.9) && real_equal<W>((W)1, len)) return component;
   if (len == (W)0) return c == 0 ? (W)1 : (W)0;
   if (len == Lim<W>::inf()) len = Lim<W>::max_value();
   return component * ((W)1 / len);
@@ -359,15 +364,20 @@ __device__ void position_change(const RCtx<R, W, SM>& x, const BatchView<R>& v, 
   const int bO = __shfl_xor_sync(0xffffffffu, b, 4);
   const bool act = on && b >= 0;
   W acc = (W)0;
-  R qr = z;
+  R qr = z, share = z;
   if (act) {
     const int b0 = i == 0 ? b : bO, b1 = i == 0 ? bO : b;
     R total = z;
     if (b0 >= 0) total += (i == 0 ? linI : linO) + (i == 0 ? angI : angO);
     if (b1 >= 0) total += (i == 0 ? linO : linI) + (i == 0 ? angO : angI);
+    // angI / total on the even lanes, linI / total on the odd ones
+    share = ((c & 1) == 0 ? angI : linI) / total;
+  }
+  const R share_o = __shfl_xor_sync(0xffffffffu, share, 1);
+  if (act) {
     const R sign = i != 0 ? (R)-1 : (R)1;
-    R am = sign * penetration * (angI / total);
-    R lm = sign * penetration * (linI / total);
+    R am = sign * penetration * ((c & 1) == 0 ? share : share_o);
+    R lm = sign * penetration * ((c & 1) == 0 ? share_o : share);
     v3<R> proj = rp;
     add_scaled(proj, n, -dot(rp, n));
     const R maxm = (R)0.2 * mag(proj);
@@ -391,17 +401,23 @@ __device__ void position_change(const RCtx<R, W, SM>& x, const BatchView<R>& v, 
     acc = x.P(3 + c, b);
     qr = cvt_fast<R>(acc);
   }
-  q4<R> q;
-  q.w = __shfl_sync(0xffffffffu, qr, src, 8);
-  q.x = __shfl_sync(0xffffffffu, qr, src + 1, 8);
-  q.y = __shfl_sync(0xffffffffu, qr, src + 2, 8);
-  q.z = __shfl_sync(0xffffffffu, qr, src + 3, 8);
+  // component c of (0, ang) * q (quaternion.go:45-53), each lane its own:
+  //   w: 0 qw - ax qx - ay qy - az qz     x: 0 qx + ax qw + ay qz - az qy
+  //   y: 0 qy + ay qw + az qx - ax qz     z: 0 qz + az qw + ax qy - ay qx
+  const R q1 = __shfl_sync(0xffffffffu, qr, src + (c == 0 ? 1 : 0), 8);
+  const R q2 = __shfl_sync(0xffffffffu, qr, src + (c == 1 ? 3 : (c == 2 ? 1 : 2)), 8);
+  const R q3 = __shfl_sync(0xffffffffu, qr, src + (c == 1 ? 2 : (c == 3 ? 1 : 3)), 8);
   if (act) {
     // Position.AddScaled(normal, linearMove), and the quaternion increment
     if (c < 3) x.P(c, b) += cvt_fast<W>(linc);
-    q4<R> t{(R)0, ang.x * (R)1, ang.y * (R)1, ang.z * (R)1};
-    t = qmul(t, q);
-    acc += cvt_fast<W>((c == 0 ? t.w : (c == 1 ? t.x : (c == 2 ? t.y : t.z))) * (R)0.5);
+    const R a1 = (c < 2 ? ang.x : (c == 2 ? ang.y : ang.z)) * q1;
+    const R a2 = (c < 2 ? ang.y : (c == 2 ? ang.z : ang.x)) * q2;
+    const R a3 = (c < 2 ? ang.z : (c == 2 ? ang.x : ang.y)) * q3;
+    R t = (R)0 * qr;
+    t = c == 0 ? t - a1 : t + a1;
+    t = c == 0 ? t - a2 : t + a2;
+    t = t - a3;
+    acc += cvt_fast<W>(t * (R)0.5);
   }
   // qnormalize_island on the four components
   const W sq = act ? acc * acc : (W)0;
