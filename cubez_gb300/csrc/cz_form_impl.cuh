@@ -342,7 +342,10 @@ static cudaError_t big_smem(int n, int max_cap, size_t budget, int* csm, size_t*
   *smem = fixed;
   if (budget > fixed) {
     const size_t fit = (budget - fixed) / big_contact_bytes<R>();
-    *csm = (int)(fit < (size_t)max_cap ? fit : (size_t)max_cap) & ~3;
+    // eight contacts a body (a settled pile has about five), and no more: the rest
+    // of the SM's memory is the records' L1
+    const size_t want = (size_t)((std::min(max_cap, 8 * n) + 15) & ~15);
+    *csm = (int)std::min(want, fit & ~(size_t)15);
     *smem = fixed + *csm * big_contact_bytes<R>();
   }
   return raise_smem_limit((const void*)k_resolve_big<R, W>, *smem);

@@ -25,6 +25,8 @@
 // inference and plan, launched before k_resolve) and the shared pieces of
 // k_resolve_big (cz_resolve_big.cuh).
 #pragma once
+#include <type_traits>
+
 #include "cz_layout.cuh"
 #include "cz_math.cuh"
 #include "cz_mlp.cuh"
@@ -324,63 +326,98 @@ template <class W> __device__ __noinline__ W normalize_component(W s, W componen
 }
 
 // applyPositionChange, contact.go:285-386, of contact k by the first eight
-// lanes (sl = 0..7) of a group with `on`; every lane of the warp calls it.
-// The four lanes 4i..4i+3 move body i: they form its inertia, its moves and
-// its changes alike (the two bodies meet by shuffles, and the total is summed
-// in the reference's order), then lane 4i + c adds position component c
-// (c < 3) and quaternion component c and squares the latter; the squares meet
-// by shuffles and every lane of the body decides the renormalisation alike
-// (the precision form's island, or Normalize in the float64 form).  A float64
-// warp instruction costs the pipe the same whatever its active lanes: two
-// adds and one multiply for both bodies' fourteen components, against seven
-// adds and four multiplies per body on one lane.  The operations on every
-// value are the one-lane formula's, so the bits are the same.  Lane 4i + c
-// returns component c of body i's linear and angular change.
+// lanes (sl = 0..7) of a group with `on`; every lane of the warp calls both
+// parts.  The four lanes 4i..4i+3 move body i: lane 4i + c (c < 3) forms
+// component c of its inertia's vectors, of its moves and of its position, and
+// (c < 4) its own component of the quaternion; the vectors meet by shuffles
+// where a dot product or a matrix row needs them whole, the two bodies where
+// the total does (summed in the reference's order), and every lane of a body
+// decides the clamps and the renormalisation alike (the precision form's
+// island, or Normalize in the float64 form).  A float64 warp instruction takes
+// its scheduler's float64 unit 64 cycles whatever its active mask, so the
+// number of them is what counts: about 110 where one lane per body's formulas
+// took 160.  The operations on every value are the one-lane formula's, so the
+// bits are the same.  Lane 4i + c returns component c of body i's linear and
+// angular change.  position_load reads what it needs, as velocity_load does.
+template <class R, class W> struct PositionIn {
+  v3<R> n, rp;         // normal, the body's relative position
+  R nc, np, nq;        // components c and the cross product's other two
+  R rc, rp1, rq1;
+  R i0, i1, i2, im;    // the body's inertia row c, inverse mass
+  R penetration;
+  W acc, at;           // quaternion component c, position component c
+  int b;
+};
 template <class R, class W, bool SM>
-__device__ void position_change(const RCtx<R, W, SM>& x, const BatchView<R>& v, int bstart, int k, bool on, int sl,
-                                R& linc, R& angc) {
-  const int i = (sl >> 2) & 1, c = sl & 3, src = sl & 4;
+__device__ __forceinline__ void position_load(const RCtx<R, W, SM>& x, PositionIn<R, W>& in, int k, int bb, bool on,
+                                              int sl) {
   const R z = (R)0;
-  linc = angc = z;
-  int b = -1;
-  v3<R> n = V<R>(z, z, z), rp = V<R>(z, z, z), ang = V<R>(z, z, z);
-  R angI = z, linI = z, penetration = z;
-  if (on) {
-    const int bb = x.pair(k);
-    b = i == 0 ? x.B0(bb) : x.B1(bb);
-    const R* r = x.rec(k);
-    const quad<R> a = ld4(r);
-    n = V<R>(a.a, a.b, a.c);
-    rp = x.rel(i, k);
-    penetration = r[CR_PEN];
-    if (b >= 0) {
-      ang = mulv(x.iit(b), cross(rp, n));
-      angI = dot(cross(ang, rp), n);
-      linI = x.body(b)[BR_INVM];
-    }
+  const int i = (sl >> 2) & 1, c4 = sl & 3, c = c4 != 3 ? c4 : 0;
+  const int p = c == 2 ? 0 : c + 1, q = c == 0 ? 2 : c - 1;
+  in.n = in.rp = V<R>(z, z, z);
+  in.nc = in.np = in.nq = in.rc = in.rp1 = in.rq1 = in.i0 = in.i1 = in.i2 = in.im = in.penetration = z;
+  in.b = -1;
+  in.acc = in.at = (W)0;
+  if (!on) return;
+  const R* r = x.rec(k);
+  const R* rel = r + (i == 0 ? CR_R0 : CR_R1);
+  in.n = V<R>(r[0], r[1], r[2]);
+  in.rp = V<R>(rel[0], rel[1], rel[2]);
+  in.nc = r[CR_N + c]; in.np = r[CR_N + p]; in.nq = r[CR_N + q];
+  in.rc = rel[c]; in.rp1 = rel[p]; in.rq1 = rel[q];
+  in.penetration = r[CR_PEN];
+  in.b = i == 0 ? x.B0(bb) : x.B1(bb);
+  if (in.b >= 0) {
+    const R* bd = x.body(in.b);
+    in.i0 = bd[BR_IIT + c]; in.i1 = bd[BR_IIT + 3 + c]; in.i2 = bd[BR_IIT + 6 + c];
+    in.im = bd[BR_INVM];
+    in.acc = x.P(3 + c4, in.b);
+    in.at = x.P(c, in.b);
   }
+}
+template <class R, class W, bool SM>
+__device__ __forceinline__ void position_change(const RCtx<R, W, SM>& x, const BatchView<R>& v,
+                                                const PositionIn<R, W>& in, int bstart, bool on, int sl, R& linc,
+                                                R& angc) {
+  const int i = (sl >> 2) & 1, c4 = sl & 3, c = c4 != 3 ? c4 : 0, src = sl & 4;
+  const int p = c == 2 ? 0 : c + 1, q = c == 0 ? 2 : c - 1;
+  const R z = (R)0;
+  auto all = [&](R a) {
+    return V<R>(__shfl_sync(0xffffffffu, a, 0, 4), __shfl_sync(0xffffffffu, a, 1, 4),
+                __shfl_sync(0xffffffffu, a, 2, 4));
+  };
+  const int b = in.b;
+  const bool act = on && b >= 0;
+  // angular inertia: dot(cross(iitWorld * cross(rp, n), rp), n)
+  const v3<R> a = all(in.rp1 * in.nq - in.rq1 * in.np);
+  const R wc = in.i0 * a.x + in.i1 * a.y + in.i2 * a.z;
+  const R wp = __shfl_sync(0xffffffffu, wc, p, 4), wq = __shfl_sync(0xffffffffu, wc, q, 4);
+  const v3<R> d = all(wp * in.rq1 - wq * in.rp1);
+  const R angI = act ? dot(d, in.n) : z;
+  const R linI = act ? in.im : z;
   const R angO = __shfl_xor_sync(0xffffffffu, angI, 4);
   const R linO = __shfl_xor_sync(0xffffffffu, linI, 4);
   const int bO = __shfl_xor_sync(0xffffffffu, b, 4);
-  const bool act = on && b >= 0;
-  W acc = (W)0;
-  R qr = z, share = z;
+  R share = z;
   if (act) {
     const int b0 = i == 0 ? b : bO, b1 = i == 0 ? bO : b;
     R total = z;
     if (b0 >= 0) total += (i == 0 ? linI : linO) + (i == 0 ? angI : angO);
     if (b1 >= 0) total += (i == 0 ? linO : linI) + (i == 0 ? angO : angI);
     // angI / total on the even lanes, linI / total on the odd ones
-    share = ((c & 1) == 0 ? angI : linI) / total;
+    share = ((c4 & 1) == 0 ? angI : linI) / total;
   }
   const R share_o = __shfl_xor_sync(0xffffffffu, share, 1);
+  const R pc = in.rc + in.nc * -dot(in.rp, in.n);  // the projection's component c
+  const v3<R> pp = all(pc * pc);
+  linc = angc = z;
+  W acc = in.acc;
+  R qr = z;
   if (act) {
     const R sign = i != 0 ? (R)-1 : (R)1;
-    R am = sign * penetration * ((c & 1) == 0 ? share : share_o);
-    R lm = sign * penetration * ((c & 1) == 0 ? share_o : share);
-    v3<R> proj = rp;
-    add_scaled(proj, n, -dot(rp, n));
-    const R maxm = (R)0.2 * mag(proj);
+    R am = sign * in.penetration * ((c4 & 1) == 0 ? share : share_o);
+    R lm = sign * in.penetration * ((c4 & 1) == 0 ? share_o : share);
+    const R maxm = (R)0.2 * sqrt_<R>(pp.x + pp.y + pp.z);
     if (am < -maxm) {
       R tm = am + lm;
       am = -maxm;
@@ -390,32 +427,28 @@ __device__ void position_change(const RCtx<R, W, SM>& x, const BatchView<R>& v, 
       am = maxm;
       lm = tm - am;
     }
-    if (am != (R)0)
-      mul_with(ang, am / angI);
-    else
-      ang = V<R>(z, z, z);
-    linc = c == 3 ? z : (c == 0 ? n.x : (c == 1 ? n.y : n.z)) * lm;
-    angc = c == 0 ? ang.x : (c == 1 ? ang.y : ang.z);
+    if (am != (R)0) angc = wc * (am / angI);
+    linc = in.nc * lm;
     // the quaternion, narrowed by its component lanes for the increment
     // (add_scaled_vector_island's first step)
-    acc = x.P(3 + c, b);
     qr = cvt_fast<R>(acc);
   }
-  // component c of (0, ang) * q (quaternion.go:45-53), each lane its own:
+  // component c4 of (0, ang) * q (quaternion.go:45-53), each lane its own:
   //   w: 0 qw - ax qx - ay qy - az qz     x: 0 qx + ax qw + ay qz - az qy
   //   y: 0 qy + ay qw + az qx - ax qz     z: 0 qz + az qw + ax qy - ay qx
-  const R q1 = __shfl_sync(0xffffffffu, qr, src + (c == 0 ? 1 : 0), 8);
-  const R q2 = __shfl_sync(0xffffffffu, qr, src + (c == 1 ? 3 : (c == 2 ? 1 : 2)), 8);
-  const R q3 = __shfl_sync(0xffffffffu, qr, src + (c == 1 ? 2 : (c == 3 ? 1 : 3)), 8);
+  const R q1 = __shfl_sync(0xffffffffu, qr, src + (c4 == 0 ? 1 : 0), 8);
+  const R q2 = __shfl_sync(0xffffffffu, qr, src + (c4 == 1 ? 3 : (c4 == 2 ? 1 : 2)), 8);
+  const R q3 = __shfl_sync(0xffffffffu, qr, src + (c4 == 1 ? 2 : (c4 == 3 ? 1 : 3)), 8);
+  const R u1 = __shfl_sync(0xffffffffu, angc, c4 < 2 ? 0 : c4 - 1, 4);
+  const R u2 = __shfl_sync(0xffffffffu, angc, c4 < 2 ? 1 : (c4 == 2 ? 2 : 0), 4);
+  const R u3 = __shfl_sync(0xffffffffu, angc, c4 < 2 ? 2 : c4 - 2, 4);
   if (act) {
     // Position.AddScaled(normal, linearMove), and the quaternion increment
-    if (c < 3) x.P(c, b) += cvt_fast<W>(linc);
-    const R a1 = (c < 2 ? ang.x : (c == 2 ? ang.y : ang.z)) * q1;
-    const R a2 = (c < 2 ? ang.y : (c == 2 ? ang.z : ang.x)) * q2;
-    const R a3 = (c < 2 ? ang.z : (c == 2 ? ang.x : ang.y)) * q3;
+    if (c4 < 3) x.P(c, b) = in.at + cvt_fast<W>(linc);
+    const R a1 = u1 * q1, a2 = u2 * q2, a3 = u3 * q3;
     R t = (R)0 * qr;
-    t = c == 0 ? t - a1 : t + a1;
-    t = c == 0 ? t - a2 : t + a2;
+    t = c4 == 0 ? t - a1 : t + a1;
+    t = c4 == 0 ? t - a2 : t + a2;
     t = t - a3;
     acc += cvt_fast<W>(t * (R)0.5);
   }
@@ -432,15 +465,15 @@ __device__ void position_change(const RCtx<R, W, SM>& x, const BatchView<R>& v, 
     } else if (sizeof(R) != sizeof(W) && ae < (W)0x1p-11) {
       acc *= (W)1 + e * ((W)-0.5 + e * ((W)0.375 + e * ((W)-0.3125 + e * (W)0.2734375)));
     } else {  // on the same sum
-      acc = normalize_component<W>(s, acc, c);
+      acc = normalize_component<W>(s, acc, c4);
     }
     asleep = !x.all_awake && !x.aw[b];
     // an asleep body's CalculateDerivedData reads the stored (R-rounded) orientation
-    x.P(3 + c, b) = asleep ? (W)(R)acc : acc;
+    x.P(3 + c4, b) = asleep ? (W)(R)acc : acc;
   }
   if (!x.all_awake && __any_sync(0xffffffffu, asleep)) {
     __syncwarp();
-    if (asleep && c == 0) derive_asleep(x, v, bstart, b);
+    if (asleep && c4 == 0) derive_asleep(x, v, bstart, b);
     __syncwarp();
   }
 }
@@ -508,82 +541,106 @@ template <class R, class W, bool SM> __device__ __forceinline__ void friction_pr
 }
 
 // applyVelocityChange, contact.go:447-494, of contact k by the first eight
-// lanes (sl = 0..7) of a group with `on`; every lane of the warp calls it.
-// Lane 4i + c (c < 3) forms component c of the friction solve's product
+// lanes (sl = 0..7) of a group with `on`; every lane of the warp calls both
+// parts.  Lane 4i + c (c < 3) forms component c of the friction solve's product
 // (calculateFrictionImpulse, contact.go:533-606, from friction_prepare's
 // matrices), of the impulse, and of body i's velocity and rotation changes,
 // which it adds to the body and returns; the vectors in between meet by
 // shuffles, and the friction cone is decided on every lane alike.  Every
 // component is the one-lane formula's (mulv's row, cross's component,
 // add_scaled), so the bits are the same; one lane forming all of them issued
-// about twice the instructions.  err collects status bits.
+// about twice the instructions.  velocity_load reads all of it, so that the
+// caller's other loads and one latency cover it.
+template <class R> struct VelocityIn {
+  R k0, k1, k2, k9, k10, k11;  // K's row c, the response's first row
+  R n, ty, tz;                 // the basis, row c
+  R rp, rq;                    // the relative position's other components
+  R i0, i1, i2, im, vel, rot;  // the body's inertia row, inverse mass, velocity and rotation c
+  R cvy, cvz, ddv;
+  int b, bb;
+};
+template <class R, class W, bool SM>
+__device__ __forceinline__ void velocity_load(const RCtx<R, W, SM>& x, VelocityIn<R>& in, int k, int bb, bool on,
+                                              int sl) {
+  const R z = (R)0;
+  const int i = (sl >> 2) & 1, c = (sl & 3) != 3 ? sl & 3 : 0;
+  const int p = c == 2 ? 0 : c + 1, q = c == 0 ? 2 : c - 1;
+  in = VelocityIn<R>{z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, -1, bb};
+  if (!on) return;
+  const R* kr = x.krow(k);
+  in.k0 = kr[c]; in.k1 = kr[3 + c]; in.k2 = kr[6 + c];
+  in.k9 = kr[9]; in.k10 = kr[10]; in.k11 = kr[11];
+  const R* r = x.rec(k);
+  const quad<R> m = ld4(r + CR_CV);
+  in.cvy = m.b; in.cvz = m.c; in.ddv = m.d;
+  in.n = r[CR_N + c]; in.ty = r[CR_TY + c]; in.tz = r[CR_TZ + c];
+  const R* rel = r + (i == 0 ? CR_R0 : CR_R1);
+  in.rp = rel[p];
+  in.rq = rel[q];
+  in.b = i == 0 ? x.B0(bb) : x.B1(bb);
+  if (in.b >= 0) {
+    const R* bd = x.body(in.b);
+    in.vel = bd[BR_VEL + c];
+    in.rot = bd[BR_ROT + c];
+    in.i0 = bd[BR_IIT + c]; in.i1 = bd[BR_IIT + 3 + c]; in.i2 = bd[BR_IIT + 6 + c];
+    in.im = bd[BR_INVM];
+  }
+}
+// err collects status bits.
 template <class R, class W, bool LEARN, bool SM>
-__device__ __forceinline__ void velocity_change(const RCtx<R, W, SM>& x, const BatchView<R>& v, int k, bool on, int sl,
-                                                R& vc, R& rc, uint32_t& err) {
+__device__ __forceinline__ void velocity_change(const RCtx<R, W, SM>& x, const BatchView<R>& v,
+                                                const VelocityIn<R>& in, int k, bool on, int sl, R& vc, R& rc,
+                                                uint32_t& err) {
   const int i = (sl >> 2) & 1;
   const bool comp = (sl & 3) != 3;
   const int c = comp ? sl & 3 : 0;
   const int p = c == 2 ? 0 : c + 1, q = c == 0 ? 2 : c - 1;  // cross component c = a_p b_q - a_q b_p
   const R z = (R)0;
-  int b = -1, o = 0;
-  R icc = z, ddv = z, fr = (R)0.9;
-  // loaded ahead of the first shuffle, so that one latency covers them: the
-  // basis rows c, the relative position's other components, the body's rows
-  R nc = z, tyc = z, tzc = z, rp = z, rq = z, i0c = z, i1c = z, i2c = z, im = z, vel = z, rot = z;
-  R k9 = z, k10 = z, k11 = z;
+  const int o = SM ? (int)((unsigned)in.bb >> 16) : k;  // the list index
+  R icc = z, fr = (R)0.9;
   bool frictionless = false;
   v3<R> ic = V<R>(z, z, z);
   if (on) {
-    const R* kr = x.krow(k);
-    const R kc0 = kr[c], kc1 = kr[3 + c], kc2 = kr[6 + c];
-    k9 = kr[9]; k10 = kr[10]; k11 = kr[11];
-    const R* r = x.rec(k);
-    const int bb = x.pair(k);
-    const int b0 = x.B0(bb), b1 = x.B1(bb);
-    b = i == 0 ? b0 : b1;
-    o = x.list_index(k);
     fr = x.friction(o);
-    const quad<R> m = ld4(r + CR_CV);
-    nc = r[CR_N + c]; tyc = r[CR_TY + c]; tzc = r[CR_TZ + c];
-    const R* rel = r + (i == 0 ? CR_R0 : CR_R1);
-    rp = rel[p];
-    rq = rel[q];
-    if (b >= 0) {
-      const R* bd = x.body(b);
-      vel = bd[BR_VEL + c];
-      rot = bd[BR_ROT + c];
-      i0c = bd[BR_IIT + c]; i1c = bd[BR_IIT + 3 + c]; i2c = bd[BR_IIT + 6 + c];
-      im = bd[BR_INVM];
-    }
-    ddv = m.d;
     frictionless = fr == z;
     if (frictionless) {
       // calculateFrictionlessImpulse, contact.go:496-531 (rare: every lane)
+      const int b0 = x.B0(in.bb);
+      const R* r = x.rec(k);
       const v3<R> r0 = x.rel(0, k), n = V<R>(r[0], r[1], r[2]);
       v3<R> d = cross(r0, n);
       d = mulv(x.iit(b0), d);
       d = cross(d, r0);
       R dvel = dot(d, n);
       dvel += x.body(b0)[BR_INVM];
-      if (b1 < 0 && sl == 0) err |= ST_FRICTIONLESS_NIL;
-      ic = V<R>(ddv / dvel, z, z);
+      if (x.B1(in.bb) < 0 && sl == 0) err |= ST_FRICTIONLESS_NIL;
+      ic = V<R>(in.ddv / dvel, z, z);
     } else {
       // component c of K * (desired delta velocity, -vy, -vz) (mulv's row c)
-      icc = kc0 * ddv + kc1 * -m.b + kc2 * -m.c;
+      icc = in.k0 * in.ddv + in.k1 * -in.cvy + in.k2 * -in.cvz;
     }
   }
   {
     const R i0 = __shfl_sync(0xffffffffu, icc, 0, 4), i1 = __shfl_sync(0xffffffffu, icc, 1, 4);
     const R i2 = __shfl_sync(0xffffffffu, icc, 2, 4);
+    // the dynamic friction of contact.go:586-604, its two quotients by the
+    // planar length on two lanes
+    R planar = z;
+    bool slides = false;
     if (on && !frictionless) {
       ic = V<R>(i0, i1, i2);
-      // the dynamic friction of contact.go:586-604
-      const R planar = sqrt_<R>(ic.y * ic.y + ic.z * ic.z);
-      if (planar > ic.x * fr) {
-        ic.y /= planar;
-        ic.z /= planar;
-        ic.x = k9 + k10 * fr * ic.y + k11 * fr * ic.z;
-        ic.x = ddv / ic.x;
+      planar = sqrt_<R>(ic.y * ic.y + ic.z * ic.z);
+      slides = planar > ic.x * fr;
+    }
+    if (__any_sync(0xffffffffu, slides)) {
+      R part = z;
+      if (slides) part = (c == 2 ? ic.z : ic.y) / planar;
+      const R py = __shfl_sync(0xffffffffu, part, 1, 4), pz = __shfl_sync(0xffffffffu, part, 2, 4);
+      if (slides) {
+        ic.y = py;
+        ic.z = pz;
+        ic.x = in.k9 + in.k10 * fr * ic.y + in.k11 * fr * ic.z;
+        ic.x = in.ddv / ic.x;
         ic.y *= fr * ic.x;
         ic.z *= fr * ic.x;
       }
@@ -596,13 +653,13 @@ __device__ __forceinline__ void velocity_change(const RCtx<R, W, SM>& x, const B
   }
   // component c of the impulse contactToWorld * ic (mulv's row c)
   R impc = z;
-  if (on) impc = nc * ic.x + tyc * ic.y + tzc * ic.z;
+  if (on) impc = in.n * ic.x + in.ty * ic.y + in.tz * ic.z;
   const R ip = __shfl_sync(0xffffffffu, impc, p, 4), iq = __shfl_sync(0xffffffffu, impc, q, 4);
-  const bool act = on && b >= 0;
+  const bool act = on && in.b >= 0;
   // component c of cross(r0, imp) (body 0) or cross(imp, r1) (body 1)
   R crc = z;
   if (act) {
-    const R m1 = rp * iq, m2 = rq * ip;
+    const R m1 = in.rp * iq, m2 = in.rq * ip;
     crc = i == 0 ? m1 - m2 : m2 - m1;
   }
   const R cx = __shfl_sync(0xffffffffu, crc, 0, 4), cy = __shfl_sync(0xffffffffu, crc, 1, 4);
@@ -610,12 +667,12 @@ __device__ __forceinline__ void velocity_change(const RCtx<R, W, SM>& x, const B
   vc = rc = z;
   if (act) {
     // rc = iitWorld * cross (mulv's row c); vc = 0 + imp * (+-inverse mass)
-    rc = i0c * cx + i1c * cy + i2c * cz;
-    vc += impc * (i == 0 ? im : -im);
+    rc = in.i0 * cx + in.i1 * cy + in.i2 * cz;
+    vc += impc * (i == 0 ? in.im : -in.im);
     if (comp && sl < 8) {
-      R* bd = x.body(b);
-      bd[BR_VEL + c] = vel + vc;
-      bd[BR_ROT + c] = rot + rc;
+      R* bd = x.body(in.b);
+      bd[BR_VEL + c] = in.vel + vc;
+      bd[BR_ROT + c] = in.rot + rc;
     }
   }
 }
@@ -635,7 +692,7 @@ __device__ __forceinline__ int2 touching(int kb0, int kb1, int d0, int d1) {
 // The update of a contact after resolving a contact between bodies d0, d1:
 // its penetration (VEL false, contact.go:254-280) or contact velocity and
 // desired delta velocity (VEL true, contact.go:412-440).  update_load reads
-// what it needs of contact k (where `valid`), which the change of the resolved
+// what it needs of contact k with pair bb (where `valid`), which the change of the resolved
 // contact does not touch, so the caller loads ahead of computing that change;
 // update_apply takes the change, of which lanes 4d + c of the group of L lanes
 // hold component c of resolved body d's, and returns the value the argmax
@@ -650,14 +707,14 @@ template <class R> struct Touched {
   quad<R> q0, q1, q2, q3, m;  // the record: basis, relative positions, penetration or frame velocity; cv, ddv
 };
 template <bool VEL, class R, class W, bool SM>
-__device__ __forceinline__ void update_load(const RCtx<R, W, SM>& x, Touched<R>& t, int k, bool valid, int d0, int d1) {
+__device__ __forceinline__ void update_load(const RCtx<R, W, SM>& x, Touched<R>& t, int k, int bb, bool valid, int d0,
+                                            int d1) {
   t.k = k;
   t.valid = valid;
   t.e = make_int2(-1, -1);
-  t.bb = 0;
+  t.bb = bb;
   t.m = t.q3 = quad<R>{(R)0, (R)0, (R)0, (R)0};
   if (!valid) return;
-  t.bb = x.pair(k);
   t.e = touching(x.B0(t.bb), x.B1(t.bb), d0, d1);
   const R* r = x.rec(k);
   if (VEL) t.m = ld4(r + CR_CV);
@@ -672,45 +729,44 @@ __device__ __forceinline__ R update_apply(const RCtx<R, W, SM>& x, Touched<R>& t
   const bool hit = t.e.x >= 0 || t.e.y >= 0, both = t.e.x >= 0 && t.e.y >= 0;
   R value = VEL ? t.m.d : t.q3.d;
   if (!__any_sync(0xffffffffu, hit)) return value;
-  const int s1 = 4 * ((t.e.x >= 0 ? t.e.x : t.e.y) > 0);
-  const v3<R> dl = V<R>(__shfl_sync(0xffffffffu, lin, s1, L), __shfl_sync(0xffffffffu, lin, s1 + 1, L),
-                        __shfl_sync(0xffffffffu, lin, s1 + 2, L));
-  const v3<R> da = V<R>(__shfl_sync(0xffffffffu, ang, s1, L), __shfl_sync(0xffffffffu, ang, s1 + 1, L),
-                        __shfl_sync(0xffffffffu, ang, s1 + 2, L));
-  const bool first0 = t.e.x >= 0;  // the first change is contact body 0's
   const m3<R> C{{t.q0.a, t.q0.b, t.q0.c, t.q0.d, t.q1.a, t.q1.b, t.q1.c, t.q1.d, t.q2.a}};
   const v3<R> n = V<R>(t.q0.a, t.q0.b, t.q0.c);
-  if (hit) {
-    v3<R> dv = cross(da, first0 ? V<R>(t.q2.b, t.q2.c, t.q2.d) : V<R>(t.q3.a, t.q3.b, t.q3.c));
+  const bool first0 = t.e.x >= 0;  // the first change is contact body 0's
+  // the change of resolved body d at relative position r, in the contact's terms
+  auto from = [&](int d) { return V<R>(__shfl_sync(0xffffffffu, lin, d, L), __shfl_sync(0xffffffffu, lin, d + 1, L),
+                                       __shfl_sync(0xffffffffu, lin, d + 2, L)); };
+  auto turn = [&](int d) { return V<R>(__shfl_sync(0xffffffffu, ang, d, L), __shfl_sync(0xffffffffu, ang, d + 1, L),
+                                       __shfl_sync(0xffffffffu, ang, d + 2, L)); };
+  auto moved = [&](const v3<R>& dl, const v3<R>& da, const v3<R>& r) {
+    v3<R> dv = cross(da, r);
     add(dv, dl);
+    if constexpr (VEL) return mulv_t(C, dv);
+    else return V<R>(dot(dv, n), (R)0, (R)0);
+  };
+  const int s1 = 4 * ((t.e.x >= 0 ? t.e.x : t.e.y) > 0);
+  const v3<R> dl = from(s1), da = turn(s1);
+  const v3<R> r1 = V<R>(t.q3.a, t.q3.b, t.q3.c);
+  const v3<R> rf = first0 ? V<R>(t.q2.b, t.q2.c, t.q2.d) : r1;
+  auto apply = [&](const v3<R>& a, bool plus) {
     if constexpr (VEL) {
-      const v3<R> a = mulv_t(C, dv);
-      t.m.a = first0 ? t.m.a + a.x : t.m.a - a.x;
-      t.m.b = first0 ? t.m.b + a.y : t.m.b - a.y;
-      t.m.c = first0 ? t.m.c + a.z : t.m.c - a.z;
+      t.m.a = plus ? t.m.a + a.x : t.m.a - a.x;
+      t.m.b = plus ? t.m.b + a.y : t.m.b - a.y;
+      t.m.c = plus ? t.m.c + a.z : t.m.c - a.z;
     } else {
-      const R a = dot(dv, n);
-      value = first0 ? value - a : value + a;
+      value = plus ? value - a.x : value + a.x;
     }
-  }
+  };
   if (__any_sync(0xffffffffu, both)) {
+    // both terms at once (independent until they are added, in order)
     const int s2 = 4 * (t.e.y > 0);
-    const v3<R> dl2 = V<R>(__shfl_sync(0xffffffffu, lin, s2, L), __shfl_sync(0xffffffffu, lin, s2 + 1, L),
-                           __shfl_sync(0xffffffffu, lin, s2 + 2, L));
-    const v3<R> da2 = V<R>(__shfl_sync(0xffffffffu, ang, s2, L), __shfl_sync(0xffffffffu, ang, s2 + 1, L),
-                           __shfl_sync(0xffffffffu, ang, s2 + 2, L));
-    if (both) {
-      v3<R> dv = cross(da2, V<R>(t.q3.a, t.q3.b, t.q3.c));
-      add(dv, dl2);
-      if constexpr (VEL) {
-        const v3<R> a = mulv_t(C, dv);
-        t.m.a -= a.x;
-        t.m.b -= a.y;
-        t.m.c -= a.z;
-      } else {
-        value += dot(dv, n);
-      }
+    const v3<R> dl2 = from(s2), da2 = turn(s2);
+    if (hit) {
+      const v3<R> a = moved(dl, da, rf), a2 = moved(dl2, da2, r1);
+      apply(a, first0);
+      if (both) apply(a2, false);
     }
+  } else if (hit) {
+    apply(moved(dl, da, rf), first0);
   }
   if (hit) {
     R* r = x.rec(t.k);
@@ -724,6 +780,59 @@ __device__ __forceinline__ R update_apply(const RCtx<R, W, SM>& x, Touched<R>& t
     }
   }
   return value;
+}
+
+// The same update (update_load and update_apply) of contact k with pair bb by
+// four lanes, lane c (of 4) the component c of the change and of the contact
+// velocity: for the float64 form, whose update is bound by the number of
+// float64 instructions, where a group has lanes to spare (14 or, with both
+// bodies touched, 24 of them for L / 4 contacts, against 34 or 64 for L).
+template <bool VEL, class R, class W, bool SM>
+__device__ __forceinline__ void update_spread(const RCtx<R, W, SM>& x, int k, int bb, bool valid, int d0, int d1, R lin,
+                                              R ang, int L, bool woke) {
+  const R z = (R)0;
+  const int c4 = threadIdx.x & 3, c = c4 != 3 ? c4 : 0;
+  const int p = c == 2 ? 0 : c + 1, q = c == 0 ? 2 : c - 1;
+  const int2 e = valid ? touching(x.B0(bb), x.B1(bb), d0, d1) : make_int2(-1, -1);
+  const bool both = e.x >= 0 && e.y >= 0, first0 = e.x >= 0;
+  R r0p = z, r0q = z, r1p = z, r1q = z, col0 = z, col1 = z, col2 = z, m = z, vfa = z;
+  if (valid) {
+    const R* r = x.rec(k);
+    r0p = r[CR_R0 + p]; r0q = r[CR_R0 + q];
+    r1p = r[CR_R1 + p]; r1q = r[CR_R1 + q];
+    const R* col = r + CR_N + (VEL ? 3 * c : 0);
+    col0 = col[0]; col1 = col[1]; col2 = col[2];
+    m = VEL ? r[CR_CV + c] : r[CR_PEN];
+    if (VEL) vfa = r[CR_VFA];
+  }
+  auto term = [&](int d, R rp, R rq) {
+    const R ap = __shfl_sync(0xffffffffu, ang, d + p, L), aq = __shfl_sync(0xffffffffu, ang, d + q, L);
+    const R dv = ap * rq - aq * rp + __shfl_sync(0xffffffffu, lin, d + c, L);
+    const R x0 = __shfl_sync(0xffffffffu, dv, 0, 4), x1 = __shfl_sync(0xffffffffu, dv, 1, 4);
+    const R x2 = __shfl_sync(0xffffffffu, dv, 2, 4);
+    return x0 * col0 + x1 * col1 + x2 * col2;
+  };
+  const R t = term(4 * ((e.x >= 0 ? e.x : e.y) > 0), first0 ? r0p : r1p, first0 ? r0q : r1q);
+  // a velocity takes body 0's term and gives body 1's back, a penetration the other way round
+  m = first0 == VEL ? m + t : m - t;
+  if (__any_sync(0xffffffffu, both)) {
+    const R t2 = term(4 * (e.y > 0), r1p, r1q);
+    if (both) m = VEL ? m - t2 : m + t2;
+  }
+  if (valid) {
+    R* r = x.rec(k);
+    if (VEL) {
+      if (woke) vfa = frame_velocity(x, x.B0(bb), x.B1(bb), V<R>(r[0], r[1], r[2]));
+      if (c4 < 3) r[CR_CV + c] = m;
+      const R value = desired_dv(m, vfa, x.restitution(SM ? (int)((unsigned)bb >> 16) : k));
+      if (c4 == 0) {
+        if (woke) r[CR_VFA] = vfa;
+        r[CR_DDV] = value;
+      }
+    } else if (c4 == 0) {
+      r[CR_PEN] = m;
+    }
+  }
 }
 
 // A world's bodies from the batch rows into the records of x, by the `step`
@@ -1321,12 +1430,19 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
     const int d0 = have ? x.B0(bb) : -2, d1 = have ? x.B1(bb) : -2;
     R lin, ang;
     bool woke = false;
+    const bool mine = have && sl < 8;
     auto change = [&]() {
+      // (loaded here: held across the first update_load they would spill)
+      std::conditional_t<VEL, VelocityIn<R>, PositionIn<R, W>> in;
+      if constexpr (VEL)
+        velocity_load(x, in, k, bb, mine, sl);
+      else
+        position_load(x, in, k, bb, mine, sl);
       woke = match_awake(x, bb, have, sl == 0);
       if constexpr (VEL)
-        velocity_change<R, W, LEARN>(x, v, k, have && sl < 8, sl, lin, ang, err);
+        velocity_change<R, W, LEARN>(x, v, in, k, mine, sl, lin, ang, err);
       else
-        position_change(x, v, bstart, k, have && sl < 8, sl, lin, ang);
+        position_change(x, v, in, bstart, mine, sl, lin, ang);
     };
     if constexpr (kGather) {
       change();
@@ -1346,11 +1462,20 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
         if (__any_sync(FULL, m > cap - L) || base + L >= len) {
           __syncwarp();
           const int mm = (int)__reduce_max_sync(FULL, (unsigned)m);
+          if (L > kIslandLanes && mm <= L / 2) {
 #pragma unroll 1
-          for (int q = sl; q - sl < mm; q += L) {
-            Touched<R> t;
-            update_load<VEL>(x, t, q < m ? ml[q] : 0, q < m, d0, d1);
-            update_apply<VEL>(x, t, lin, ang, L, woke);
+            for (int q = sl >> 2; q - (sl >> 2) < mm; q += L / 4) {
+              const int j = q < m ? ml[q] : 0;
+              update_spread<VEL>(x, j, q < m ? x.pair(j) : 0, q < m, d0, d1, lin, ang, L, woke);
+            }
+          } else {
+#pragma unroll 1
+            for (int q = sl; q - sl < mm; q += L) {
+              Touched<R> t;
+              const int j = q < m ? ml[q] : 0;
+              update_load<VEL>(x, t, j, q < m ? x.pair(j) : 0, q < m, d0, d1);
+              update_apply<VEL>(x, t, lin, ang, L, woke);
+            }
           }
           __syncwarp();
           m = 0;
@@ -1364,7 +1489,9 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
       for (int base = 0; base < len; base += L) {
         // the first contacts' records load while the change is computed
         Touched<R> t;
-        update_load<VEL>(x, t, s + base + sl, have && s + base + sl < e, d0, d1);
+        const int j = s + base + sl;
+        const bool valid = have && j < e;
+        update_load<VEL>(x, t, j, valid ? x.pair(j) : 0, valid, d0, d1);
         if (base == 0) change();
         const R value = update_apply<VEL>(x, t, lin, ang, L, woke);
         if (t.valid) consider(t.k, t.bb, value);

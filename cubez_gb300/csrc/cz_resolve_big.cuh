@@ -5,9 +5,9 @@
 // one chain, and what counts is the latency of an iteration.
 //   * Body and contact records are in global memory (L1/L2); a record is two
 //     cache lines at most, where rows took a line per value.
-//   * The argmax is over chunk maxima in shared memory (at most kBigChunks),
-//     kept by refreshing the chunks of the contacts an iteration changed,
-//     instead of a scan over every contact's value.
+//   * The argmax is over two levels of chunk maxima in shared memory, kept by
+//     refreshing the chunks of the contacts an iteration changed, instead of a
+//     scan over every contact's value.
 //   * After prepareContacts every body gets the list of its contacts (counting
 //     sort by body), so the update after each resolved contact visits only the
 //     contacts of the two resolved bodies: the reference's loop over every
@@ -24,36 +24,82 @@
 namespace cz {
 
 constexpr int kBigChunks = 512;  // chunks of a world's contacts (16 each up to 8192 contacts)
+constexpr int kBigTops = kBigChunks / 16;  // groups of 16 chunks: one per lane
 
-// shared memory ahead of the per-contact arrays: chunk maxima and their first
-// contacts, list starts and ends of n bodies
+// shared memory ahead of the per-contact arrays: maxima and their contacts of
+// the chunks and of the groups of chunks, list starts and ends of n bodies
 template <class R> __host__ __device__ inline size_t big_fixed_bytes(int n) {
-  return (size_t)kBigChunks * (sizeof(R) + sizeof(int)) + (size_t)2 * ((n + 3) & ~3) * sizeof(int);
+  return (size_t)(kBigChunks + kBigTops) * (sizeof(R) + sizeof(int)) + (size_t)2 * ((n + 3) & ~3) * sizeof(int);
 }
 // per contact: key, packed bodies, two list entries
 template <class R> __host__ __device__ constexpr size_t big_contact_bytes() { return sizeof(R) + 3 * sizeof(int); }
 
-// The chunk maxima of a world's keys and the first contact holding each.
+__device__ __forceinline__ void prefetch_line(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+// The first maximum of 16 consecutive keys (16-byte aligned): adjacent pairs,
+// so that the left one of equals is the earlier.
+template <class Key> __device__ __forceinline__ void first_max16(const Key* p, Key& best, int& at) {
+  constexpr int V = 16 / (int)sizeof(Key);
+  union {
+    uint4 v[16 / V];
+    Key k[16];
+  } u;
+#pragma unroll
+  for (int i = 0; i < 16 / V; ++i) u.v[i] = reinterpret_cast<const uint4*>(p)[i];
+  int ix[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) ix[i] = i;
+#pragma unroll
+  for (int w = 8; w > 0; w >>= 1)
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const bool right = u.k[2 * i + 1] > u.k[2 * i];
+      u.k[i] = right ? u.k[2 * i + 1] : u.k[2 * i];
+      ix[i] = right ? ix[2 * i + 1] : ix[2 * i];
+    }
+  best = u.k[0];
+  at = ix[0];
+}
+
+// The maxima of a world's keys by chunk and by group of 16 chunks, with the
+// first contact holding each: the world's argmax is one load per lane and the
+// warp reductions.
 template <class Key> struct BigKeys {
-  Key* key;     // [C]
-  Key* cmax;    // [kBigChunks]
-  int* cfirst;  // [kBigChunks]
+  Key* key;      // [C], zeros up to a whole chunk where `padded`
+  Key* cmax;     // [kBigChunks] (zeros beyond the last chunk)
+  int* cfirst;   // [kBigChunks]
+  Key* tmax;     // [kBigTops]
+  int* tfirst;   // [kBigTops]
   int C, shift;  // chunk of contact k: k >> shift
-  // the chunk's first maximum again, by one lane
-  __device__ __forceinline__ void refresh(int ch) const {
-    const int k0 = ch << shift, k1 = min(C, k0 + (1 << shift));
+  bool padded;   // chunks of 16, whole
+  // a chunk's first maximum again, by one lane
+  __device__ __forceinline__ void refresh_chunk(int ch) const {
     Key best = 0;
-    int at = k0;
-#pragma unroll 4
-    for (int k = k0; k < k1; ++k) {
-      const Key q = key[k];
-      if (q > best) {
-        best = q;
-        at = k;
+    int at = 0;
+    const int k0 = ch << shift;
+    if (padded) {
+      first_max16(key + k0, best, at);
+      at += k0;
+    } else {
+      const int k1 = min(C, k0 + (1 << shift));
+#pragma unroll 1
+      for (int k = k0; k < k1; ++k) {
+        const Key q = key[k];
+        if (q > best) {
+          best = q;
+          at = k;
+        }
       }
     }
     cmax[ch] = best;
     cfirst[ch] = at;
+  }
+  __device__ __forceinline__ void refresh_top(int t) const {
+    Key best;
+    int at;
+    first_max16(cmax + 16 * t, best, at);
+    tmax[t] = best;
+    tfirst[t] = cfirst[16 * t + at];
   }
 };
 
@@ -65,59 +111,73 @@ __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const Batch
                                          int max_it, uint32_t& err) {
   const int lane = threadIdx.x;
   const int C = bk.C;
-  const int nch = (C + (1 << bk.shift) - 1) >> bk.shift;
   for (int k = lane; k < C; k += 32) bk.key[k] = key_of(x.rec(k)[VEL ? CR_DDV : CR_PEN], (R)0.01);
+  if (bk.padded && C + lane < ((C + 15) & ~15)) bk.key[C + lane] = 0;
   __syncwarp();
-  for (int ch = lane; ch < nch; ch += 32) bk.refresh(ch);
+  const int nch = (C + (1 << bk.shift) - 1) >> bk.shift;
+  for (int ch = lane; ch < kBigChunks; ch += 32) {
+    if (ch < nch) {
+      bk.refresh_chunk(ch);
+    } else {
+      bk.cmax[ch] = 0;
+      bk.cfirst[ch] = 0;
+    }
+  }
+  __syncwarp();
+  bk.refresh_top(lane);
   __syncwarp();
   int used = 0;
   while (used < max_it) {
-    Key best = 0;
-    int ch = 0x7fffffff;
-    for (int c = lane; c < nch; c += 32) {
-      const Key q = bk.cmax[c];
-      if (q > best) {
-        best = q;
-        ch = c;
-      }
-    }
-    warp_first_max(best, ch);
+    Key best = bk.tmax[lane];
+    int k = bk.tfirst[lane];
+    warp_first_max(best, k);
     if (best == 0) break;
-    const int k = bk.cfirst[ch];
     const int bb = x.pair(k);
     const int d0 = x.B0(bb), d1 = x.B1(bb);
     const int o0 = off[d0], l0 = end[d0] - o0;
     const int o1 = d1 >= 0 ? off[d1] : 0, l1 = d1 >= 0 ? end[d1] - o1 : 0;
     // this lane's contact of the two bodies' lists (32 at a time); one that
     // touches both bodies is visited in d0's list
+    int q, qb;
     auto entry = [&](int e) {
-      if (e >= l0 + l1) return -1;
-      const int q = e < l0 ? adj[o0 + e] : adj[o1 + e - l0];
-      if (e >= l0) {
-        const int qb = x.pair(q);
-        if (x.B0(qb) == d0 || x.B1(qb) == d0) return -1;
-      }
-      return q;
+      q = -1;
+      qb = 0;
+      if (e >= l0 + l1) return;
+      q = e < l0 ? adj[o0 + e] : adj[o1 + e - l0];
+      qb = x.pair(q);
+      if (e >= l0 && (x.B0(qb) == d0 || x.B1(qb) == d0)) q = -1;
     };
-    // its record loads while the resolved contact's change is computed
+    entry(lane);
+    // what the change needs, then the touched records: they load while the
+    // change is computed
+    std::conditional_t<VEL, VelocityIn<R>, PositionIn<R, W>> in;
+    if constexpr (VEL)
+      velocity_load(x, in, k, bb, lane < 8, lane);
+    else
+      position_load(x, in, k, bb, lane < 8, lane);
     Touched<R> t;
-    const int q = entry(lane);
-    update_load<VEL>(x, t, q, q >= 0, d0, d1);
+    update_load<VEL>(x, t, q, qb, q >= 0, d0, d1);
     const bool woke = match_awake(x, bb, true, lane == 0);
     R lin, ang;
     if constexpr (VEL)
-      velocity_change<R, W, false>(x, v, k, lane < 8, lane, lin, ang, err);
+      velocity_change<R, W, false>(x, v, in, k, lane < 8, lane, lin, ang, err);
     else
-      position_change(x, v, bstart, k, lane < 8, lane, lin, ang);
+      position_change(x, v, in, bstart, lane < 8, lane, lin, ang);
     for (int base = 0; base < l0 + l1; base += 32) {
       if (base > 0) {
-        const int r = entry(base + lane);
-        update_load<VEL>(x, t, r, r >= 0, d0, d1);
+        entry(base + lane);
+        update_load<VEL>(x, t, q, qb, q >= 0, d0, d1);
       }
       const R value = update_apply<VEL>(x, t, lin, ang, 32, woke);
-      if (t.valid) bk.key[t.k] = key_of(value, (R)0.01);
+      if (t.valid) {
+        bk.key[t.k] = key_of(value, (R)0.01);
+        // the next contact to resolve is mostly one of these
+        if (VEL) prefetch_line(x.krow(t.k));
+      }
       __syncwarp();
-      if (t.valid) bk.refresh(t.k >> bk.shift);  // lanes of one chunk find the same
+      if (t.valid) bk.refresh_chunk(t.k >> bk.shift);  // lanes of one chunk find the same
+      __syncwarp();
+      if (t.valid) bk.refresh_top(t.k >> bk.shift >> 4);
       __syncwarp();
     }
     ++used;
@@ -125,33 +185,25 @@ __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const Batch
   return used;
 }
 
-template <class R, class W>
-__global__ void __launch_bounds__(32, 4) k_resolve_big(BatchView<R> v, R dt, int csm) {
+// One world of C contacts by its warp.  TILE: its per-contact arrays are in
+// shared memory, which the compiler then knows (csm: their capacity).
+template <class R, class W, bool TILE>
+__device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, int w, int C, unsigned char* smem) {
   using Key = decltype(key_of((R)0, (R)0));
-  extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x;
-  const int w = v.big_list[blockIdx.x];
   const int n = v.body_count[w];
   const int bstart = v.body_start[w];
   const long long cst = v.contact_start[w];
-  int C = v.contact_count[w];
-  if (C > v.contact_cap[w]) C = v.contact_cap[w];  // the world is already flagged ST_CAPACITY
-  if (C <= 0 || dt <= (R)0) {                      // ResolveContacts guards, contact.go:210-212
-    if (lane == 0) {
-      v.pos_iters[w] = 0;
-      v.vel_iters[w] = 0;
-      atomicAdd(&v.counters[3], (unsigned long long)C);
-    }
-    return;
-  }
   BigKeys<Key> bk;
   bk.C = C;
   bk.shift = 4;
   while (((C - 1) >> bk.shift) >= kBigChunks) ++bk.shift;
   bk.cmax = reinterpret_cast<Key*>(smem);
-  bk.cfirst = reinterpret_cast<int*>(bk.cmax + kBigChunks);
+  bk.tmax = bk.cmax + kBigChunks;
+  bk.cfirst = reinterpret_cast<int*>(bk.tmax + kBigTops);
+  bk.tfirst = bk.cfirst + kBigChunks;
   // list starts and ends (first the counts, then the fill cursors)
-  int* off = bk.cfirst + kBigChunks;
+  int* off = bk.tfirst + kBigTops;
   int* end = off + ((n + 3) & ~3);
   unsigned char* tile = reinterpret_cast<unsigned char*>(end + ((n + 3) & ~3));
   RCtx<R, W, false> x;
@@ -168,7 +220,8 @@ __global__ void __launch_bounds__(32, 4) k_resolve_big(BatchView<R> v, R dt, int
   x.wst = x.jst = 0;
   x.kw = v.kmat + cst * K_ROW;
   int* adj;
-  if (C <= csm) {
+  bk.padded = TILE;
+  if (TILE) {
     bk.key = reinterpret_cast<Key*>(tile);
     x.cb = reinterpret_cast<int*>(bk.key + csm);
     adj = x.cb + csm;
@@ -236,6 +289,25 @@ __global__ void __launch_bounds__(32, 4) k_resolve_big(BatchView<R> v, R dt, int
   if (v.contact_writeback)
     for (int k = lane; k < C; k += 32) write_back_contact(x, v, cst, k);
   store_bodies(x, v, bstart, n, lane, 32);
+}
+
+template <class R, class W>
+__global__ void __launch_bounds__(32, 4) k_resolve_big(BatchView<R> v, R dt, int csm) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int w = v.big_list[blockIdx.x];
+  int C = v.contact_count[w];
+  if (C > v.contact_cap[w]) C = v.contact_cap[w];  // the world is already flagged ST_CAPACITY
+  if (C <= 0 || dt <= (R)0) {                      // ResolveContacts guards, contact.go:210-212
+    if (threadIdx.x == 0) {
+      v.pos_iters[w] = 0;
+      v.vel_iters[w] = 0;
+      atomicAdd(&v.counters[3], (unsigned long long)C);
+    }
+  } else if (C <= csm && C <= 16 * kBigChunks) {
+    big_world<R, W, true>(v, dt, csm, w, C, smem);
+  } else {
+    big_world<R, W, false>(v, dt, csm, w, C, smem);
+  }
 }
 
 }  // namespace cz
