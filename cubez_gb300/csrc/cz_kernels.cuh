@@ -147,6 +147,33 @@ template <class R> struct SatResult {
 };
 constexpr int kSatApart = -1;
 
+// penetrationOnAxis, colliders.go:445-456, of two boxes whose centres are tc apart
+template <class R>
+__device__ __forceinline__ R axis_penetration(const xf<R>& t1, const v3<R>& h1, const xf<R>& t2, const v3<R>& h2,
+                                              const v3<R>& tc, v3<R> axis) {
+  normalize(axis);
+  const R one = transform_to_axis(t1, h1, axis);
+  const R two = transform_to_axis(t2, h2, axis);
+  const R dist = fabs_<R>(dot(tc, axis));
+  return one + two - dist;
+}
+
+// Whether one of box i1's own axes separates the boxes: the first three of
+// their axes, by one lane.
+template <class R> __device__ __forceinline__ bool sat_apart_first(const NPTile<R>& tl, int i1, int i2) {
+  const xf<R> t1 = tl.xform(i1), t2 = tl.xform(i2);
+  const v3<R> h1 = tl.half(i1), h2 = tl.half(i2);
+  v3<R> tc = t2.axis(3);
+  sub(tc, t1.axis(3));
+  bool apart = false;
+#pragma unroll 1
+  for (int q = 0; q < 3 && !apart; ++q) {
+    const v3<R> axis = tl.axis(i1, q);
+    apart = !(sqmag(axis) < Lim<R>::eps()) && axis_penetration(t1, h1, t2, h2, tc, axis) < (R)0;
+  }
+  return apart;
+}
+
 // tryAxis (colliders.go:458-477) for the fifteen axes of a pair of boxes, an
 // axis per lane of a group of 16 (l = 0..15), the smallest penetration (the
 // first of equal ones, as the reference's loop keeps) by shuffles.  Every lane
@@ -170,13 +197,7 @@ __device__ __forceinline__ SatResult<R> sat_axes(const NPTile<R>& tl, int i1, in
   sub(tc, t1.axis(3));
   R p = (R)0;
   bool tried = l < 15 && !(sqmag(axis) < Lim<R>::eps());
-  if (tried) {
-    normalize(axis);
-    const R one = transform_to_axis(t1, h1, axis);
-    const R two = transform_to_axis(t2, h2, axis);
-    const R dist = fabs_<R>(dot(tc, axis));
-    p = one + two - dist;  // penetrationOnAxis, colliders.go:445-456
-  }
+  if (tried) p = axis_penetration(t1, h1, t2, h2, tc, axis);
   SatResult<R> r;
   r.pen = (R)0;
   r.code = kSatApart;
@@ -709,7 +730,21 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
     }
     perm[dst] = tid;
     __syncthreads();
-    // cube pairs: an axis per lane
+    // Cube pairs: an axis per lane.  With Offsets, cubes whose Offset is not
+    // rigid are never culled and most of their pairs are apart: where there are
+    // more than two passes, a lane per pair tries three axes first (1000 worlds
+    // of 31 bodies, float32: 54 -> 41 us; without Offsets the culls leave near
+    // pairs, and 8192 x 32 settled bodies took 187 us with it, 175 without).
+    const bool pre = v.offset != nullptr && n4 > bd >> 3;
+    if (pre) {
+      if (tid < n4) {
+        const int at = perm[n0 + n1 + n23 + tid];
+        const int uu = surv[sb + at];
+        const int i = uu / n, k = uu - i * n;
+        satc[at] = sat_apart_first(tl, i, k - 1 >= i ? k : k - 1) ? kSatApart : 0;
+      }
+      __syncthreads();
+    }
 #pragma unroll 1
     for (int g = tid >> 4; g < ((n4 + 1) & ~1); g += bd >> 4) {  // both groups of a warp together
       const bool on = g < n4;
@@ -719,12 +754,13 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
       const int j = k - 1 >= i ? k : k - 1;
       // (i, j) with i > j takes the outcome of (j, i) where the chunk has it
       int other = -1;
-      if (on && i > j)
+      const bool apart = pre && satc[at] == kSatApart;
+      if (on && i > j && !apart)
         for (int q = l; q < m; q += 16)
           if (surv[sb + q] == j * n + i) other = q;  // j's k is i: i > j
       const unsigned have = __ballot_sync(FULL, other >= 0) & (0xFFFFu << (lane & 16));
       other = __shfl_sync(FULL, other, have ? __ffs(have) - 1 : lane);
-      const bool need = on && !have;
+      const bool need = on && !have && !apart;
       if (__any_sync(FULL, need)) {
         const SatResult<R> r = sat_axes(tl, i, j, l);
         if (need && l == 0) {
@@ -734,7 +770,9 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
       }
       if (on && l == 0) satr[at] = have ? other : at;
     }
-    // half-space with a cube: a vertex per lane, kept by the last pass
+    // half-space with a cube: a vertex per lane; in float64 the last pass keeps
+    // its contacts (in float32 they are computed again: held, they cost a CTA per SM)
+    constexpr bool kKeep = sizeof(R) == 8;
     NPContact<R> vc;
     bool vhit = false;
     const int passes = (8 * n1 + bd - 1) / bd;
@@ -784,7 +822,7 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
       const int g = (q * bd + tid) >> 3;
       if (g < n1) {
         const int at = perm[n0 + g];
-        if (q < passes - 1) vhit = plane_vertex(tl, surv[sb + at] / n, tid & 7, v, vc);
+        if (!kKeep || q < passes - 1) vhit = plane_vertex(tl, surv[sb + at] / n, tid & 7, v, vc);
         if (vhit) np_emit<R>(v, cs, cap, out + cntb[at] + __popc((unsigned)satr[at] & ((1u << (tid & 7)) - 1u)), vc);
       }
     }
@@ -1071,11 +1109,12 @@ __device__ void np_world(const NPTile<R>& tl, const BatchView<R>& v, int w, int 
 
 // GRID = false compiles the all-pairs path alone (worlds too small for the
 // grid), so its registers and occupancy stay those of that path; in float32
-// it is bounded to 80 registers (6 CTAs of 128 threads per SM; a few registers
-// spill): 0.190 ms for 8192 worlds of 32 bodies, against 0.200 with 64 (320
-// bytes spilled) and 0.201 with 109 (no spills, 4 CTAs).
+// it is bounded to 64 registers (8 CTAs of 128 threads per SM; 240 bytes
+// spilled): with few contacts a world is a chain of staging and barriers, and
+// 16384 worlds of 14 bodies took 155 us against 178 with 80 registers (6 CTAs);
+// 8192 worlds of 32 settled bodies 175 against 170, and 200 unbounded.
 template <class R, bool GRID>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 && !GRID ? 3 : 0) k_narrowphase(BatchView<R> v, int nbs) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 && !GRID ? 4 : 0) k_narrowphase(BatchView<R> v, int nbs) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem);
   NPTile<R> tl;
