@@ -837,14 +837,16 @@ __device__ __forceinline__ void update_spread(const RCtx<R, W, SM>& x, int k, in
 
 // A world's bodies from the batch rows into the records of x, by the `step`
 // lanes of a group (lane index `first`).
-// Returns whether this lane's bodies are all awake.
+// Returns whether this lane's bodies are all awake.  With `lab`, all but the
+// bodies of label `keep`.
 template <class R, class W, bool SM>
 __device__ __forceinline__ bool load_bodies(const RCtx<R, W, SM>& x, const BatchView<R>& v, long long bstart, int n,
-                                            int first, int step) {
+                                            int first, int step, const uint8_t* lab = nullptr, int keep = -1) {
   const long long S = v.nb_pad;
   bool awake = true;
 #pragma unroll 1
   for (int i = first; i < n; i += step) {
+    if (lab && lab[i] == keep) continue;
     const R* g = v.body + bstart + i;
     auto F = [&](int r) { return g[(long long)r * S]; };
     x.P(0, i) = (W)F(B_PX); x.P(1, i) = (W)F(B_PY); x.P(2, i) = (W)F(B_PZ);
@@ -1336,26 +1338,45 @@ struct Progress {
   int rounds;  // rounds this world took part in
   bool over;   // the world wants more than max_it iterations
 };
+template <class R> using KeyOf = decltype(key_of((R)0, (R)0));
+// What a phase runs: the records [s, e) as one list for all lanes (`list`), or
+// the islands, leaving out the one that starts at record s; each until its
+// first value's key is below `stop`.
+template <class Key> struct Span {
+  bool list;
+  int s, e;
+  Key stop;
+};
+// Of the islands under way when the budget ended, the one to go on from: its
+// records, its iterations, and the smallest key among theirs and its next, the
+// largest of the islands'.  tie: some list met a first value of key Span::stop.
+template <class Key> struct Resume {
+  Key stop;
+  int s, e, its;
+  bool tie;
+};
 template <class R, class W, int G, bool VEL, bool LEARN>
-__device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, const BatchView<R>& v, int bstart, int C,
-                                                  int gl, int max_it, bool run, bool whole, int ni,
-                                                  const uint16_t* ist, int* ml_world, uint32_t& err) {
-  using Key = decltype(key_of((R)0, (R)0));
+__device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, const BatchView<R>& v, int bstart, int gl,
+                                                  int max_it, bool run, Span<KeyOf<R>> sp, int ni, const uint16_t* ist,
+                                                  int* ml_world, uint32_t& err, Resume<KeyOf<R>>& rs) {
+  using Key = KeyOf<R>;
+  constexpr bool kResume = G == 32;
   constexpr bool kGather = gathers_updates<R>();
   constexpr int kValue = VEL ? CR_DDV : CR_PEN;
   const int lane = threadIdx.x & 31;
   const unsigned wmask = G == 32 ? FULL : (((1u << G) - 1u) << (lane - gl));
   Progress pr{0, 0, false};
-  int L = G, sl = gl, s = 0, e = C, next = 0, len = 0, cap = kTouchList;
+  int L = G, sl = gl, s = sp.s, e = sp.e, next = 0, len = 0, cap = kTouchList, its = 0;
+  Key low = ~(Key)0;  // smallest key of the island's iterations
   unsigned lmask = wmask;
   int* ml = ml_world;
-  if (G > kIslandLanes && !whole) {
+  if (G > kIslandLanes && !sp.list) {
     L = kIslandLanes;
     sl = gl % L;
     lmask = 0xFFu << (lane - sl);
     cap = kTouchList / (G / L);
     ml = ml_world + gl / L * cap;
-    e = 0;  // no island yet: the first round's maxima are zero
+    s = e = 0;  // no island yet: the first round's maxima are zero
   } else {
     ni = 0;
   }
@@ -1387,17 +1408,20 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
     else
       group_first_max<G>(best, bidx);
     const unsigned leaders = __ballot_sync(FULL, sl == 0) & wmask;
-    const bool fin = have && best == 0;
+    const bool fin = have && best < sp.stop;
     const unsigned done = __ballot_sync(FULL, fin);
     if (done) {
       const unsigned m = done & leaders;
       if (fin) {  // the next island, in the order of the groups
-        const int isl = next + __popc(m & ((1u << (lane - sl)) - 1u));
+        int isl = next + __popc(m & ((1u << (lane - sl)) - 1u));
         have = isl < ni;
         if (have) {
+          if (kResume && ist[isl] >= sp.s) ++isl;
           s = ist[isl];
           e = ist[isl + 1];
         }
+        its = 0;
+        low = ~(Key)0;
         scan = true;
       }
       next += __popc(m);
@@ -1412,6 +1436,10 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
       const int from = held ? __ffs(held) - 1 : lane;
       s = __shfl_sync(FULL, s, from);
       e = __shfl_sync(FULL, e, from);
+      if (kResume) {
+        its = __shfl_sync(FULL, its, from);
+        low = __shfl_sync(FULL, low, from);
+      }
       have = held != 0;
       L = G;
       sl = gl;
@@ -1421,7 +1449,27 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
       scan = true;
       continue;
     }
-    if (act && pr.used + act > max_it) pr.over = true;
+    if (kResume) {
+      rs.tie = rs.tie || (have && best == sp.stop);
+      low = best < low ? best : low;
+    }
+    if (act && pr.used + act > max_it) {
+      pr.over = true;
+      if (kResume) {
+        Key c = have ? low : 0;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+          const Key y = __shfl_xor_sync(FULL, c, d);
+          c = y > c ? y : c;
+        }
+        const int from = __ffs(__ballot_sync(FULL, have && low == c)) - 1;
+        rs.stop = c;
+        rs.s = __shfl_sync(FULL, s, from);
+        rs.e = __shfl_sync(FULL, e, from);
+        rs.its = __shfl_sync(FULL, its, from);
+      }
+    }
+    ++its;
     pr.used += act;
     pr.rounds += act > 0;
     if (pr.over) have = false;
@@ -1505,31 +1553,115 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
 // A phase of the worlds with `run` set: their islands side by side (unless
 // they are all `hard`: their last solve ran out of iterations); then, as
 // one list, the worlds whose islands want more iterations than the budget,
-// after restart(over) has put them back (not with `once`: such a world only
-// reports the whole budget used).
+// after restart(over, ...) has put them back (not with `once`: such a world
+// only reports the whole budget used; nor a world of one island, whose list
+// it is).
+//
+// With a world per warp less is put back.  The reference
+// resolves the contact with the first value, over all islands: island j's
+// t-th iteration comes in the order of m_j(t), the smallest of the island's
+// first values so far (what follows a smaller value but is larger is resolved
+// before any other island's value that the smaller one was ahead of).  When
+// the budget ends, let U be the island under way whose smallest value so far,
+// its next included, is the largest, c.  Every iteration U has had is ahead of
+// every other island's from its first value below c on; so U has had none too
+// many, and of the others only those with m_j > c come before U's next.  The
+// others are put back and run to their first value below c; U goes on from
+// where it is until its first value is below c; and if the budget has not
+// ended by then, the world stands as the one list would have it, and goes on
+// as that.  The whole world is put back where a value equals c (its place is
+// then a matter of list order), where the others do not reach c within the
+// budget (islands not begun), and where an error flag was set.  Half of the
+// worlds out of budget were not in the frame before, and one of them is the
+// chain that its launch waits for: 8192 worlds of 32 bodies took 1.20 ms at
+// frame 120 and 1.19 at 300 with the whole world put back, 0.97 and 0.88 so
+// (float64: 4.52 and 4.80, 3.99 and 4.16).
 template <class R, class W, int G, bool VEL, bool LEARN, class F>
 __device__ __forceinline__ Progress resolve_worlds(const RCtx<R, W, true>& x, const BatchView<R>& v, int bstart, int C,
                                                    int gl, int max_it, bool run, int ni, const uint16_t* ist, int* ml,
                                                    bool hard, bool once, uint32_t& err, F&& restart) {
+  using Key = KeyOf<R>;
+  constexpr int kNone = 0x7fffffff;
   Progress pr{0, 0, false};
   uint32_t er = 0;
-  bool on = run;
+  if constexpr (G == 32) {
+    Span<Key> sp{false, kNone, C, 1};
+    int part = 0, others = ni, ls = 0, le = 0;
+    bool over = false;
 #pragma unroll 1
-  for (bool whole = G == kIslandLanes || __all_sync(FULL, !run || hard);; whole = true) {
-    const Progress p = resolve_phase<R, W, G, VEL, LEARN>(x, v, bstart, C, gl, max_it, on, whole, ni, ist, ml, er);
-    if (on) {
+    for (;;) {
+      Resume<Key> rs{0, 0, 0, 0, false};
+      const Progress p = resolve_phase<R, W, G, VEL, LEARN>(x, v, bstart, gl, max_it - pr.used, run, sp, others, ist,
+                                                            ml, er, rs);
       pr.rounds += p.rounds;
-      pr.used = p.over ? max_it : p.used;
+      over = over || p.over;
+      const bool bad = __any_sync(FULL, er != 0 || (part == 1 && rs.tie));
+      if (part == 0 && p.over && !once && ni > 1 && !bad) {
+        ls = rs.s;
+        le = rs.e;
+        pr.used = rs.its;
+        sp = Span<Key>{false, ls, C, rs.stop};
+        others = ni - 1;
+        restart(true, ls, le);
+        part = 1;
+      } else if ((part == 0 && p.over && !once && ni > 1) || (part == 1 && (p.over || bad))) {
+        restart(true, 0, 0);
+        er = 0;
+        pr.used = 0;
+        sp = Span<Key>{true, 0, C, 1};
+        part = 3;
+      } else {
+        pr.used += p.used;
+        if (part == 0 || part == 3 || p.over) break;
+        sp = part == 1 ? Span<Key>{true, ls, le, sp.stop} : Span<Key>{true, 0, C, 1};
+        ++part;
+      }
     }
-    // as one list, the budget's end is the reference's
-    pr.over = pr.over || (on && p.over);
-    on = on && p.over && !whole && !once;
-    if (!__any_sync(FULL, on)) break;
-    restart(on);
-    if (on) er = 0;
+    pr.over = over;
+    if (over) pr.used = max_it;
+  } else {
+    bool on = run;
+#pragma unroll 1
+    for (bool whole = G == kIslandLanes || __all_sync(FULL, !run || hard);; whole = true) {
+      Resume<Key> rs{0, 0, 0, 0, false};
+      const Progress p = resolve_phase<R, W, G, VEL, LEARN>(
+          x, v, bstart, gl, max_it, on, Span<Key>{whole, whole ? 0 : kNone, C, 1}, ni, ist, ml, er, rs);
+      if (on) {
+        pr.rounds += p.rounds;
+        pr.used = p.over ? max_it : p.used;
+      }
+      // as one list, the budget's end is the reference's
+      pr.over = pr.over || (on && p.over);
+      on = on && p.over && !whole && !once && ni > 1;
+      if (!__any_sync(FULL, on)) break;
+      restart(on, 0, 0);
+      if (on) er = 0;
+    }
   }
   err |= er;
   return pr;
+}
+
+// label of the island of records [ks, ke), -1 for none
+template <class R, class W>
+__device__ __forceinline__ int island_label(const RCtx<R, W, true>& x, int ks, int ke, const uint8_t* lab) {
+  if (ks >= ke) return -1;
+  const int bb = x.pair(ks);
+  return lab[x.B0(bb) < 0 ? x.B1(bb) : x.B0(bb)];
+}
+// Puts the worlds with `on` back to the state adjustPositions starts from, all
+// but the island of the records [ks, ke), if any.  (Out of the kernel's code,
+// as restart_velocities.)
+template <class R, class W, int G>
+__device__ __noinline__ void restart_positions(RCtx<R, W, true> x, const BatchView<R>& v, long long bstart,
+                                               long long cst, int n, int C, int gl, bool on, int ks, int ke,
+                                               const uint8_t* lab) {
+  __syncwarp();
+  if (on) load_bodies(x, v, bstart, n, gl, G, lab, island_label(x, ks, ke, lab));
+#pragma unroll 1
+  for (int k = gl; on && k < C; k += G)
+    if (k < ks || k >= ke) x.rec(k)[CR_PEN] = v.contact[C_PEN * v.nc_total + cst + x.list_index(k)];
+  __syncwarp();
 }
 
 // Puts the worlds with `on` back to the state adjustVelocities starts from:
@@ -1537,16 +1669,19 @@ __device__ __forceinline__ Progress resolve_worlds(const RCtx<R, W, true>& x, co
 // values before the solve; awake_bits are the flags after adjustPositions,
 // whose matchAwakeState may have woken bodies), and the contact velocities and
 // desired delta velocities prepareContacts left (same velocities, relative
-// positions, basis and awake flags).  Harvested impulse totals start again at
+// positions, basis and awake flags); all but the island of the records
+// [ks, ke), if any.  Harvested impulse totals start again at
 // zero.  Every lane of the warp calls it.
 // (Rare, so its code stays out of the kernel's: __noinline__, by value.)
 template <class R, class W, int G>
 __device__ __noinline__ void restart_velocities(RCtx<R, W, true> x, const R* body, const uint8_t* awake, long long S,
                                                 long long bstart, int n, int C, int gl, bool on, unsigned awake_bits,
-                                                bool harvest) {
+                                                bool harvest, int ks, int ke, const uint8_t* lab) {
   const R* g = body + bstart;
+  const int keep = island_label(x, ks, ke, lab);
   __syncwarp();
   for (int i = gl; on && i < n; i += G) {
+    if (lab[i] == keep) continue;
     R* b = x.body(i);
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
@@ -1557,6 +1692,7 @@ __device__ __noinline__ void restart_velocities(RCtx<R, W, true> x, const R* bod
   }
   __syncwarp();
   for (int k = gl; on && k < C; k += G) {
+    if (k >= ks && k < ke) continue;
     const int bb = x.pair(k), o = x.list_index(k);
     const int b0 = x.B0(bb), b1 = x.B1(bb);
     const m3<R> Ck = x.basis(k);
@@ -1572,12 +1708,14 @@ __device__ __noinline__ void restart_velocities(RCtx<R, W, true> x, const R* bod
   }
   __syncwarp();
   for (int i = gl, j = 0; on && i < n; i += G, ++j) {
+    if (lab[i] == keep) continue;
     const bool was = x.aw[i] != 0, now = (awake_bits >> j) & 1u;
     x.body(i)[BR_MOTION] = now && !was ? (R)(0.3 * 2.0) : g[B_MOTION * S + i];
     if (now && !was) x.aw[i] = 1;
   }
   __syncwarp();
   for (int k = gl; on && k < C; k += G) {
+    if (k >= ks && k < ke) continue;
     const int bb = x.pair(k);
     const R* r = x.rec(k);
     x.rec(k)[CR_VFA] = frame_velocity(x, x.B0(bb), x.B1(bb), V<R>(r[0], r[1], r[2]));
@@ -1682,7 +1820,7 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
     int C = has ? v.contact_count[w] : 0;
     // about half of the worlds whose adjustVelocities ran out of its budget do
     // so again in the next frame: they are solved as one list at once
-    const bool hard = has && (v.cost[w] & kExhausted) != 0;
+    const bool hard = G < 32 && has && (v.cost[w] & kExhausted) != 0;
     if (has) {
       const int cap = v.contact_cap[w];
       if (C > cap) C = cap;  // the world is already flagged ST_CAPACITY
@@ -1728,14 +1866,8 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
     uint32_t err = 0;
     // ---------------- adjustPositions, contact.go:231-283
     const Progress pos = resolve_worlds<R, W, G, false, LEARN>(
-        x, v, bstart, C, gl, max_it, solve, ni, sl.ist, sl.ml, false, false, err, [&](bool over) {
-          if (over) {
-            load_bodies(x, v, bstart, n, gl, G);
-#pragma unroll 1
-            for (int k = gl; k < C; k += G)
-              x.rec(k)[CR_PEN] = v.contact[C_PEN * v.nc_total + cst + x.list_index(k)];
-          }
-          __syncwarp();
+        x, v, bstart, C, gl, max_it, solve, ni, sl.ist, sl.ml, false, false, err, [&](bool over, int ks, int ke) {
+          restart_positions<R, W, G>(x, v, bstart, cst, n, C, gl, over, ks, ke, sl.lab);
         });
     const int pos_used = pos.used;
     if (active && v.contact_writeback)  // the caller's Contact.Penetration after ResolveContacts
@@ -1784,10 +1916,10 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
       warmed = group_sum<G>(nw) > 0;
     }
     // ---------------- adjustVelocities, contact.go:388-445
-    auto restart = [&](bool over) {
+    auto restart = [&](bool over, int ks, int ke) {
       if (__any_sync(FULL, over))
         restart_velocities<R, W, G>(x, v.body, v.awake, v.nb_pad, bstart, n, C, gl, over, awake_bits,
-                                    LEARN && mode == 1);
+                                    LEARN && mode == 1, ks, ke, sl.lab);
     };
     int vel_used = 0, rounds = 2 * pos.rounds;
     bool exhausted = false;
@@ -1809,7 +1941,7 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
           if (again && gl == 0) atomicAdd(&v.counters[4], 1ull);
         }
       }
-      if (LEARN) restart(again);
+      if (LEARN) restart(again, 0, 0);
       todo = again;
     }
     if (LEARN && mode == 2 && warm_ok && gl == 0) atomicAdd(&v.counters[5], 1ull);
