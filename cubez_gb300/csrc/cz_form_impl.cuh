@@ -273,6 +273,13 @@ static cudaError_t resolve(const HostView& h, int nbs, int cs, int lanes, int gr
   return cudaGetLastError();
 }
 
+static size_t wide_smem(int nbs, int cs) { return wide_smem_bytes<R, W>(nbs, cs); }
+static cudaError_t wide_prepare(size_t smem) { return raise_smem_limit((const void*)k_resolve_wide<R, W>, smem); }
+static cudaError_t resolve_wide(const HostView& h, int nbs, int cs, int grid, size_t smem, double dt, cudaStream_t s) {
+  k_resolve_wide<R, W><<<grid, 32 * kWideWarps, smem, s>>>(view_of(h), nbs, cs, (R)dt);
+  return cudaGetLastError();
+}
+
 static size_t frame_smem(int nbs, int cs) { return frame_slot_bytes<R, W>(nbs, cs); }
 
 static cudaError_t frame_occupancy(int* blocks, size_t smem) {
@@ -410,6 +417,9 @@ const FormOps CZ_FORM_OBJ = {sizeof(CZ_R),
                              CZ_FORM_NS::resolve_big,
                              CZ_FORM_NS::big_smem,
                              CZ_FORM_NS::resolve,
+                             CZ_FORM_NS::wide_smem,
+                             CZ_FORM_NS::wide_prepare,
+                             CZ_FORM_NS::resolve_wide,
                              CZ_FORM_NS::upload,
                              CZ_FORM_NS::download,
                              CZ_FORM_NS::occupancy,

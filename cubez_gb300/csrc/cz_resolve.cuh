@@ -1316,7 +1316,9 @@ __device__ __forceinline__ int next_record(const BatchView<R>& v, long long cst,
 // take that one (L = G): the islands left last are the long ones, and a round
 // of theirs is then one update pass instead of one per eight contacts.  With
 // `whole`, the world is one list for all G lanes from the start, the
-// reference's own order of work.  Equal values go to the contact that comes
+// reference's own order of work.  WARPS > 1: the world is shared by as many
+// warps; a group of lanes starts on island `seat` and takes further ones from
+// shared[0], and shared[1] counts the world's iterations.  Equal values go to the contact that comes
 // first in the narrowphase's list.  `over` is set when the iterations wanted
 // exceed max_it.
 //
@@ -1355,10 +1357,11 @@ template <class Key> struct Resume {
   int s, e, its;
   bool tie;
 };
-template <class R, class W, int G, bool VEL, bool LEARN>
+template <class R, class W, int G, bool VEL, bool LEARN, int WARPS = 1>
 __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, const BatchView<R>& v, int bstart, int gl,
                                                   int max_it, bool run, Span<KeyOf<R>> sp, int ni, const uint16_t* ist,
-                                                  int* ml_world, uint32_t& err, Resume<KeyOf<R>>& rs) {
+                                                  int* ml_world, uint32_t& err, Resume<KeyOf<R>>& rs, int seat = 0,
+                                                  int* shared = nullptr) {
   using Key = KeyOf<R>;
   constexpr bool kResume = G == 32;
   constexpr bool kGather = gathers_updates<R>();
@@ -1413,7 +1416,18 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
     if (done) {
       const unsigned m = done & leaders;
       if (fin) {  // the next island, in the order of the groups
-        int isl = next + __popc(m & ((1u << (lane - sl)) - 1u));
+        int isl;
+        if constexpr (WARPS > 1) {
+          isl = seat;
+          if (seat < 0) {
+            if (sl == 0) isl = atomicAdd(&shared[0], 1);
+            isl = __shfl_sync(lmask, isl, lane - sl);
+          }
+          seat = -1;
+          next = isl;
+        } else {
+          isl = next + __popc(m & ((1u << (lane - sl)) - 1u));
+        }
         have = isl < ni;
         if (have) {
           if (kResume && ist[isl] >= sp.s) ++isl;
@@ -1424,13 +1438,14 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
         low = ~(Key)0;
         scan = true;
       }
-      next += __popc(m);
+      if (WARPS == 1) next += __popc(m);
       continue;
     }
     const unsigned live = __ballot_sync(FULL, have);
     if (!live) break;
     const int act = __popc(live & leaders);
-    if (G > kIslandLanes && L == kIslandLanes && __all_sync(FULL, act <= 1 && next >= ni)) {
+    if (G > kIslandLanes && L == kIslandLanes &&
+        (WARPS == 1 ? __all_sync(FULL, act <= 1 && next >= ni) : act <= 1 && __any_sync(FULL, next >= ni))) {
       // all lanes of the world on its last island
       const unsigned held = live & wmask;
       const int from = held ? __ffs(held) - 1 : lane;
@@ -1453,7 +1468,12 @@ __device__ __forceinline__ Progress resolve_phase(const RCtx<R, W, true>& x, con
       rs.tie = rs.tie || (have && best == sp.stop);
       low = best < low ? best : low;
     }
-    if (act && pr.used + act > max_it) {
+    int before = pr.used;
+    if (WARPS > 1) {
+      if (lane == 0) before = atomicAdd(&shared[1], act);
+      before = __shfl_sync(FULL, before, 0);
+    }
+    if (act && before + act > max_it) {
       pr.over = true;
       if (kResume) {
         Key c = have ? low : 0;
@@ -1972,6 +1992,209 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
   }
 }
 
+
+// ---------------------------------------------------------------- k_resolve_wide
+// The resolver for batches of fewer worlds than SMs: four warps to a world,
+// one CTA each.  With one warp a small batch leaves three of an SM's four
+// schedulers idle, and in float64 each scheduler has its own quarter of the
+// SM's float64 rate, so a warp on its own is bound by its scheduler's unit.
+// The preparation is split over the warps, and so are the world's islands
+// (side by side within a warp where there are more than warps); bodies, records, friction matrices and
+// lists are in shared memory, which such a batch has to spare.  A world whose
+// islands want more iterations than its budget is put back and solved as one
+// list by the first warp, as in resolve_worlds.
+constexpr int kWideWarps = 4;
+// What the warps share: the next island, the iterations (resolve_phase), then
+// per call the sum of the iterations, the most rounds, whether a warp met the
+// budget, a tie or an error flag, and each warp's island to go on from.
+template <class Key> struct WideShared {
+  int island, count, used, rounds, over, tie, err, world, islands;
+  Resume<Key> rs[kWideWarps];
+};
+// shared memory of one world, with tiles of cs contacts
+template <class R, class W> __host__ __device__ inline size_t wide_smem_bytes(int nbs, int cs) {
+  size_t b = rs_slot_bytes<R, W>(nbs, cs);
+  b += (size_t)K_ROW * cs * sizeof(R);
+  b += (size_t)kWideWarps * kTouchList * sizeof(int);
+  b += (size_t)kWideWarps * nbs * sizeof(uint16_t);
+  b = (b + 15) & ~(size_t)15;
+  return b + sizeof(WideShared<KeyOf<R>>);
+}
+
+// resolve_worlds for one world by the CTA's warps
+template <class R, class W, bool VEL, class F>
+__device__ __forceinline__ Progress wide_phase(const RCtx<R, W, true>& x, const BatchView<R>& v, int bstart, int C,
+                                               int max_it, int ni, const uint16_t* ist, int* ml,
+                                               WideShared<KeyOf<R>>* sh, uint32_t& err, F&& restart) {
+  using Key = KeyOf<R>;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  Span<Key> sp{false, 0x7fffffff, C, 1};
+  int part = 0, others = ni, ls = 0, le = 0;
+  Progress pr{0, 0, false};
+  bool over = false;
+  uint32_t er = 0;
+#pragma unroll 1
+  for (;;) {
+    if (threadIdx.x == 0) {
+      sh->island = kWideWarps * (32 / kIslandLanes);
+      sh->count = sh->used = sh->rounds = sh->over = sh->tie = sh->err = 0;
+    }
+    if (lane == 0) sh->rs[wid].stop = 0;
+    __syncthreads();
+    Resume<Key> rs{0, 0, 0, 0, false};
+    const Progress p = resolve_phase<R, W, 32, VEL, false, kWideWarps>(
+        x, v, bstart, lane, max_it - pr.used, !sp.list || wid == 0, sp, others, ist, ml, er, rs,
+        wid + kWideWarps * (lane / kIslandLanes), &sh->island);
+    if (rs.tie) sh->tie = 1;
+    if (er) sh->err = 1;
+    if (lane == 0) {
+      atomicAdd(&sh->used, p.used);
+      atomicMax(&sh->rounds, p.rounds);
+      if (p.over) {
+        sh->over = 1;
+        sh->rs[wid] = rs;
+      }
+    }
+    __syncthreads();
+    const int used = sh->used;
+    const bool out = sh->over != 0, bad = sh->err != 0 || (part == 1 && sh->tie != 0);
+    pr.rounds += sh->rounds;
+    over = over || out;
+    rs = sh->rs[0];
+#pragma unroll
+    for (int q = 1; q < kWideWarps; ++q)
+      if (sh->rs[q].stop > rs.stop) rs = sh->rs[q];
+    __syncthreads();
+    if (part == 0 && out && ni > 1 && !bad) {
+      ls = rs.s;
+      le = rs.e;
+      pr.used = rs.its;
+      sp = Span<Key>{false, ls, C, rs.stop};
+      others = ni - 1;
+      restart(ls, le);
+      part = 1;
+    } else if ((part == 0 && out && ni > 1) || (part == 1 && (out || bad))) {
+      restart(0, 0);
+      er = 0;
+      pr.used = 0;
+      sp = Span<Key>{true, 0, C, 1};
+      part = 3;
+    } else {
+      pr.used += used;
+      if (part == 0 || part == 3 || out) break;
+      sp = part == 1 ? Span<Key>{true, ls, le, sp.stop} : Span<Key>{true, 0, C, 1};
+      ++part;
+    }
+    __syncthreads();
+  }
+  pr.over = over;
+  if (over) pr.used = max_it;
+  err |= er;
+  return pr;
+}
+
+template <class R, class W>
+__global__ void __launch_bounds__(32 * kWideWarps, 1) k_resolve_wide(BatchView<R> v, int nbs, int cs, R dt) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int T = 32 * kWideWarps;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  Slot<R, W> sl = make_slot<R, W>(smem, nbs, cs, dt);
+  RCtx<R, W, true>& x = sl.x;
+  R* k_tile = reinterpret_cast<R*>(smem + rs_slot_bytes<R, W>(nbs, cs));
+  int* ml = reinterpret_cast<int*>(k_tile + (size_t)K_ROW * cs) + wid * kTouchList;
+  uint16_t* curs = reinterpret_cast<uint16_t*>(reinterpret_cast<int*>(k_tile + (size_t)K_ROW * cs) +
+                                               kWideWarps * kTouchList);
+  uint16_t* cur = curs + wid * nbs;
+  WideShared<KeyOf<R>>* sh = reinterpret_cast<WideShared<KeyOf<R>>*>(
+      smem + (((size_t)(reinterpret_cast<unsigned char*>(curs + kWideWarps * nbs) - smem) + 15) & ~(size_t)15));
+  for (;;) {
+    if (tid == 0) sh->world = (int)atomicAdd(&v.queue[1], 1u);
+    __syncthreads();
+    const int qi = sh->world;
+    if (qi >= v.num_worlds) break;
+    const int w = v.order_rs[qi];
+    const int n = v.body_count[w];
+    if (n > nbs) {  // a world of k_resolve_big
+      __syncthreads();
+      continue;
+    }
+    const int bstart = v.body_start[w];
+    int C = v.contact_count[w];
+    if (C > v.contact_cap[w]) C = v.contact_cap[w];  // the world is already flagged ST_CAPACITY
+    const bool active = C > 0 && dt > (R)0;  // ResolveContacts guards, contact.go:210-212
+    int pos_used = 0, vel_used = 0, cost = 0;
+    uint32_t err = 0;
+    if (active) {
+      const long long cst = v.contact_start[w];
+      bind_contacts(sl, v, C, cs, cst);
+      if (C <= cs) x.kw = k_tile;
+      x.all_awake = __syncthreads_and(load_bodies(x, v, bstart, n, tid, T));
+      if (wid == 0) {
+        const int ni = build_islands<32>(v, cst, n, nbs, C, lane, reinterpret_cast<int*>(sl.cr_s), sl.ist, sl.cur,
+                                         sl.lab);
+        if (lane == 0) sh->islands = ni;
+      }
+      __syncthreads();
+      const int ni = sh->islands;
+      // every warp counts the places of all contacts, and prepares its share
+      for (int i = lane; i < n; i += 32) cur[i] = sl.cur[i];
+      __syncwarp();
+#pragma unroll 1
+      for (int base = 0; base < C; base += 32) {
+        const int k = base + lane;
+        const int p = next_record<32>(v, cst, k, k < C, lane, cur, sl.lab);
+        if ((base >> 5) % kWideWarps == wid && k < C) prepare_contact(x, v, cst + k, p, k);
+      }
+      __syncthreads();
+      const int max_it = v.max_iterations >= 0 ? v.max_iterations : C * v.iter_mult;
+      if (max_it > 0) {
+        const Progress pos = wide_phase<R, W, false>(
+            x, v, bstart, C, max_it, ni, sl.ist, ml, sh, err, [&](int ks, int ke) {
+              load_bodies(x, v, bstart, n, tid, T, sl.lab, island_label(x, ks, ke, sl.lab));
+              for (int k = tid; k < C; k += T)
+                if (k < ks || k >= ke) x.rec(k)[CR_PEN] = v.contact[C_PEN * v.nc_total + cst + x.list_index(k)];
+            });
+        pos_used = pos.used;
+        cost = 2 * pos.rounds;
+      }
+      if (v.contact_writeback)  // the caller's Contact.Penetration after ResolveContacts
+        for (int k = tid; k < C; k += T) v.contact[C_PEN * v.nc_total + cst + x.list_index(k)] = x.rec(k)[CR_PEN];
+      __syncthreads();
+      if (max_it > 0) {
+#pragma unroll 1
+        for (int k = tid; k < C; k += T) friction_prepare(x, k);
+        // awake flags after adjustPositions, of the first warp's lanes' bodies
+        unsigned awake_bits = 0;
+        for (int i = lane, j = 0; i < n; i += 32, ++j) awake_bits |= (x.aw[i] ? 1u : 0u) << j;
+        __syncthreads();
+        const Progress vel = wide_phase<R, W, true>(
+            x, v, bstart, C, max_it, ni, sl.ist, ml, sh, err, [&](int ks, int ke) {
+              if (wid == 0)
+                restart_velocities<R, W, 32>(x, v.body, v.awake, v.nb_pad, bstart, n, C, lane, true, awake_bits, false,
+                                             ks, ke, sl.lab);
+            });
+        vel_used = vel.used;
+        cost += vel.rounds;
+      }
+      if (err) {
+        atomicOr(&v.world_status[w], err);
+        atomicOr(v.status, err);
+      }
+      if (v.contact_writeback)
+        for (int k = tid; k < C; k += T) write_back_contact(x, v, cst, k);
+      store_bodies(x, v, bstart, n, tid, T);
+    }
+    if (tid == 0) {
+      v.pos_iters[w] = pos_used;
+      v.vel_iters[w] = vel_used;
+      v.cost[w] = cost;
+      atomicAdd(&v.counters[1], (unsigned long long)pos_used);
+      atomicAdd(&v.counters[2], (unsigned long long)vel_used);
+      atomicAdd(&v.counters[3], (unsigned long long)C);
+    }
+    __syncthreads();
+  }
+}
 
 // ---------------------------------------------------------------- k_warm_features
 // Shared-memory copy of the inference weights (fragment layouts of MlpDev).
