@@ -93,7 +93,7 @@ struct FormOps {
   // the learned paths' features / predictions ahead of the resolver (k_warm_features)
   cudaError_t (*warm_features)(const HostView& v, int nbs, int grid, double dt, cudaStream_t s);
   int (*warm_features_blocks)(int nbs);  // resident CTAs per SM
-  // worlds above the shared-memory slot, one warp each; smem bytes hold csm contacts' arrays (big_smem)
+  // worlds above the shared-memory slot, a CTA each; smem bytes hold csm contacts' arrays (big_smem)
   cudaError_t (*resolve_big)(const HostView& v, int nbig, int csm, size_t smem, double dt, cudaStream_t s);
   // the contacts whose arrays fit `budget` bytes beside those of n bodies, and the bytes for them (0: none fit)
   cudaError_t (*big_smem)(int n, int max_cap, size_t budget, int* csm, size_t* smem);

@@ -788,8 +788,8 @@ __device__ __forceinline__ R update_apply(const RCtx<R, W, SM>& x, Touched<R>& t
 // float64 instructions, where a group has lanes to spare (14 or, with both
 // bodies touched, 24 of them for L / 4 contacts, against 34 or 64 for L).
 template <bool VEL, class R, class W, bool SM>
-__device__ __forceinline__ void update_spread(const RCtx<R, W, SM>& x, int k, int bb, bool valid, int d0, int d1, R lin,
-                                              R ang, int L, bool woke) {
+__device__ __forceinline__ R update_spread(const RCtx<R, W, SM>& x, int k, int bb, bool valid, int d0, int d1, R lin,
+                                           R ang, int L, bool woke) {
   const R z = (R)0;
   const int c4 = threadIdx.x & 3, c = c4 != 3 ? c4 : 0;
   const int p = c == 2 ? 0 : c + 1, q = c == 0 ? 2 : c - 1;
@@ -819,12 +819,13 @@ __device__ __forceinline__ void update_spread(const RCtx<R, W, SM>& x, int k, in
     const R t2 = term(4 * (e.y > 0), r1p, r1q);
     if (both) m = VEL ? m - t2 : m + t2;
   }
+  R value = m;
   if (valid) {
     R* r = x.rec(k);
     if (VEL) {
       if (woke) vfa = frame_velocity(x, x.B0(bb), x.B1(bb), V<R>(r[0], r[1], r[2]));
       if (c4 < 3) r[CR_CV + c] = m;
-      const R value = desired_dv(m, vfa, x.restitution(SM ? (int)((unsigned)bb >> 16) : k));
+      value = desired_dv(m, vfa, x.restitution(SM ? (int)((unsigned)bb >> 16) : k));
       if (c4 == 0) {
         if (woke) r[CR_VFA] = vfa;
         r[CR_DDV] = value;
@@ -833,6 +834,7 @@ __device__ __forceinline__ void update_spread(const RCtx<R, W, SM>& x, int k, in
       r[CR_PEN] = m;
     }
   }
+  return value;
 }
 
 // A world's bodies from the batch rows into the records of x, by the `step`

@@ -1,8 +1,9 @@
 // ResolveContacts (contact.go:204-445) for worlds whose bodies do not fit the
 // shared-memory slot of k_resolve (hundreds to thousands of bodies).
 //
-// One warp per world: such a world is mostly one island, so its iterations are
-// one chain, and what counts is the latency of an iteration.
+// One warp per world (four in float64, sharing each iteration): such a world is
+// mostly one island, so its iterations are one chain, and what counts is the
+// latency of an iteration.
 //   * Body and contact records are in global memory (L1/L2); a record is two
 //     cache lines at most, where rows took a line per value.
 //   * The argmax is over two levels of chunk maxima in shared memory, kept by
@@ -26,10 +27,13 @@ namespace cz {
 constexpr int kBigChunks = 512;  // chunks of a world's contacts (16 each up to 8192 contacts)
 constexpr int kBigTops = kBigChunks / 16;  // groups of 16 chunks: one per lane
 
+// the change shared between the warps (16-byte multiple)
+template <class R> __host__ __device__ constexpr size_t big_change_bytes() { return 16 * sizeof(R) + 16; }
 // shared memory ahead of the per-contact arrays: maxima and their contacts of
 // the chunks and of the groups of chunks, list starts and ends of n bodies
 template <class R> __host__ __device__ inline size_t big_fixed_bytes(int n) {
-  return (size_t)(kBigChunks + kBigTops) * (sizeof(R) + sizeof(int)) + (size_t)2 * ((n + 3) & ~3) * sizeof(int);
+  return (size_t)(kBigChunks + kBigTops) * (sizeof(R) + sizeof(int)) + (size_t)2 * ((n + 3) & ~3) * sizeof(int) +
+         big_change_bytes<R>();
 }
 // per contact: key, packed bodies, two list entries
 template <class R> __host__ __device__ constexpr size_t big_contact_bytes() { return sizeof(R) + 3 * sizeof(int); }
@@ -103,19 +107,38 @@ template <class Key> struct BigKeys {
   }
 };
 
+// Warps per world.  In float64 each of an SM's four schedulers has its own
+// quarter of the float64 rate, and a warp alone is bound by its own: four
+// warps share an iteration's updates, four lanes to a contact (update_spread),
+// while its argmax and the resolved contact's change stay with one chain:
+// 64 piles of 1024 cubes x 3 frames 128.8 -> 113.7 ms, 600 of 72 cubes (two
+// worlds to a scheduler) 14.4 -> 13.7.  In float32 the updates are a sixth of
+// an iteration, about what the barriers cost.
+template <class R> __host__ __device__ constexpr int big_warps() { return sizeof(R) == 8 ? 4 : 1; }
+// the resolved contact's change, for the other warps
+template <class R> struct BigChange {
+  R lin[8], ang[8];
+  int woke;
+};
+template <int NW> __device__ __forceinline__ void big_sync() {
+  if (NW > 1) __syncthreads();
+  else __syncwarp();
+}
+
 // adjustPositions (VEL false) or adjustVelocities (VEL true) of one world by
-// its warp; returns the iterations used.
+// its warps; returns the iterations used.
 template <class R, class W, bool VEL, class Key>
 __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const BatchView<R>& v, int bstart,
                                          const BigKeys<Key>& bk, const int* off, const int* end, const int* adj,
-                                         int max_it, uint32_t& err) {
-  const int lane = threadIdx.x;
+                                         int max_it, BigChange<R>* chg, uint32_t& err) {
+  constexpr int NW = big_warps<R>(), T = 32 * NW;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int C = bk.C;
-  for (int k = lane; k < C; k += 32) bk.key[k] = key_of(x.rec(k)[VEL ? CR_DDV : CR_PEN], (R)0.01);
-  if (bk.padded && C + lane < ((C + 15) & ~15)) bk.key[C + lane] = 0;
-  __syncwarp();
+  for (int k = tid; k < C; k += T) bk.key[k] = key_of(x.rec(k)[VEL ? CR_DDV : CR_PEN], (R)0.01);
+  if (bk.padded && C + tid < ((C + 15) & ~15)) bk.key[C + tid] = 0;
+  big_sync<NW>();
   const int nch = (C + (1 << bk.shift) - 1) >> bk.shift;
-  for (int ch = lane; ch < kBigChunks; ch += 32) {
+  for (int ch = tid; ch < kBigChunks; ch += T) {
     if (ch < nch) {
       bk.refresh_chunk(ch);
     } else {
@@ -123,9 +146,9 @@ __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const Batch
       bk.cfirst[ch] = 0;
     }
   }
-  __syncwarp();
-  bk.refresh_top(lane);
-  __syncwarp();
+  big_sync<NW>();
+  if (wid == 0) bk.refresh_top(lane);
+  big_sync<NW>();
   int used = 0;
   while (used < max_it) {
     Key best = bk.tmax[lane];
@@ -147,50 +170,102 @@ __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const Batch
       qb = x.pair(q);
       if (e >= l0 && (x.B0(qb) == d0 || x.B1(qb) == d0)) q = -1;
     };
-    entry(lane);
-    // what the change needs, then the touched records: they load while the
-    // change is computed
-    std::conditional_t<VEL, VelocityIn<R>, PositionIn<R, W>> in;
-    if constexpr (VEL)
-      velocity_load(x, in, k, bb, lane < 8, lane);
-    else
-      position_load(x, in, k, bb, lane < 8, lane);
-    Touched<R> t;
-    update_load<VEL>(x, t, q, qb, q >= 0, d0, d1);
-    const bool woke = match_awake(x, bb, true, lane == 0);
     R lin, ang;
-    if constexpr (VEL)
-      velocity_change<R, W, false>(x, v, in, k, lane < 8, lane, lin, ang, err);
-    else
-      position_change(x, v, in, bstart, lane < 8, lane, lin, ang);
-    for (int base = 0; base < l0 + l1; base += 32) {
-      if (base > 0) {
-        entry(base + lane);
-        update_load<VEL>(x, t, q, qb, q >= 0, d0, d1);
+    if constexpr (NW > 1) {
+      // every warp's contacts, eight at a time; the first warp's change
+      const int first = 8 * wid + (lane >> 2);
+      const bool lead = (lane & 3) == 0;
+      entry(first);
+      if (q >= 0) prefetch_line(x.rec(q) + 16 * (lane & 1));
+      if (wid == 0) {
+        std::conditional_t<VEL, VelocityIn<R>, PositionIn<R, W>> in;
+        if constexpr (VEL)
+          velocity_load(x, in, k, bb, lane < 8, lane);
+        else
+          position_load(x, in, k, bb, lane < 8, lane);
+        const bool woke = match_awake(x, bb, true, lane == 0);
+        if constexpr (VEL)
+          velocity_change<R, W, false>(x, v, in, k, lane < 8, lane, lin, ang, err);
+        else
+          position_change(x, v, in, bstart, lane < 8, lane, lin, ang);
+        if (lane < 8) {
+          chg->lin[lane] = lin;
+          chg->ang[lane] = ang;
+        }
+        if (lane == 0) chg->woke = woke;
       }
-      const R value = update_apply<VEL>(x, t, lin, ang, 32, woke);
-      if (t.valid) {
-        bk.key[t.k] = key_of(value, (R)0.01);
-        // the next contact to resolve is mostly one of these
-        if (VEL) prefetch_line(x.krow(t.k));
+      __syncthreads();
+      lin = chg->lin[lane & 7];
+      ang = chg->ang[lane & 7];
+      const bool woke = chg->woke != 0;
+      for (int base = 0; base < l0 + l1; base += 8 * NW) {
+        if (base > 0) entry(base + first);
+        if (base + 8 * wid < l0 + l1) {
+          const R value = update_spread<VEL>(x, q < 0 ? 0 : q, qb, q >= 0, d0, d1, lin, ang, 32, woke);
+          if (q >= 0 && lead) {
+            bk.key[q] = key_of(value, (R)0.01);
+            if (VEL) prefetch_line(x.krow(q));
+          }
+        }
       }
-      __syncwarp();
-      if (t.valid) bk.refresh_chunk(t.k >> bk.shift);  // lanes of one chunk find the same
-      __syncwarp();
-      if (t.valid) bk.refresh_top(t.k >> bk.shift >> 4);
-      __syncwarp();
+      const bool again = l0 + l1 > 8 * NW;
+      __syncthreads();
+      for (int base = 0; base < l0 + l1; base += 8 * NW) {
+        if (again) entry(base + first);
+        if (q >= 0 && lead) bk.refresh_chunk(q >> bk.shift);  // lanes of one chunk find the same
+      }
+      __syncthreads();
+      for (int base = 0; base < l0 + l1; base += 8 * NW) {
+        if (again) entry(base + first);
+        if (q >= 0 && lead) bk.refresh_top(q >> bk.shift >> 4);
+      }
+      __syncthreads();
+    } else {
+      entry(lane);
+      // what the change needs, then the touched records: they load while the
+      // change is computed
+      std::conditional_t<VEL, VelocityIn<R>, PositionIn<R, W>> in;
+      if constexpr (VEL)
+        velocity_load(x, in, k, bb, lane < 8, lane);
+      else
+        position_load(x, in, k, bb, lane < 8, lane);
+      Touched<R> t;
+      update_load<VEL>(x, t, q, qb, q >= 0, d0, d1);
+      const bool woke = match_awake(x, bb, true, lane == 0);
+      if constexpr (VEL)
+        velocity_change<R, W, false>(x, v, in, k, lane < 8, lane, lin, ang, err);
+      else
+        position_change(x, v, in, bstart, lane < 8, lane, lin, ang);
+      for (int base = 0; base < l0 + l1; base += 32) {
+        if (base > 0) {
+          entry(base + lane);
+          update_load<VEL>(x, t, q, qb, q >= 0, d0, d1);
+        }
+        const R value = update_apply<VEL>(x, t, lin, ang, 32, woke);
+        if (t.valid) {
+          bk.key[t.k] = key_of(value, (R)0.01);
+          // the next contact to resolve is mostly one of these
+          if (VEL) prefetch_line(x.krow(t.k));
+        }
+        __syncwarp();
+        if (t.valid) bk.refresh_chunk(t.k >> bk.shift);  // lanes of one chunk find the same
+        __syncwarp();
+        if (t.valid) bk.refresh_top(t.k >> bk.shift >> 4);
+        __syncwarp();
+      }
     }
     ++used;
   }
   return used;
 }
 
-// One world of C contacts by its warp.  TILE: its per-contact arrays are in
+// One world of C contacts by its warps.  TILE: its per-contact arrays are in
 // shared memory, which the compiler then knows (csm: their capacity).
 template <class R, class W, bool TILE>
 __device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, int w, int C, unsigned char* smem) {
   using Key = decltype(key_of((R)0, (R)0));
-  const int lane = threadIdx.x;
+  constexpr int NW = big_warps<R>(), T = 32 * NW;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int n = v.body_count[w];
   const int bstart = v.body_start[w];
   const long long cst = v.contact_start[w];
@@ -205,7 +280,8 @@ __device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, 
   // list starts and ends (first the counts, then the fill cursors)
   int* off = bk.tfirst + kBigTops;
   int* end = off + ((n + 3) & ~3);
-  unsigned char* tile = reinterpret_cast<unsigned char*>(end + ((n + 3) & ~3));
+  BigChange<R>* chg = reinterpret_cast<BigChange<R>*>(end + ((n + 3) & ~3));
+  unsigned char* tile = reinterpret_cast<unsigned char*>(chg) + big_change_bytes<R>();
   RCtx<R, W, false> x;
   x.nbs = n;
   x.dt = dt;
@@ -230,20 +306,21 @@ __device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, 
     x.cb = v.work_bodies + cst;
     adj = v.big_adj + 2 * cst;
   }
-  x.all_awake = __all_sync(FULL, load_bodies(x, v, bstart, n, lane, 32));
-  __syncwarp();
-  for (int k = lane; k < C; k += 32) prepare_contact(x, v, cst + k, k, k);
-  for (int i = lane; i < n; i += 32) end[i] = 0;
-  __syncwarp();
+  const bool awake = load_bodies(x, v, bstart, n, tid, T);
+  x.all_awake = NW > 1 ? __syncthreads_and(awake) != 0 : __all_sync(FULL, awake) != 0;
+  big_sync<NW>();
+  for (int k = tid; k < C; k += T) prepare_contact(x, v, cst + k, k, k);
+  for (int i = tid; i < n; i += T) end[i] = 0;
+  big_sync<NW>();
   // contact lists per body: count, exclusive scan, fill
-  for (int k = lane; k < C; k += 32) {
+  for (int k = tid; k < C; k += T) {
     const int bb = x.pair(k);
     atomicAdd(&end[x.B0(bb)], 1);
     if (x.B1(bb) >= 0) atomicAdd(&end[x.B1(bb)], 1);
   }
-  __syncwarp();
+  big_sync<NW>();
   int carry = 0;
-  for (int base = 0; base < n; base += 32) {
+  for (int base = 0; tid < 32 && base < n; base += 32) {
     const int i = base + lane;
     const int c = i < n ? end[i] : 0;
     int s = c;
@@ -258,28 +335,28 @@ __device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, 
     }
     carry += __shfl_sync(FULL, s, 31);
   }
-  __syncwarp();
-  for (int k = lane; k < C; k += 32) {
+  big_sync<NW>();
+  for (int k = tid; k < C; k += T) {
     const int bb = x.pair(k);
     adj[atomicAdd(&end[x.B0(bb)], 1)] = k;
     if (x.B1(bb) >= 0) adj[atomicAdd(&end[x.B1(bb)], 1)] = k;
   }
-  __syncwarp();
+  big_sync<NW>();
   const int max_it = v.max_iterations >= 0 ? v.max_iterations : C * v.iter_mult;
   uint32_t err = 0;
-  const int pos_used = big_phase<R, W, false>(x, v, bstart, bk, off, end, adj, max_it, err);
-  __syncwarp();
+  const int pos_used = big_phase<R, W, false>(x, v, bstart, bk, off, end, adj, max_it, chg, err);
+  big_sync<NW>();
   if (v.contact_writeback)
-    for (int k = lane; k < C; k += 32) v.contact[C_PEN * v.nc_total + cst + k] = x.rec(k)[CR_PEN];
-  for (int k = lane; k < C; k += 32) friction_prepare(x, k);
-  __syncwarp();
-  const int vel_used = big_phase<R, W, true>(x, v, bstart, bk, off, end, adj, max_it, err);
-  __syncwarp();
+    for (int k = tid; k < C; k += T) v.contact[C_PEN * v.nc_total + cst + k] = x.rec(k)[CR_PEN];
+  for (int k = tid; k < C; k += T) friction_prepare(x, k);
+  big_sync<NW>();
+  const int vel_used = big_phase<R, W, true>(x, v, bstart, bk, off, end, adj, max_it, chg, err);
+  big_sync<NW>();
   if (err) {
     atomicOr(&v.world_status[w], err);
     atomicOr(v.status, err);
   }
-  if (lane == 0) {
+  if (tid == 0) {
     v.pos_iters[w] = pos_used;
     v.vel_iters[w] = vel_used;
     atomicAdd(&v.counters[1], (unsigned long long)pos_used);
@@ -287,12 +364,12 @@ __device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, 
     atomicAdd(&v.counters[3], (unsigned long long)C);
   }
   if (v.contact_writeback)
-    for (int k = lane; k < C; k += 32) write_back_contact(x, v, cst, k);
-  store_bodies(x, v, bstart, n, lane, 32);
+    for (int k = tid; k < C; k += T) write_back_contact(x, v, cst, k);
+  store_bodies(x, v, bstart, n, tid, T);
 }
 
 template <class R, class W>
-__global__ void __launch_bounds__(32, 4) k_resolve_big(BatchView<R> v, R dt, int csm) {
+__global__ void __launch_bounds__(32 * big_warps<R>(), big_warps<R>() > 1 ? 2 : 4) k_resolve_big(BatchView<R> v, R dt, int csm) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int w = v.big_list[blockIdx.x];
   int C = v.contact_count[w];
