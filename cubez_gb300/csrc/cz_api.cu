@@ -14,6 +14,7 @@
 #include <map>
 #include <numeric>
 #include <string>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -353,6 +354,49 @@ int finish(cz_batch* b) {
   return st;
 }
 
+// Copies between the caller's arrays and the pinned staging, in equal shares
+// of at least 1 MB on up to eight threads, which end with the call: one thread
+// copied, and faulted in the pages of fresh arrays, at 12 to 20 GB/s (147k
+// bodies up 2.42 -> 0.97 ms, down 2.88 -> 1.29; the state of 524k bodies down
+// 5.85 -> 2.20, of which a part is that only the fields asked for leave the GPU).
+struct HostCopy {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+struct HostCopies {
+  HostCopy c[20];
+  int n = 0;
+  void add(void* dst, const void* src, size_t bytes) { c[n++] = {dst, src, bytes}; }
+};
+void copy_share(const HostCopies& list, size_t from, size_t to) {
+  size_t at = 0;
+  for (int i = 0; i < list.n; ++i) {
+    const HostCopy& c = list.c[i];
+    const size_t a = std::max(from, at), e = std::min(to, at + c.bytes);
+    if (a < e) std::memcpy(static_cast<char*>(c.dst) + (a - at), static_cast<const char*>(c.src) + (a - at), e - a);
+    at += c.bytes;
+  }
+}
+void host_copy(const HostCopies& list) {
+  size_t total = 0;
+  for (int i = 0; i < list.n; ++i) total += list.c[i].bytes;
+  size_t shares = std::min<size_t>(total >> 20, 8);
+  if (shares > 1) shares = std::min<size_t>(shares, std::thread::hardware_concurrency());
+  shares = std::max<size_t>(shares, 1);
+  auto cut = [&](size_t q) { return total / 64 * q / shares * 64 + (q == shares ? total % 64 : 0); };
+  std::thread t[8];
+  size_t started = 1;  // share 0 is this thread's
+  try {
+    for (; started < shares; ++started)
+      t[started] = std::thread(copy_share, std::cref(list), cut(started), cut(started + 1));
+  } catch (...) {  // no more threads: the rest is this thread's too
+  }
+  copy_share(list, 0, cut(1));
+  if (started < shares) copy_share(list, cut(started), total);
+  for (size_t q = 1; q < started; ++q) t[q].join();
+}
+
 int reset_status(cz_batch* b) {
   CZ_CUDA(cudaMemsetAsync(b->d_status, 0, sizeof(uint32_t), b->stream));
   return CZ_OK;
@@ -364,10 +408,17 @@ int ensure_pows(cz_batch* b, double dt) {
   if (b->pow_dt == dt) return CZ_OK;
   const long long P = b->nb_pad;
   for (long long i = 0; i < 2 * P; ++i) b->h_pow[i] = 1.0;
+  // a pow for each run of equal values (by bits: -0 and NaN keep theirs), which
+  // is most of them: 2.78 -> 0.29 ms for 147k bodies
+  double lin = 0.0, ang = 0.0, lin_pow = 0.0, ang_pow = 0.0;
   for (long long h = 0; h < b->nb; ++h) {
     const long long p = b->h2p[h];
-    b->h_pow[p] = std::pow(b->lin_damp[h], dt);
-    b->h_pow[P + p] = std::pow(b->ang_damp[h], dt);
+    if (h == 0 || std::memcmp(&b->lin_damp[h], &lin, sizeof lin) != 0)
+      lin_pow = std::pow(lin = b->lin_damp[h], dt);
+    if (h == 0 || std::memcmp(&b->ang_damp[h], &ang, sizeof ang) != 0)
+      ang_pow = std::pow(ang = b->ang_damp[h], dt);
+    b->h_pow[p] = lin_pow;
+    b->h_pow[P + p] = ang_pow;
   }
   CZ_CUDA(cudaMemcpyAsync(b->d_pow, b->h_pow, sizeof(double) * 2 * P, cudaMemcpyHostToDevice, b->stream));
   CZ_CUDA(b->ops->set_rows(b->view(), cz::B_LINPOW, 2, b->d_pow, b->stream));
@@ -866,24 +917,27 @@ int cz_upload_bodies(cz_batch* b, const cz_bodies* in) {
     if (in->shape[h] != CZ_SHAPE_SPHERE && in->shape[h] != CZ_SHAPE_CUBE)
       return fail(CZ_ERR_BAD_ARG, "cz_upload_bodies: unknown shape");
   double* sg = b->h_stage;
-  std::memcpy(sg + cz::SG_POS * n, in->position, sizeof(double) * 3 * n);
-  std::memcpy(sg + cz::SG_Q * n, in->orientation, sizeof(double) * 4 * n);
-  std::memcpy(sg + cz::SG_VEL * n, in->velocity, sizeof(double) * 3 * n);
-  std::memcpy(sg + cz::SG_ROT * n, in->rotation, sizeof(double) * 3 * n);
-  std::memcpy(sg + cz::SG_ACC * n, in->acceleration, sizeof(double) * 3 * n);
-  std::memcpy(sg + cz::SG_IB * n, in->inverse_inertia, sizeof(double) * 9 * n);
-  std::memcpy(sg + cz::SG_INVM * n, in->inverse_mass, sizeof(double) * n);
-  if (in->motion) std::memcpy(sg + cz::SG_MOTION * n, in->motion, sizeof(double) * n);
-  else for (long long h = 0; h < n; ++h) sg[cz::SG_MOTION * n + h] = 0.3 * 2.0;
-  std::memcpy(sg + cz::SG_HALF * n, in->half_size, sizeof(double) * 3 * n);
-  std::memcpy(sg + cz::SG_RAD * n, in->radius, sizeof(double) * n);
   const int has_iw = in->inverse_inertia_world != nullptr;
   const int has_lfa = in->last_frame_acceleration != nullptr;
-  if (has_iw) std::memcpy(sg + cz::SG_IW * n, in->inverse_inertia_world, sizeof(double) * 9 * n);
-  if (has_lfa) std::memcpy(sg + cz::SG_LFA * n, in->last_frame_acceleration, sizeof(double) * 3 * n);
-  std::memcpy(b->h_stage_u8, in->is_awake, n);
-  std::memcpy(b->h_stage_u8 + n, in->can_sleep, n);
-  std::memcpy(b->h_stage_i32, in->shape, sizeof(int) * n);
+  HostCopies list;
+  auto add = [&](int blk, const double* src, int width) {
+    if (src) list.add(sg + (long long)blk * n, src, sizeof(double) * width * n);
+  };
+  add(cz::SG_POS, in->position, 3);
+  add(cz::SG_Q, in->orientation, 4);
+  add(cz::SG_VEL, in->velocity, 3);
+  add(cz::SG_ROT, in->rotation, 3);
+  add(cz::SG_ACC, in->acceleration, 3);
+  add(cz::SG_IB, in->inverse_inertia, 9);
+  add(cz::SG_INVM, in->inverse_mass, 1);
+  add(cz::SG_MOTION, in->motion, 1);
+  add(cz::SG_HALF, in->half_size, 3);
+  add(cz::SG_RAD, in->radius, 1);
+  add(cz::SG_IW, in->inverse_inertia_world, 9);
+  add(cz::SG_LFA, in->last_frame_acceleration, 3);
+  list.add(b->h_stage_u8, in->is_awake, (size_t)n);
+  list.add(b->h_stage_u8 + n, in->can_sleep, (size_t)n);
+  list.add(b->h_stage_i32, in->shape, sizeof(int) * n);
   const bool has_off = in->collider_offset != nullptr;
   if (has_off && !b->d_offset) {
     const size_t rows = b->ops->real_size * 12 * std::max<long long>(b->nb_pad, 1);
@@ -905,15 +959,25 @@ int cz_upload_bodies(cz_batch* b, const cz_bodies* in) {
     drop_graphs(b);  // the narrowphase's view changes
     b->has_offset = has_off;
   }
+  if (has_off) list.add(b->h_off_stage, in->collider_offset, sizeof(double) * 12 * n);
+  host_copy(list);
+  if (!in->motion)
+    for (long long h = 0; h < n; ++h) sg[cz::SG_MOTION * n + h] = 0.3 * 2.0;
   if (has_off) {
-    std::memcpy(b->h_off_stage, in->collider_offset, sizeof(double) * 12 * n);
     CZ_CUDA(cudaMemcpyAsync(b->d_off_stage, b->h_off_stage, sizeof(double) * 12 * n, cudaMemcpyHostToDevice,
                             b->stream));
   }
   b->lin_damp.assign(in->linear_damping, in->linear_damping + n);
   b->ang_damp.assign(in->angular_damping, in->angular_damping + n);
   b->pow_dt = std::nan("");
-  CZ_CUDA(cudaMemcpyAsync(b->d_stage, sg, sizeof(double) * cz::SG_NDOUBLES * n, cudaMemcpyHostToDevice, b->stream));
+  // the blocks the caller gave: all up to SG_IW, and the last two
+  auto send = [&](int blk, int width) {
+    const long long at = (long long)blk * n;
+    return cudaMemcpyAsync(b->d_stage + at, sg + at, sizeof(double) * width * n, cudaMemcpyHostToDevice, b->stream);
+  };
+  CZ_CUDA(send(0, cz::SG_IW));
+  if (has_iw) CZ_CUDA(send(cz::SG_IW, 9));
+  if (has_lfa) CZ_CUDA(send(cz::SG_LFA, 3));
   CZ_CUDA(cudaMemcpyAsync(b->d_stage_u8, b->h_stage_u8, 2 * n, cudaMemcpyHostToDevice, b->stream));
   CZ_CUDA(cudaMemcpyAsync(b->d_stage_i32, b->h_stage_i32, sizeof(int) * n, cudaMemcpyHostToDevice, b->stream));
   CZ_CUDA(b->ops->upload(b->view(), b->d_stage, b->d_stage_u8, b->d_stage_i32, b->d_h2p, (int)n, has_iw, has_lfa,
@@ -935,38 +999,51 @@ int cz_download_bodies(cz_batch* b, cz_bodies* out) {
   if (want_off)
     CZ_CUDA(cudaMemcpyAsync(b->h_off_stage, b->d_off_stage, sizeof(double) * 12 * n, cudaMemcpyDeviceToHost,
                             b->stream));
-  CZ_CUDA(cudaMemcpyAsync(b->h_stage, b->d_stage, sizeof(double) * cz::SG_NDOUBLES * n, cudaMemcpyDeviceToHost,
-                          b->stream));
-  CZ_CUDA(cudaMemcpyAsync(b->h_stage_u8, b->d_stage_u8, 2 * n, cudaMemcpyDeviceToHost, b->stream));
-  CZ_CUDA(cudaMemcpyAsync(b->h_stage_i32, b->d_stage_i32, sizeof(int) * n, cudaMemcpyDeviceToHost, b->stream));
-  CZ_CUDA(cudaStreamSynchronize(b->stream));
-  const double* sg = b->h_stage;
-  auto cp = [&](double* dst, int blk, int width) {
-    if (dst) std::memcpy(dst, sg + (long long)blk * n, sizeof(double) * width * n);
+  // only the blocks the caller wants, in one copy where what lies between is short
+  const struct {
+    int blk, width;
+    double* dst;
+  } fields[] = {{cz::SG_POS, 3, out->position},        {cz::SG_Q, 4, out->orientation},
+                {cz::SG_VEL, 3, out->velocity},        {cz::SG_ROT, 3, out->rotation},
+                {cz::SG_ACC, 3, out->acceleration},    {cz::SG_IB, 9, out->inverse_inertia},
+                {cz::SG_INVM, 1, out->inverse_mass},   {cz::SG_MOTION, 1, out->motion},
+                {cz::SG_HALF, 3, out->half_size},      {cz::SG_RAD, 1, out->radius},
+                {cz::SG_IW, 9, out->inverse_inertia_world},
+                {cz::SG_LFA, 3, out->last_frame_acceleration}};
+  HostCopies list;
+  int first = 0, next = 0;  // blocks [first, next) are still to be copied
+  auto fetch = [&]() {
+    const long long at = (long long)first * n;
+    if (first == next) return cudaSuccess;
+    return cudaMemcpyAsync(b->h_stage + at, b->d_stage + at, sizeof(double) * (next - first) * n,
+                           cudaMemcpyDeviceToHost, b->stream);
   };
-  cp(out->position, cz::SG_POS, 3);
-  cp(out->orientation, cz::SG_Q, 4);
-  cp(out->velocity, cz::SG_VEL, 3);
-  cp(out->rotation, cz::SG_ROT, 3);
-  cp(out->acceleration, cz::SG_ACC, 3);
-  cp(out->inverse_inertia, cz::SG_IB, 9);
-  cp(out->inverse_mass, cz::SG_INVM, 1);
-  cp(out->motion, cz::SG_MOTION, 1);
-  cp(out->half_size, cz::SG_HALF, 3);
-  cp(out->radius, cz::SG_RAD, 1);
-  cp(out->inverse_inertia_world, cz::SG_IW, 9);
-  cp(out->last_frame_acceleration, cz::SG_LFA, 3);
-  if (out->linear_damping) std::memcpy(out->linear_damping, b->lin_damp.data(), sizeof(double) * n);
-  if (out->angular_damping) std::memcpy(out->angular_damping, b->ang_damp.data(), sizeof(double) * n);
-  if (out->is_awake) std::memcpy(out->is_awake, b->h_stage_u8, n);
-  if (out->can_sleep) std::memcpy(out->can_sleep, b->h_stage_u8 + n, n);
-  if (want_off) {
-    std::memcpy(out->collider_offset, b->h_off_stage, sizeof(double) * 12 * n);
-  } else if (out->collider_offset) {
+  for (const auto& f : fields) {
+    if (!f.dst) continue;
+    list.add(f.dst, b->h_stage + (long long)f.blk * n, sizeof(double) * f.width * n);
+    if (sizeof(double) * (f.blk - next) * n > 32768) {
+      CZ_CUDA(fetch());
+      first = f.blk;
+    }
+    next = f.blk + f.width;
+  }
+  CZ_CUDA(fetch());
+  if (out->is_awake || out->can_sleep)
+    CZ_CUDA(cudaMemcpyAsync(b->h_stage_u8, b->d_stage_u8, 2 * n, cudaMemcpyDeviceToHost, b->stream));
+  if (out->shape)
+    CZ_CUDA(cudaMemcpyAsync(b->h_stage_i32, b->d_stage_i32, sizeof(int) * n, cudaMemcpyDeviceToHost, b->stream));
+  if (out->linear_damping) list.add(out->linear_damping, b->lin_damp.data(), sizeof(double) * n);
+  if (out->angular_damping) list.add(out->angular_damping, b->ang_damp.data(), sizeof(double) * n);
+  if (out->is_awake) list.add(out->is_awake, b->h_stage_u8, (size_t)n);
+  if (out->can_sleep) list.add(out->can_sleep, b->h_stage_u8 + n, (size_t)n);
+  if (out->shape) list.add(out->shape, b->h_stage_i32, sizeof(int) * n);
+  if (want_off) list.add(out->collider_offset, b->h_off_stage, sizeof(double) * 12 * n);
+  CZ_CUDA(cudaStreamSynchronize(b->stream));
+  host_copy(list);
+  if (out->collider_offset && !want_off) {
     static const double id[12] = {1, 0, 0, 0, 1, 0, 0, 0, 1, 0, 0, 0};
     for (long long h = 0; h < n; ++h) std::memcpy(out->collider_offset + 12 * h, id, sizeof id);
   }
-  if (out->shape) std::memcpy(out->shape, b->h_stage_i32, sizeof(int) * n);
   return CZ_OK;
 }
 
