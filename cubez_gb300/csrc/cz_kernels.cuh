@@ -553,7 +553,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 constexpr int kSurvivors = 1280;
 // np_flush's scratch for a CTA of bd threads: the box pairs' penetrations,
 // outcomes and the unit that holds them, the chunk's order by kind of test, its
-// counts, and per-kind counts of each warp (6 kinds x 8 warps)
+// counts, and per-kind counts of each warp (7 kinds x 8 warps)
 template <class R> __host__ __device__ constexpr int np_sort_ints(int bd) {
   return (int)(sizeof(R) / 4) * bd + 4 * bd + 64;
 }
@@ -675,7 +675,8 @@ __device__ __forceinline__ void np_emit(const BatchView<R>& v, long long cs, int
 // half-space, else the pair with j = k - 1, skipping i), in chunks of the
 // CTA's size, emitting their contacts in list order at out onwards.  Within a
 // chunk the units are taken in order of their kind of test (half-space with a
-// sphere, with a cube; sphere-sphere, sphere-cube, cube-cube), stably, so the
+// sphere, with a cube; sphere-sphere, sphere-cube, cube-cube with i < j, then
+// with i > j, which mostly take the other order's axes), stably, so the
 // lanes of a warp mostly run one test's code; the counts are then scanned in
 // list order, so every contact lands where the list order puts it (the
 // reference's contact order).  The two tests with many parts are spread over
@@ -684,8 +685,8 @@ __device__ __forceinline__ void np_emit(const BatchView<R>& v, long long cs, int
 // axes take sixteen (sat_axes).  On a thread each, a warp ran the eight
 // vertices twice (count, write) and the fifteen axes one after the other for
 // whatever few lanes had them.  Narrowphase of 8192 worlds x 32 bodies, float64
-// 1.50 -> 0.73 ms a frame, float32 0.176 -> 0.170; of one world of 20 cubes in
-// float64 84 -> 43 us.  sortw: np_sort_ints(blockDim.x) ints.
+// 1.50 -> 0.69 ms a frame (0.73 with the two orders of the pairs mixed); of one
+// world of 20 cubes in float64 84 -> 39 us.  sortw: np_sort_ints(blockDim.x) ints.
 template <class R>
 __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart, int n, long long cs, int cap,
                          const int* surv, int nsurv, int* scan, int& parity, int& out, uint32_t& err, int* sortw) {
@@ -698,7 +699,7 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
   int* wcnt = cntb + bd;  // [kind * 8 + warp]
   for (int sb = 0; sb < nsurv; sb += bd) {
     const int m = nsurv - sb < bd ? nsurv - sb : bd;
-    int key = 5;  // no unit
+    int key = 6;  // no unit
     if (tid < m) {
       const int uu = surv[sb + tid];
       const int i = uu / n, k = uu - i * n;
@@ -708,11 +709,12 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
         int j = k - 1;
         if (j >= i) ++j;
         key = 2 + (tl.shape[i] != 0 ? 1 : 0) + (tl.shape[j] != 0 ? 1 : 0);
+        if (key == 4 && i > j) key = 5;
       }
     }
     int rank = 0;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) {
+    for (int q = 0; q < 7; ++q) {
       const unsigned bal = __ballot_sync(FULL, key == q);
       if (key == q) rank = __popc(bal & ((1u << lane) - 1u));
       if (lane == 0) wcnt[q * 8 + wid] = __popc(bal);
@@ -721,11 +723,13 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
     int dst = rank, n0 = 0, n1 = 0, n23 = 0, n4 = 0;
     for (int w2 = 0; w2 < nwarps; ++w2) {
       const int a = wcnt[w2], b = wcnt[8 + w2], c2 = wcnt[16 + w2], c3 = wcnt[24 + w2], d = wcnt[32 + w2];
+      const int e = wcnt[40 + w2];
       n0 += a;
       n1 += b;
       n23 += c2 + c3;
-      n4 += d;
-      dst += (key > 0 ? a : 0) + (key > 1 ? b : 0) + (key > 2 ? c2 : 0) + (key > 3 ? c3 : 0) + (key > 4 ? d : 0);
+      n4 += d + e;
+      dst += (key > 0 ? a : 0) + (key > 1 ? b : 0) + (key > 2 ? c2 : 0) + (key > 3 ? c3 : 0) + (key > 4 ? d : 0) +
+             (key > 5 ? e : 0);
       if (w2 < wid) dst += wcnt[key * 8 + w2];
     }
     perm[dst] = tid;
