@@ -339,7 +339,7 @@ static int warm_features_blocks(int nbs) {
 
 static cudaError_t resolve_big(const HostView& h, int nbig, int csm, size_t smem, double dt, cudaStream_t s) {
   if (nbig <= 0) return cudaSuccess;
-  k_resolve_big<R, W><<<nbig, 32 * big_warps<R>(), smem, s>>>(view_of(h), (R)dt, csm);
+  k_resolve_big<R, W><<<nbig, kBigThreads, smem, s>>>(view_of(h), (R)dt, csm);
   return cudaGetLastError();
 }
 
