@@ -164,6 +164,7 @@ struct cz_batch {
   int warm_shift = 2;        // warm-start worlds whose last solve used <= max_it >> warm_shift
   size_t np_smem = 0, rs_smem = 0;  // per narrowphase CTA; per resolver warp
   int rs_wpc = 1;                    // warps per resolver CTA
+  bool rs_cs_set = false;            // the caller chose rs_cs (tile_rule otherwise)
   size_t wide_smem = 0;              // k_resolve_wide's shared memory per world (0: not used)
   int wide_cs = 0;                   // its contact tile
 
@@ -542,6 +543,18 @@ int part_rule(int form, int num_worlds) {
   return std::max(1, std::min(num_worlds / 64, form == CZ_FORM_FP64 ? 32 : 8));
 }
 
+// Contacts of the resolver's shared-memory tile: three a body, which a settled
+// heap of cubes reaches (2.6 to 2.8), at least 96.  A world with more keeps all
+// its records in global memory, and its iterations then load through what L1
+// the tiles leave: 4096 worlds of 62 bodies x 10 frames, float32, took 29.4 ms
+// with 96 and 22.6 with 192 although 9 worlds fit an SM then instead of 12; 48
+// bodies 16.2 and 14.0 (160), 40 bodies 11.0 and 9.6 (128); 4096 worlds of 8 to
+// 64 bodies x 30 45.1 and 39.1.  More than that only costs occupancy: 16384
+// worlds of 32 bodies x 30 51.2 with 96, 52.9 with 128.  float64: 1024 x 62
+// bodies 35.9 -> 31.6, 4096 x 8 to 64 125.5 -> 124.8.  Narrower groups have
+// several worlds' tiles to a warp, and stay with 96.
+int tile_rule(int nbs, int lanes) { return lanes < 32 ? 96 : std::max(96, (int)round_up(3 * nbs, 32)); }
+
 // The captured graphs hold the kernels' parameters (the batch view); drop them
 // whenever those change.
 void drop_graphs(cz_batch* b) {
@@ -556,6 +569,7 @@ void drop_graphs(cz_batch* b) {
 
 int configure(cz_batch* b) {
   // resolver shared-memory tile: shrink the contact capacity until it fits
+  if (!b->rs_cs_set) b->rs_cs = tile_rule(b->rs_nbs, b->run_lanes());
   int cs = std::min<long long>(b->rs_cs, round_up(b->max_cap, 32));
   cs = std::max(cs, 32);
   while (cs > 32 && b->ops->rs_smem(b->rs_nbs, cs, b->run_lanes()) > b->smem_optin) cs -= 32;
@@ -727,7 +741,6 @@ int cz_batch_create(const cz_batch_desc* d, cz_batch** out) {
   b->np_threads = b->max_n >= 256 ? 256 : 128;
   // a world per warp: its islands share the warp's instructions (the tuner may
   // change it)
-  b->rs_cs = 96;
   b->rs_lanes = 32;
   // world queue: decreasing body count (pair work grows as n^2)
   std::vector<int> order(b->num_worlds);
@@ -853,7 +866,10 @@ int cz_set_tuning(cz_batch* b, const cz_tuning* t) {
       return fail(CZ_ERR_BAD_ARG, "narrowphase_threads must be a multiple of 32, at most 256");
     b->np_threads = t->narrowphase_threads;
   }
-  if (t->resolver_contacts > 0) b->rs_cs = (int)round_up(t->resolver_contacts, 32);
+  if (t->resolver_contacts > 0) {
+    b->rs_cs = (int)round_up(t->resolver_contacts, 32);
+    b->rs_cs_set = true;
+  }
   if (t->resolver_lanes > 0) {
     if (t->resolver_lanes != 4 && t->resolver_lanes != 8 && t->resolver_lanes != 16 && t->resolver_lanes != 32)
       return fail(CZ_ERR_BAD_ARG, "resolver_lanes must be 4, 8, 16 or 32");
