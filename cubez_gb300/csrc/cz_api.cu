@@ -166,7 +166,7 @@ struct cz_batch {
   int rs_wpc = 1;                    // warps per resolver CTA
   bool rs_cs_set = false;            // the caller chose rs_cs (tile_rule otherwise)
   size_t wide_smem = 0;              // k_resolve_wide's shared memory per world (0: not used)
-  int wide_cs = 0;                   // its contact tile
+  int wide_cs = 0, wide_per_sm = 0;  // its contact tile, worlds per SM (wide_rule)
 
   // graph cache: (nsteps, dt) -> executable graph
   std::map<std::pair<int, double>, cudaGraphExec_t> graphs;
@@ -496,7 +496,7 @@ int launch_resolve(cz_batch* b, const Chain& c, double dt, bool reset) {
       g_launches++;
     }
     if (b->wide_smem > 0 && c.v.mode == 0)
-      CZ_CUDA(b->ops->resolve_wide(c.v, b->rs_nbs, b->wide_cs, std::min(c.nsmall, b->sm_count), b->wide_smem, dt, c.s));
+      CZ_CUDA(b->ops->resolve_wide(c.v, b->rs_nbs, b->wide_cs, b->wide_per_sm, c.nsmall, b->wide_smem, dt, c.s));
     else
       CZ_CUDA(b->ops->resolve(c.v, b->rs_nbs, b->rs_cs, b->run_lanes(),
                               chain_grid(c.v.num_worlds, worlds_per_warp * b->rs_wpc, b->rs_grid), b->rs_wpc,
@@ -555,6 +555,24 @@ int part_rule(int form, int num_worlds) {
 // several worlds' tiles to a warp, and stay with 96.
 int tile_rule(int nbs, int lanes) { return lanes < 32 ? 96 : std::max(96, (int)round_up(3 * nbs, 32)); }
 
+// Worlds per SM that k_resolve_wide holds, four warps to each; 0: k_resolve
+// takes the batch, one warp to a world.  Up to one world per SM that is where
+// they have more than a dozen bodies: one world of 20 cubes, float64, 278 ->
+// 215 us a frame; 61 worlds of 8 to 64 bodies, float32, 604 -> 494; 150 of 62
+// bodies x 20 frames, float64, 28.1 -> 24.8 ms (150 of 8, float32, 2.18 ->
+// 2.24: few islands, and one warp is as good).  Up to three worlds per SM where
+// their tiles leave an SM few warps otherwise, x 10 frames: 450 of 62 bodies,
+// float64 34.4 -> 26.5 ms, float32 13.4 -> 11.4; 450 of 8 to 64 33.4 -> 23.3 and
+// 11.9 -> 9.4; but 300 freshly landed ones of 24 bodies x 3, float32, 0.47 ->
+// 0.49.  Beyond, fresh worlds of few contacts do with one warp (600 of 31 bodies
+// x 4, float32, 1.16 -> 1.20 ms), and with many worlds one warp is better
+// throughout (4096 of 62, 11.8 -> 14.3).
+int wide_rule(int worlds, int nbs, int lanes, int sms) {
+  if (lanes != 32 || worlds <= 0) return 0;
+  const int per_sm = (worlds + sms - 1) / sms;
+  return (per_sm == 1 && nbs >= 16) || (per_sm <= 3 && nbs >= 36) ? per_sm : 0;
+}
+
 // The captured graphs hold the kernels' parameters (the batch view); drop them
 // whenever those change.
 void drop_graphs(cz_batch* b) {
@@ -598,19 +616,19 @@ int configure(cz_batch* b) {
       b->rs_wpc = wpc;
     }
   }
-  // Four warps to a world where every world has an SM to itself and is of more
-  // than a dozen bodies: one world of 20 cubes, float64, 278 -> 215 us a frame;
-  // 61 worlds of 8 to 64 bodies, float32, 604 -> 494; 150 worlds of 62 bodies x
-  // 20 frames, 28.1 -> 24.8 ms in float64.  Worlds of few bodies have few
-  // islands, and one warp is as good: 150 of 8 bodies, float32, 2.18 -> 2.24 ms.
-  // The tile holds eight contacts a body, with their friction matrices.
+  // Four warps to a world (wide_rule), in tiles of eight contacts a body with
+  // their friction matrices, or what lets the SMs hold all the worlds at once.
   b->wide_smem = 0;
-  if (lanes == 32 && b->rs_nbs >= 16 && b->nsmall > 0 && b->nsmall <= b->sm_count) {
+  const int per_sm = wide_rule(b->nsmall, b->rs_nbs, lanes, b->sm_count);
+  if (per_sm > 0) {
     b->wide_cs = std::max(b->rs_cs, std::min((int)round_up(b->max_cap, 32), 8 * b->rs_nbs));
-    while (b->wide_cs > b->rs_cs && b->ops->wide_smem(b->rs_nbs, b->wide_cs) > b->smem_optin) b->wide_cs -= 32;
+    while (b->wide_cs > b->rs_cs &&
+           (b->ops->wide_smem(b->rs_nbs, b->wide_cs) + 1024) * per_sm > b->smem_optin + 1024)
+      b->wide_cs -= 32;
     const size_t bytes = b->ops->wide_smem(b->rs_nbs, b->wide_cs);
     if (bytes <= b->smem_optin) {
-      CZ_CUDA(b->ops->wide_prepare(bytes));
+      CZ_CUDA(b->ops->wide_prepare(per_sm, bytes));
+      b->wide_per_sm = per_sm;
       b->wide_smem = bytes;
     }
   }

@@ -274,9 +274,16 @@ static cudaError_t resolve(const HostView& h, int nbs, int cs, int lanes, int gr
 }
 
 static size_t wide_smem(int nbs, int cs) { return wide_smem_bytes<R, W>(nbs, cs); }
-static cudaError_t wide_prepare(size_t smem) { return raise_smem_limit((const void*)k_resolve_wide<R, W>, smem); }
-static cudaError_t resolve_wide(const HostView& h, int nbs, int cs, int grid, size_t smem, double dt, cudaStream_t s) {
-  k_resolve_wide<R, W><<<grid, 32 * kWideWarps, smem, s>>>(view_of(h), nbs, cs, (R)dt);
+static const void* wide_kernel(int per_sm) {
+  return per_sm == 1 ? (const void*)k_resolve_wide<R, W, 1> : (const void*)k_resolve_wide<R, W, 3>;
+}
+static cudaError_t wide_prepare(int per_sm, size_t smem) { return raise_smem_limit(wide_kernel(per_sm), smem); }
+static cudaError_t resolve_wide(const HostView& h, int nbs, int cs, int per_sm, int grid, size_t smem, double dt,
+                                cudaStream_t s) {
+  if (per_sm == 1)
+    k_resolve_wide<R, W, 1><<<grid, 32 * kWideWarps, smem, s>>>(view_of(h), nbs, cs, (R)dt);
+  else
+    k_resolve_wide<R, W, 3><<<grid, 32 * kWideWarps, smem, s>>>(view_of(h), nbs, cs, (R)dt);
   return cudaGetLastError();
 }
 

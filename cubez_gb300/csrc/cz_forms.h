@@ -100,10 +100,11 @@ struct FormOps {
   // grid CTAs of wpc warps each, smem bytes per warp
   cudaError_t (*resolve)(const HostView& v, int nbs, int cs, int lanes, int grid, int wpc, size_t smem, double dt,
                          cudaStream_t s);
-  // four warps to a world, for batches of fewer worlds than SMs (k_resolve_wide)
+  // four warps to a world, for small batches (k_resolve_wide)
   size_t (*wide_smem)(int nbs, int cs);
-  cudaError_t (*wide_prepare)(size_t smem);
-  cudaError_t (*resolve_wide)(const HostView& v, int nbs, int cs, int grid, size_t smem, double dt, cudaStream_t s);
+  cudaError_t (*wide_prepare)(int per_sm, size_t smem);
+  cudaError_t (*resolve_wide)(const HostView& v, int nbs, int cs, int per_sm, int grid, size_t smem, double dt,
+                              cudaStream_t s);
   // `off` ([n][12] doubles, the collider Offsets) may be null; the upload
   // writes the Offset rows only when both it and v.offset are set
   cudaError_t (*upload)(const HostView& v, const double* stage, const uint8_t* u8, const int* i32, const int* h2p,

@@ -1996,15 +1996,16 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
 
 
 // ---------------------------------------------------------------- k_resolve_wide
-// The resolver for batches of fewer worlds than SMs: four warps to a world,
+// The resolver for batches of up to three worlds per SM: four warps to a world,
 // one CTA each.  With one warp a small batch leaves three of an SM's four
 // schedulers idle, and in float64 each scheduler has its own quarter of the
 // SM's float64 rate, so a warp on its own is bound by its scheduler's unit.
 // The preparation is split over the warps, and so are the world's islands
-// (side by side within a warp where there are more than warps); bodies, records, friction matrices and
-// lists are in shared memory, which such a batch has to spare.  A world whose
-// islands want more iterations than its budget is put back and solved as one
-// list by the first warp, as in resolve_worlds.
+// (side by side within a warp where there are more than warps); bodies,
+// records, friction matrices and lists are in shared memory, which such a batch
+// has to spare.  A world whose islands want more iterations than its budget
+// goes on as in resolve_worlds, the one island and the one list by the first
+// warp.
 constexpr int kWideWarps = 4;
 // What the warps share: the next island, the iterations (resolve_phase), then
 // per call the sum of the iterations, the most rounds, whether a warp met the
@@ -2095,8 +2096,10 @@ __device__ __forceinline__ Progress wide_phase(const RCtx<R, W, true>& x, const 
   return pr;
 }
 
-template <class R, class W>
-__global__ void __launch_bounds__(32 * kWideWarps, 1) k_resolve_wide(BatchView<R> v, int nbs, int cs, R dt) {
+// PER_SM worlds fit an SM's registers: one of its own keeps 1.5 % with the
+// registers it wants (float64 180, float32 179; three leave 168).
+template <class R, class W, int PER_SM>
+__global__ void __launch_bounds__(32 * kWideWarps, PER_SM) k_resolve_wide(BatchView<R> v, int nbs, int cs, R dt) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int T = 32 * kWideWarps;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;

@@ -1,4 +1,4 @@
-"""Batches of fewer worlds than SMs are resolved with four warps to a world
+"""Batches of up to three worlds per SM are resolved with four warps to a world
 (k_resolve_wide): the same bits as the same worlds give in a larger batch, one
 warp to a world, with budgets that run out, sleeping bodies, worlds of one to
 many islands, empty worlds, and contact lists past the shared tile."""
@@ -32,7 +32,7 @@ def _scene(worlds, seed):
 
 
 @pytest.mark.parametrize("form", [0, 1])
-@pytest.mark.parametrize("worlds,budget", [(8, 0), (40, 0), (150, 0), (40, 1), (40, 30), (40, 200)])
+@pytest.mark.parametrize("worlds,budget", [(8, 0), (40, 0), (150, 0), (400, 0), (40, 1), (40, 30), (40, 200)])
 def test_wide_equals_one_warp_per_world(form, worlds, budget, cuda_lib):
     from cubez_gb300.batch import WorldBatch
     scene = _scene(worlds, 90 + worlds)
