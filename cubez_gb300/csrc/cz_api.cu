@@ -564,13 +564,16 @@ int tile_rule(int nbs, int lanes) { return lanes < 32 ? 96 : std::max(96, (int)r
 // their tiles leave an SM few warps otherwise, x 10 frames: 450 of 62 bodies,
 // float64 34.4 -> 26.5 ms, float32 13.4 -> 11.4; 450 of 8 to 64 33.4 -> 23.3 and
 // 11.9 -> 9.4; but 300 freshly landed ones of 24 bodies x 3, float32, 0.47 ->
-// 0.49.  Beyond, fresh worlds of few contacts do with one warp (600 of 31 bodies
-// x 4, float32, 1.16 -> 1.20 ms), and with many worlds one warp is better
-// throughout (4096 of 62, 11.8 -> 14.3).
+// 0.49.  Up to seven per SM (three at a time) where they are nearly the largest:
+// 1000 of 62 settled bodies x 3, float64 12.8 -> 11.1 ms, float32 4.62 -> 4.27,
+// of 8 to 64 float32 4.70 -> 3.73, fresh ones the same; 1000 of 40 gain 5 to 10 %
+// settled and lose 4 fresh.  With many worlds one warp is better throughout
+// (4096 of 62, float32, 11.8 -> 14.3).
 int wide_rule(int worlds, int nbs, int lanes, int sms) {
   if (lanes != 32 || worlds <= 0) return 0;
   const int per_sm = (worlds + sms - 1) / sms;
-  return (per_sm == 1 && nbs >= 16) || (per_sm <= 3 && nbs >= 36) ? per_sm : 0;
+  if (per_sm == 1) return nbs >= 16 ? 1 : 0;
+  return (per_sm <= 3 && nbs >= 36) || (per_sm <= 7 && nbs >= 52) ? std::min(per_sm, 3) : 0;
 }
 
 // The captured graphs hold the kernels' parameters (the batch view); drop them

@@ -32,11 +32,11 @@ def _scene(worlds, seed):
 
 
 @pytest.mark.parametrize("form", [0, 1])
-@pytest.mark.parametrize("worlds,budget", [(8, 0), (40, 0), (150, 0), (400, 0), (40, 1), (40, 30), (40, 200)])
+@pytest.mark.parametrize("worlds,budget", [(8, 0), (40, 0), (150, 0), (400, 0), (700, 0), (40, 1), (40, 30), (40, 200)])
 def test_wide_equals_one_warp_per_world(form, worlds, budget, cuda_lib):
     from cubez_gb300.batch import WorldBatch
     scene = _scene(worlds, 90 + worlds)
-    filler = scenes.precision(num_worlds=600, bodies=2, seed=5)
+    filler = scenes.precision(num_worlds=1200, bodies=2, seed=5)
     both = scenes.Scene.concat([scene, filler])
     kw = {"form": form, "max_iterations": budget, "contact_capacity": 1024}
     a, b = WorldBatch.from_scene(scene, **kw), WorldBatch.from_scene(both, **kw)
