@@ -1,8 +1,9 @@
 // Kernels of the batched rigid-body step, templated on the bulk type R and the
 // island type W (plain form: double/double; precision form: float/double).
 //
-//   k_integrate    one thread per body: RigidBody.Integrate +
-//                  CalculateDerivedData (rigidbody.go:213-299)
+//   k_integrate    one thread per body (four in small float64 batches):
+//                  RigidBody.Integrate + CalculateDerivedData
+//                  (rigidbody.go:213-299)
 //   k_narrowphase  one CTA per world, worlds pulled from a device queue; body
 //                  rows staged in shared memory with bulk async copies; the
 //                  plane test and all ordered pairs in the reference's loop
@@ -91,6 +92,110 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_integrate(Batch
   if (i < 4) v.queue[i] = 0;
   if (i >= v.nb_run) return;
   integrate_body<R, W>(v, v.first_body + i, dt, sleep_bias);
+}
+
+// integrate_body by four lanes, for small float64 batches: lane c (c < 3) has
+// component c of the vectors and row c of the world inertia, lane c (c < 4)
+// component c of the quaternion; what a sum needs whole meets by shuffles.
+// Each component is the one-lane formula's.  A float64 warp instruction costs
+// its scheduler the same for any mask, and a body on one lane takes about 300
+// of them, on four 110.  Every lane of the warp calls it; `valid` where i is a
+// body.
+template <class R>
+__device__ __forceinline__ void integrate_body_spread(const BatchView<R>& v, long long i, bool valid, R dt,
+                                                      R sleep_bias) {
+  const int c4 = threadIdx.x & 3, c = c4 != 3 ? c4 : 0;
+  const bool on = valid && v.awake[i];  // rigidbody.go:214-216
+  const bool sleeps = on && v.can_sleep[i];
+  const long long S = v.nb_pad;
+  R* b = v.body + i;
+#define F(r) b[(long long)(r) * S]
+  const R zero = (R)0;
+  R lfa = zero, vel = zero, rot = zero, pos = zero, acc = zero, motion = zero;
+  R i0 = zero, i1 = zero, i2 = zero, i3 = zero, i4 = zero, i5 = zero, i6 = zero, i7 = zero, i8 = zero;
+  if (on) {
+    lfa = F(B_AX + c) + zero * F(B_INVM);
+    const R ang = F(B_IW0 + c) * zero + F(B_IW0 + 3 + c) * zero + F(B_IW0 + 6 + c) * zero;
+    vel = (F(B_VX + c) + lfa * dt) * F(B_LINPOW);
+    rot = (F(B_RX + c) + ang * dt) * F(B_ANGPOW);
+    pos = F(B_PX + c) + vel * dt;
+    acc = F(B_QW + c4);
+    i0 = F(B_IB0); i1 = F(B_IB0 + 1); i2 = F(B_IB0 + 2);
+    i3 = F(B_IB0 + 3); i4 = F(B_IB0 + 4); i5 = F(B_IB0 + 5);
+    i6 = F(B_IB0 + 6); i7 = F(B_IB0 + 7); i8 = F(B_IB0 + 8);
+    if (sleeps) motion = F(B_MOTION);
+  }
+  auto get = [&](R a, int from) { return __shfl_sync(FULL, a, from, 4); };
+  // Quaternion.AddScaledVector (quaternion.go:18-33): component c4 of (0, rot dt) * q
+  {
+    const R turn = rot * dt;
+    const R q1 = get(acc, c4 == 0 ? 1 : 0), q2 = get(acc, c4 == 1 ? 3 : (c4 == 2 ? 1 : 2));
+    const R q3 = get(acc, c4 == 1 ? 2 : (c4 == 3 ? 1 : 3));
+    const R u1 = get(turn, c4 < 2 ? 0 : c4 - 1), u2 = get(turn, c4 < 2 ? 1 : (c4 == 2 ? 2 : 0));
+    const R u3 = get(turn, c4 < 2 ? 2 : c4 - 2);
+    const R a1 = u1 * q1, a2 = u2 * q2, a3 = u3 * q3;
+    R t = zero * acc;
+    t = c4 == 0 ? t - a1 : t + a1;
+    t = c4 == 0 ? t - a2 : t + a2;
+    t = t - a3;
+    acc += t * (R)0.5;
+  }
+  // CalculateDerivedData: renormalise, transform, world inertia (row c)
+  {
+    const R sq = acc * acc;
+    const R s0 = get(sq, 0), s1 = get(sq, 1), s2 = get(sq, 2), s3 = get(sq, 3);
+    if (on) acc = normalize_component<R>(s0 + s1 + s2 + s3, acc, c4);
+  }
+  const q4<R> q{get(acc, 0), get(acc, 1), get(acc, 2), get(acc, 3)};
+  R r[9];
+  rotation_of(q, r);
+  const R ra = c == 0 ? r[0] : (c == 1 ? r[1] : r[2]), rb = c == 0 ? r[3] : (c == 1 ? r[4] : r[5]);
+  const R rc = c == 0 ? r[6] : (c == 1 ? r[7] : r[8]);
+  const R ta = ra * i0 + rb * i1 + rc * i2, tb = ra * i3 + rb * i4 + rc * i5, tc = ra * i6 + rb * i7 + rc * i8;
+  const R w0 = ta * r[0] + tb * r[3] + tc * r[6], w3 = ta * r[1] + tb * r[4] + tc * r[7];
+  const R w6 = ta * r[2] + tb * r[5] + tc * r[8];
+  // sleep bookkeeping, rigidbody.go:248-258
+  bool falls = false;
+  if (__any_sync(FULL, sleeps)) {
+    const R vv = vel * vel, rr = rot * rot;
+    const R cm = (get(vv, 0) + get(vv, 1) + get(vv, 2)) + (get(rr, 0) + get(rr, 1) + get(rr, 2));
+    if (sleeps) {
+      motion = sleep_bias * motion + ((R)1 - sleep_bias) * cm;
+      falls = motion < (R)0.3;
+      if (falls) vel = rot = zero;
+      else if (motion > (R)3.0) motion = (R)3.0;
+    }
+  }
+  __syncwarp();
+  if (!on) return;
+  F(B_QW + c4) = acc;
+  if (c4 == 3) {
+    if (sleeps) F(B_MOTION) = motion;
+    if (falls) v.awake[i] = 0;
+    return;
+  }
+  F(B_PX + c) = pos;
+  F(B_VX + c) = vel;
+  F(B_RX + c) = rot;
+  F(B_LX + c) = lfa;
+  F(B_IW0 + c) = w0;
+  F(B_IW0 + 3 + c) = w3;
+  F(B_IW0 + 6 + c) = w6;
+#undef F
+}
+
+// Four lanes per body for float64 batches of up to kSpreadBodies, where a
+// scheduler has one such warp at most: one world of 20 cubes 14 -> 10 us a
+// frame, 60 falling worlds of 30 bodies x 10 frames 1469 -> 1332 us (with CTAs
+// of 256 threads 12 us and 1372).  With more bodies the float64 pipes are full
+// and the lanes' idle quarter counts (4 x 110 instructions per 32 bodies for 300).
+constexpr long long kSpreadBodies = 8192;
+template <class R>
+__global__ void __launch_bounds__(256) k_integrate_spread(BatchView<R> v, R dt, R sleep_bias) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < 4) v.queue[t] = 0;
+  const long long i = t >> 2;
+  integrate_body_spread<R>(v, v.first_body + (i < v.nb_run ? i : 0), i < v.nb_run, dt, sleep_bias);
 }
 
 // ============================================================== narrowphase

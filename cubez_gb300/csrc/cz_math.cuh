@@ -196,6 +196,22 @@ template <class R, class W> __device__ __forceinline__ void qnormalize_island(q4
   }
 }
 
+// Normalize (quaternion.go:77-99) of component c (w first) of a quaternion
+// whose squares sum to s: the component after it.  Out of line: in the
+// precision form's island it is rare.
+// RealEqual(1, len) is |1 - len| / (1 + len) < 1e-7: certain without the
+// division below 1e-7 (1 + len is at least 1) and above 4e-7 (with len < 2.9
+// the divisor is at most 3.9), which is nearly always.
+template <class W> __device__ __noinline__ W normalize_component(W s, W component, int c) {
+  W len = sqrt_<W>(s);
+  const W diff = fabs_<W>((W)1 - len);
+  if (diff < (W)1e-7) return component;
+  if (!(diff > (W)4e-7 && len < (W)2.9) && real_equal<W>((W)1, len)) return component;
+  if (len == (W)0) return c == 0 ? (W)1 : (W)0;
+  if (len == Lim<W>::inf()) len = Lim<W>::max_value();
+  return component * ((W)1 / len);
+}
+
 // matrix.go:79-86
 template <class R> __device__ __forceinline__ v3<R> mulv(const m3<R>& a, const v3<R>& v) {
   return v3<R>{a.m[0] * v.x + a.m[3] * v.y + a.m[6] * v.z, a.m[1] * v.x + a.m[4] * v.y + a.m[7] * v.z,

@@ -309,22 +309,6 @@ __device__ __noinline__ void derive_asleep(RCtx<R, W, SM> x, const BatchView<R>&
   x.P(3, body) = (W)q.w; x.P(4, body) = (W)q.x; x.P(5, body) = (W)q.y; x.P(6, body) = (W)q.z;
 }
 
-// Normalize (quaternion.go:77-99) of component c (w first) of a quaternion
-// whose squares sum to s: the component after it.  Out of line: in the
-// precision form's island it is rare.
-// RealEqual(1, len) is |1 - len| / (1 + len) < 1e-7: certain without the
-// division below 1e-7 (1 + len is at least 1) and above 4e-7 (with len < 2.9
-// the divisor is at most 3.9), which is nearly always.
-template <class W> __device__ __noinline__ W normalize_component(W s, W component, int c) {
-  W len = sqrt_<W>(s);
-  const W diff = fabs_<W>((W)1 - len);
-  if (diff < (W)1e-7) return component;
-  if (!(diff > (W)4e-7 && len < (W)2.9) && real_equal<W>((W)1, len)) return component;
-  if (len == (W)0) return c == 0 ? (W)1 : (W)0;
-  if (len == Lim<W>::inf()) len = Lim<W>::max_value();
-  return component * ((W)1 / len);
-}
-
 // applyPositionChange, contact.go:285-386, of contact k by the first eight
 // lanes (sl = 0..7) of a group with `on`; every lane of the warp calls both
 // parts.  The four lanes 4i..4i+3 move body i: lane 4i + c (c < 3) forms
