@@ -134,7 +134,7 @@ template <int NW> __device__ __forceinline__ void big_sync() {
 // its warps; returns the iterations used.
 template <class R, class W, bool VEL, class Key>
 __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const BatchView<R>& v, int bstart,
-                                         const BigKeys<Key>& bk, const int* off, const int* end, const int* adj,
+                                         const BigKeys<Key>& bk, const int2* span, const int* adj,
                                          int max_it, BigChange<R>* chg, uint32_t& err) {
   constexpr int NW = big_warps<R>(), T = 32 * NW;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -162,8 +162,15 @@ __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const Batch
     if (best == 0) break;
     const int bb = x.pair(k);
     const int d0 = x.B0(bb), d1 = x.B1(bb);
-    const int o0 = off[d0], l0 = end[d0] - o0;
-    const int o1 = d1 >= 0 ? off[d1] : 0, l1 = d1 >= 0 ? end[d1] - o1 : 0;
+    // the two bodies' lists
+    int o0, l0, o1, l1;
+    auto spans = [&]() {
+      const int2 a = span[d0], b = d1 >= 0 ? span[d1] : make_int2(0, 0);
+      o0 = a.x;
+      l0 = a.y - a.x;
+      o1 = b.x;
+      l1 = b.y - b.x;
+    };
     // this lane's contact of the two bodies' lists (32 at a time); one that
     // touches both bodies is visited in d0's list
     int q, qb;
@@ -180,14 +187,17 @@ __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const Batch
       // every warp's contacts, eight at a time; the first warp's change
       const int first = 8 * wid + (lane >> 2);
       const bool lead = (lane & 3) == 0;
-      entry(first);
-      if (q >= 0) prefetch_line(x.rec(q) + 16 * (lane & 1));
+      std::conditional_t<VEL, VelocityIn<R>, PositionIn<R, W>> in;
       if (wid == 0) {
-        std::conditional_t<VEL, VelocityIn<R>, PositionIn<R, W>> in;
         if constexpr (VEL)
           velocity_load(x, in, k, bb, lane < 8, lane);
         else
           position_load(x, in, k, bb, lane < 8, lane);
+      }
+      spans();
+      entry(first);
+      if (q >= 0) prefetch_line(x.rec(q) + 16 * (lane & 1));
+      if (wid == 0) {
         const bool woke = match_awake(x, bb, true, lane == 0);
         if constexpr (VEL)
           velocity_change<R, W, false>(x, v, in, k, lane < 8, lane, lin, ang, err);
@@ -226,7 +236,6 @@ __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const Batch
       }
       __syncthreads();
     } else {
-      entry(lane);
       // what the change needs, then the touched records: they load while the
       // change is computed
       std::conditional_t<VEL, VelocityIn<R>, PositionIn<R, W>> in;
@@ -234,6 +243,8 @@ __device__ __forceinline__ int big_phase(const RCtx<R, W, false>& x, const Batch
         velocity_load(x, in, k, bb, lane < 8, lane);
       else
         position_load(x, in, k, bb, lane < 8, lane);
+      spans();
+      entry(lane);
       Touched<R> t;
       update_load<VEL>(x, t, q, qb, q >= 0, d0, d1);
       const bool woke = match_awake(x, bb, true, lane == 0);
@@ -283,9 +294,8 @@ __device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, 
   bk.cfirst = reinterpret_cast<int*>(bk.tmax + kBigTops);
   bk.tfirst = bk.cfirst + kBigChunks;
   // list starts and ends (first the counts, then the fill cursors)
-  int* off = bk.tfirst + kBigTops;
-  int* end = off + ((n + 3) & ~3);
-  BigChange<R>* chg = reinterpret_cast<BigChange<R>*>(end + ((n + 3) & ~3));
+  int2* span = reinterpret_cast<int2*>(bk.tfirst + kBigTops);
+  BigChange<R>* chg = reinterpret_cast<BigChange<R>*>(span + ((n + 3) & ~3));
   unsigned char* tile = reinterpret_cast<unsigned char*>(chg) + big_change_bytes<R>();
   RCtx<R, W, false> x;
   x.nbs = n;
@@ -314,19 +324,19 @@ __device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, 
   const bool awake = load_bodies(x, v, bstart, n, tid, T);
   x.all_awake = __syncthreads_and(awake) != 0;
   for (int k = tid; k < C; k += T) prepare_contact(x, v, cst + k, k, k);
-  for (int i = tid; i < n; i += T) end[i] = 0;
+  for (int i = tid; i < n; i += T) span[i].y = 0;
   __syncthreads();
   // contact lists per body: count, exclusive scan, fill
   for (int k = tid; k < C; k += T) {
     const int bb = x.pair(k);
-    atomicAdd(&end[x.B0(bb)], 1);
-    if (x.B1(bb) >= 0) atomicAdd(&end[x.B1(bb)], 1);
+    atomicAdd(&span[x.B0(bb)].y, 1);
+    if (x.B1(bb) >= 0) atomicAdd(&span[x.B1(bb)].y, 1);
   }
   __syncthreads();
   int carry = 0;
   for (int base = 0; tid < 32 && base < n; base += 32) {
     const int i = base + lane;
-    const int c = i < n ? end[i] : 0;
+    const int c = i < n ? span[i].y : 0;
     int s = c;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -334,28 +344,27 @@ __device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, 
       if (lane >= d) s += y;
     }
     if (i < n) {
-      off[i] = carry + s - c;
-      end[i] = carry + s - c;
+      span[i] = make_int2(carry + s - c, carry + s - c);
     }
     carry += __shfl_sync(FULL, s, 31);
   }
   __syncthreads();
   for (int k = tid; k < C; k += T) {
     const int bb = x.pair(k);
-    adj[atomicAdd(&end[x.B0(bb)], 1)] = k;
-    if (x.B1(bb) >= 0) adj[atomicAdd(&end[x.B1(bb)], 1)] = k;
+    adj[atomicAdd(&span[x.B0(bb)].y, 1)] = k;
+    if (x.B1(bb) >= 0) adj[atomicAdd(&span[x.B1(bb)].y, 1)] = k;
   }
   __syncthreads();
   const int max_it = v.max_iterations >= 0 ? v.max_iterations : C * v.iter_mult;
   uint32_t err = 0;
   const bool solves = tid < 32 * big_warps<R>();
-  const int pos_used = !solves ? 0 : big_phase<R, W, false>(x, v, bstart, bk, off, end, adj, max_it, chg, err);
+  const int pos_used = !solves ? 0 : big_phase<R, W, false>(x, v, bstart, bk, span, adj, max_it, chg, err);
   __syncthreads();
   if (v.contact_writeback)
     for (int k = tid; k < C; k += T) v.contact[C_PEN * v.nc_total + cst + k] = x.rec(k)[CR_PEN];
   for (int k = tid; k < C; k += T) friction_prepare(x, k);
   __syncthreads();
-  const int vel_used = !solves ? 0 : big_phase<R, W, true>(x, v, bstart, bk, off, end, adj, max_it, chg, err);
+  const int vel_used = !solves ? 0 : big_phase<R, W, true>(x, v, bstart, bk, span, adj, max_it, chg, err);
   __syncthreads();
   if (err) {
     atomicOr(&v.world_status[w], err);
@@ -374,7 +383,7 @@ __device__ __forceinline__ void big_world(const BatchView<R>& v, R dt, int csm, 
 }
 
 template <class R, class W>
-__global__ void __launch_bounds__(kBigThreads, sizeof(R) == 8 ? 2 : 4) k_resolve_big(BatchView<R> v, R dt, int csm) {
+__global__ void __launch_bounds__(kBigThreads, sizeof(R) == 8 ? 3 : 4) k_resolve_big(BatchView<R> v, R dt, int csm) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int w = v.big_list[blockIdx.x];
   int C = v.contact_count[w];
