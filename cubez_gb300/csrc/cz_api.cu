@@ -636,7 +636,7 @@ int configure(cz_batch* b) {
     }
   }
   CZ_CUDA(b->ops->occupancy(&npb, b->np_threads, b->np_smem,
-                            b->grid_min_bodies > 0 && b->max_n >= b->grid_min_bodies));
+                            cz::np_mode(b->grid_min_bodies, b->max_n)));
   npb = std::max(npb, 1);
   rsb = std::max(rsb, 1);
   if (b->rs_ctas_per_sm > 0) rsb = std::min(rsb, b->rs_ctas_per_sm);

@@ -222,15 +222,17 @@ static cudaError_t raise_smem_limit(const void* f, size_t bytes) {
 
 // The narrowphase instantiation a batch runs: with the grid only when one of
 // its worlds is large enough for it.
-static bool uses_grid(const HostView& h) { return h.grid_min_bodies > 0 && h.max_bodies >= h.grid_min_bodies; }
-static const void* narrowphase_fn(bool grid) {
-  return grid ? (const void*)k_narrowphase<R, true> : (const void*)k_narrowphase<R, false>;
+static const void* narrowphase_fn(NPMode mode) {
+  return mode == NP_GRID    ? (const void*)k_narrowphase<R, NP_GRID>
+         : mode == NP_LARGE ? (const void*)k_narrowphase<R, NP_LARGE>
+                            : (const void*)k_narrowphase<R, NP_SMALL>;
 }
 
 static cudaError_t prepare(size_t np, size_t rs, int lanes) {
-  cudaError_t e = raise_smem_limit(narrowphase_fn(false), np);
+  cudaError_t e = raise_smem_limit(narrowphase_fn(NP_SMALL), np);
   if (e != cudaSuccess) return e;
-  if ((e = raise_smem_limit(narrowphase_fn(true), np)) != cudaSuccess) return e;
+  if ((e = raise_smem_limit(narrowphase_fn(NP_LARGE), np)) != cudaSuccess) return e;
+  if ((e = raise_smem_limit(narrowphase_fn(NP_GRID), np)) != cudaSuccess) return e;
   for (int mode = 0; mode <= 1; ++mode) {
     const void* f = resolve_fn_mode(lanes, mode);
     if (!f) return cudaErrorInvalidValue;
@@ -261,10 +263,11 @@ static cudaError_t integrate(const HostView& h, double dt, double bias, int thre
 }
 
 static cudaError_t narrowphase(const HostView& h, int nbs, int threads, int grid, size_t smem, cudaStream_t s) {
-  if (uses_grid(h))
-    k_narrowphase<R, true><<<grid, threads, smem, s>>>(view_of(h), nbs);
-  else
-    k_narrowphase<R, false><<<grid, threads, smem, s>>>(view_of(h), nbs);
+  switch (np_mode(h.grid_min_bodies, h.max_bodies)) {
+    case NP_GRID: k_narrowphase<R, NP_GRID><<<grid, threads, smem, s>>>(view_of(h), nbs); break;
+    case NP_LARGE: k_narrowphase<R, NP_LARGE><<<grid, threads, smem, s>>>(view_of(h), nbs); break;
+    default: k_narrowphase<R, NP_SMALL><<<grid, threads, smem, s>>>(view_of(h), nbs);
+  }
   return cudaGetLastError();
 }
 
@@ -393,8 +396,8 @@ static cudaError_t download(const HostView& h, double* sg, uint8_t* u8, int* i32
   return cudaGetLastError();
 }
 
-static cudaError_t occupancy(int* npb, int np_threads, size_t nps, int grid) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(npb, narrowphase_fn(grid != 0), np_threads, nps);
+static cudaError_t occupancy(int* npb, int np_threads, size_t nps, int mode) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(npb, narrowphase_fn((NPMode)mode), np_threads, nps);
 }
 
 static cudaError_t rs_occupancy(int* rsb, int wpc, size_t rss, int lanes, int mode) {

@@ -334,6 +334,35 @@ __device__ __forceinline__ SatResult<R> sat_axes(const NPTile<R>& tl, int i1, in
   return r;
 }
 
+// The same axes on one lane, in the reference's loop (an axis apart ends it),
+// for the order (i1, i2) alone.
+template <class R> __device__ __forceinline__ SatResult<R> sat_serial(const NPTile<R>& tl, int i1, int i2) {
+  const xf<R> t1 = tl.xform(i1), t2 = tl.xform(i2);
+  const v3<R> h1 = tl.half(i1), h2 = tl.half(i2);
+  v3<R> tc = t2.axis(3);
+  sub(tc, t1.axis(3));
+  SatResult<R> r;
+  r.pen = Lim<R>::max_value();
+  r.code = kSatApart;
+  int best = 255, single = 255;
+#pragma unroll 1
+  for (int l = 0; l < 15; ++l) {
+    v3<R> axis = tl.axis(l < 3 || l > 5 ? i1 : i2, l < 3 ? l : (l < 6 ? l - 3 : (l - 6) / 3));
+    if (l > 5) axis = cross(axis, tl.axis(i2, (l - 6) % 3));
+    if (!(sqmag(axis) < Lim<R>::eps())) {
+      const R p = axis_penetration(t1, h1, t2, h2, tc, axis);
+      if (p < (R)0) return r;
+      if (p < r.pen) {
+        r.pen = p;
+        best = l;
+      }
+    }
+    if (l == 5) single = best;
+  }
+  r.code = best | single << 8;
+  return r;
+}
+
 // fillPointFaceBoxBox, colliders.go:479-517, of boxes one and two
 template <class R>
 __device__ __forceinline__ void fill_point_face(const NPTile<R>& tl, int one, int two, const v3<R>& tc, int best, R pen,
@@ -780,8 +809,8 @@ __device__ __forceinline__ void np_emit(const BatchView<R>& v, long long cs, int
 // half-space, else the pair with j = k - 1, skipping i), in chunks of the
 // CTA's size, emitting their contacts in list order at out onwards.  Within a
 // chunk the units are taken in order of their kind of test (half-space with a
-// sphere, with a cube; sphere-sphere, sphere-cube, cube-cube with i < j, then
-// with i > j, which mostly take the other order's axes), stably, so the
+// sphere, with a cube; sphere-sphere, sphere-cube, cube-cube, in float64 with
+// i < j ahead of i > j, which mostly take the other order's axes), stably, so the
 // lanes of a warp mostly run one test's code; the counts are then scanned in
 // list order, so every contact lands where the list order puts it (the
 // reference's contact order).  The two tests with many parts are spread over
@@ -792,7 +821,7 @@ __device__ __forceinline__ void np_emit(const BatchView<R>& v, long long cs, int
 // whatever few lanes had them.  Narrowphase of 8192 worlds x 32 bodies, float64
 // 1.50 -> 0.69 ms a frame (0.73 with the two orders of the pairs mixed); of one
 // world of 20 cubes in float64 84 -> 39 us.  sortw: np_sort_ints(blockDim.x) ints.
-template <class R>
+template <class R, bool LARGE>
 __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart, int n, long long cs, int cap,
                          const int* surv, int nsurv, int* scan, int& parity, int& out, uint32_t& err, int* sortw) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, bd = blockDim.x, nwarps = (bd + 31) >> 5;
@@ -804,7 +833,8 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
   int* wcnt = cntb + bd;  // [kind * 8 + warp]
   for (int sb = 0; sb < nsurv; sb += bd) {
     const int m = nsurv - sb < bd ? nsurv - sb : bd;
-    int key = 6;  // no unit
+    constexpr bool kOrders = sizeof(R) == 8;  // (in float32 the kind costs what it saves)
+    int key = kOrders ? 6 : 5;  // no unit
     if (tid < m) {
       const int uu = surv[sb + tid];
       const int i = uu / n, k = uu - i * n;
@@ -814,12 +844,12 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
         int j = k - 1;
         if (j >= i) ++j;
         key = 2 + (tl.shape[i] != 0 ? 1 : 0) + (tl.shape[j] != 0 ? 1 : 0);
-        if (key == 4 && i > j) key = 5;
+        if (kOrders && key == 4 && i > j) key = 5;
       }
     }
     int rank = 0;
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
+    for (int q = 0; q < (kOrders ? 7 : 6); ++q) {
       const unsigned bal = __ballot_sync(FULL, key == q);
       if (key == q) rank = __popc(bal & ((1u << lane) - 1u));
       if (lane == 0) wcnt[q * 8 + wid] = __popc(bal);
@@ -828,13 +858,13 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
     int dst = rank, n0 = 0, n1 = 0, n23 = 0, n4 = 0;
     for (int w2 = 0; w2 < nwarps; ++w2) {
       const int a = wcnt[w2], b = wcnt[8 + w2], c2 = wcnt[16 + w2], c3 = wcnt[24 + w2], d = wcnt[32 + w2];
-      const int e = wcnt[40 + w2];
+      const int e = kOrders ? wcnt[40 + w2] : 0;
       n0 += a;
       n1 += b;
       n23 += c2 + c3;
       n4 += d + e;
       dst += (key > 0 ? a : 0) + (key > 1 ? b : 0) + (key > 2 ? c2 : 0) + (key > 3 ? c3 : 0) + (key > 4 ? d : 0) +
-             (key > 5 ? e : 0);
+             (kOrders && key > 5 ? e : 0);
       if (w2 < wid) dst += wcnt[key * 8 + w2];
     }
     perm[dst] = tid;
@@ -844,7 +874,27 @@ __device__ void np_flush(const NPTile<R>& tl, const BatchView<R>& v, int bstart,
     // more than two passes, a lane per pair tries three axes first (1000 worlds
     // of 31 bodies, float32: 54 -> 41 us; without Offsets the culls leave near
     // pairs, and 8192 x 32 settled bodies took 187 us with it, 175 without).
-    const bool pre = v.offset != nullptr && n4 > bd >> 3;
+    // In a world of more than kPairedBodies the chunks are full of pairs whose
+    // other order is in another chunk.  float32 then takes a lane per pair for
+    // all its axes, float64 the three axes first (LARGE: the code is left out where
+    // no world needs it).  64 piles of 1024 cubes, falling and settled: float32
+    // 1.24 -> 0.91 and 2.19 -> 1.73 ms a frame, float64 3.90 -> 1.69 and 7.43 ->
+    // 6.05; 600 of 72, float64, 0.82 -> 0.27 and 1.53 -> 1.33.
+    const bool large = LARGE && n > kPairedBodies;
+    const bool serial = sizeof(R) == 4 && large;
+    if (serial) {
+      if (tid < n4) {
+        const int at = perm[n0 + n1 + n23 + tid];
+        const int uu = surv[sb + at];
+        const int i = uu / n, k = uu - i * n;
+        const SatResult<R> r = sat_serial(tl, i, k - 1 >= i ? k : k - 1);
+        satp[at] = r.pen;
+        satc[at] = r.code;
+        satr[at] = at;
+      }
+      n4 = 0;
+    }
+    const bool pre = (v.offset != nullptr || large) && n4 > bd >> 3;
     if (pre) {
       if (tid < n4) {
         const int at = perm[n0 + n1 + n23 + tid];
@@ -1124,7 +1174,7 @@ __device__ int np_grid_units(const NPTile<R>& tl, const BatchView<R>& v, const N
 // culled, the kept ones listed (scap of them at a time) and tested, the
 // contacts emitted in the reference's order; sets the world's contact count.
 // Every thread of the CTA calls it.
-template <class R, bool GRID>
+template <class R, NPMode MODE>
 __device__ void np_world(const NPTile<R>& tl, const BatchView<R>& v, int w, int n, int bstart, int* scan,
                          int& chunk_parity, int* surv, int scap) {
   const int tid = threadIdx.x;
@@ -1134,7 +1184,7 @@ __device__ void np_world(const NPTile<R>& tl, const BatchView<R>& v, int w, int 
   int out = 0, nsurv = 0;
   uint32_t err = 0;
   const NPGrid g = np_grid_scratch(tl);
-  if (GRID && v.grid_min_bodies > 0 && n >= v.grid_min_bodies && np_grid_build(tl, n, g, scan, chunk_parity)) {
+  if (MODE == NP_GRID && v.grid_min_bodies > 0 && n >= v.grid_min_bodies && np_grid_build(tl, n, g, scan, chunk_parity)) {
     // Grid: each body's kept units (counted, then listed and sorted), as
     // many bodies at a time as the list holds, then their full tests.
     for (int ib = 0; ib < n;) {
@@ -1161,7 +1211,7 @@ __device__ void np_world(const NPTile<R>& tl, const BatchView<R>& v, int w, int 
       }
       __syncthreads();
       nsurv = g.info[5];
-      np_flush(tl, v, bstart, n, cs, cap, surv, nsurv, scan, chunk_parity, out, err, surv + scap);
+      np_flush<R, MODE != NP_SMALL>(tl, v, bstart, n, cs, cap, surv, nsurv, scan, chunk_parity, out, err, surv + scap);
       __syncthreads();
       ib += m;
     }
@@ -1197,7 +1247,7 @@ __device__ void np_world(const NPTile<R>& tl, const BatchView<R>& v, int w, int 
       nsurv += total;
       if (nsurv <= scap - round && base + round < U) continue;
       __syncthreads();
-      np_flush(tl, v, bstart, n, cs, cap, surv, nsurv, scan, chunk_parity, out, err, surv + scap);
+      np_flush<R, MODE != NP_SMALL>(tl, v, bstart, n, cs, cap, surv, nsurv, scan, chunk_parity, out, err, surv + scap);
       nsurv = 0;
       __syncthreads();
     }
@@ -1216,14 +1266,14 @@ __device__ void np_world(const NPTile<R>& tl, const BatchView<R>& v, int w, int 
   }
 }
 
-// GRID = false compiles the all-pairs path alone (worlds too small for the
-// grid), so its registers and occupancy stay those of that path; in float32
+// NP_SMALL and NP_LARGE compile the all-pairs path alone (worlds too small for
+// the grid), so its registers and occupancy stay those of that path; in float32
 // it is bounded to 64 registers (8 CTAs of 128 threads per SM; 240 bytes
 // spilled): with few contacts a world is a chain of staging and barriers, and
 // 16384 worlds of 14 bodies took 155 us against 178 with 80 registers (6 CTAs);
 // 8192 worlds of 32 settled bodies 175 against 170, and 200 unbounded.
-template <class R, bool GRID>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 && !GRID ? 4 : 0) k_narrowphase(BatchView<R> v, int nbs) {
+template <class R, NPMode MODE>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 && MODE != NP_GRID ? 4 : 0) k_narrowphase(BatchView<R> v, int nbs) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem);
   NPTile<R> tl;
@@ -1292,7 +1342,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 && !GRID ? 4 : 0) k_narrow
     }
     np_build_tile(tl, n, v.offset ? v.offset + bstart : nullptr, v.nb_pad);
     __syncthreads();
-    np_world<R, GRID>(tl, v, w, n, bstart, scan, chunk_parity, surv, np_surv_cap(nbs));
+    np_world<R, MODE>(tl, v, w, n, bstart, scan, chunk_parity, surv, np_surv_cap(nbs));
     __syncthreads();
   }
 }
@@ -1345,7 +1395,7 @@ __global__ void __launch_bounds__(256) k_collide(BatchView<R> v, int w, const in
     nsurv += total;
     if (nsurv + (int)blockDim.x <= scap && base + (int)blockDim.x < nunits) continue;
     __syncthreads();
-    np_flush(tl, v, bstart, n, cs, cap, surv, nsurv, scan, parity, out, err, surv + scap);
+    np_flush<R, true>(tl, v, bstart, n, cs, cap, surv, nsurv, scan, parity, out, err, surv + scap);
     nsurv = 0;
     __syncthreads();
   }

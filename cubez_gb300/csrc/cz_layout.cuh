@@ -80,6 +80,16 @@ enum : uint32_t {
 
 // in BatchView::cost: the world's last adjustVelocities used its whole budget
 constexpr int kExhausted = 1 << 30;
+// Worlds of more bodies than this list more units for the narrowphase than a
+// chunk or two of its CTA hold (np_flush).
+constexpr int kPairedBodies = 64;
+// k_narrowphase's instantiation for a batch: worlds of up to kPairedBodies
+// bodies, larger ones, or with the grid
+enum NPMode { NP_SMALL, NP_LARGE, NP_GRID };
+inline NPMode np_mode(int grid_min_bodies, int max_bodies) {
+  if (grid_min_bodies > 0 && max_bodies >= grid_min_bodies) return NP_GRID;
+  return max_bodies > kPairedBodies ? NP_LARGE : NP_SMALL;
+}
 
 // packed body pair of a contact: low 16 bits body 0, high 16 bits body 1
 // (0xFFFF = nil).  World-local indices, so a world holds at most 65535 bodies.

@@ -1779,7 +1779,7 @@ __device__ void frame_front(const BatchView<R>& v, int w, int n, int bstart, int
   np_build_tile(tl, n, v.offset ? v.offset + bstart : nullptr, v.nb_pad);
   __syncwarp();
   int parity = 0;
-  np_world<R, false>(tl, v, w, n, bstart, scan, parity, surv, kFrameSurvivors);
+  np_world<R, NP_SMALL>(tl, v, w, n, bstart, scan, parity, surv, kFrameSurvivors);
   __syncwarp();
 }
 
