@@ -21,9 +21,10 @@
 // adjustVelocities and are computed once per contact, off the chain
 // (friction_prepare).
 //
-// Also here: k_warm_features (the learned warm start's features, tensor-core
-// inference and plan, launched before k_resolve) and the shared pieces of
-// k_resolve_big (cz_resolve_big.cuh).
+// Also here: k_resolve_wide (small batches: four warps to a world),
+// k_warm_features (the learned warm start's features, tensor-core inference and
+// plan, launched before k_resolve) and the shared pieces of k_resolve_big
+// (cz_resolve_big.cuh).
 #pragma once
 #include <type_traits>
 

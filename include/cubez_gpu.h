@@ -262,7 +262,8 @@ int cz_mlp_predict(cz_mlp* mlp, const float* features, int64_t n, float* impulse
 /* Tuning knobs picked by the autotuner (0 keeps the current value). */
 typedef struct cz_tuning {
   int32_t narrowphase_threads; /* CTA size of the narrowphase */
-  int32_t resolver_contacts;   /* contacts kept in shared memory per world */
+  int32_t resolver_contacts;   /* contacts kept in shared memory per world (by default three per body of the
+                                  largest world up to 64 bodies, at least 96) */
   int32_t resolver_ctas_per_sm;/* resident resolver CTAs per SM (a CTA is 1 warp, or up to 8 independent ones in
                                   the float32 form with 32 lanes per world) */
   int32_t integrate_threads;
@@ -271,7 +272,7 @@ typedef struct cz_tuning {
   int32_t warm_start_budget_shift; /* learned warm start: a world is warm-started when its last
                                       solve used at most max_iterations >> shift iterations
                                       (1 to 8; default 2) */
-  int32_t large_world_lanes;   /* worlds of more than 64 bodies: 32 (the default) or 16; one warp per world
+  int32_t large_world_lanes;   /* worlds of more than 64 bodies: 32 (the default) or 16; a CTA per world
                                   either way */
   int32_t broadphase_min_bodies; /* the narrowphase bins the bodies of worlds of at least this many
                                     bodies in a uniform grid and tests only pairs of neighbouring
