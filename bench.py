@@ -56,10 +56,11 @@ DT = 1.0 / 60.0
 L2_BYTES = 126 * 1024 * 1024
 # DRAM bytes (read + write) of one resolver launch at steady state on the
 # default workload (16384 worlds x 32 bodies), per form, from an ncu capture
-# of the resolver instantiation that form runs (frame 381 of a 400-frame
-# rollout): the roofline's measured traffic beside its algorithmic bytes.
+# of the resolver instantiation that form runs (settled worlds, frame 216, one
+# launch over all of them): the roofline's measured traffic beside its
+# algorithmic bytes.
 RESOLVE_TRAFFIC = {
-    "fp32_mlp": {"bytes": 255.9e6, "kernel": "k_resolve<float, double, 32, true>",
+    "fp32_mlp": {"bytes": 234.1e6, "kernel": "k_resolve<float, double, 32, true>",
                  "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch"},
 }
 

@@ -569,11 +569,16 @@ int tile_rule(int nbs, int lanes) { return lanes < 32 ? 96 : std::max(96, (int)r
 // of 8 to 64 float32 4.70 -> 3.73, fresh ones the same; 1000 of 40 gain 5 to 10 %
 // settled and lose 4 fresh.  With many worlds one warp is better throughout
 // (4096 of 62, float32, 11.8 -> 14.3).
-int wide_rule(int worlds, int nbs, int lanes, int sms) {
+// In float64, whose rate one warp reaches a quarter of, up to seven per SM from
+// 24 slots on: 1001 worlds of 24 bodies with Offsets x 20 20.3 -> 19.4 ms, 600
+// settled of 31 x 4 5.95 -> 5.21, 1000 settled of 32 x 5 7.55 -> 6.63, against
+// fresh ones of 24 to 40 bodies, 0.99 to 1.04 times (300 of 24 x 3, 1.05 -> 1.08).
+int wide_rule(int form, int worlds, int nbs, int lanes, int sms) {
   if (lanes != 32 || worlds <= 0) return 0;
   const int per_sm = (worlds + sms - 1) / sms;
   if (per_sm == 1) return nbs >= 16 ? 1 : 0;
-  return (per_sm <= 3 && nbs >= 36) || (per_sm <= 7 && nbs >= 52) ? std::min(per_sm, 3) : 0;
+  const bool wide = form == CZ_FORM_FP64 ? nbs >= 24 : nbs >= (per_sm <= 3 ? 36 : 52);
+  return wide && per_sm <= 7 ? std::min(per_sm, 3) : 0;
 }
 
 // The captured graphs hold the kernels' parameters (the batch view); drop them
@@ -622,7 +627,7 @@ int configure(cz_batch* b) {
   // Four warps to a world (wide_rule), in tiles of eight contacts a body with
   // their friction matrices, or what lets the SMs hold all the worlds at once.
   b->wide_smem = 0;
-  const int per_sm = wide_rule(b->nsmall, b->rs_nbs, lanes, b->sm_count);
+  const int per_sm = wide_rule(b->form, b->nsmall, b->rs_nbs, lanes, b->sm_count);
   if (per_sm > 0) {
     b->wide_cs = std::max(b->rs_cs, std::min((int)round_up(b->max_cap, 32), 8 * b->rs_nbs));
     while (b->wide_cs > b->rs_cs &&
