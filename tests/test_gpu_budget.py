@@ -1,6 +1,6 @@
-"""Worlds that run out of their iteration budget, solved by a warp each
-(resolve_worlds in cz_resolve.cuh goes on from one island and puts the others
-back): the oracle's bits, for budgets that end in either phase, worlds of many
+"""Worlds that run out of their iteration budget, solved by a warp each or, the
+larger ones, by four (resolve_worlds and wide_phase in cz_resolve.cuh go on from
+one island and put the others back): the oracle's bits, for budgets that end in either phase, worlds of many
 islands, equal values on different islands, and sleeping bodies."""
 import numpy as np
 import pytest
@@ -33,15 +33,19 @@ def _alike(seed):
     return s
 
 
-def _spread(seed):
-    s = scenes.mixed(num_worlds=WORLDS, seed=seed, min_bodies=2, max_bodies=48)
+def _spread(seed, bodies=20):
+    s = scenes.mixed(num_worlds=WORLDS, seed=seed, min_bodies=2, max_bodies=bodies)
     s.position[:, (0, 2)] *= 1.6  # more islands
     s.can_sleep[::4] = 1
     return s
 
 
+def _spread_large(seed):
+    return _spread(seed, 48)
+
+
 @pytest.mark.parametrize("form", [0, 1])
-@pytest.mark.parametrize("make,settle", [(_alike, 0), (_spread, 90)])
+@pytest.mark.parametrize("make,settle", [(_alike, 0), (_spread, 90), (_spread_large, 90)])
 @pytest.mark.parametrize("budget", [0, 3, 12, 40, 90])
 def test_out_of_budget_bit_exact(form, make, settle, budget, cuda_lib):
     from cubez_gb300.batch import WorldBatch
