@@ -155,7 +155,8 @@ class WorldBatch:
         check(self.L.cz_restore(self.h))
 
     def step_timed(self, nsteps, dt=1.0 / 60.0):
-        """Run a captured rollout; returns (total_ms, [integrate, narrowphase, resolve] ms)."""
+        """step with events between the phases; returns (total_ms, [integrate,
+        narrowphase, resolve] ms), shares of the total where parts overlap."""
         tot = C.c_double(0.0)
         ph = np.zeros(3)
         check(self.L.cz_step_timed(self.h, int(nsteps), float(dt), C.byref(tot), _ptr(ph)))

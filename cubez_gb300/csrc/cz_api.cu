@@ -170,10 +170,11 @@ struct cz_batch {
 
   // graph cache: (nsteps, dt) -> executable graph
   std::map<std::pair<int, double>, cudaGraphExec_t> graphs;
-  // rollouts with event-record nodes between the phases (cz_step_timed)
+  // the same rollouts with event-record nodes between the phases (cz_step_timed)
   struct Timed {
     cudaGraphExec_t exec = nullptr;
-    std::vector<cudaEvent_t> ev;  // 3 * nsteps + 1
+    int chains = 1;               // chains of launches with events
+    std::vector<cudaEvent_t> ev;  // 3 * nsteps + 1 a chain, then the rollout's start and end
   };
   std::map<std::pair<int, double>, Timed> timed;
   // on-device copy of the body state (cz_snapshot / cz_restore)
@@ -438,6 +439,13 @@ bool uses_frame(const cz_batch* b) {
 // Frames in one graph where the batch runs in parts (longer rollouts launch it
 // again: the parts meet that often, and the graph has at most 4096 launches).
 constexpr int kPartFrames = 32;
+// Parts whose phases cz_step_timed brackets, evenly spaced.  Event nodes in
+// many branches keep a graph's branches from running side by side: 4096 worlds
+// of 32 bodies x 60 frames, float64, 140 ms by cz_step, and timed with the
+// events of 1, 2, 4, 8 and 32 of the 32 parts 141, 142, 142, 187 and 280 ms
+// (float32, 8 parts: 16384 worlds 99.3 and 99.5 to 99.7, 1000 worlds 23.5 and
+// 23.8, 24.1, 24.4 and 25.0).
+constexpr int kTimedParts = 4;
 // The re-queue by cost matters where a launch's worlds do not all start at once.
 constexpr int kReorderWorlds = 256;
 
@@ -463,9 +471,9 @@ int chain_grid(int worlds, int per_cta, int most) {
 int launches_of(const cz_batch* b, int nsmall, int nbig, bool requeue) {
   return 2 + (nsmall > 0 ? 1 + (requeue ? 1 : 0) + (b->mode != 0 ? 1 : 0) : 0) + (nbig > 0 ? 1 : 0);
 }
-int launches_per_step(const cz_batch* b, bool in_parts) {
+int launches_per_step(const cz_batch* b) {
   if (uses_frame(b)) return 1 + (b->nsmall > 1 ? 1 : 0);
-  if (!in_parts || b->parts.size() == 1)
+  if (b->parts.size() == 1)
     return launches_of(b, b->nsmall, (int)b->big_ids.size(), requeues(b, b->nsmall));
   int n = 0;
   for (const auto& p : b->parts) n += launches_of(b, p.nsmall, p.nbig, p.nsmall > kReorderWorlds);
@@ -1117,17 +1125,33 @@ int cz_resolve(cz_batch* b, double dt) {
   return finish(b);
 }
 
-// One frame of a chain.
-static int launch_step(cz_batch* b, const Chain& c, double dt) {
+// Marks where a timed rollout records event k (`t` null: an untimed one).
+static int record_event(cz_batch::Timed* t, size_t k, cudaStream_t s) {
+  if (t) CZ_CUDA(cudaEventRecordWithFlags(t->ev[k], s, cudaEventRecordExternal));
+  return CZ_OK;
+}
+
+// One frame of a chain; in a timed rollout, events at + 1 to at + 3 end its phases.
+static int launch_step(cz_batch* b, const Chain& c, double dt, cz_batch::Timed* t = nullptr, size_t at = 0) {
   int st = launch_integrate(b, c, dt);
+  if (!st) st = record_event(t, at + 1, c.s);
   if (!st) st = launch_narrowphase(b, c, false);
+  if (!st) st = record_event(t, at + 2, c.s);
   if (!st) st = launch_resolve(b, c, dt, false);
+  if (!st) st = record_event(t, at + 3, c.s);
+  return st;
+}
+// `nsteps` of them, chain number `index` of the rollout.
+static int launch_chain(cz_batch* b, const Chain& c, int nsteps, double dt, cz_batch::Timed* t, size_t index) {
+  const size_t at = index * (3 * (size_t)nsteps + 1);
+  int st = record_event(t, at, c.s);
+  for (int s = 0; s < nsteps && !st; ++s) st = launch_step(b, c, dt, t, at + 3 * (size_t)s);
   return st;
 }
 
 // The batch's parts as parallel branches of the graph being captured on its
 // stream, each its own chain of frames.
-static int capture_parts(cz_batch* b, int nsteps, double dt) {
+static int capture_parts(cz_batch* b, int nsteps, double dt, cz_batch::Timed* t) {
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> joins;
   auto run = [&]() -> int {
@@ -1138,8 +1162,9 @@ static int capture_parts(cz_batch* b, int nsteps, double dt) {
       const Chain c{b->view(part, (int)p), part.nsmall, part.nbig, part.nsmall > kReorderWorlds,
                     p == 0 ? b->stream : b->part_streams[p - 1]};
       if (p > 0) CZ_CUDA(cudaStreamWaitEvent(c.s, fork, 0));
-      for (int s = 0; s < nsteps; ++s)
-        if (int st = launch_step(b, c, dt)) return st;
+      const size_t every = t ? b->parts.size() / t->chains : 1, index = p / every;
+      const bool timed = t && p % every == 0 && index < (size_t)t->chains;
+      if (int st = launch_chain(b, c, nsteps, dt, timed ? t : nullptr, index)) return st;
       if (p > 0) {
         cudaEvent_t e = nullptr;
         CZ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1161,6 +1186,44 @@ static int graph_frames(const cz_batch* b, int left) {
   return !uses_frame(b) && b->parts.size() > 1 ? std::min(left, kPartFrames) : left;
 }
 
+// A rollout's launches, on the batch's stream: the fused frames, the parts, or
+// one chain over the whole batch.  With `t`, the events around its phases (a
+// fused frame, one launch, is its resolve phase).
+static int launch_rollout(cz_batch* b, int nsteps, double dt, cz_batch::Timed* t) {
+  if (!uses_frame(b)) {
+    if (b->parts.size() > 1) return capture_parts(b, nsteps, dt, t);
+    return launch_chain(b, whole(b), nsteps, dt, t, 0);
+  }
+  int st = record_event(t, 0, b->stream);
+  for (int s = 0; s < nsteps && !st; ++s) {
+    st = record_event(t, 3 * (size_t)s + 1, b->stream);
+    if (!st) st = record_event(t, 3 * (size_t)s + 2, b->stream);
+    if (!st) st = launch_frame(b, dt);
+    if (!st) st = record_event(t, 3 * (size_t)s + 3, b->stream);
+  }
+  return st;
+}
+
+static int capture_rollout(cz_batch* b, int nsteps, double dt, cz_batch::Timed* t, cudaGraphExec_t* exec) {
+  CZ_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+  const long long before = g_launches.load();
+  const size_t ends = t ? t->ev.size() - 2 : 0;
+  int cst = record_event(t, ends, b->stream);
+  if (!cst) cst = launch_rollout(b, nsteps, dt, t);
+  if (!cst) cst = record_event(t, ends + 1, b->stream);
+  g_launches.store(before);  // captured launches are counted when the graph runs
+  cudaGraph_t graph = nullptr;
+  cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
+  if (cst != CZ_OK || e != cudaSuccess) {
+    if (graph) cudaGraphDestroy(graph);
+    return cst != CZ_OK ? cst : fail(CZ_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+  }
+  e = cudaGraphInstantiate(exec, graph, 0);
+  cudaGraphDestroy(graph);
+  if (e != cudaSuccess) return fail(CZ_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+  return CZ_OK;
+}
+
 // Capture (once per (nsteps, dt)) the plain rollout graph.
 static int get_graph(cz_batch* b, int nsteps, double dt, cudaGraphExec_t* out) {
   auto key = std::make_pair(nsteps, dt);
@@ -1169,36 +1232,12 @@ static int get_graph(cz_batch* b, int nsteps, double dt, cudaGraphExec_t* out) {
     *out = it->second;
     return CZ_OK;
   }
-  CZ_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  const long long before = g_launches.load();
-  int cst = CZ_OK;
-  const bool fused = uses_frame(b);
-  if (fused) {
-    for (int s = 0; s < nsteps && cst == CZ_OK; ++s) cst = launch_frame(b, dt);
-  } else if (b->parts.size() > 1) {
-    cst = capture_parts(b, nsteps, dt);
-  } else {
-    const Chain c = whole(b);
-    for (int s = 0; s < nsteps && cst == CZ_OK; ++s) cst = launch_step(b, c, dt);
-  }
-  g_launches.store(before);  // captured launches are counted when the graph runs
-  cudaGraph_t graph = nullptr;
-  cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
-  if (cst != CZ_OK) {
-    if (graph) cudaGraphDestroy(graph);
-    return cst;
-  }
-  if (e != cudaSuccess) return fail(CZ_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-  cudaGraphExec_t exec = nullptr;
-  e = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (e != cudaSuccess) return fail(CZ_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-  b->graphs.emplace(key, exec);
-  *out = exec;
+  if (int st = capture_rollout(b, nsteps, dt, nullptr, out)) return st;
+  b->graphs.emplace(key, *out);
   return CZ_OK;
 }
 
-// Capture the rollout with event-record nodes around every phase.
+// The same graph with event-record nodes around every phase.
 static int get_timed(cz_batch* b, int nsteps, double dt, cz_batch::Timed** out) {
   auto key = std::make_pair(nsteps, dt);
   auto it = b->timed.find(key);
@@ -1207,45 +1246,16 @@ static int get_timed(cz_batch* b, int nsteps, double dt, cz_batch::Timed** out) 
     return CZ_OK;
   }
   cz_batch::Timed t;
-  t.ev.resize(3 * (size_t)nsteps + 1);
-  for (auto& e : t.ev) CZ_CUDA(cudaEventCreate(&e));
-  CZ_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  const long long before = g_launches.load();
-  auto record = [&](int k) {
-    return cudaEventRecordWithFlags(t.ev[k], b->stream, cudaEventRecordExternal) == cudaSuccess ? CZ_OK
-                                                                                                : CZ_ERR_CUDA;
-  };
-  int cst = record(0);
-  const bool fused = uses_frame(b);
-  const Chain c = whole(b);
-  for (int s = 0; s < nsteps && cst == CZ_OK; ++s) {
-    if (fused) {  // one launch: its time is reported as the resolve phase
-      cst = record(3 * s + 1);
-      if (!cst) cst = record(3 * s + 2);
-      if (!cst) cst = launch_frame(b, dt);
-      if (!cst) cst = record(3 * s + 3);
-      continue;
-    }
-    cst = launch_integrate(b, c, dt);
-    if (!cst) cst = record(3 * s + 1);
-    if (!cst) cst = launch_narrowphase(b, c, false);
-    if (!cst) cst = record(3 * s + 2);
-    if (!cst) cst = launch_resolve(b, c, dt, false);
-    if (!cst) cst = record(3 * s + 3);
-  }
-  g_launches.store(before);
-  cudaGraph_t graph = nullptr;
-  cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
-  if (cst != CZ_OK || e != cudaSuccess) {
-    if (graph) cudaGraphDestroy(graph);
-    for (auto& ev : t.ev) cudaEventDestroy(ev);
-    return fail(CZ_ERR_CUDA, "timed graph capture failed");
-  }
-  e = cudaGraphInstantiate(&t.exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (e != cudaSuccess) {
-    for (auto& ev : t.ev) cudaEventDestroy(ev);
-    return fail(CZ_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+  t.chains = uses_frame(b) ? 1 : std::min((int)b->parts.size(), kTimedParts);
+  t.ev.resize(t.chains * (3 * (size_t)nsteps + 1) + 2);
+  cudaError_t e = cudaSuccess;
+  for (size_t k = 0; k < t.ev.size() && e == cudaSuccess; ++k) e = cudaEventCreate(&t.ev[k]);
+  int st = e == cudaSuccess ? capture_rollout(b, nsteps, dt, &t, &t.exec)
+                            : fail(CZ_ERR_CUDA, std::string("event: ") + cudaGetErrorString(e));
+  if (st) {
+    for (cudaEvent_t ev : t.ev)
+      if (ev) cudaEventDestroy(ev);
+    return st;
   }
   *out = &b->timed.emplace(key, std::move(t)).first->second;
   return CZ_OK;
@@ -1265,7 +1275,7 @@ int cz_step(cz_batch* b, int32_t nsteps, double dt) {
     CZ_CUDA(cudaGraphLaunch(exec, b->stream));
     left -= n;
   }
-  g_launches += (long long)launches_per_step(b, true) * nsteps;
+  g_launches += (long long)launches_per_step(b) * nsteps;
   return finish(b);
 }
 
@@ -1274,12 +1284,12 @@ int cz_prepare_rollout(cz_batch* b, int32_t nsteps, double dt) {
   CZ_CUDA(cudaSetDevice(b->device));
   int st = ensure_pows(b, dt);
   if (st) return st;
-  cudaGraphExec_t exec = nullptr;
-  if ((st = get_graph(b, graph_frames(b, nsteps), dt, &exec))) return st;
-  const int rest = nsteps % graph_frames(b, nsteps);
-  if (rest > 0 && (st = get_graph(b, rest, dt, &exec))) return st;
-  cz_batch::Timed* t = nullptr;
-  return get_timed(b, nsteps, dt, &t);
+  for (int n : {graph_frames(b, nsteps), nsteps % graph_frames(b, nsteps)}) {
+    cudaGraphExec_t exec = nullptr;
+    cz_batch::Timed* t = nullptr;
+    if (n > 0 && ((st = get_graph(b, n, dt, &exec)) || (st = get_timed(b, n, dt, &t)))) return st;
+  }
+  return CZ_OK;
 }
 
 int cz_contact_counts(cz_batch* b, int32_t* counts) {
@@ -1425,26 +1435,38 @@ int cz_step_timed(cz_batch* b, int32_t nsteps, double dt, double* total_ms, doub
   int st = ensure_pows(b, dt);
   if (st) return st;
   if ((st = reset_status(b))) return st;
-  cz_batch::Timed* t = nullptr;
-  if ((st = get_timed(b, nsteps, dt, &t))) return st;
-  CZ_CUDA(cudaGraphLaunch(t->exec, b->stream));
-  g_launches += (long long)launches_per_step(b, false) * nsteps;
-  st = finish(b);
-  double ph[3] = {0, 0, 0};
   const bool fused = uses_frame(b);
-  for (int s = 0; s < nsteps; ++s)
-    if (fused) {  // the whole frame (with the gaps between its event nodes) is the resolve phase
+  double tot = 0, ph[3] = {0, 0, 0};
+  for (int left = nsteps; left > 0;) {
+    const int n = graph_frames(b, left);
+    cz_batch::Timed* t = nullptr;
+    if ((st = get_timed(b, n, dt, &t))) return st;
+    CZ_CUDA(cudaGraphLaunch(t->exec, b->stream));
+    CZ_CUDA(cudaStreamSynchronize(b->stream));  // the next launch records the same events
+    auto between = [&](size_t from, size_t to, double* sum) -> int {
       float ms = 0.f;
-      CZ_CUDA(cudaEventElapsedTime(&ms, t->ev[3 * s], t->ev[3 * s + 3]));
-      ph[2] += ms;
-    } else
-      for (int k = 0; k < 3; ++k) {
-        float ms = 0.f;
-        CZ_CUDA(cudaEventElapsedTime(&ms, t->ev[3 * s + k], t->ev[3 * s + k + 1]));
-        ph[k] += ms;
-      }
-  float tot = 0.f;
-  CZ_CUDA(cudaEventElapsedTime(&tot, t->ev[0], t->ev[3 * (size_t)nsteps]));
+      CZ_CUDA(cudaEventElapsedTime(&ms, t->ev[from], t->ev[to]));
+      *sum += ms;
+      return CZ_OK;
+    };
+    double whole_ms = 0, part[3] = {0, 0, 0};
+    if ((st = between(t->ev.size() - 2, t->ev.size() - 1, &whole_ms))) return st;
+    for (int c = 0; c < t->chains; ++c)
+      for (int s = 0; s < n; ++s)
+        for (int k = 0; k < 3; ++k) {
+          const size_t at = c * (3 * (size_t)n + 1) + 3 * (size_t)s + k;
+          // a fused frame, with the gaps between its event nodes, is all resolve
+          if ((st = between(at, at + 1, &part[fused ? 2 : k]))) return st;
+        }
+    // parts overlap: their phases' times are shares of the rollout's
+    const double sum = part[0] + part[1] + part[2];
+    const double scale = !fused && b->parts.size() > 1 && sum > 0 ? whole_ms / sum : 1.0;
+    tot += whole_ms;
+    for (int k = 0; k < 3; ++k) ph[k] += part[k] * scale;
+    left -= n;
+  }
+  g_launches += (long long)launches_per_step(b) * nsteps;
+  st = finish(b);
   if (total_ms) *total_ms = tot;
   if (phase_ms)
     for (int k = 0; k < 3; ++k) phase_ms[k] = ph[k];

@@ -123,7 +123,9 @@ int cz_download_bodies(cz_batch* batch, cz_bodies* out);
  * Integrate + collider derived data for every body, the ordered all-pairs
  * narrowphase (plane first, then every other body), and ResolveContacts per
  * world.  The sequence is captured once as a CUDA graph per (nsteps, dt) and
- * replayed.  Blocking; returns the first error status seen. */
+ * replayed; batches of 128 worlds or more run as several parts, consecutive
+ * worlds each, in parallel branches of a graph of up to 32 frames, which
+ * longer calls launch again.  Blocking; returns the first error status seen. */
 int cz_step(cz_batch* batch, int32_t nsteps, double dt);
 
 /* Compute the damping factors for dt and capture the rollout graphs of
@@ -161,9 +163,12 @@ int cz_resolve_contacts(cz_batch* batch, int32_t max_iterations, cz_contact* con
 int cz_snapshot(cz_batch* batch);
 int cz_restore(cz_batch* batch);
 
-/* cz_step with CUDA events recorded on the batch stream around every phase
- * inside the captured rollout: total_ms = whole rollout, phase_ms[0..2] =
- * integrate, narrowphase, resolve summed over the steps. */
+/* cz_step with CUDA events recorded inside the captured rollout: total_ms =
+ * the whole rollout (without the host's gaps between its graphs),
+ * phase_ms[0..2] = integrate, narrowphase, resolve summed over the steps.
+ * Where the batch runs in parts side by side (cz_step), the phases of
+ * different parts overlap: phase_ms is then total_ms, shared out in the ratio
+ * of the times each phase took in up to four of the parts. */
 int cz_step_timed(cz_batch* batch, int32_t nsteps, double dt, double* total_ms, double* phase_ms);
 
 /* Running totals since creation or the last reset: [0] contacts generated,
