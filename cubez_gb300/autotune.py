@@ -4,8 +4,8 @@ Searches, on the caller's own batch and scene state, over
   * resolver lanes per world G (worlds per warp = 32 / G),
   * the resolver's shared-memory contact tile (contacts per world kept on chip),
   * the narrowphase CTA size,
-  * with worlds of more than 64 bodies in the batch, the large-world
-    resolver's lanes per world (32, or 16 = two worlds per warp),
+  * with worlds of more than 64 bodies in the batch, the caller's list of
+    large_world_lanes (by default the one setting: both run the same kernel),
   * with one world per warp, the fused frame (one launch per frame) or the
     three launches,
   * with the learned warm start enabled, optionally the warm-start budget
@@ -24,10 +24,10 @@ import itertools
 
 import numpy as np
 
-DEFAULT_LANES = (4, 8, 16, 32)
+DEFAULT_LANES = (8, 16, 32)  # 4 runs as 8
 DEFAULT_TILES = (64, 96, 128, 192)
 DEFAULT_NP_THREADS = (32, 64, 128, 256)
-DEFAULT_LARGE_LANES = (32, 16)
+DEFAULT_LARGE_LANES = (32,)  # both settings run the same kernel
 BIG_WORLD = 64  # worlds of more bodies than this go to the large-world resolver
 
 

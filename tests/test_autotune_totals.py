@@ -36,3 +36,10 @@ def test_whole_rollouts_decide():
     b = OverlappingBatch()
     cfg, _ = autotune.tune(b, frames=2)
     assert cfg == {"narrowphase_threads": 64, "resolver_contacts": 128, "resolver_lanes": 32, "fused_frame": -1}
+
+
+def test_every_default_setting_runs_other_launches():
+    """resolver_lanes 4 runs as 8, and both large_world_lanes settings run the
+    same kernel: trying them would let noise pick."""
+    assert autotune.DEFAULT_LANES == (8, 16, 32)
+    assert len(autotune.DEFAULT_LARGE_LANES) == 1
