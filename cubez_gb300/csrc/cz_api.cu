@@ -436,6 +436,9 @@ bool uses_frame(const cz_batch* b) {
   return b->fused && b->fr_smem > 0 && b->big_ids.empty() && b->rs_lanes == 32 && b->mode == 0 && b->nsmall > 0;
 }
 
+// Whether the resolver launch is k_resolve_wide (wide_rule, the plain resolver).
+bool uses_wide(const cz_batch* b, int mode) { return b->wide_smem > 0 && mode == 0; }
+
 // Frames in one graph where the batch runs in parts (longer rollouts launch it
 // again: the parts meet that often, and the graph has at most 4096 launches).
 constexpr int kPartFrames = 32;
@@ -503,7 +506,7 @@ int launch_resolve(cz_batch* b, const Chain& c, double dt, bool reset) {
       CZ_CUDA(b->ops->warm_features(c.v, b->rs_nbs, chain_grid(c.v.num_worlds, 1, b->wf_grid), dt, c.s));
       g_launches++;
     }
-    if (b->wide_smem > 0 && c.v.mode == 0)
+    if (uses_wide(b, c.v.mode))
       CZ_CUDA(b->ops->resolve_wide(c.v, b->rs_nbs, b->wide_cs, b->wide_per_sm, c.nsmall, b->wide_smem, dt, c.s));
     else
       CZ_CUDA(b->ops->resolve(c.v, b->rs_nbs, b->rs_cs, b->run_lanes(),
@@ -1597,9 +1600,10 @@ int cz_batch_info(cz_batch* b, int64_t* info) {
   info[3] = (int64_t)b->ops->real_size;
   info[4] = b->sm_count;
   info[5] = b->np_grid;
-  info[6] = b->rs_grid;
+  const bool wide = uses_wide(b, b->mode);
+  info[6] = wide ? b->nsmall : b->rs_grid;
   info[7] = (int64_t)b->np_smem;
-  info[8] = (int64_t)(b->rs_wpc * b->rs_smem);
+  info[8] = (int64_t)(wide ? b->wide_smem : b->rs_wpc * b->rs_smem);
   return CZ_OK;
 }
 

@@ -182,7 +182,8 @@ int cz_counters(cz_batch* batch, int64_t* out /* [8] */, int32_t reset);
 
 /* Sizes: [0] bodies, [1] padded bodies, [2] contact slots, [3] bytes per real,
  * [4] SMs, [5] narrowphase CTAs, [6] resolver CTAs, [7] narrowphase shared
- * bytes, [8] resolver shared bytes. */
+ * bytes, [8] resolver shared bytes, [6] and [8] of the kernel that the plain
+ * or, if set, the warm-started step runs for worlds of up to 64 bodies. */
 int cz_batch_info(cz_batch* batch, int64_t* info /* [9] */);
 
 /* ResolveContacts for one world without allocating any memory.  This entry
