@@ -167,6 +167,7 @@ struct cz_batch {
   bool rs_cs_set = false;            // the caller chose rs_cs (tile_rule otherwise)
   size_t wide_smem = 0;              // k_resolve_wide's shared memory per world (0: not used)
   int wide_cs = 0, wide_per_sm = 0;  // its contact tile, worlds per SM (wide_rule)
+  int wide_grid = 0;                 // its CTAs: a world's each, or what rs_ctas_per_sm allows
 
   // graph cache: (nsteps, dt) -> executable graph
   std::map<std::pair<int, double>, cudaGraphExec_t> graphs;
@@ -507,7 +508,8 @@ int launch_resolve(cz_batch* b, const Chain& c, double dt, bool reset) {
       g_launches++;
     }
     if (uses_wide(b, c.v.mode))
-      CZ_CUDA(b->ops->resolve_wide(c.v, b->rs_nbs, b->wide_cs, b->wide_per_sm, c.nsmall, b->wide_smem, dt, c.s));
+      CZ_CUDA(b->ops->resolve_wide(c.v, b->rs_nbs, b->wide_cs, b->wide_per_sm, chain_grid(c.nsmall, 1, b->wide_grid),
+                                   b->wide_smem, dt, c.s));
     else
       CZ_CUDA(b->ops->resolve(c.v, b->rs_nbs, b->rs_cs, b->run_lanes(),
                               chain_grid(c.v.num_worlds, worlds_per_warp * b->rs_wpc, b->rs_grid), b->rs_wpc,
@@ -648,6 +650,9 @@ int configure(cz_batch* b) {
     if (bytes <= b->smem_optin) {
       CZ_CUDA(b->ops->wide_prepare(per_sm, bytes));
       b->wide_per_sm = per_sm;
+      b->wide_grid = b->nsmall;
+      if (b->rs_ctas_per_sm > 0)
+        b->wide_grid = (int)std::min<long long>(b->nsmall, (long long)b->rs_ctas_per_sm * b->sm_count);
       b->wide_smem = bytes;
     }
   }
@@ -1601,7 +1606,7 @@ int cz_batch_info(cz_batch* b, int64_t* info) {
   info[4] = b->sm_count;
   info[5] = b->np_grid;
   const bool wide = uses_wide(b, b->mode);
-  info[6] = wide ? b->nsmall : b->rs_grid;
+  info[6] = wide ? b->wide_grid : b->rs_grid;
   info[7] = (int64_t)b->np_smem;
   info[8] = (int64_t)(wide ? b->wide_smem : b->rs_wpc * b->rs_smem);
   return CZ_OK;

@@ -270,8 +270,9 @@ typedef struct cz_tuning {
   int32_t narrowphase_threads; /* CTA size of the narrowphase */
   int32_t resolver_contacts;   /* contacts kept in shared memory per world (by default three per body of the
                                   largest world up to 64 bodies, at least 96) */
-  int32_t resolver_ctas_per_sm;/* resident resolver CTAs per SM (a CTA is 1 warp, or up to 8 independent ones in
-                                  the float32 form with 32 lanes per world) */
+  int32_t resolver_ctas_per_sm;/* most resolver CTAs per SM (a CTA is 1 warp, or up to 8 independent ones in
+                                  the float32 form with 32 lanes per world, or, in small batches with 32 lanes
+                                  per world, 4 that share one) */
   int32_t integrate_threads;
   int32_t resolver_lanes;      /* lanes per world in the resolver: 4, 8, 16 or 32 (its islands of touching
                                   bodies take 8 lanes each; 4 runs as 8) */
