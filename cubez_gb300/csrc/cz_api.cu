@@ -137,7 +137,8 @@ struct cz_batch {
   int max_iterations = -1;
 
   // tuning
-  int np_threads = 128, np_grid = 1, rs_cs = 128, rs_grid = 1, rs_ctas_per_sm = 0, int_threads = 256;
+  int np_threads = 128, np_grid = 1, rs_cs = 128, rs_grid = 1, rs_ctas_per_sm = 0;
+  int int_threads = 0;  // integrate_threads as set (0: integrate_cta)
   int rs_lanes = 8;  // resolver_lanes as set
   // lanes per world in the resolver (32 / run_lanes() worlds per warp): an island takes eight
   int run_lanes() const { return std::max(rs_lanes, 8); }
@@ -484,8 +485,19 @@ int launches_per_step(const cz_batch* b) {
   return n;
 }
 
+// Integrate's CTA size unless the caller sets one: a warp per CTA in batches of
+// up to 32768 body rows, so that few warps have an SM each, and 256 threads
+// above, where the launch covers the GPU anyway.  By the batch's rows, not the
+// launch's: a rollout's parts are on the GPU together.  float64, 20 frames from
+// the fall, with 256 and with 32: 500 worlds of 30 bodies 3.02 and 2.84 ms,
+// 1000 of 32 3.41 and 3.31, 1300 of 32 3.89 and 3.86, 2000 of 24 4.38 and 4.49,
+// 2000 of 32 5.26 and 5.46; one launch (with its call) over 20000 rows 36.7 and
+// 28.2 us, over 32000 36.8 both.  float32: one launch over 15600 rows 24.5 and
+// 16.3 us, from 25000 rows on and in rollouts the same.
+int integrate_cta(const cz_batch* b) { return b->int_threads > 0 ? b->int_threads : (b->nb_pad <= 32768 ? 32 : 256); }
+
 int launch_integrate(cz_batch* b, const Chain& c, double dt) {
-  CZ_CUDA(b->ops->integrate(c.v, dt, std::pow(0.5, dt), b->int_threads, c.s));
+  CZ_CUDA(b->ops->integrate(c.v, dt, std::pow(0.5, dt), integrate_cta(b), c.s));
   g_launches++;
   return CZ_OK;
 }
@@ -953,7 +965,7 @@ int cz_get_tuning(cz_batch* b, cz_tuning* t) {
   t->narrowphase_threads = b->np_threads;
   t->resolver_contacts = b->rs_cs;
   t->resolver_ctas_per_sm = b->rs_grid / std::max(b->sm_count, 1);
-  t->integrate_threads = b->int_threads;
+  t->integrate_threads = integrate_cta(b);
   t->resolver_lanes = b->rs_lanes;
   t->warm_start_budget_shift = b->warm_shift;
   t->broadphase_min_bodies = b->grid_min_bodies > 0 ? b->grid_min_bodies : -1;

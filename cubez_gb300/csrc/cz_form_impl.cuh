@@ -245,15 +245,12 @@ template <class T>
 static cudaError_t integrate_as(const HostView& h, double dt, double bias, int threads, cudaStream_t s) {
   const long long nb = h.nb_run;
   if constexpr (sizeof(T) == 8) {
-    if (nb <= kSpreadBodies) {
-      const int spread = (int)std::max<long long>(1, (4 * nb + 31) / 32);
-      k_integrate_spread<T><<<spread, 32, 0, s>>>(view_of(h), (T)dt, (T)bias);
+    if (nb <= kSpreadBodies && h.nb_pad <= 2 * kSpreadBodies) {
+      const int spread = (int)std::max<long long>(1, (4 * nb + threads - 1) / threads);
+      k_integrate_spread<T><<<spread, threads, 0, s>>>(view_of(h), (T)dt, (T)bias);
       return cudaGetLastError();
     }
   }
-  // a warp per CTA, so that few warps have an SM each: 60 falling worlds of 30
-  // bodies x 10 frames, float32, 656 -> 644 us; 500 of 30, float64, 1644 -> 1557
-  if (nb <= 2 * kSpreadBodies) threads = 32;
   const int grid = (int)std::max<long long>(1, (nb + threads - 1) / threads);
   k_integrate<T, W><<<grid, threads, 0, s>>>(view_of(h), (T)dt, (T)bias);
   return cudaGetLastError();

@@ -184,11 +184,17 @@ __device__ __forceinline__ void integrate_body_spread(const BatchView<R>& v, lon
 #undef F
 }
 
-// Four lanes per body for float64 batches of up to kSpreadBodies, where a
-// scheduler has one such warp at most: one world of 20 cubes 14 -> 10 us a
-// frame, 60 falling worlds of 30 bodies x 10 frames 1469 -> 1332 us (with CTAs
-// of 256 threads 12 us and 1372).  With more bodies the float64 pipes are full
-// and the lanes' idle quarter counts (4 x 110 instructions per 32 bodies for 300).
+// Four lanes per body in float64 for launches of up to kSpreadBodies rows,
+// where a scheduler has one or two such warps: one world of 20 cubes 14 -> 10 us
+// a frame, 60 falling worlds of 30 bodies x 10 frames 1469 -> 1332 us (with CTAs
+// of 256 threads 12 us and 1372); one launch over 10000 rows takes 24.5 us
+// either way, over 15600 24.5 with a lane per body and 36.4 so.  With more
+// bodies the float64 pipes are full and the lanes' idle quarter counts (4 x 110
+// instructions per 32 bodies for 300).  A rollout's parts share the GPU, but
+// not in step: up to twice as many rows in the batch.  20 frames from the fall,
+// a lane per body and four: 200 worlds of 30 bodies 2.67 and 2.61 ms, 500 of 30
+// 2.84 and 2.83, 600 of 30 2.91 both, 1000 of 32 3.31 and 3.39, 4096 of 8 to 64
+// 10.5 and 11.3.
 constexpr long long kSpreadBodies = 8192;
 template <class R>
 __global__ void __launch_bounds__(256) k_integrate_spread(BatchView<R> v, R dt, R sleep_bias) {

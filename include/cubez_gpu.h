@@ -273,7 +273,8 @@ typedef struct cz_tuning {
   int32_t resolver_ctas_per_sm;/* most resolver CTAs per SM (a CTA is 1 warp, or up to 8 independent ones in
                                   the float32 form with 32 lanes per world, or, in small batches with 32 lanes
                                   per world, 4 that share one) */
-  int32_t integrate_threads;
+  int32_t integrate_threads;   /* CTA size of the integrate launches (by default 32 in batches of up to 32768
+                                  bodies, else 256) */
   int32_t resolver_lanes;      /* lanes per world in the resolver: 4, 8, 16 or 32 (its islands of touching
                                   bodies take 8 lanes each; 4 runs as 8) */
   int32_t warm_start_budget_shift; /* learned warm start: a world is warm-started when its last
