@@ -964,7 +964,8 @@ int cz_get_tuning(cz_batch* b, cz_tuning* t) {
   if (!b || !t) return fail(CZ_ERR_BAD_ARG, "cz_get_tuning: null argument");
   t->narrowphase_threads = b->np_threads;
   t->resolver_contacts = b->rs_cs;
-  t->resolver_ctas_per_sm = b->rs_grid / std::max(b->sm_count, 1);
+  const int sms = std::max(b->sm_count, 1);
+  t->resolver_ctas_per_sm = uses_wide(b, b->mode) ? (b->wide_grid + sms - 1) / sms : b->rs_grid / sms;
   t->integrate_threads = integrate_cta(b);
   t->resolver_lanes = b->rs_lanes;
   t->warm_start_budget_shift = b->warm_shift;

@@ -43,3 +43,13 @@ def test_ctas_per_sm_bounds_the_launch(form, cuda_lib):
     for k in FIELDS:
         assert np.array_equal(x[k], y[k]), k
     assert a.counters() == b.counters()
+
+
+@pytest.mark.parametrize("form", [0, 1])
+def test_reported_tuning_set_again_changes_nothing(form, cuda_lib):
+    from cubez_gb300.batch import WorldBatch
+    for worlds in (1, 40, 200, 311):
+        b = WorldBatch([62] * worlds, form=form)
+        before = b.info()
+        b.set_tuning(**b.get_tuning())
+        assert b.info() == before, worlds
