@@ -7,21 +7,21 @@ U[-1,1]^3), ground plane y = 0, dt = 1/60, ResolveContacts(4 * len(contacts)).
 Synthetic seeded scenes (there is no dataset).
 
 One benchmark "step" is one 600-frame rollout of all worlds from the same
-initial state, captured as one CUDA graph (integrate -> narrowphase -> resolve
-per frame).  The metric is body-steps/s = bodies x frames / time.
+initial state, captured as CUDA graphs (integrate -> narrowphase -> resolve per
+frame; up to 32 frames a graph, the batch in parallel parts).  The metric is body-steps/s = bodies x frames / time.
 
   value       precision form (float32 bulk, float64 islands) with the learned
               warm start of adjustVelocities (network trained before timing,
               on the GPU, on contacts harvested from scenes of other seeds),
-              device time of the rollout graph (CUDA events recorded on the
-              batch stream inside the graph), inputs resident in HBM
+              device time of the rollout's graphs (CUDA events recorded
+              inside them), inputs resident in HBM
   e2e         the same through the C ABI with host buffers: cz_upload_bodies
               (host -> device) + cz_step + cz_download_bodies (device -> host)
   fp32_plain  the precision form without the warm start, measured the same way
   fp64        the plain float64 form measured the same way (reported beside it)
   accuracy    both precision variants against the float64 form
-  roofline    the dominant kernel, algorithmic bytes per launch / its average
-              CUDA-event duration over the timed rollouts
+  roofline    the dominant phase, its algorithmic bytes in a frame / its share
+              of a frame's time (CUDA events; the parts' launches overlap)
   cpu_baseline  the oracle (C++ restatement of the reference's float64 Go path)
               on the host's cores, one thread per world, on a bounded sample
 
@@ -194,8 +194,21 @@ def accuracy(scene, frames, batches, forms=("fp32_mlp", "fp32")):
     return out
 
 
+def _copied_bytes(nbodies, padded):
+    """(host to device, device to host) bytes of an upload of a scene's arrays,
+    a rollout and a download of the default fields, which copy only those."""
+    # position 3, orientation 4, velocity 3, rotation 3, acceleration 3, inverse inertia 9, inverse mass 1,
+    # motion 1, half size 3, radius 1; two flags, the shape; two damping factors per padded body
+    up = 31 * 8 * nbodies + 2 * nbodies + 4 * nbodies + 2 * 8 * int(padded)
+    # position 3, orientation 4, velocity 3, rotation 3, motion 1, inverse inertia (world) 9, last
+    # acceleration 3; two flags; the status word
+    down = 26 * 8 * nbodies + 2 * nbodies + 4
+    return up, down
+
+
 def _alg_bytes(phase, real, nbodies, counters, frames, rollouts):
-    """Algorithmic HBM bytes per launch of a phase (the minimum each kernel must move)."""
+    """Algorithmic HBM bytes of a phase in one frame (the minimum its launch over
+    all worlds, or its parts' launches together, must move)."""
     launches = frames * rollouts
     contacts = counters["contacts"] / launches
     resolved = counters["contacts_resolved"] / launches
@@ -319,8 +332,7 @@ def run_ours(args):
             out = b.download()
         barrier()
         e2e_s = (time.perf_counter() - t0) / args.steps
-        real_h2d = 43 * 8 * nb + 2 * nb + 4 * nb + 2 * 8 * int(b.info()["padded_bodies"])
-        real_d2h = 43 * 8 * nb + 2 * nb + 4 * nb + 4
+        real_h2d, real_d2h = _copied_bytes(nb, b.info()["padded_bodies"])
         e2e = {"value": nb * frames * ws / e2e_s, "unit": UNIT, "h2d_bytes_per_step": real_h2d,
                "d2h_bytes_per_step": real_d2h, "ms_per_step": e2e_s * 1e3}
         del C, out
@@ -638,8 +650,8 @@ def run_piles(args):
 def run_batched(args):
     """The batched configuration: 4096 worlds of U{8..64} spheres and cubes in
     the plain float64 form (bit-exact with the reference's arithmetic), one
-    600-frame rollout per step captured as one CUDA graph, restarted from the
-    same device-resident state; e2e through the C ABI with host buffers; the
+    600-frame rollout per step captured as CUDA graphs, restarted from the same
+    device-resident state; e2e through the C ABI with host buffers; the
     oracle on the host's cores beside it."""
     import torch
     ws, rank, local = _dist()
@@ -720,8 +732,7 @@ def run_batched(args):
             b.download()
         barrier()
         e2e_s = (time.perf_counter() - t0) / args.steps
-        h2d = 43 * 8 * nb + 2 * nb + 4 * nb + 2 * 8 * int(b.info()["padded_bodies"])
-        d2h = 43 * 8 * nb + 2 * nb + 4 * nb + 4
+        h2d, d2h = _copied_bytes(nb, b.info()["padded_bodies"])
         e2e = {"value": nb * frames * ws / e2e_s, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                "ms_per_step": e2e_s * 1e3}
     info = b.info()
