@@ -23,7 +23,7 @@
 #include "cz_layout.cuh"
 
 // Worlds of more bodies than this are resolved by k_resolve_big (bodies and
-// contacts in global memory, 32 or 16 lanes per world).
+// contacts in global memory, a CTA of four warps per world).
 constexpr int kBigWorld = 64;
 
 namespace {
@@ -142,7 +142,7 @@ struct cz_batch {
   int rs_lanes = 8;  // resolver_lanes as set
   // lanes per world in the resolver (32 / run_lanes() worlds per warp): an island takes eight
   int run_lanes() const { return std::max(rs_lanes, 8); }
-  int big_lanes = 32; // large_world_lanes as set (both settings run one warp per world)
+  int big_lanes = 32; // large_world_lanes as set (both settings run a CTA of four warps per world)
   int wait_limit = 1 << 22;  // polls of the narrowphase's bounded wait
   int wait_extra_tx = 0;     // test hook: bytes that wait expects beyond its copies
   int grid_min_bodies = 128; // narrowphase grid for worlds of at least this many bodies (0: never)
@@ -442,7 +442,8 @@ bool uses_frame(const cz_batch* b) {
 bool uses_wide(const cz_batch* b, int mode) { return b->wide_smem > 0 && mode == 0; }
 
 // Frames in one graph where the batch runs in parts (longer rollouts launch it
-// again: the parts meet that often, and the graph has at most 4096 launches).
+// again: the parts meet that often, and the graph has 6144 launches at most: 32
+// parts of six, with the sort, the warm start's features and large worlds).
 constexpr int kPartFrames = 32;
 // Parts whose phases cz_step_timed brackets, evenly spaced.  Event nodes in
 // many branches keep a graph's branches from running side by side: 4096 worlds
@@ -597,7 +598,16 @@ int tile_rule(int nbs, int lanes) { return lanes < 32 ? 96 : std::max(96, (int)r
 // In float64, whose rate one warp reaches a quarter of, up to seven per SM from
 // 24 slots on: 1001 worlds of 24 bodies with Offsets x 20 20.3 -> 19.4 ms, 600
 // settled of 31 x 4 5.95 -> 5.21, 1000 settled of 32 x 5 7.55 -> 6.63, against
-// fresh ones of 24 to 40 bodies, 0.99 to 1.04 times (300 of 24 x 3, 1.05 -> 1.08).
+// fresh ones of 24 to 40 bodies, 0.97 to 1.04 times (300 of 24 x 3, 1.05 -> 1.08).
+// Around the ends, 6 frames from frame 60 and from 240, one warp's time over
+// four warps': float64, 24 bodies, 450 worlds 0.99 and 1.16, 1000 (7 per SM)
+// 0.99 and 1.04, 1200 (8) 0.98 and 1.03, 1500 0.97 and 1.06, 2100 0.93 and 0.99;
+// 62 bodies, 1000 1.06 and 1.11, 1500 1.04 and 1.22, 2100 1.01 and 1.14; 20
+// bodies, 300 1.02 and 1.01, 1000 1.01 and 0.99; 16 bodies, 450 1.02 and 1.04,
+// 1000 1.00 and 0.97, 1500 0.97 and 0.93.  float32, 62 bodies, 1000 1.10 and
+// 1.12, 1500 1.04 and 1.09; 450 of 36 0.98 and 1.14, 450 of 32 0.97 and 1.08.
+// So from eight per SM on small falling worlds lose what they gain at rest (the
+// largest would still gain), and below 24 slots nothing is gained by seven.
 int wide_rule(int form, int worlds, int nbs, int lanes, int sms) {
   if (lanes != 32 || worlds <= 0) return 0;
   const int per_sm = (worlds + sms - 1) / sms;

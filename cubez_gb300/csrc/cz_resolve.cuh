@@ -1981,8 +1981,8 @@ __global__ void __launch_bounds__(32 * rs_wpc<R, G, FRAME>(),
 
 
 // ---------------------------------------------------------------- k_resolve_wide
-// The resolver for batches of up to three worlds per SM: four warps to a world,
-// one CTA each.  With one warp a small batch leaves three of an SM's four
+// The resolver for small batches, up to seven worlds per SM (wide_rule in
+// cz_api.cu): four warps to a world, one CTA each.  With one warp a small batch leaves three of an SM's four
 // schedulers idle, and in float64 each scheduler has its own quarter of the
 // SM's float64 rate, so a warp on its own is bound by its scheduler's unit.
 // The preparation is split over the warps, and so are the world's islands
