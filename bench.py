@@ -13,8 +13,8 @@ frame; up to 32 frames a graph, the batch in parallel parts).  The metric is bod
   value       precision form (float32 bulk, float64 islands) with the learned
               warm start of adjustVelocities (network trained before timing,
               on the GPU, on contacts harvested from scenes of other seeds),
-              device time of the rollout's graphs (CUDA events recorded
-              inside them), inputs resident in HBM
+              device time of the rollout (CUDA events around its graphs),
+              inputs resident in HBM
   e2e         the same through the C ABI with host buffers: cz_upload_bodies
               (host -> device) + cz_step + cz_download_bodies (device -> host)
   fp32_plain  the precision form without the warm start, measured the same way

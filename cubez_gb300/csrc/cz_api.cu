@@ -172,13 +172,16 @@ struct cz_batch {
 
   // graph cache: (nsteps, dt) -> executable graph
   std::map<std::pair<int, double>, cudaGraphExec_t> graphs;
-  // the same rollouts with event-record nodes between the phases (cz_step_timed)
+  // the same rollouts with marks between the phases (cz_step_timed): event-record
+  // nodes in one chain, stamps (k_stamp) in parts
   struct Timed {
     cudaGraphExec_t exec = nullptr;
-    int chains = 1;               // chains of launches with events
-    std::vector<cudaEvent_t> ev;  // 3 * nsteps + 1 a chain, then the rollout's start and end
+    std::vector<cudaEvent_t> ev;  // 3 * nsteps + 1
   };
   std::map<std::pair<int, double>, Timed> timed;
+  unsigned long long* stamps = nullptr;  // [kTimedParts][1 + stamp_cap]: how many, then the times
+  size_t stamp_cap = 0;
+  cudaEvent_t roll_ev[2] = {};  // around a rollout in parts
   // on-device copy of the body state (cz_snapshot / cz_restore)
   void* snap_body = nullptr;
   uint8_t* snap_u8 = nullptr;  // awake, can_sleep
@@ -324,11 +327,13 @@ void free_batch(cz_batch* b) {
     cudaGraphExecDestroy(kv.second.exec);
     for (cudaEvent_t e : kv.second.ev) cudaEventDestroy(e);
   }
+  for (cudaEvent_t e : b->roll_ev)
+    if (e) cudaEventDestroy(e);
   void* dev[] = {
       b->d_offset,  b->d_off_stage, b->ws_feat,   b->d_units,     b->d_big,      b->big_bw,      b->big_br,
       b->big_aw,    b->big_adj,     b->big_key,   b->ws_imp,      b->ws_rows,    b->ws_int,
       b->ws_world,  b->mlp_mem,     b->hv_features, b->hv_labels, b->hv_count,   b->snap_body,   b->snap_u8,
-      b->body,      b->awake,       b->can_sleep, b->shape,       b->d_bstart,   b->d_bcount,    b->d_ccap,
+      b->stamps,    b->body,      b->awake,       b->can_sleep, b->shape,       b->d_bstart,   b->d_bcount,    b->d_ccap,
       b->d_ccount,  b->d_cstart,    b->d_wstatus, b->d_piters,    b->d_viters,    b->d_cost,   b->contact,     b->cbodies,
       b->work,      b->wbodies,     b->kmat,      b->d_order,    b->d_order_rs,  b->d_order_part, b->d_order_rs_part, b->d_queue,
       b->d_status,  b->d_counters,  b->d_h2p,     b->d_stage,     b->d_stage_u8, b->d_stage_i32, b->d_cstage,
@@ -441,16 +446,13 @@ bool uses_frame(const cz_batch* b) {
 // Whether the resolver launch is k_resolve_wide (wide_rule, the plain resolver).
 bool uses_wide(const cz_batch* b, int mode) { return b->wide_smem > 0 && mode == 0; }
 
+// Whether a rollout runs the batch in parts.
+bool in_parts(const cz_batch* b) { return !uses_frame(b) && b->parts.size() > 1; }
 // Frames in one graph where the batch runs in parts (longer rollouts launch it
 // again: the parts meet that often, and the graph has 6144 launches at most: 32
 // parts of six, with the sort, the warm start's features and large worlds).
 constexpr int kPartFrames = 32;
-// Parts whose phases cz_step_timed brackets, evenly spaced.  Event nodes in
-// many branches keep a graph's branches from running side by side: 4096 worlds
-// of 32 bodies x 60 frames, float64, 140 ms by cz_step, and timed with the
-// events of 1, 2, 4, 8 and 32 of the 32 parts 141, 142, 142, 187 and 280 ms
-// (float32, 8 parts: 16384 worlds 99.3 and 99.5 to 99.7, 1000 worlds 23.5 and
-// 23.8, 24.1, 24.4 and 25.0).
+// Parts whose phases cz_step_timed marks, evenly spaced.
 constexpr int kTimedParts = 4;
 // The re-queue by cost matters where a launch's worlds do not all start at once.
 constexpr int kReorderWorlds = 256;
@@ -616,16 +618,19 @@ int wide_rule(int form, int worlds, int nbs, int lanes, int sms) {
   return wide && per_sm <= 7 ? std::min(per_sm, 3) : 0;
 }
 
-// The captured graphs hold the kernels' parameters (the batch view); drop them
-// whenever those change.
-void drop_graphs(cz_batch* b) {
-  for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
-  b->graphs.clear();
+void drop_timed(cz_batch* b) {
   for (auto& kv : b->timed) {
     cudaGraphExecDestroy(kv.second.exec);
     for (cudaEvent_t e : kv.second.ev) cudaEventDestroy(e);
   }
   b->timed.clear();
+}
+// The captured graphs hold the kernels' parameters (the batch view); drop them
+// whenever those change.
+void drop_graphs(cz_batch* b) {
+  for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
+  b->graphs.clear();
+  drop_timed(b);
 }
 
 int configure(cz_batch* b) {
@@ -1156,33 +1161,59 @@ int cz_resolve(cz_batch* b, double dt) {
   return finish(b);
 }
 
-// Marks where a timed rollout records event k (`t` null: an untimed one).
-static int record_event(cz_batch::Timed* t, size_t k, cudaStream_t s) {
-  if (t) CZ_CUDA(cudaEventRecordWithFlags(t->ev[k], s, cudaEventRecordExternal));
-  return CZ_OK;
+// The end of a phase in a part's chain of a timed rollout: the time, appended to
+// the part's log.  With event nodes the branches of a graph did not run side by
+// side: 4096 worlds of 32 bodies x 60 frames, float64, 137 ms by cz_step, 138.6
+// timed so, 142 to 280 with events in 4 to 32 of the 32 parts; 4096 of 8 to 64
+// bodies x 600 frames 2177, 2167 and 2620 and more.
+__global__ void k_stamp(unsigned long long* log, size_t cap) {
+  unsigned long long now;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+  const unsigned long long at = log[0];
+  if (at < cap) log[1 + at] = now;
+  log[0] = at + 1;
 }
 
-// One frame of a chain; in a timed rollout, events at + 1 to at + 3 end its phases.
-static int launch_step(cz_batch* b, const Chain& c, double dt, cz_batch::Timed* t = nullptr, size_t at = 0) {
+// What a timed rollout leaves between the phases of a chain (an untimed one:
+// nothing).
+struct Marks {
+  const std::vector<cudaEvent_t>* ev = nullptr;
+  unsigned long long* log = nullptr;
+  size_t cap = 0, next = 0;
+  int mark(cudaStream_t s) {
+    if (ev) CZ_CUDA(cudaEventRecordWithFlags((*ev)[next++], s, cudaEventRecordExternal));
+    if (log) {
+      k_stamp<<<1, 1, 0, s>>>(log, cap);
+      CZ_CUDA(cudaGetLastError());
+    }
+    return CZ_OK;
+  }
+};
+
+// One frame of a chain.
+static int launch_step(cz_batch* b, const Chain& c, double dt, Marks* m = nullptr) {
+  Marks none;
+  if (!m) m = &none;
   int st = launch_integrate(b, c, dt);
-  if (!st) st = record_event(t, at + 1, c.s);
+  if (!st) st = m->mark(c.s);
   if (!st) st = launch_narrowphase(b, c, false);
-  if (!st) st = record_event(t, at + 2, c.s);
+  if (!st) st = m->mark(c.s);
   if (!st) st = launch_resolve(b, c, dt, false);
-  if (!st) st = record_event(t, at + 3, c.s);
+  if (!st) st = m->mark(c.s);
   return st;
 }
-// `nsteps` of them, chain number `index` of the rollout.
-static int launch_chain(cz_batch* b, const Chain& c, int nsteps, double dt, cz_batch::Timed* t, size_t index) {
-  const size_t at = index * (3 * (size_t)nsteps + 1);
-  int st = record_event(t, at, c.s);
-  for (int s = 0; s < nsteps && !st; ++s) st = launch_step(b, c, dt, t, at + 3 * (size_t)s);
+static int launch_chain(cz_batch* b, const Chain& c, int nsteps, double dt, Marks m) {
+  int st = m.mark(c.s);
+  for (int s = 0; s < nsteps && !st; ++s) st = launch_step(b, c, dt, &m);
   return st;
 }
+
+// The parts whose chains a timed rollout marks: every so many, the first kTimedParts of them.
+static int timed_parts(const cz_batch* b) { return std::min((int)b->parts.size(), kTimedParts); }
 
 // The batch's parts as parallel branches of the graph being captured on its
 // stream, each its own chain of frames.
-static int capture_parts(cz_batch* b, int nsteps, double dt, cz_batch::Timed* t) {
+static int capture_parts(cz_batch* b, int nsteps, double dt, bool timed) {
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> joins;
   auto run = [&]() -> int {
@@ -1193,9 +1224,13 @@ static int capture_parts(cz_batch* b, int nsteps, double dt, cz_batch::Timed* t)
       const Chain c{b->view(part, (int)p), part.nsmall, part.nbig, part.nsmall > kReorderWorlds,
                     p == 0 ? b->stream : b->part_streams[p - 1]};
       if (p > 0) CZ_CUDA(cudaStreamWaitEvent(c.s, fork, 0));
-      const size_t every = t ? b->parts.size() / t->chains : 1, index = p / every;
-      const bool timed = t && p % every == 0 && index < (size_t)t->chains;
-      if (int st = launch_chain(b, c, nsteps, dt, timed ? t : nullptr, index)) return st;
+      const size_t every = b->parts.size() / timed_parts(b), index = p / every;
+      Marks m;
+      if (timed && p % every == 0 && index < (size_t)timed_parts(b)) {
+        m.log = b->stamps + index * (1 + b->stamp_cap);
+        m.cap = b->stamp_cap;
+      }
+      if (int st = launch_chain(b, c, nsteps, dt, m)) return st;
       if (p > 0) {
         cudaEvent_t e = nullptr;
         CZ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1213,35 +1248,30 @@ static int capture_parts(cz_batch* b, int nsteps, double dt, cz_batch::Timed* t)
 }
 
 // Frames the next graph of a rollout with `left` frames to go holds.
-static int graph_frames(const cz_batch* b, int left) {
-  return !uses_frame(b) && b->parts.size() > 1 ? std::min(left, kPartFrames) : left;
-}
+static int graph_frames(const cz_batch* b, int left) { return in_parts(b) ? std::min(left, kPartFrames) : left; }
 
 // A rollout's launches, on the batch's stream: the fused frames, the parts, or
-// one chain over the whole batch.  With `t`, the events around its phases (a
+// one chain over the whole batch.  With `t`, the marks between its phases (a
 // fused frame, one launch, is its resolve phase).
-static int launch_rollout(cz_batch* b, int nsteps, double dt, cz_batch::Timed* t) {
-  if (!uses_frame(b)) {
-    if (b->parts.size() > 1) return capture_parts(b, nsteps, dt, t);
-    return launch_chain(b, whole(b), nsteps, dt, t, 0);
-  }
-  int st = record_event(t, 0, b->stream);
+static int launch_rollout(cz_batch* b, int nsteps, double dt, const cz_batch::Timed* t) {
+  if (in_parts(b)) return capture_parts(b, nsteps, dt, t != nullptr);
+  Marks m;
+  if (t) m.ev = &t->ev;
+  if (!uses_frame(b)) return launch_chain(b, whole(b), nsteps, dt, m);
+  int st = m.mark(b->stream);
   for (int s = 0; s < nsteps && !st; ++s) {
-    st = record_event(t, 3 * (size_t)s + 1, b->stream);
-    if (!st) st = record_event(t, 3 * (size_t)s + 2, b->stream);
+    st = m.mark(b->stream);
+    if (!st) st = m.mark(b->stream);
     if (!st) st = launch_frame(b, dt);
-    if (!st) st = record_event(t, 3 * (size_t)s + 3, b->stream);
+    if (!st) st = m.mark(b->stream);
   }
   return st;
 }
 
-static int capture_rollout(cz_batch* b, int nsteps, double dt, cz_batch::Timed* t, cudaGraphExec_t* exec) {
+static int capture_rollout(cz_batch* b, int nsteps, double dt, const cz_batch::Timed* t, cudaGraphExec_t* exec) {
   CZ_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   const long long before = g_launches.load();
-  const size_t ends = t ? t->ev.size() - 2 : 0;
-  int cst = record_event(t, ends, b->stream);
-  if (!cst) cst = launch_rollout(b, nsteps, dt, t);
-  if (!cst) cst = record_event(t, ends + 1, b->stream);
+  const int cst = launch_rollout(b, nsteps, dt, t);
   g_launches.store(before);  // captured launches are counted when the graph runs
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
@@ -1268,7 +1298,7 @@ static int get_graph(cz_batch* b, int nsteps, double dt, cudaGraphExec_t* out) {
   return CZ_OK;
 }
 
-// The same graph with event-record nodes around every phase.
+// The same graph with marks around every phase.
 static int get_timed(cz_batch* b, int nsteps, double dt, cz_batch::Timed** out) {
   auto key = std::make_pair(nsteps, dt);
   auto it = b->timed.find(key);
@@ -1277,8 +1307,7 @@ static int get_timed(cz_batch* b, int nsteps, double dt, cz_batch::Timed** out) 
     return CZ_OK;
   }
   cz_batch::Timed t;
-  t.chains = uses_frame(b) ? 1 : std::min((int)b->parts.size(), kTimedParts);
-  t.ev.resize(t.chains * (3 * (size_t)nsteps + 1) + 2);
+  if (!in_parts(b)) t.ev.resize(3 * (size_t)nsteps + 1);
   cudaError_t e = cudaSuccess;
   for (size_t k = 0; k < t.ev.size() && e == cudaSuccess; ++k) e = cudaEventCreate(&t.ev[k]);
   int st = e == cudaSuccess ? capture_rollout(b, nsteps, dt, &t, &t.exec)
@@ -1289,6 +1318,20 @@ static int get_timed(cz_batch* b, int nsteps, double dt, cz_batch::Timed** out) 
     return st;
   }
   *out = &b->timed.emplace(key, std::move(t)).first->second;
+  return CZ_OK;
+}
+
+// Room in the log for the marks of a rollout of nsteps frames: three a frame, and
+// one a graph.  The graphs hold its address, so those of a shorter one go.
+static int ensure_stamps(cz_batch* b, int nsteps) {
+  const size_t need = 3 * (size_t)nsteps + ((size_t)nsteps + kPartFrames - 1) / kPartFrames;
+  if (!in_parts(b) || need <= b->stamp_cap) return CZ_OK;
+  drop_timed(b);
+  CZ_CUDA(cudaFree(b->stamps));
+  b->stamps = nullptr;
+  b->stamp_cap = 0;
+  CZ_CUDA(cudaMalloc((void**)&b->stamps, sizeof(unsigned long long) * kTimedParts * (1 + need)));
+  b->stamp_cap = need;
   return CZ_OK;
 }
 
@@ -1315,6 +1358,7 @@ int cz_prepare_rollout(cz_batch* b, int32_t nsteps, double dt) {
   CZ_CUDA(cudaSetDevice(b->device));
   int st = ensure_pows(b, dt);
   if (st) return st;
+  if ((st = ensure_stamps(b, nsteps))) return st;
   for (int n : {graph_frames(b, nsteps), nsteps % graph_frames(b, nsteps)}) {
     cudaGraphExec_t exec = nullptr;
     cz_batch::Timed* t = nullptr;
@@ -1466,38 +1510,53 @@ int cz_step_timed(cz_batch* b, int32_t nsteps, double dt, double* total_ms, doub
   int st = ensure_pows(b, dt);
   if (st) return st;
   if ((st = reset_status(b))) return st;
-  const bool fused = uses_frame(b);
-  double tot = 0, ph[3] = {0, 0, 0};
+  const bool fused = uses_frame(b), parts = in_parts(b);
+  if ((st = ensure_stamps(b, nsteps))) return st;
+  for (cudaEvent_t& e : b->roll_ev)
+    if (parts && !e) CZ_CUDA(cudaEventCreate(&e));
+  if (parts) {
+    CZ_CUDA(cudaMemset2DAsync(b->stamps, sizeof(*b->stamps) * (1 + b->stamp_cap), 0, sizeof(*b->stamps), kTimedParts,
+                              b->stream));
+    CZ_CUDA(cudaEventRecord(b->roll_ev[0], b->stream));
+  }
+  cz_batch::Timed* t = nullptr;
   for (int left = nsteps; left > 0;) {
     const int n = graph_frames(b, left);
-    cz_batch::Timed* t = nullptr;
     if ((st = get_timed(b, n, dt, &t))) return st;
     CZ_CUDA(cudaGraphLaunch(t->exec, b->stream));
-    CZ_CUDA(cudaStreamSynchronize(b->stream));  // the next launch records the same events
-    auto between = [&](size_t from, size_t to, double* sum) -> int {
-      float ms = 0.f;
-      CZ_CUDA(cudaEventElapsedTime(&ms, t->ev[from], t->ev[to]));
-      *sum += ms;
-      return CZ_OK;
-    };
-    double whole_ms = 0, part[3] = {0, 0, 0};
-    if ((st = between(t->ev.size() - 2, t->ev.size() - 1, &whole_ms))) return st;
-    for (int c = 0; c < t->chains; ++c)
-      for (int s = 0; s < n; ++s)
-        for (int k = 0; k < 3; ++k) {
-          const size_t at = c * (3 * (size_t)n + 1) + 3 * (size_t)s + k;
-          // a fused frame, with the gaps between its event nodes, is all resolve
-          if ((st = between(at, at + 1, &part[fused ? 2 : k]))) return st;
-        }
-    // parts overlap: their phases' times are shares of the rollout's
-    const double sum = part[0] + part[1] + part[2];
-    const double scale = !fused && b->parts.size() > 1 && sum > 0 ? whole_ms / sum : 1.0;
-    tot += whole_ms;
-    for (int k = 0; k < 3; ++k) ph[k] += part[k] * scale;
     left -= n;
   }
+  if (parts) CZ_CUDA(cudaEventRecord(b->roll_ev[1], b->stream));
   g_launches += (long long)launches_per_step(b) * nsteps;
   st = finish(b);
+  float ms = 0.f;
+  double tot = 0, ph[3] = {0, 0, 0};
+  if (parts) {
+    CZ_CUDA(cudaEventElapsedTime(&ms, b->roll_ev[0], b->roll_ev[1]));
+    tot = ms;
+    // the parts overlap: their phases' times are shares of the rollout's
+    const size_t row = 1 + b->stamp_cap;
+    std::vector<unsigned long long> log(timed_parts(b) * row);
+    CZ_CUDA(cudaMemcpy(log.data(), b->stamps, sizeof(log[0]) * log.size(), cudaMemcpyDeviceToHost));
+    for (size_t p = 0; p < log.size(); p += row) {
+      const unsigned long long* at = &log[p + 1];
+      for (int left = nsteps; left > 0; ++at) {  // (a graph's first mark)
+        const int n = graph_frames(b, left);
+        for (int k = 0; k < 3 * n; ++k, ++at) ph[k % 3] += (double)(at[1] - at[0]);
+        left -= n;
+      }
+    }
+    const double sum = ph[0] + ph[1] + ph[2];
+    for (double& x : ph) x = sum > 0 ? x * tot / sum : 0;
+  } else {
+    for (size_t k = 0; k + 1 < t->ev.size(); ++k) {
+      CZ_CUDA(cudaEventElapsedTime(&ms, t->ev[k], t->ev[k + 1]));
+      // a fused frame, with the gaps between its event nodes, is all resolve
+      ph[fused ? 2 : k % 3] += ms;
+    }
+    CZ_CUDA(cudaEventElapsedTime(&ms, t->ev.front(), t->ev.back()));
+    tot = ms;
+  }
   if (total_ms) *total_ms = tot;
   if (phase_ms)
     for (int k = 0; k < 3; ++k) phase_ms[k] = ph[k];

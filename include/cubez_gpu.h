@@ -163,12 +163,11 @@ int cz_resolve_contacts(cz_batch* batch, int32_t max_iterations, cz_contact* con
 int cz_snapshot(cz_batch* batch);
 int cz_restore(cz_batch* batch);
 
-/* cz_step with CUDA events recorded inside the captured rollout: total_ms =
- * the whole rollout (without the host's gaps between its graphs),
- * phase_ms[0..2] = integrate, narrowphase, resolve summed over the steps.
- * Where the batch runs in parts side by side (cz_step), the phases of
- * different parts overlap: phase_ms is then total_ms, shared out in the ratio
- * of the times each phase took in up to four of the parts. */
+/* cz_step with CUDA events: total_ms = the whole rollout, phase_ms[0..2] =
+ * integrate, narrowphase, resolve summed over the steps, from events between
+ * the phases.  Where the batch runs in parts side by side (cz_step), the phases
+ * of different parts overlap: phase_ms is then total_ms, shared out in the
+ * ratio of the times each phase took in up to four of the parts. */
 int cz_step_timed(cz_batch* batch, int32_t nsteps, double dt, double* total_ms, double* phase_ms);
 
 /* Running totals since creation or the last reset: [0] contacts generated,
