@@ -562,11 +562,19 @@ int launch_frame(cz_batch* b, double dt) {
 // launch over all of them ends with its longest world, and a frame's next
 // launch waited for that: half of a resolver launch was its tail (8192 worlds
 // of 32 bodies, float32: 0.62 of 1.2 ms with the SMs busy).  With parts, one
-// part's tail runs beside the others' work.  At least 64 worlds each; at most
-// 32 parts in float64, where 4096 worlds of 8 to 64 bodies x 30 frames took
-// 221, 189, 179 and 165 ms with 1, 4, 8 and 32 parts, and 8 in float32, whose
-// launches are short (16384 x 32 bodies x 60 frames: 142, 119, 122 and 132 ms;
-// 8192 worlds with the warm start x 30: 48.3, 40.2, 39.3 and 40.7 ms).
+// part's tail runs beside the others' work.  At least 64 worlds each, at most 32
+// parts in float64 and 8 in float32, whose launches are short.  32 frames from
+// the fall, from frame 120 and from 400, with 1, 8 and 32 parts, ms:
+//   float64  1001 x 24       6.4  38.0  27.8    5.0  27.7  25.7    4.7  26.1  23.9 (15 parts)
+//            2000 x 32      12.1  62.0  46.9    9.0  50.3  40.0    9.8  47.3  42.7
+//            4096 x 8 to 64 20.3 142.5 114.3   16.0 119.7 114.7   18.3 128.7 129.2
+//            8192 x 32      27.8 159.9 140.7   23.7 134.3 124.1   26.3 147.3 140.0
+//   float32  1000 x 32       3.4  16.4  11.4    2.9  13.8  11.2    2.9  13.6  11.3
+//            4096 x 8 to 64  7.5  48.0  43.0    6.3  41.0  40.4    7.6  36.8  40.4
+//           16384 x 32      15.9  65.2  59.0   14.6  56.4  50.1   17.5  66.5  60.7
+// (float64's 32 were the fastest of these while a resolver launch took twice as
+// long; from some 2000 worlds on eight now are, and a settled mixed batch of
+// 4096 is 13 % faster in one part than in 32.)
 int part_rule(int form, int num_worlds) {
   return std::max(1, std::min(num_worlds / 64, form == CZ_FORM_FP64 ? 32 : 8));
 }
